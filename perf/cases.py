@@ -136,6 +136,15 @@ def tolerance(case):
 # ---------------------------------------------------------------------------------------------------- state
 
 
+def _decode_inputs(case, seed):
+    """Norm weights, the per-head ones of q and k, and the hidden state."""
+    g = torch.Generator("cuda").manual_seed((seed << 8) + 1)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g)  # noqa: E731
+    norms = {n: 1.0 + 0.1 * rand(case["hidden"]) for n in ("attn", "post_attn", "ffn", "post_ffn")}
+    q_norm, k_norm = 0.0884 + 0.01 * rand(HEAD_DIM), 1.0 + 0.1 * rand(HEAD_DIM)
+    return norms, q_norm, k_norm, rand(case["tokens"], case["hidden"])
+
+
 class _Decode:
     def __init__(self, case, seed):
         t, p = case["tokens"], _projections(case)
@@ -143,11 +152,7 @@ class _Decode:
         self.ctx = op.Context(0, workspace_bytes=1 << 20)
         self.kern = op.CudaKernels(self.ctx)
         self.w = _kquant_weights(self.ctx, p, seed)
-        g = torch.Generator("cuda").manual_seed((seed << 8) + 1)
-        rand = lambda *s: torch.randn(s, device="cuda", generator=g)  # noqa: E731
-        self.norms = {n: 1.0 + 0.1 * rand(case["hidden"]) for n in ("attn", "post_attn", "ffn", "post_ffn")}
-        self.q_norm, self.k_norm = 0.0884 + 0.01 * rand(HEAD_DIM), 1.0 + 0.1 * rand(HEAD_DIM)
-        self.embedding = rand(t, case["hidden"])
+        self.norms, self.q_norm, self.k_norm, self.embedding = _decode_inputs(case, seed)
         new = lambda n: torch.empty((t, n), device="cuda")  # noqa: E731
         self.hidden, self.y, self.proj, self.down = (new(case["hidden"]) for _ in range(4))
         self.out = {n: new(p[n][1]) for n in ("q", "k", "v", "gate")}
@@ -174,10 +179,16 @@ class _Decode:
         return {"hidden": self.hidden, "y": self.y, "proj": self.proj, "act": self.act, "down": self.down, **self.out}
 
 
+INPUT = {"q": "attn", "k": "attn", "v": "attn", "o": "o", "ffn_gate": "ffn", "ffn_up": "ffn", "ffn_down": "down"}
+
+
+def _projection_inputs(case, seed):
+    p, g = _projections(case), torch.Generator("cuda").manual_seed((seed << 8) + 1)
+    return {i: torch.randn((case["tokens"], p[n][0]), device="cuda", generator=g).to(DTYPES[case.get("dtype", "bf16")]) for n, i in INPUT.items()}
+
+
 class _Projections:
     """The seven projections of a layer, each on its own input (q, k and v share one, gate and up another)."""
-
-    INPUT = {"q": "attn", "k": "attn", "v": "attn", "o": "o", "ffn_gate": "ffn", "ffn_up": "ffn", "ffn_down": "down"}
 
     def __init__(self, case, seed):
         t, p = case["tokens"], _projections(case)
@@ -187,15 +198,20 @@ class _Projections:
         self.kern = op.CudaKernels(self.ctx)
         self.w = _nvfp4_weights(self.ctx, p, seed, {})[0] if a16 else _kquant_weights(self.ctx, p, seed)
         self.encode = self.kern.encode_nvfp4_matmul if a16 else self.kern.encode_quantized_matmul
-        g = torch.Generator("cuda").manual_seed((seed << 8) + 1)
-        dtype = DTYPES[case.get("dtype", "bf16")]
-        self.x = {i: torch.randn((t, p[n][0]), device="cuda", generator=g).to(dtype) for n, i in self.INPUT.items()}
+        self.x = _projection_inputs(case, seed)
         self.y = {n: torch.empty((t, p[n][1]), device="cuda", dtype=torch.float16 if a16 else torch.float32) for n in p}
 
     def run(self):
         for n, y in self.y.items():
-            self.encode(self.w[n], self.x[self.INPUT[n]], y, self.t)
+            self.encode(self.w[n], self.x[INPUT[n]], y, self.t)
         return self.y
+
+
+def _lm_head_inputs(case, seed):
+    k, n, dt = case["hidden"], case["vocab"], QUANTS[case["quant"]]
+    rows = -(-n // 8)
+    raw = torch.cat([synth.quantize_kquant(synth.normal_weights(min(rows, n - r), k, seed=seed, stream=90 + r, device="cuda"), dt) for r in range(0, n, rows)])
+    return raw, synth.normal_activations(case["tokens"], k, seed=seed, device="cuda")
 
 
 class _LmHead:
@@ -204,16 +220,21 @@ class _LmHead:
         self.t = case["tokens"]
         self.ctx = op.Context(0, workspace_bytes=1 << 20)
         self.kern = op.CudaKernels(self.ctx)
-        rows = -(-n // 8)
-        raw = torch.cat([synth.quantize_kquant(synth.normal_weights(min(rows, n - r), k, seed=seed, stream=90 + r, device="cuda"), dt)
-                         for r in range(0, n, rows)])
+        raw, self.x = _lm_head_inputs(case, seed)
         self.w = op.Weight(self.ctx, op.TensorView(raw, dt, k, n))
-        self.x = synth.normal_activations(self.t, k, seed=seed, device="cuda")
         self.logits = torch.empty((self.t, n), device="cuda")
 
     def run(self):
         picked = self.kern.encode_lm_head_argmax(self.w, self.x, self.t, logits=self.logits, out_scale=0.5, softcap=30.0)
         return [*picked, self.logits]
+
+
+def _nvfp4_inputs(case, seed):
+    """The hidden state, the two norms' weights and rows to calibrate with."""
+    h, g = case["hidden"], torch.Generator("cuda").manual_seed((seed << 8) + 1)
+    x = torch.randn((case["tokens"], h), device="cuda", generator=g).to(torch.bfloat16)
+    norms = [1.0 + 0.1 * torch.randn(h, device="cuda", generator=g) for _ in range(2)]
+    return x, norms, torch.randn((128, h), device="cuda", generator=g)
 
 
 class _Nvfp4Layer:
@@ -223,10 +244,7 @@ class _Nvfp4Layer:
         self.t = t
         self.ctx = op.Context(0, workspace_bytes=(t + 128) * (a // 2 + a // 16) + (1 << 20))
         self.kern = op.CudaKernels(self.ctx)
-        g = torch.Generator("cuda").manual_seed((seed << 8) + 1)
-        self.x = torch.randn((t, h), device="cuda", generator=g).to(torch.bfloat16)
-        self.norms = [1.0 + 0.1 * torch.randn(h, device="cuda", generator=g) for _ in range(2)]
-        sample = torch.randn((128, h), device="cuda", generator=g)
+        self.x, self.norms, sample = _nvfp4_inputs(case, seed)
         self.w, self.isi = _nvfp4_weights(self.ctx, p, seed, {"sample": sample, "norms": self.norms})
         new = lambda n: torch.empty((t, n), device="cuda", dtype=torch.bfloat16)  # noqa: E731
         self.q, self.k, self.v, self.h1, self.h2 = new(a), new(p["k"][1]), new(p["v"][1]), new(h), new(h)
@@ -245,17 +263,19 @@ class _Nvfp4Layer:
         return [self.q, self.k, self.v, self.h1, self.h2]
 
 
+def _kquant_raw(p, seed):
+    """name -> K-quant blocks of the projection's weights."""
+    return {name: synth.quantize_kquant(synth.normal_weights(n, k, seed=seed, stream=i, device="cuda"), dt) for i, (name, (k, n, dt)) in enumerate(p.items())}
+
+
 def _kquant_weights(ctx, p, seed):
-    w = {}
-    for i, (name, (k, n, dt)) in enumerate(p.items()):
-        raw = synth.quantize_kquant(synth.normal_weights(n, k, seed=seed, stream=i, device="cuda"), dt)
-        w[name] = op.Weight(ctx, op.TensorView(raw, dt, k, n))
-    return w
+    return {name: op.Weight(ctx, op.TensorView(raw, p[name][2], p[name][0], p[name][1])) for name, raw in _kquant_raw(p, seed).items()}
 
 
-def _nvfp4_weights(ctx, p, seed, calibration):
-    """Weights and, given calibration rows, each projection's input_scale_inv as a checkpoint stores it (from the largest
-    magnitude that the sample shows at that input, with a margin); without them the weight-only form."""
+def _nvfp4_raw(p, seed, calibration):
+    """name -> (codes, scales, scale2) and, given calibration rows, each projection's input_scale_inv as a checkpoint
+    stores it (from the largest magnitude that the sample shows at that input, with a margin); without them the
+    weight-only form."""
     dense = {n: synth.normal_weights(o, i, seed=seed, stream=s, device="cuda") for s, (n, (i, o, _)) in enumerate(p.items())}
     isi = dict.fromkeys(p)
     if calibration:
@@ -266,11 +286,12 @@ def _nvfp4_weights(ctx, p, seed, calibration):
         isi.update({n: synth.activation_input_scale_inv(1.25 * v) for n, v in inputs.items()})
         isi["k"] = isi["v"] = isi["q"]
         isi["ffn_up"] = isi["ffn_gate"]
-    w = {}
-    for n, (i, o, _) in p.items():
-        packed, scales, scale2 = synth.nvfp4_weight(dense.pop(n))
-        w[n] = op.Weight(ctx, op.TensorView(packed, op.NVFP4, i, o, scales, scale2, isi[n]))
-    return w, isi
+    return {n: synth.nvfp4_weight(dense.pop(n)) for n in p}, isi
+
+
+def _nvfp4_weights(ctx, p, seed, calibration):
+    raw, isi = _nvfp4_raw(p, seed, calibration)
+    return {n: op.Weight(ctx, op.TensorView(packed, op.NVFP4, p[n][0], p[n][1], scales, scale2, isi[n])) for n, (packed, scales, scale2) in raw.items()}, isi
 
 
 def prepare(case, seed):
@@ -279,3 +300,130 @@ def prepare(case, seed):
 
 def run(state):
     return state.run()
+
+
+# ---------------------------------------------------------------------------------------------------- in 64 bits
+
+
+def _f16_pairs(b):
+    return b.contiguous().view(torch.float16).double()
+
+
+def _dense64(raw, dt):
+    """[rows][blocks * bytes] K-quant blocks -> f64 weights."""
+    b = raw.reshape(raw.shape[0], -1, synth.BLOCK_BYTES[dt])
+    if dt == synth.Q6_K:
+        ql, qh = b[..., :128].reshape(*b.shape[:2], 2, 2, 32), b[..., 128:192].reshape(*b.shape[:2], 2, 32)
+        lo = torch.stack([ql[..., 0, :] & 15, ql[..., 1, :] & 15, ql[..., 0, :] >> 4, ql[..., 1, :] >> 4], -2)
+        hi = torch.stack([(qh >> s) & 3 for s in (0, 2, 4, 6)], -2)
+        q = (lo | (hi << 4)).reshape(*b.shape[:2], 16, 16).double() - 32.0
+        sc = b[..., 192:208].contiguous().view(torch.int8).double()
+        return (q * (sc * _f16_pairs(b[..., 208:210])).unsqueeze(-1)).reshape(b.shape[0], -1)
+    packed = b[..., 4:16]
+    low, mid, top = packed[..., 0:4], packed[..., 4:8], packed[..., 8:12]
+    sc = torch.cat([low & 63, (top & 15) | ((low >> 6) << 4)], -1).double() * _f16_pairs(b[..., 0:2])
+    mn = torch.cat([mid & 63, (top >> 4) | ((mid >> 6) << 4)], -1).double() * _f16_pairs(b[..., 2:4])
+    qs = b[..., -128:].reshape(*b.shape[:2], 4, 32)
+    q = torch.stack([qs & 15, qs >> 4], -2).reshape(*b.shape[:2], 8, 32)
+    if dt == synth.Q5_K:
+        q = q | torch.stack([((b[..., 16:48] >> j) & 1) << 4 for j in range(8)], -2)
+    return (q.double() * sc.unsqueeze(-1) - mn.unsqueeze(-1)).reshape(b.shape[0], -1)
+
+
+def _product64(x, rows, decode):
+    """x [tokens][n_in] times the weights' transpose, decoded some rows at a time."""
+    step = max(1, (1 << 26) // x.shape[1])
+    return torch.cat([x.double() @ decode(r, min(rows, r + step)).t() for r in range(0, rows, step)], 1)
+
+
+def _kquant64(raw, dt, x):
+    return _product64(x, raw.shape[0], lambda a, b: _dense64(raw[a:b], dt))
+
+
+def _norm64(x, w, eps):
+    x = x.double()
+    return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * w.double()
+
+
+_E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0)
+
+
+def _fp4_values(packed, scales):
+    """Codes and their E4M3 scales, one per 16 -> f64 values."""
+    codes = torch.stack([packed & 15, packed >> 4], -1).reshape(packed.shape[0], -1, 16)
+    return (torch.tensor(_E2M1, dtype=torch.float64, device=packed.device)[codes.int()] * scales.view(torch.float8_e4m3fn).double().unsqueeze(-1)).flatten(1)
+
+
+def _nvfp4_dot64(w, x):
+    """x (codes times scales, or any f64 values) times an NVFP4 weight."""
+    packed, scales, scale2 = w
+    return _product64(x, packed.shape[0], lambda a, b: _fp4_values(packed[a:b], scales[a:b])) * scale2
+
+
+def _fp4_round(x, isi):
+    """x as the W4A4 lane's inputs: each 16 values of f16(x) * isi as E2M1 codes times an E4M3 scale, over isi."""
+    r = x.half().float().reshape(x.shape[0], -1, 16)
+    isi = torch.tensor(isi, dtype=torch.float32, device=x.device)
+    scale = (r.abs().amax(-1) * torch.tensor(1.0 / 6.0, dtype=torch.float32, device=x.device) * isi).clamp_max(448.0).to(torch.float8_e4m3fn).float().unsqueeze(-1)
+    mag, code = r.abs() * isi, 0
+    for edge, inclusive in ((0.25, False), (0.75, True), (1.25, False), (1.75, True), (2.5, False), (3.5, True), (5.0, False)):
+        code = code + ((mag >= scale * edge) if inclusive else (mag > scale * edge)).int()
+    value = torch.tensor(_E2M1[:8], dtype=torch.float64, device=x.device)[code] * scale
+    return torch.copysign(value, r.double()).flatten(1) / isi.double()
+
+
+def _int8_round(x):
+    """x as the weight-only lane's inputs: each 256 values of f16(x) as int8 against the first of largest magnitude."""
+    r = x.half().float().reshape(x.shape[0], -1, 256)
+    inverse = -127.0 / r.gather(-1, r.abs().argmax(-1, keepdim=True))
+    return (torch.round(inverse.double() * r.double()).clamp_max(127.0) * (1.0 / inverse).double()).flatten(1)
+
+
+def _exact_decode(case, seed):
+    p = _projections(case)
+    raw = _kquant_raw(p, seed)
+    norms, q_norm, k_norm, hidden = _decode_inputs(case, seed)
+    dot = lambda n, x: _kquant64(raw[n], p[n][2], x)  # noqa: E731
+    heads = lambda x, w: _norm64(x.reshape(case["tokens"], -1, HEAD_DIM), w, EPS).flatten(1)  # noqa: E731
+    x = _norm64(hidden, norms["attn"], EPS)
+    q, k, v, gate = heads(dot("q", x), q_norm), heads(dot("k", x), k_norm), dot("v", x), dot("gate", x)
+    q = q * torch.sigmoid(gate)
+    proj = dot("o", q)
+    hidden = hidden.double() + _norm64(proj, norms["post_attn"], EPS_POST)
+    y = _norm64(hidden, norms["ffn"], EPS)
+    act = torch.nn.functional.silu(dot("ffn_gate", y)) * dot("ffn_up", y)
+    down = dot("ffn_down", act)
+    return {"hidden": hidden + _norm64(down, norms["post_ffn"], EPS_POST), "y": y, "proj": proj, "act": act, "down": down, "q": q, "k": k, "v": v, "gate": gate}
+
+
+def _exact_projections(case, seed):
+    p, x = _projections(case), _projection_inputs(case, seed)
+    if case["kind"] == "verify":
+        raw = _kquant_raw(p, seed)
+        return {n: _kquant64(raw[n], p[n][2], x[INPUT[n]]) for n in p}
+    raw = _nvfp4_raw(p, seed, {})[0]
+    return {n: _nvfp4_dot64(raw[n], _int8_round(x[INPUT[n]])) for n in p}
+
+
+def _exact_lm_head(case, seed):
+    raw, x = _lm_head_inputs(case, seed)
+    logits = 30.0 * torch.tanh(_kquant64(raw, QUANTS[case["quant"]], x) * 0.5 / 30.0)
+    return [None, logits.amax(-1), None, logits]
+
+
+def _exact_nvfp4(case, seed):
+    """What one entry point hands to the next has the type that the caller's buffers have: bf16, or 4-bit codes."""
+    x, norms, sample = _nvfp4_inputs(case, seed)
+    w, isi = _nvfp4_raw(_projections(case), seed, {"sample": sample, "norms": norms})
+    stored = lambda v: v.float().bfloat16()  # noqa: E731
+    a = _fp4_round(_norm64(x, norms[0], EPS), isi["q"])
+    q, k, v = (_nvfp4_dot64(w[n], a) for n in ("q", "k", "v"))
+    h1 = _nvfp4_dot64(w["o"], _fp4_round(stored(q), isi["o"])) + x.double()
+    a = _fp4_round(_norm64(stored(h1), norms[1], EPS), isi["ffn_gate"])
+    act = torch.nn.functional.silu(_nvfp4_dot64(w["ffn_gate"], a).half().double()) * _nvfp4_dot64(w["ffn_up"], a).half().double()
+    return [q, k, v, h1, _nvfp4_dot64(w["ffn_down"], _fp4_round(act, isi["ffn_down"])) + stored(h1).double()]
+
+
+def exact(case, seed):
+    """run()'s outputs for prepare(case, seed)'s inputs in plain 64-bit arithmetic, from the formats' definitions."""
+    return {"decode": _exact_decode, "verify": _exact_projections, "nvfp4_a16": _exact_projections, "lm_head": _exact_lm_head, "nvfp4": _exact_nvfp4}[case["kind"]](case, seed)
