@@ -7,45 +7,69 @@
 
 namespace muser {
 
-__device__ __forceinline__ float e4m3_to_f32(uint32_t code) { // finite, non-negative codes only
-    const uint32_t ex = (code >> 3) & 15u, man = code & 7u;
-    if (ex == 0) return (float)man * (1.0f / 512.0f);
-    return __fmul_rn(1.0f + (float)man * 0.125f, __uint_as_float((ex + 120u) << 23));
-}
-
-__device__ __forceinline__ uint32_t e2m1_code(float r, float isi, float scale) {
-    const uint32_t sign = (__float_as_uint(r) >> 31) << 3;
-    if (scale == 0.0f) return sign;
-    const float m = __fmul_rn(fabsf(r), isi);
-    uint32_t code = 0;
-    code += m > __fmul_rn(scale, 0.25f);
-    code += m >= __fmul_rn(scale, 0.75f);
-    code += m > __fmul_rn(scale, 1.25f);
-    code += m >= __fmul_rn(scale, 1.75f);
-    code += m > __fmul_rn(scale, 2.5f);
-    code += m >= __fmul_rn(scale, 3.5f);
-    code += m > __fmul_rn(scale, 5.0f);
-    return sign | code;
+// Eight magnitudes-with-sign -> one word of E2M1 codes, the first in the low nibble: nearest, ties to the even code,
+// saturating, the sign of a zero kept.
+__device__ __forceinline__ uint32_t e2m1_word(const float (&q)[8]) {
+    uint32_t w;
+    asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+        "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+        : "=r"(w) : "f"(q[0]), "f"(q[1]), "f"(q[2]), "f"(q[3]), "f"(q[4]), "f"(q[5]), "f"(q[6]), "f"(q[7]));
+    return w;
 }
 
 // Quantizes one group of 16 values: writes its 8 code bytes and returns its E4M3 scale code.
-__device__ __forceinline__ uint32_t quantize_group(float (&r)[16], float isi, uint8_t *codes) {
-    float amax = 0.0f;
+//
+// The reference compares m = |r| * isi with scale * {0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5} by > and >= in turn.  Those
+// products are exact (a 4-bit and a 3-bit significand), the bounds are the midpoints between neighbouring E2M1 values
+// and the >= ones belong to the even code: the chain is "m / scale to the nearest E2M1 value, ties to even", which is
+// one conversion instruction.  The quotient has to be the correctly rounded one: two floats m and scale * bound that
+// differ, differ by more than half a unit of the bound's last place after the division, so the rounded quotient meets a
+// midpoint only where m met it.  It is made without a divide, by the residual of a product with the rounded
+// reciprocal (tests/test_nvfp4_codec_cpu.py runs every scale against the floats around every bound).  The chain (seven
+// multiplies, compares and adds a value) bounded both quantizer kernels and the GEMM epilogue that quantizes: norm +
+// quantize of 32768 x 5120 286 -> 166 us, quantize 270 -> 148 (the memory alone: 66), gate/up + quantize 6.14 -> 4.82 ms.
+__device__ __forceinline__ uint32_t quantize_group(const float (&r)[16], float isi, uint8_t *codes) {
+    __half2 h[8], top = __floats2half2_rn(0.0f, 0.0f);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        r[i] = __half2float(__float2half_rn(r[i]));
-        amax = fmaxf(amax, fabsf(r[i]));
+    for (int i = 0; i < 8; ++i) {
+        h[i] = __floats2half2_rn(r[2 * i], r[2 * i + 1]);
+        top = __hmax2_nan(top, __habs2(h[i]));
+    }
+    const float2 top2 = __half22float2(top);
+    float amax = fmaxf(top2.x, top2.y);
+    float m[16], v[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float2 f = __half22float2(h[i]);
+        v[2 * i] = f.x, v[2 * i + 1] = f.y;
+        m[2 * i] = __fmul_rn(fabsf(f.x), isi), m[2 * i + 1] = __fmul_rn(fabsf(f.y), isi);
+    }
+    // A NaN is left out of the maximum and compares false all along (code 0 with its sign); an infinity, or a product
+    // that overflows, is above every bound: the former become 0, the latter a number that still is.
+    if (!(__fmul_rn(top2.x, isi) <= 1e30f && __fmul_rn(top2.y, isi) <= 1e30f)) {
+        amax = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            amax = fmaxf(amax, fabsf(v[i]));
+            m[i] = m[i] > 0.0f ? fminf(m[i], 1e30f) : 0.0f;
+        }
     }
     const float target = fminf(__fmul_rn(__fmul_rn(amax, 1.0f / 6.0f), isi), 448.0f);
     const uint32_t scale_code = __nv_cvt_float_to_fp8(target, __NV_SATFINITE, __NV_E4M3) & 0x7Fu;
-    const float scale = e4m3_to_f32(scale_code);
-    uint32_t lo = 0, hi = 0;
+    const float scale = __half2float(__half(__nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)scale_code, __NV_E4M3)));
+    const float inv = scale > 0.0f ? __frcp_rn(scale) : 0.0f; // no scale: only the signs remain
+    float q[2][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        lo |= e2m1_code(r[i], isi, scale) << (4 * i);
-        hi |= e2m1_code(r[8 + i], isi, scale) << (4 * i);
+    for (int i = 0; i < 16; ++i) {
+        const float q0 = __fmul_rn(m[i], inv);
+        const float q1 = __fmaf_rn(__fmaf_rn(-q0, scale, m[i]), inv, q0);
+        q[i >> 3][i & 7] = __uint_as_float(__float_as_uint(q1) | (__float_as_uint(v[i]) & 0x80000000u));
     }
-    *reinterpret_cast<uint2 *>(codes) = make_uint2(lo, hi);
+    *reinterpret_cast<uint2 *>(codes) = make_uint2(e2m1_word(q[0]), e2m1_word(q[1]));
     return scale_code;
 }
 
