@@ -9,19 +9,22 @@
 // then four FMAs in a fixed order turn it into f32, the blocks are added front to back, and the result is rounded
 // to f16.  Nothing here is approximate, so outputs are compared for equal bits.
 //
-// This is the lane for checkpoints without activation scales, not the prefill hot path: one warp per output row,
-// the row's codes read once per group of eight tokens, every weight byte read with 4-byte loads.  The activations
-// of a call are quantized once into the context workspace by a kernel of their own.
+// This is the lane for checkpoints without activation scales, not the prefill hot path.  The activations of a call are
+// quantized once into the context workspace by a kernel of their own; the contraction runs on the int8 tensor pipe.
+#include <cuda_fp8.h>
+
 #include "common.cuh"
 
 namespace muser {
 
 // int8 codes [tokens][n_in] followed by one f32 d per (token, 256-block)
-__global__ void __launch_bounds__(256) nvfp4_q8_quantize_kernel(const void *__restrict__ x, uint32_t x_f32, uint32_t n_in,
-                                                                int8_t *__restrict__ qs, float *__restrict__ ds) {
+__global__ void __launch_bounds__(256) nvfp4_q8_quantize_kernel(const void *x, uint32_t x_f32, uint32_t n_in,
+                                                                int8_t *qs, float *ds) {
     __shared__ float s_mag[8];
     __shared__ uint32_t s_idx[8];
     __shared__ float s_val[8];
+    pdl_wait();
+    pdl_release(); // the contraction may start fetching its weights
     const uint32_t block = blockIdx.x, tok = blockIdx.y, i = threadIdx.x, blocks = n_in / 256;
     const size_t at = (size_t)tok * n_in + (size_t)block * 256 + i;
     const float raw = x_f32 ? reinterpret_cast<const float *>(x)[at] : __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(x)[at]);
@@ -54,75 +57,196 @@ __global__ void __launch_bounds__(256) nvfp4_q8_quantize_kernel(const void *__re
     if (i == 0) ds[(size_t)tok * blocks + block] = d;
 }
 
-__device__ __forceinline__ int e2m1_q1(uint32_t nibble) { // the code's value in halves (quant/nvfp4.rs:16-30)
-    const int m = (int)((0xC8643210u >> (4 * (nibble & 7))) & 15u); // 0, 1, 2, 3, 4, 6, 8, 12
-    return (nibble & 8) ? -m : m;
-}
-__device__ __forceinline__ int e4m3_q9(uint32_t code) { // a finite, non-negative scale code in units of 2^-9 (nvfp4.rs:33-51)
-    const uint32_t ex = (code >> 3) & 15u, man = code & 7u;
-    return ex == 0 ? (int)man : (int)((8u + man) << (ex - 1));
-}
-
 struct A16Args {
     const uint8_t *packed, *scales; // the repacked image: codes [n_out_pad][n_in/2], swizzled unsigned scales
     const int8_t *qs;
     const float *ds;
     void *y;
     float scale2;
-    uint32_t n_out, n_in, kt, tokens, y_dtype;
+    uint32_t n_out, n_in, kt, tokens, y_dtype, ksplit, row_tiles;
 };
 
-// One warp per output row, eight tokens at a time.  Lane l takes bytes 4l .. 4l+3 of every 128-byte (256-value) block
-// of the row, i.e. half of 16-group l / 2.
-__global__ void __launch_bounds__(256) nvfp4_a16_kernel(const A16Args a) {
-    const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= a.n_out) return;
+// Four E2M1 codes (the low 16 bits of w, one per nibble) -> four int8 of the codes' values in halves
+// (quant/nvfp4.rs:16-30).  A byte permute looks the magnitude up by the nibble's low three bits; with the nibble's
+// sign bit set it replicates the looked-up byte's top bit instead, i.e. gives 0.  One permute on the codes as they are
+// yields the positive values, one on the codes with their sign bits flipped the negative ones' magnitudes; the bias
+// keeps the borrows of the 32-bit difference inside their bytes.
+__device__ __forceinline__ uint32_t e2m1_halves(uint32_t w, uint32_t w_flipped) {
+    uint32_t pos, neg; // (the __byte_perm intrinsic uses three bits of a selector)
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(pos) : "r"(0x03020100u), "r"(0x0C080604u), "r"(w));
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(neg) : "r"(0x03020100u), "r"(0x0C080604u), "r"(w_flipped));
+    return (pos + 0x80808080u - neg) ^ 0x80808080u;
+}
+__device__ __forceinline__ void imma_k32(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Four unsigned, finite E4M3 scale codes in units of 2^-9 (nvfp4.rs:33-51), at most 229376: through f16, exact.
+__device__ __forceinline__ void e4m3_q9(uint32_t codes, int (&q9)[4]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float2 f = __half22float2(__half2(__nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(codes >> (16 * i)), __NV_E4M3)));
+        q9[2 * i] = __float_as_int(__fmaf_rn(f.x, 512.0f, 12582912.0f)) - 0x4B400000;
+        q9[2 * i + 1] = __float_as_int(__fmaf_rn(f.y, 512.0f, 12582912.0f)) - 0x4B400000;
+    }
+}
+__device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return (&v.x)[i]; } // compile-time i only
+
+constexpr int kA16Warps = 8;
+
+// A warp contracts one 256-value block of 16 weight rows with 2 * PAIRS tokens at a time.  The codes come as they lie in
+// memory: lane (g, t) loads 16 bytes of row g (and of row g + 8) of each 128-value chunk, which are the two 16-groups
+// 2t and 2t + 1.  Word i of the four lanes of a row feeds one m16n8k32 product, so its 32 inputs belong to FOUR groups;
+// they are told apart by the columns: column (token, q) carries the token's int8 inputs in lane q of the four and zeros
+// in the others.  Three quarters of such a product are zeros, but the tensor pipe has the time (8 cycles a product and
+// 4 products for 2 tokens beside ~145 other instructions), nothing is regrouped, and weights go from memory to
+// registers.  Two products accumulate a group; its exact sum then meets the group's scale in a 64-bit multiply-add.
+//
+// CTA: 8 / ksplit row tiles; the ksplit warps of a tile take neighbouring blocks, leave their f32 contributions in
+// shared memory, meet at a named barrier, and every (row, token) sum is continued front to back by one thread, so the
+// order of the additions is the reference's whatever ksplit is.
+//
+// Two tokens: 27648 x 5120 151 -> 35 us, 5120 x 27648 222 -> 58, 1024 x 5120 23 -> 6.5, a layer's seven calls 699 -> 167
+// (bound by instruction issue; the weights' bytes take 12 us each for the large ones).  The earlier form, one warp per
+// row with eight scalar multiply-adds per lane and a 64-bit shuffle tree per token and block, had about five times the
+// instructions per weight.
+template <int PAIRS>
+__global__ void __launch_bounds__(kA16Warps * 32, 2) nvfp4_a16_kernel(const __grid_constant__ A16Args a) {
+    __shared__ float contrib[2][kA16Warps][2 * PAIRS * 16];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t slot = warp / a.ksplit, part = warp % a.ksplit, slots = kA16Warps / a.ksplit;
+    const uint32_t rt = blockIdx.x * slots + slot;
+    // Tile u of a 128-row group holds rows 32 (m & 3) + 4 u + (m >> 2), m = 0..15: four rows that share 16 bytes of the
+    // swizzled scale plane sit side by side.
+    const uint32_t tile_row = (rt / 8) * 128 + 4 * (rt % 8);
+    auto row_of = [&](uint32_t m) { return tile_row + 32 * (m & 3) + (m >> 2); };
+    if (rt >= a.row_tiles || tile_row >= a.n_out) return; // whole slots leave; barriers are per slot
     const uint32_t blocks = a.n_in / 256;
-    const uint8_t *codes = a.packed + (size_t)row * (a.n_in / 2);
-    for (uint32_t t0 = 0; t0 < a.tokens; t0 += 8) {
-        float total[8];
+    const uint8_t *code0 = a.packed + (size_t)row_of(g) * (a.n_in / 2) + 16 * t, *code1 = a.packed + (size_t)row_of(g + 8) * (a.n_in / 2) + 16 * t;
+    auto scale_ptr = [&](uint32_t row) {
+        return a.scales + (size_t)(row / 128) * ((size_t)a.kt * 512) + (row % 32) * 16 + ((row % 128) / 32) * 4 + (t & 1) * 512;
+    };
+    const uint8_t *sc0 = scale_ptr(row_of(g)), *sc1 = scale_ptr(row_of(g + 8));
+    struct Block {
+        uint4 c[2][2];    // [chunk][row g, row g + 8]
+        uint32_t s[2][2];
+    };
+    auto fetch = [&](uint32_t b, Block &k) {
 #pragma unroll
-        for (int t = 0; t < 8; ++t) total[t] = 0.0f;
-        for (uint32_t b = 0; b < blocks; ++b) {
-            const uint32_t w = *reinterpret_cast<const uint32_t *>(codes + (size_t)b * 128 + 4 * lane);
-            const uint32_t grp = b * 16 + lane / 2;
-            const size_t soff = (size_t)(row / 128) * ((size_t)a.kt * 512) + (size_t)(grp / 4) * 512 + (row % 32) * 16 + ((row % 128) / 32) * 4 + grp % 4;
-            const long long q9 = e4m3_q9(a.scales[soff]);
-            int wq[8];
+        for (int ch = 0; ch < 2; ++ch) {
+            k.c[ch][0] = __ldg(reinterpret_cast<const uint4 *>(code0 + (size_t)b * 128 + ch * 64));
+            k.c[ch][1] = __ldg(reinterpret_cast<const uint4 *>(code1 + (size_t)b * 128 + ch * 64));
+            k.s[ch][0] = __ldg(reinterpret_cast<const uint32_t *>(sc0 + (size_t)(4 * b + 2 * ch) * 512));
+            k.s[ch][1] = __ldg(reinterpret_cast<const uint32_t *>(sc1 + (size_t)(4 * b + 2 * ch) * 512));
+        }
+    };
+    Block cur, nxt;
+    if (part < blocks) fetch(part, nxt);
+    pdl_wait(); // the int8 activations come from the kernel before this one; weights are constants
+    // (released behind the wait, so that whatever starts early starts when the kernel before THIS one is complete: no
+    // line of a buffer that is about to be rewritten can enter an SM's L1 after its launch)
+    pdl_release();
+    for (uint32_t t0 = 0; t0 < a.tokens; t0 += 2 * PAIRS) {
+        if (t0 > 0 && part < blocks) fetch(part, nxt);
+        const uint32_t live = min(a.tokens - t0, 2u * PAIRS);
+        float total[PAIRS];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) wq[i] = e2m1_q1((w >> (4 * i)) & 15u); // low nibble = even element
+        for (int i = 0; i < PAIRS; ++i) total[i] = 0.0f;
+        uint32_t step = 0;
+        for (uint32_t b0 = 0; b0 < blocks; b0 += a.ksplit, ++step) {
+            const uint32_t b = b0 + part;
+            float *mine = contrib[step & 1][warp];
+            if (b < blocks) {
+                cur = nxt;
+                if (b + a.ksplit < blocks) fetch(b + a.ksplit, nxt);
+                long long sum[PAIRS][2];
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                if (t0 + t >= a.tokens) break; // warp-uniform
-                const float d = a.ds[(size_t)(t0 + t) * blocks + b];
-                const int2 q = *reinterpret_cast<const int2 *>(a.qs + (size_t)(t0 + t) * a.n_in + (size_t)b * 256 + 8 * lane);
-                int dot = 0;
+                for (int p = 0; p < PAIRS; ++p) sum[p][0] = sum[p][1] = 0;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) dot += wq[i] * (int)(int8_t)(((i < 4 ? q.x : q.y) >> (8 * (i & 3))) & 0xFF);
-                dot += __shfl_xor_sync(0xffffffffu, dot, 1); // the two halves of a 16-group
-                long long part = (lane & 1) ? 0ll : (long long)dot * q9;
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t av[4][4];
 #pragma unroll
-                for (int o = 2; o < 32; o <<= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-                if (d != 0.0f) { // a block of zeros is skipped (nvfp4.rs:356-358)
-                    float c = __fmaf_rn(__ll2float_rn(part), 1.0f / 1024.0f, 0.0f);
-                    c = __fmaf_rn(c, d, 0.0f);
-                    c = __fmaf_rn(c, a.scale2, 0.0f);
-                    total[t] = __fmaf_rn(1.0f, c, total[t]);
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const uint32_t w = word(cur.c[ch][r], i), f = w ^ 0x88888888u;
+                            av[i][r] = e2m1_halves(w, f);
+                            av[i][2 + r] = e2m1_halves(w >> 16, f >> 16);
+                        }
+                    int q0[4], q1[4]; // groups 4 (t & 1) .. + 3 of the chunk, rows g and g + 8
+                    e4m3_q9(cur.s[ch][0], q0);
+                    e4m3_q9(cur.s[ch][1], q1);
+#pragma unroll
+                    for (int p = 0; p < PAIRS; ++p) {
+                        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+                        const uint32_t tok = 2 * p + (g >> 2);
+                        if ((g & 3) == t && tok < live) {
+                            const uint4 *src = reinterpret_cast<const uint4 *>(a.qs + (size_t)(t0 + tok) * a.n_in + (size_t)b * 256 + ch * 128 + 32 * t);
+                            x0 = ld_after_wait(src), x1 = ld_after_wait(src + 1);
+                        }
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) { // groups 2q + h of the four lanes q
+                            int d[4] = {0, 0, 0, 0};
+                            const uint4 &x = h ? x1 : x0;
+                            imma_k32(d, av[2 * h][0], av[2 * h][1], av[2 * h][2], av[2 * h][3], x.x, x.y);
+                            imma_k32(d, av[2 * h + 1][0], av[2 * h + 1][1], av[2 * h + 1][2], av[2 * h + 1][3], x.z, x.w);
+                            sum[p][0] += (long long)d[0] * q0[h] + (long long)d[1] * q0[2 + h];
+                            sum[p][1] += (long long)d[2] * q1[h] + (long long)d[3] * q1[2 + h];
+                        }
+                    }
+                }
+                // lanes t and t ^ 1 hold the two halves of the block for token 2 p + (t >> 1): the even one ends up with
+                // row g, the odd one with row g + 8
+                const uint32_t odd = t & 1, m = g + 8 * odd;
+#pragma unroll
+                for (int p = 0; p < PAIRS; ++p) {
+                    const long long other = __shfl_xor_sync(0xffffffffu, odd ? sum[p][0] : sum[p][1], 1);
+                    const long long whole = (odd ? sum[p][1] : sum[p][0]) + other;
+                    const uint32_t tok = 2 * p + (t >> 1);
+                    float c = -0.0f; // a block of zeros is skipped (nvfp4.rs:356-358): adding -0 changes nothing
+                    const float d = tok < live ? ld_after_wait(a.ds + (size_t)(t0 + tok) * blocks + b) : 0.0f;
+                    if (d != 0.0f) {
+                        c = __fmaf_rn(__ll2float_rn(whole), 1.0f / 1024.0f, 0.0f);
+                        c = __fmaf_rn(c, d, 0.0f);
+                        c = __fmaf_rn(c, a.scale2, 0.0f);
+                    }
+                    mine[tok * 16 + m] = c;
                 }
             }
-        }
-        if (lane == 0) {
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(a.ksplit * 32) : "memory");
+            // (two buffers in turn: a warp writes a buffer again only behind the next step's barrier)
+            const uint32_t n_here = min(a.ksplit, blocks - b0);
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                if (t0 + t >= a.tokens) break;
-                const __half h = __float2half_rn(total[t]); // the lane's output boundary (nvfp4.rs:378)
-                const size_t o = (size_t)(t0 + t) * a.n_out + row;
-                if (a.y_dtype == MUSER_DTYPE_F16) reinterpret_cast<__half *>(a.y)[o] = h;
-                else if (a.y_dtype == MUSER_DTYPE_BF16) reinterpret_cast<__nv_bfloat16 *>(a.y)[o] = __float2bfloat16_rn(__half2float(h));
-                else reinterpret_cast<float *>(a.y)[o] = __half2float(h);
+            for (int i = 0; i < PAIRS; ++i) {
+                const uint32_t e = part * 32 + lane + (uint32_t)i * a.ksplit * 32;
+                if (e < 32u * PAIRS)
+                    for (uint32_t s = 0; s < n_here; ++s) total[i] = __fmaf_rn(1.0f, contrib[step & 1][slot * a.ksplit + s][e], total[i]);
             }
         }
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            const uint32_t e = part * 32 + lane + (uint32_t)i * a.ksplit * 32, tok = e / 16, row = row_of(e % 16);
+            if (e >= 32u * PAIRS || tok >= live || row >= a.n_out) continue;
+            const __half h = __float2half_rn(total[i]); // the lane's output boundary (nvfp4.rs:378)
+            const size_t o = (size_t)(t0 + tok) * a.n_out + row;
+            if (a.y_dtype == MUSER_DTYPE_F16) reinterpret_cast<__half *>(a.y)[o] = h;
+            else if (a.y_dtype == MUSER_DTYPE_BF16) reinterpret_cast<__nv_bfloat16 *>(a.y)[o] = __float2bfloat16_rn(__half2float(h));
+            else reinterpret_cast<float *>(a.y)[o] = __half2float(h);
+        }
     }
+}
+
+// Warps per row tile: the split with the fewest rounds of (CTAs on the GPU) x (blocks in turn), two CTAs an SM.  Few
+// rows (attn_k: 64 tiles) want all eight warps on one tile, 27648 rows of 20 blocks four (15 rounds against 20 and 18).
+static uint32_t a16_ksplit(uint32_t row_tiles, uint32_t blocks, int sm_count) {
+    uint32_t best = 1, best_rounds = ~0u;
+    for (uint32_t ks = 1; ks <= kA16Warps; ks *= 2) {
+        const uint32_t ctas = (row_tiles + kA16Warps / ks - 1) / (kA16Warps / ks);
+        const uint32_t rounds = (ctas + 2 * sm_count - 1) / (2 * sm_count) * ((blocks + ks - 1) / ks);
+        if (rounds < best_rounds) best = ks, best_rounds = rounds;
+    }
+    return best;
 }
 
 // x: [tokens][n_in] f32 or bf16; the int8 codes and block scales pass through `workspace`.
@@ -136,14 +260,19 @@ muser_cuda_status launch_nvfp4_a16(Ctx *ctx, const Weight *w, const void *x, uin
         return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "context workspace holds " + std::to_string(workspace_bytes) + " bytes, this call needs " + std::to_string(q_bytes + d_bytes));
     int8_t *qs = reinterpret_cast<int8_t *>(workspace);
     float *ds = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(workspace) + q_bytes);
-    nvfp4_q8_quantize_kernel<<<dim3((unsigned)(w->n_in / 256), tokens), 256, 0, stream>>>(x, x_dtype == MUSER_DTYPE_F32, (uint32_t)w->n_in, qs, ds);
-    MUSER_CUDA_TRY(ctx, cudaGetLastError());
+    MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_q8_quantize_kernel, dim3((unsigned)(w->n_in / 256), tokens), dim3(256), 0, stream, x,
+                                   (uint32_t)(x_dtype == MUSER_DTYPE_F32), (uint32_t)w->n_in, qs, ds));
     A16Args a;
     a.packed = w->packed, a.scales = w->scales, a.qs = qs, a.ds = ds, a.y = y;
     a.scale2 = w->scale2;
     a.n_out = (uint32_t)w->n_out, a.n_in = (uint32_t)w->n_in, a.kt = (uint32_t)((w->n_in + 63) / 64), a.tokens = tokens, a.y_dtype = y_dtype;
-    nvfp4_a16_kernel<<<(unsigned)((w->n_out + 7) / 8), 256, 0, stream>>>(a);
-    MUSER_CUDA_TRY(ctx, cudaGetLastError());
+    a.row_tiles = (a.n_out + 127) / 128 * 8;
+    a.ksplit = a16_ksplit(a.row_tiles, a.n_in / 256, ctx->sm_count);
+    const dim3 grid((a.row_tiles * a.ksplit + kA16Warps - 1) / kA16Warps), threads(kA16Warps * 32);
+    if (tokens <= 2) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<1>, grid, threads, 0, stream, a));
+    else if (tokens <= 4) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<2>, grid, threads, 0, stream, a));
+    else if (tokens <= 8) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<4>, grid, threads, 0, stream, a));
+    else MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<8>, grid, threads, 0, stream, a));
     return MUSER_CUDA_OK;
 }
 
