@@ -10,7 +10,7 @@
 // 4-stage shared-memory ring; warp 1 copies each K = 64 block's scale factors into tensor memory (tcgen05.cp) and
 // issues its tcgen05.mma kind::mxf4nvf4 right behind them into a 128 x 256 f32 accumulator in tensor memory (both
 // warps run their loops converged and issue through an elected lane: tcgen05.cuh);
-// warps 2-9 read the accumulator back (tcgen05.ld), apply the two tensor scales and the fused epilogue, and
+// warps 2-17 read the accumulator back (tcgen05.ld), apply the two tensor scales and the fused epilogue, and
 // store.  Every mbarrier wait is bounded: on expiry the CTA records a code in the context's status word,
 // stops issuing work, waits (bounded) for its own copies in flight, frees its tensor memory and returns.
 #include <cuda.h>
@@ -51,6 +51,7 @@ constexpr int kSfbBytes = 2 * 4 * 512;           // 256 rows x 16 scales
 constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
 constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
 static_assert(kSmemBytes <= 227 * 1024, "stage ring exceeds the shared memory of one CTA");
+constexpr int kEpiWarps = 16, kGemmThreads = 32 * (2 + kEpiWarps);
 constexpr uint32_t kTmemCols = 512;              // 256 accumulator + 16 SFA + 32 SFB, rounded to a power of two
 constexpr uint32_t kSfCol = 256, kSfBufCols = 48, kSfBufs = 4; // scale buffers of 16 (SFA) + 32 (SFB) columns behind the accumulator
 
@@ -129,6 +130,37 @@ __device__ __forceinline__ void mma_nvf4_elect(uint32_t tmem_d, uint64_t desc_a,
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
         : "memory");
 }
+__device__ __forceinline__ void ld_32b(const void *p, uint32_t (&r)[8]) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_32b(void *p, const uint32_t (&r)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+// Sixteen neighbouring 16-bit outputs in one 32-byte store (a lane's row is its own: narrower stores write half
+// sectors), with the residual, fetched the same way, added in f32.
+template <typename T>
+__device__ __forceinline__ void store_16_wide(const float *v, T *y, const uint32_t *res) {
+    uint32_t o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        float a = v[2 * i], b = v[2 * i + 1];
+        if constexpr (std::is_same<T, __half>::value) {
+            if (res) {
+                const float2 r = __half22float2(*reinterpret_cast<const __half2 *>(res + i));
+                a += r.x, b += r.y;
+            }
+            const __half2 h = __floats2half2_rn(a, b);
+            o[i] = *reinterpret_cast<const uint32_t *>(&h);
+        } else {
+            if (res) a += __uint_as_float(res[i] << 16), b += __uint_as_float(res[i] & 0xFFFF0000u);
+            const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+            o[i] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+    }
+    st_32b(y, o);
+}
 // One 32-column strip of one accumulator row: scale, fuse, convert, store (16-byte stores when the row allows).
 template <typename T>
 __device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T *res, uint32_t valid, bool vec_ok) {
@@ -200,7 +232,7 @@ __device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T 
 // tiles form one tile space, so the small ones fill the SMs that a launch of their own would leave idle.  Plain
 // outputs only (no fused tail, row scale or residual).
 template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false>
-__global__ void __launch_bounds__(352, 1)
+__global__ void __launch_bounds__(kGemmThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_b3,
                   const __grid_constant__ CUtensorMap map_b4, const GemmArgs g) {
@@ -224,7 +256,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_acc_full, 1);
-        mbar_init(bar_acc_empty, 8); // one arrival per epilogue warp
+        mbar_init(bar_acc_empty, kEpiWarps); // one arrival per epilogue warp
         for (int b = 0; b < (int)kSfBufs; ++b) {
             mbar_init(bar_sf_full + 8 * b, 1);
             mbar_init(bar_sf_empty + 8 * b, 1);
@@ -323,15 +355,6 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     const uint64_t da = operand_desc(st), db = operand_desc(st + kABytes);
                     const uint32_t nkb = min(4u, g.kt64 - 4 * kt);
                     const uint32_t buf = it % kSfBufs, sf = tmem + kSfCol + buf * kSfBufCols;
-#ifdef MUSER_GEMM_COPIER_WARP
-                    // the scale factors of this slab were copied into tensor memory by the copier warp
-                    PROF_BEGIN ok = mbar_wait_warp(bar_sf_full + 8 * buf, (it / kSfBufs) & 1, abort_flag); PROF_END(2)
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (uint32_t kb = 0; kb < nkb; ++kb) // 64 values = 32 bytes further along the swizzled 128-byte rows: +2 in 16-byte units
-                        mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, (kt | kb) != 0);
-                    mma_commit_elect(bar_sf_empty + 8 * buf);
-#else
                     // Each MMA's scale factors go to tensor memory right in front of it, from the same lane: the tensor
                     // pipe takes both in issue order, so no barrier stands between a copy and the MMA that reads it, and
                     // the copies run under the MMAs before them (691 cycles per slab in isolation against 548 for the
@@ -343,7 +366,6 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         tmem_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
                         mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, (kt | kb) != 0);
                     }
-#endif
                     mma_commit_elect(bar_empty + 8 * s); // the stage may be overwritten once these MMAs have read it
                 }
                 if (ok) mma_commit_elect(bar_acc_full);
@@ -354,45 +376,17 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 atomicExch(g.status + 1, 102);
             }
         }
-    } else if (warp == 10) {
-#ifdef MUSER_GEMM_COPIER_WARP
-        // ---------------------------------------------------------------- scale copier (development alternative)
-        // tcgen05.cp of the slab's scale factors into one of the tensor-memory buffers, issued by a warp of its own.
-        {
-            uint32_t it = 0;
-            bool ok = true; PROF_DECL
-            for (uint32_t tile = blockIdx.x; tile < n_tiles_total && ok; tile += gridDim.x) {
-                for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
-                    const uint32_t s = it % kStages, round = it / kStages, buf = it % kSfBufs;
-                    PROF_BEGIN ok = mbar_wait_warp(bar_full + 8 * s, round & 1, abort_flag); PROF_END(0)
-                    PROF_BEGIN if (ok && it >= kSfBufs) ok = mbar_wait_warp(bar_sf_empty + 8 * buf, ((it / kSfBufs) - 1) & 1, abort_flag); PROF_END(1)
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t st = base + s * kStageBytes, sfa = st + kABytes + kBBytes, sfb = sfa + kSfaBytes;
-                    const uint32_t sf = tmem + kSfCol + buf * kSfBufCols, nkb = min(4u, g.kt64 - 4 * kt);
-                    for (uint32_t kb = 0; kb < nkb; ++kb) {
-                        tmem_cp_scales_elect(sf + 4 * kb, scale_desc(sfa + 512 * kb));
-                        tmem_cp_scales_elect(sf + 16 + 8 * kb, scale_desc(sfb + 512 * kb));
-                        tmem_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
-                    }
-                    mma_commit_elect(bar_sf_full + 8 * buf);
-                }
-            }
-            if (lane == 0) { PROF_FLUSH(2) }
-            if (!ok && lane == 0) {
-                *abort_flag = 1;
-                atomicCAS(g.status + 1, 0, 105);
-            }
-        }
-#endif
     } else {
-        // ---------------------------------------------------------------- epilogue (warps 2..9)
-        // Eight warps: two per 32-lane quarter of the accumulator, one for each half of the tile's output columns.
-        // There is room for one accumulator only, so the MMA warp cannot start the next tile before the last
-        // tcgen05.ld of this one.
+        // ---------------------------------------------------------------- epilogue (warps 2..17)
+        // Sixteen warps: four per 32-lane quarter of the accumulator, one for each quarter of the tile's output columns
+        // (64, or 32 gate + 32 up).  There is room for one accumulator only, so the MMA warp cannot start the next tile
+        // before the last tcgen05.ld of this one, and the rest of the epilogue runs under the next tile's products: it
+        // must not take longer than those do.  With eight warps it did wherever it does more than store: gate/up +
+        // quantize at 32768 tokens had two warps a scheduler waiting on each other's chains of conversions, and o_proj
+        // waited for its residual behind the accumulator.
         const uint32_t quad = warp & 3;                 // the 32 accumulator lanes this warp may read
-        const uint32_t part = (uint32_t)(warp - 2) >> 2; // which half of the output columns
-        constexpr uint32_t kOutCols = DUAL ? BN / 2 : BN, kPartCols = kOutCols / 2;
+        const uint32_t part = (uint32_t)(warp - 2) >> 2; // which quarter of the output columns
+        constexpr uint32_t kOutCols = DUAL ? BN / 2 : BN, kPartCols = kOutCols / 4, kStrips = kPartCols / 32;
         uint32_t local = 0;
         for (uint32_t tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++local) {
             uint32_t tile_m, tile_n;
@@ -405,6 +399,22 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 tile_n -= g.grp_tile0[p];
                 n_out = g.grp_n_out[p], y_out = g.grp_y[p], scale2 = g.grp_scale2[p];
             }
+            const uint32_t tok = tile_m * BM + quad * 32 + lane, col0 = part * kPartCols, out0 = tile_n * kOutCols + col0;
+            const bool live = tok < g.tokens && out0 < n_out;
+            // 16-bit rows whose 16-value pieces are whole 32-byte sectors
+            const bool wide = live && g.y_dtype != MUSER_DTYPE_F32 && (n_out & 15) == 0 && out0 + kPartCols <= n_out &&
+                              ((reinterpret_cast<uintptr_t>(y_out) | reinterpret_cast<uintptr_t>(g.residual)) & 31) == 0;
+            // the residual is fetched while the products still run: the first strip's to registers, the second's to L2
+            uint32_t res[2][8];
+            const bool wide_res = !DUAL && !GROUP && wide && g.residual;
+            const uint8_t *res_at = reinterpret_cast<const uint8_t *>(g.residual) + ((size_t)tok * n_out + out0) * 2;
+            auto load_res = [&](uint32_t s) {
+                if (wide_res) ld_32b(res_at + 64 * s, res[0]), ld_32b(res_at + 64 * s + 32, res[1]);
+            };
+            if constexpr (!DUAL && !GROUP) {
+                load_res(0);
+                if (wide_res) asm volatile("prefetch.global.L2 [%0];" ::"l"(res_at + 64));
+            }
             const bool ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_full, local & 1, abort_flag));
             if (!ok) {
                 if (lane == 0) {
@@ -414,76 +424,83 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tok = tile_m * BM + quad * 32 + lane;
             const float rs = (g.row_scale && tok < g.tokens) ? g.row_scale[tok] : 1.0f;
             const bool vec_ok = (n_out & 7) == 0;
-            const uint32_t lane_base = tmem + ((quad * 32) << 16), col0 = part * kPartCols;
-            // All of this warp's part of the accumulator goes to registers first (128 values a thread) and the
+            const uint32_t lane_base = tmem + ((quad * 32) << 16);
+            // All of this warp's part of the accumulator goes to registers first (64 values a thread) and the
             // accumulator is handed back at once: the MMA warp cannot start the next tile before that, so nothing
             // that touches global memory may sit in between.
-            uint32_t r[4][32];
+            uint32_t r[2][32];
 #pragma unroll
-            for (uint32_t s = 0; s < 4; ++s) // fused form: strips 0, 1 are gate columns, 2, 3 the same columns of up
-                tmem_ld32(lane_base + col0 + (DUAL ? (s & 1) * 32 + (s >> 1) * kOutCols : 32 * s), r[s]);
+            for (uint32_t s = 0; s < 2; ++s) // fused form: strip 0 is gate columns, strip 1 the same columns of up
+                tmem_ld32(lane_base + col0 + s * (DUAL ? kOutCols : 32), r[s]);
             tmem_ld_wait();
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
-            uint32_t q_word = 0; // QOUT: the four scale bytes of this thread's 64 outputs
-#pragma unroll
-            for (uint32_t s = 0; s < kPartCols / 32; ++s) {
-                const uint32_t c0 = col0 + 32 * s;
-                uint32_t(&cur)[32] = r[s];
-                uint32_t(&r_up)[32] = r[DUAL ? 2 + s : s];
-                const uint32_t n0 = tile_n * kOutCols + c0;
-                if constexpr (QOUT) {
-                    // rows of the last 128-token block that hold no token get zero scale bytes: the next GEMM reads the
-                    // block's whole scale chunk (their codes come from TMA's zero fill)
-                    if (n0 < n_out) {
+            if constexpr (QOUT) {
+                // rows of the last 128-token block that hold no token get zero scale bytes: the next GEMM reads the
+                // block's whole scale chunk (their codes come from TMA's zero fill)
+                if (out0 < n_out) {
+                    uint32_t q_scales = 0; // the two scale bytes of this thread's 32 outputs
+                    if (tok < g.tokens) {
                         float v[32];
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const float gate = __half2float(__float2half_rn(__fmul_rn(__fmul_rn(__uint_as_float(cur[i]), scale2), g.inv_input_scale)));
-                            const float up = __half2float(__float2half_rn(__fmul_rn(__fmul_rn(__uint_as_float(r_up[i]), g.scale2_up), g.inv_input_scale)));
+                            const float gate = __half2float(__float2half_rn(__fmul_rn(__fmul_rn(__uint_as_float(r[0][i]), scale2), g.inv_input_scale)));
+                            const float up = __half2float(__float2half_rn(__fmul_rn(__fmul_rn(__uint_as_float(r[1][i]), g.scale2_up), g.inv_input_scale)));
                             v[i] = __fdiv_rn(gate, 1.0f + expf(-gate)) * up;
                         }
-                        if (tok < g.tokens) {
-                            uint8_t *codes = g.q_packed + (size_t)tok * (n_out / 2) + n0 / 2;
-                            float(&lo)[16] = *reinterpret_cast<float(*)[16]>(&v[0]);
-                            float(&hi)[16] = *reinterpret_cast<float(*)[16]>(&v[16]);
-                            q_word |= quantize_group(lo, g.q_isi, codes) << (16 * s);
-                            q_word |= quantize_group(hi, g.q_isi, codes + 8) << (16 * s + 8);
-                        }
+                        uint8_t *codes = g.q_packed + (size_t)tok * (n_out / 2) + out0 / 2;
+                        float(&lo)[16] = *reinterpret_cast<float(*)[16]>(&v[0]);
+                        float(&hi)[16] = *reinterpret_cast<float(*)[16]>(&v[16]);
+                        q_scales = quantize_group(lo, g.q_isi, codes);
+                        q_scales |= quantize_group(hi, g.q_isi, codes + 8) << 8;
                     }
-                    if (s + 1 == kPartCols / 32 && tile_n * kOutCols + col0 < n_out)
-                        *reinterpret_cast<uint32_t *>(g.q_scales + swizzled_scale_offset(tok, (tile_n * kOutCols + col0) / 16, g.q_kt)) = q_word;
-                    continue;
+                    *reinterpret_cast<uint16_t *>(g.q_scales + swizzled_scale_offset(tok, out0 / 16, g.q_kt)) = (uint16_t)q_scales;
                 }
-                if (tok < g.tokens && n0 < n_out) {
-                    const size_t o = (size_t)tok * n_out + n0;
-                    const uint32_t valid = min(32u, n_out - n0);
-                    float v[32];
+                continue;
+            }
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) { // quant/nvfp4.rs:334-336: tensor scales applied one after the other
-                        v[i] = __fmul_rn(__fmul_rn(__uint_as_float(cur[i]), scale2), g.inv_input_scale);
-                        if constexpr (DUAL) {
-                            const float gate = __half2float(__float2half_rn(v[i]));
-                            const float up = __half2float(__float2half_rn(
-                                __fmul_rn(__fmul_rn(__uint_as_float(r_up[i]), g.scale2_up), g.inv_input_scale)));
-                            v[i] = __fdiv_rn(gate, 1.0f + expf(-gate)) * up; // silu_fast, quant/helpers.rs:72
-                        }
-                        v[i] *= rs;
-                        if constexpr (TAIL) v[i] = logit_tail(v[i], g.out_scale, g.softcap);
+            for (uint32_t s = 0; s < kStrips; ++s) {
+                const uint32_t n0 = out0 + 32 * s;
+                if (tok >= g.tokens || n0 >= n_out) continue;
+                if constexpr (!DUAL && !GROUP) {
+                    if (s > 0) load_res(s);
+                }
+                const size_t o = (size_t)tok * n_out + n0;
+                const uint32_t valid = min(32u, n_out - n0);
+                float v[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) { // quant/nvfp4.rs:334-336: tensor scales applied one after the other
+                    v[i] = __fmul_rn(__fmul_rn(__uint_as_float(r[s][i]), scale2), g.inv_input_scale);
+                    if constexpr (DUAL) {
+                        const float gate = __half2float(__float2half_rn(v[i]));
+                        const float up = __half2float(__float2half_rn(__fmul_rn(__fmul_rn(__uint_as_float(r[1][i]), g.scale2_up), g.inv_input_scale)));
+                        v[i] = __fdiv_rn(gate, 1.0f + expf(-gate)) * up; // silu_fast, quant/helpers.rs:72
                     }
-                    if (g.y_dtype == MUSER_DTYPE_F32)
-                        store_strip<float>(v, reinterpret_cast<float *>(y_out) + o,
-                                           g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
-                    else if (g.y_dtype == MUSER_DTYPE_BF16)
-                        store_strip<__nv_bfloat16>(v, reinterpret_cast<__nv_bfloat16 *>(y_out) + o,
-                                                   g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
-                    else
-                        store_strip<__half>(v, reinterpret_cast<__half *>(y_out) + o,
-                                            g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
+                    v[i] *= rs;
+                    if constexpr (TAIL) v[i] = logit_tail(v[i], g.out_scale, g.softcap);
+                }
+                if (g.y_dtype == MUSER_DTYPE_F32) {
+                    store_strip<float>(v, reinterpret_cast<float *>(y_out) + o,
+                                       g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
+                } else if (g.y_dtype == MUSER_DTYPE_BF16) {
+                    __nv_bfloat16 *y = reinterpret_cast<__nv_bfloat16 *>(y_out) + o;
+                    if (wide) {
+                        store_16_wide(v, y, wide_res ? res[0] : nullptr);
+                        store_16_wide(v + 16, y + 16, wide_res ? res[1] : nullptr);
+                    } else {
+                        store_strip<__nv_bfloat16>(v, y, g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
+                    }
+                } else {
+                    __half *y = reinterpret_cast<__half *>(y_out) + o;
+                    if (wide) {
+                        store_16_wide(v, y, wide_res ? res[0] : nullptr);
+                        store_16_wide(v + 16, y + 16, wide_res ? res[1] : nullptr);
+                    } else {
+                        store_strip<__half>(v, y, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
+                    }
                 }
             }
         }
@@ -1152,13 +1169,13 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     if (qout) {
         const void *qfn = reinterpret_cast<const void *>(nvfp4_gemm_kernel<true, false, true>);
         MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(qfn, ctx->device, kSmemBytes));
-        nvfp4_gemm_kernel<true, false, true><<<grid, 352, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
+        nvfp4_gemm_kernel<true, false, true><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
     } else if (w_up)
-        nvfp4_gemm_kernel<true, false><<<grid, 352, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g); // (the fused FFN form has no tail)
+        nvfp4_gemm_kernel<true, false><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g); // (the fused FFN form has no tail)
     else if (tail)
-        nvfp4_gemm_kernel<false, true><<<grid, 352, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
+        nvfp4_gemm_kernel<false, true><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
     else
-        nvfp4_gemm_kernel<false, false><<<grid, 352, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
+        nvfp4_gemm_kernel<false, false><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
     return MUSER_CUDA_OK;
 }
@@ -1205,7 +1222,7 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
     const void *kfn = reinterpret_cast<const void *>(nvfp4_gemm_kernel<false, false, false, true>);
     MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(kfn, ctx->device, kSmemBytes));
-    nvfp4_gemm_kernel<false, false, false, true><<<grid, 352, kSmemBytes, stream>>>(map_a, *maps[0], *maps[1], *maps[2], *maps[3], g);
+    nvfp4_gemm_kernel<false, false, false, true><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, *maps[0], *maps[1], *maps[2], *maps[3], g);
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
     return MUSER_CUDA_OK;
 }
