@@ -119,6 +119,13 @@ __device__ __forceinline__ uint4 ld_after_wait(const uint4 *p) {
     asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
+// The same from L2, past the SM's L1: for kernels that may have been launched while a kernel two back was still running
+// (its reads of the buffer's former contents could sit in L1).
+__device__ __forceinline__ uint4 ld_fresh(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ float ld_after_wait(const float *p) {
     float v;
     asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");

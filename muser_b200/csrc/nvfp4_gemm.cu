@@ -279,40 +279,57 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         {
             uint32_t it = 0, issued = 0; // k slabs issued so far, over all tiles
             bool ok = true; PROF_DECL
-            for (uint32_t tile = blockIdx.x; tile < n_tiles_total && ok; tile += gridDim.x) {
-                uint32_t tile_m, tile_n;
+            uint32_t tile_m, tile_n;
+            const uint8_t *sfa, *sfb0, *sfb1;
+            const CUtensorMap *mb;
+            auto locate = [&](uint32_t tile) {
                 tile_coords(tile, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
                 const uint8_t *b_scales = g.b_scales;
-                const CUtensorMap *mb = &map_b;
+                mb = &map_b;
                 if constexpr (GROUP) {
                     const uint32_t p = (tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3]);
                     tile_n -= g.grp_tile0[p];
                     b_scales = g.grp_b_scales[p];
                     mb = p == 0 ? &map_b : p == 1 ? &map_b2 : p == 2 ? &map_b3 : &map_b4;
                 }
-                const uint8_t *sfa = g.a_scales + (size_t)tile_m * g.kt64 * 512;
-                const uint8_t *sfb0 = b_scales + (size_t)(DUAL ? tile_n : 2 * tile_n) * g.kt64 * 512;
-                const uint8_t *sfb1 = DUAL ? g.b2_scales + (size_t)tile_n * g.kt64 * 512 : sfb0 + (size_t)g.kt64 * 512;
+                sfa = g.a_scales + (size_t)tile_m * g.kt64 * 512;
+                sfb0 = b_scales + (size_t)(DUAL ? tile_n : 2 * tile_n) * g.kt64 * 512;
+                sfb1 = DUAL ? g.b2_scales + (size_t)tile_n * g.kt64 * 512 : sfb0 + (size_t)g.kt64 * 512;
+            };
+            // the last slab may hold fewer than four 64-value blocks: the operand boxes are zero-filled past the row
+            // end, and only the scale chunks that exist are fetched
+            auto sf_bytes = [&](uint32_t kt) { return min(4u, g.kt64 - 4 * kt) * 512; };
+            auto load_weights = [&](uint32_t kt, uint32_t s) {
+                const uint32_t st = base + s * kStageBytes, full = bar_full + 8 * s;
+                mbar_expect_tx_elect(full, kABytes + kBBytes + 3 * sf_bytes(kt));
+                if constexpr (DUAL) {
+                    tma_load_2d_elect(st + kABytes, &map_b, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
+                    tma_load_2d_elect(st + kABytes + kBBytes / 2, &map_b2, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
+                } else {
+                    tma_load_2d_elect(st + kABytes, mb, (int)(kt * (BK / 2)), (int)(tile_n * BN), full);
+                }
+                bulk_load_elect(st + kABytes + kBBytes + kSfaBytes, sfb0 + (size_t)kt * 2048, sf_bytes(kt), full);
+                bulk_load_elect(st + kABytes + kBBytes + kSfaBytes + 2048, sfb1 + (size_t)kt * 2048, sf_bytes(kt), full);
+            };
+            auto load_activations = [&](uint32_t kt, uint32_t s) {
+                const uint32_t st = base + s * kStageBytes, full = bar_full + 8 * s;
+                tma_load_2d_elect(st, &map_a, (int)(kt * (BK / 2)), (int)(tile_m * BM), full);
+                bulk_load_elect(st + kABytes + kBBytes, sfa + (size_t)kt * kSfaBytes, sf_bytes(kt), full);
+            };
+            // weights are constants: the first stages' are on their way before the kernel that makes the activations is done
+            locate(blockIdx.x);
+            const uint32_t ahead = min((uint32_t)kStages, g.k_tiles);
+            for (uint32_t kt = 0; kt < ahead; ++kt) load_weights(kt, kt);
+            pdl_wait();
+            pdl_release(); // (behind the wait: what starts early starts when the kernel before this one is complete)
+            for (uint32_t tile = blockIdx.x; tile < n_tiles_total && ok; tile += gridDim.x) {
+                locate(tile);
                 for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
                     const uint32_t s = it % kStages, round = it / kStages;
                     PROF_BEGIN if (round > 0) ok = mbar_wait_warp(bar_empty + 8 * s, (round - 1) & 1, abort_flag); PROF_END(0)
                     if (!ok) break;
-                    const uint32_t st = base + s * kStageBytes;
-                    const uint32_t full = bar_full + 8 * s;
-                    // the last slab may hold fewer than four 64-value blocks: the operand boxes are zero-filled
-                    // past the row end, and only the scale chunks that exist are fetched
-                    const uint32_t nkb = min(4u, g.kt64 - 4 * kt), sf_bytes = nkb * 512;
-                    mbar_expect_tx_elect(full, kABytes + kBBytes + 3 * sf_bytes);
-                    tma_load_2d_elect(st, &map_a, (int)(kt * (BK / 2)), (int)(tile_m * BM), full);
-                    if constexpr (DUAL) {
-                        tma_load_2d_elect(st + kABytes, &map_b, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
-                        tma_load_2d_elect(st + kABytes + kBBytes / 2, &map_b2, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
-                    } else {
-                        tma_load_2d_elect(st + kABytes, mb, (int)(kt * (BK / 2)), (int)(tile_n * BN), full);
-                    }
-                    bulk_load_elect(st + kABytes + kBBytes, sfa + (size_t)kt * kSfaBytes, sf_bytes, full);
-                    bulk_load_elect(st + kABytes + kBBytes + kSfaBytes, sfb0 + (size_t)kt * 2048, sf_bytes, full);
-                    bulk_load_elect(st + kABytes + kBBytes + kSfaBytes + 2048, sfb1 + (size_t)kt * 2048, sf_bytes, full);
+                    if (it >= ahead) load_weights(kt, s);
+                    load_activations(kt, s);
                     issued = it + 1;
                 }
             }
@@ -388,6 +405,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const uint32_t part = (uint32_t)(warp - 2) >> 2; // which quarter of the output columns
         constexpr uint32_t kOutCols = DUAL ? BN / 2 : BN, kPartCols = kOutCols / 4, kStrips = kPartCols / 32;
         uint32_t local = 0;
+        pdl_wait(); // the residual and row scales come from, and the outputs may still be read by, earlier kernels
         for (uint32_t tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++local) {
             uint32_t tile_m, tile_n;
             tile_coords(tile, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
@@ -415,7 +433,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 load_res(0);
                 if (wide_res) asm volatile("prefetch.global.L2 [%0];" ::"l"(res_at + 64));
             }
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_full, local & 1, abort_flag));
+            // (with a sleep between the polls: sixteen polling warps cost the SM power that the products could use)
+            const bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64));
             if (!ok) {
                 if (lane == 0) {
                     *abort_flag = 1;
@@ -1169,13 +1188,13 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     if (qout) {
         const void *qfn = reinterpret_cast<const void *>(nvfp4_gemm_kernel<true, false, true>);
         MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(qfn, ctx->device, kSmemBytes));
-        nvfp4_gemm_kernel<true, false, true><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<true, false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g));
     } else if (w_up)
-        nvfp4_gemm_kernel<true, false><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g); // (the fused FFN form has no tail)
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<true, false>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g)); // (the fused FFN form has no tail)
     else if (tail)
-        nvfp4_gemm_kernel<false, true><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g));
     else
-        nvfp4_gemm_kernel<false, false><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, mb, mb2, mb, mb, g);
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, false>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g));
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
     return MUSER_CUDA_OK;
 }
@@ -1222,7 +1241,7 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
     const void *kfn = reinterpret_cast<const void *>(nvfp4_gemm_kernel<false, false, false, true>);
     MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(kfn, ctx->device, kSmemBytes));
-    nvfp4_gemm_kernel<false, false, false, true><<<grid, kGemmThreads, kSmemBytes, stream>>>(map_a, *maps[0], *maps[1], *maps[2], *maps[3], g);
+    MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, false, false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, *maps[0], *maps[1], *maps[2], *maps[3], g));
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
     return MUSER_CUDA_OK;
 }

@@ -29,36 +29,23 @@ __device__ __forceinline__ void store_scale_quad(uint32_t scale_code, uint32_t r
 // One thread per 16-value group; the four threads of a 64-value span merge their scale bytes into one
 // aligned 32-bit store.  Rows tokens..tokens_pad-1 only clear their scale slots.
 template <bool XF32>
-__global__ void nvfp4_quantize_kernel(const void *__restrict__ x, uint32_t tokens, uint32_t tokens_pad, uint32_t n_in,
-                                      uint32_t kt, float isi, uint8_t *__restrict__ packed,
-                                      uint8_t *__restrict__ scales) {
+__global__ void nvfp4_quantize_kernel(const void *x, uint32_t tokens, uint32_t tokens_pad, uint32_t n_in, uint32_t kt, float isi, uint8_t *packed,
+                                      uint8_t *scales) {
+    pdl_wait();
+    pdl_release();
     const uint32_t groups_pad = kt * 4; // group slots per row in the swizzled plane
     const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (idx >= (uint64_t)tokens_pad * groups_pad) return; // groups_pad % 4 == 0: quads never straddle the edge
     const uint32_t row = (uint32_t)(idx / groups_pad), grp = (uint32_t)(idx % groups_pad);
     uint32_t scale_code = 0;
     if (row < tokens && grp * 16 < n_in) {
+        const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
+                              : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
         float r[16];
-        if constexpr (XF32) {
-            const float4 *p = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(x) + (size_t)row * n_in + grp * 16);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 v = __ldg(p + i);
-                r[4 * i] = v.x, r[4 * i + 1] = v.y, r[4 * i + 2] = v.z, r[4 * i + 3] = v.w;
-            }
-        } else {
-            const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in + grp * 16);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const uint4 v = __ldg(p + i);
-                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    r[8 * i + 2 * j] = __uint_as_float(w[j] << 16);
-                    r[8 * i + 2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
-                }
-            }
-        }
+        float(&lo)[8] = *reinterpret_cast<float(*)[8]>(&r[0]);
+        float(&hi)[8] = *reinterpret_cast<float(*)[8]>(&r[8]);
+        load8<XF32>(xr, 2 * grp, lo);
+        load8<XF32>(xr, 2 * grp + 1, hi);
         scale_code = quantize_group(r, isi, packed + (size_t)row * (n_in / 2) + grp * 8);
     }
     store_scale_quad(scale_code, row, grp, kt, scales);
@@ -72,8 +59,9 @@ __global__ void nvfp4_quantize_kernel(const void *__restrict__ x, uint32_t token
 // rows at a time through shared memory (asynchronous copies, two buffers), so that global loads stay coalesced
 // (consecutive threads read consecutive 16 bytes of one row) while the sums stay sequential.
 template <bool XF32>
-__global__ void __launch_bounds__(32) rms_rows_sequential_kernel(const void *__restrict__ x, uint32_t tokens, uint32_t n_in, float eps,
-                                                                 float *__restrict__ inv_rms) {
+__global__ void __launch_bounds__(32) rms_rows_sequential_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms) {
+    pdl_wait();
+    pdl_release();
     constexpr int kRows = 32, kChunk = 256;                       // rows per block (one warp), inputs per row and step
     constexpr int kParts = kChunk * (XF32 ? 4 : 2) / 16;          // 16-byte pieces per row and step
     constexpr int kStride = kParts + 1;                           // row stride in pieces: conflict-free 16-byte reads down a column
@@ -139,22 +127,14 @@ static cudaError_t launch_rms_rows_sequential(Ctx *ctx, const void *x, uint32_t 
     const void *fn = f32 ? reinterpret_cast<const void *>(rms_rows_sequential_kernel<true>) : reinterpret_cast<const void *>(rms_rows_sequential_kernel<false>);
     const cudaError_t e = ensure_dynamic_smem(fn, ctx->device, smem);
     if (e != cudaSuccess) return e;
-    if (f32) rms_rows_sequential_kernel<true><<<blocks, 32, smem, stream>>>(x, tokens, n_in, eps, inv_rms);
-    else rms_rows_sequential_kernel<false><<<blocks, 32, smem, stream>>>(x, tokens, n_in, eps, inv_rms);
-    return cudaGetLastError();
+    return launch_pdl(f32 ? rms_rows_sequential_kernel<true> : rms_rows_sequential_kernel<false>, dim3(blocks), dim3(32), smem, stream, x, tokens, n_in, eps, inv_rms);
 }
 
-// The same quantizer behind a fused input RMSNorm (reference.rs:73-80): one block per token row quantizes
-// (x * inv_rms) * w group by group, inv_rms from the pass above.  Blocks of the padding rows only clear scales.
+// (x * inv_rms) * w of one row, quantized group by group by the whole block; rows past `tokens` only clear their scales.
 template <bool XF32>
-__global__ void __launch_bounds__(256) nvfp4_norm_quantize_kernel(const void *__restrict__ x, uint32_t tokens, uint32_t n_in,
-                                                                  uint32_t kt, float isi, const float *__restrict__ norm_w,
-                                                                  const float *__restrict__ inv_rms, uint8_t *__restrict__ packed,
-                                                                  uint8_t *__restrict__ scales) {
-    const uint32_t row = blockIdx.x, groups_pad = kt * 4;
-    const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
-                          : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
-    const float inv = row < tokens ? inv_rms[row] : 0.0f;
+__device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
+                                                  const float *__restrict__ norm_w, float inv, uint8_t *packed, uint8_t *scales) {
+    const uint32_t groups_pad = kt * 4;
     for (uint32_t g0 = 0; g0 < groups_pad; g0 += blockDim.x) { // blockDim % 4 == 0: quads stay together
         const uint32_t grp = g0 + threadIdx.x;
         uint32_t scale_code = 0;
@@ -177,6 +157,140 @@ __global__ void __launch_bounds__(256) nvfp4_norm_quantize_kernel(const void *__
         store_scale_quad(scale_code, row, grp, kt, scales, grp < groups_pad);
     }
 }
+
+// The same quantizer behind a fused input RMSNorm (reference.rs:59-80): one block per token row adds the row's squares as
+// rms_norm does, FRONT TO BACK in f32 with one rounding per step (why that order: rms_rows_sequential_kernel), and
+// quantizes (x * inv_rms) * w group by group.
+//
+// A chain of n dependent additions takes 4 cycles each at best.  It is cut into 128 segments, one per thread.  While the
+// running sum S stays inside one binade, adding s moves S up by a whole number of units u of its last place:
+// s / u rounded to nearest, where a tie goes by the parity of S / u.  So a segment acts on S's bit pattern as "add c0 if S is
+// even, c1 if odd", which its thread can work out without S, given the binade.  The binade is guessed from a parallel
+// prefix sum; then one warp walks the 128 segments, checks for each that S was in the guessed binade before and is
+// after (else it adds that segment's squares one by one: about one segment per power of two that the sum passes), and
+// ends with exactly the chain's sum.  Up to 500 rows of 5120 values: 31 us for the chain kernel and 3 to 5 for a quantizer
+// behind it -> about 12 (a layer at 16 tokens 202 -> 145 us, together with the launches that follow one another closer).
+constexpr int kNormThreads = 128;
+template <bool XF32>
+__global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
+                                                                           const float *__restrict__ norm_w, float eps, uint32_t keep, uint8_t *packed,
+                                                                           uint8_t *scales) {
+    extern __shared__ float4 norm_squares[]; // n_in squares, if they fit
+    __shared__ float warp_sum[kNormThreads / 32];
+    __shared__ uint2 seg_add[kNormThreads];
+    __shared__ uint32_t seg_binade[kNormThreads]; // exponent field the additions hold for, 0: one by one
+    __shared__ float inv_rms;
+    pdl_wait();
+    pdl_release();
+    const uint32_t row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
+                          : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
+    float inv = 0.0f;
+    if (row < tokens) { // (uniform over the block)
+        const uint32_t len8 = (n_in / 8 + kNormThreads - 1) / kNormThreads; // eights per segment
+        const uint32_t first8 = min(tid * len8, n_in / 8), end8 = min(first8 + len8, n_in / 8);
+        float sum = 0.0f;
+        for (uint32_t i = first8; i < end8; ++i) {
+            float v[8];
+            load8<XF32>(xr, i, v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(v[k], v[k]), sum += v[k];
+            if (keep) {
+                norm_squares[2 * i] = make_float4(v[0], v[1], v[2], v[3]);
+                norm_squares[2 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        }
+        auto squares = [&](uint32_t i, float (&v)[8]) {
+            if (keep) {
+                const float4 p = norm_squares[2 * i], q = norm_squares[2 * i + 1];
+                v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = p.w, v[4] = q.x, v[5] = q.y, v[6] = q.z, v[7] = q.w;
+            } else {
+                load8<XF32>(xr, i, v);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(v[k], v[k]);
+            }
+        };
+        float before = sum; // sum of the segments up to and including this one, then without it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float up = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= (uint32_t)o) before += up;
+        }
+        if (lane == 31) warp_sum[tid >> 5] = before;
+        __syncthreads();
+        float carry = 0.0f;
+        for (uint32_t w = 0; w < (tid >> 5); ++w) carry += warp_sum[w];
+        const float after = carry + before;
+        before = __shfl_up_sync(0xffffffffu, before, 1);
+        before = lane ? carry + before : carry;
+        const uint32_t binade = __float_as_uint(before) >> 23; // (sums of squares: no sign; infinities and NaN are 255)
+        uint32_t add0 = 0, add1 = 1; // additions to an even and, counted from 1, to an odd pattern
+        const bool guess = binade == (__float_as_uint(after) >> 23) && binade >= 24 && binade < 255;
+        if (guess) {
+            const float per_unit = __uint_as_float((277 - binade) << 23); // 1 / u = 2^(150 - binade)
+            for (uint32_t i = first8; i < end8; ++i) {
+                float v[8];
+                squares(i, v);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float units = v[k] * per_unit, whole = floorf(units), rest = units - whole; // all exact
+                    const uint32_t q = (uint32_t)whole, up = rest > 0.5f, tie = rest == 0.5f;
+                    add0 += q, add1 += q;
+                    add0 += up | (tie & add0), add1 += up | (tie & add1); // (bit 0 of tie & add: odd)
+                }
+            }
+        }
+        seg_add[tid] = make_uint2(add0, add1 - 1);
+        seg_binade[tid] = guess ? binade : 0;
+        __syncthreads();
+        if (tid < 32) {
+            uint32_t s = 0; // the running sum's bit pattern, the same in every lane
+            for (uint32_t base = 0; base < kNormThreads; base += 32) {
+                const uint2 my_add = seg_add[base + lane];
+                const uint32_t my_binade = seg_binade[base + lane];
+#pragma unroll 8
+                for (uint32_t j = 0; j < 32; ++j) {
+                    const uint32_t a0 = __shfl_sync(0xffffffffu, my_add.x, j), a1 = __shfl_sync(0xffffffffu, my_add.y, j);
+                    const uint32_t e = __shfl_sync(0xffffffffu, my_binade, j);
+                    const uint32_t next = s + ((s & 1) ? a1 : a0);
+                    if (e && (s >> 23) == e && (next >> 23) == e) {
+                        s = next;
+                    } else {
+                        const uint32_t f = min((base + j) * len8, n_in / 8), l = min(f + len8, n_in / 8);
+                        float t = __uint_as_float(s);
+                        for (uint32_t i = f; i < l; ++i) {
+                            float v[8];
+                            squares(i, v);
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) t = __fadd_rn(t, v[k]);
+                        }
+                        s = __float_as_uint(t);
+                    }
+                }
+            }
+            if (lane == 0) inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(__uint_as_float(s), (float)n_in), eps)));
+        }
+        __syncthreads();
+        inv = inv_rms;
+    }
+    norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, inv, packed, scales);
+}
+
+// The same behind rms_rows_sequential_kernel, whose 32 chains a warp do less work per row than the segments above and
+// take 30 us however few the rows: the better form from about 1500 rows of 5120 (20.5 ns a row for the kernel above,
+// 7.6 for these two; 2048 rows 50 us either way).
+template <bool XF32>
+__global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
+                                                                    const float *__restrict__ norm_w, const float *inv_rms, uint8_t *packed,
+                                                                    uint8_t *scales) {
+    pdl_wait();
+    pdl_release();
+    const uint32_t row = blockIdx.x;
+    const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
+                          : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
+    norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
+}
+constexpr uint32_t kNormSegmentRows = 1536; // up to here the segmented kernel
 
 // Plain rows: out[t][k] = (x[t][k] * inv_rms_t) * w[k] in f32, for the kernels that read their activations as they go.
 template <bool XF32>
@@ -220,21 +334,25 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
     if (norm_weight) {
         float *inv = ctx->inv_rms;
         if (!inv || tokens > ctx->inv_rms_rows) return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: more rows than the context's per-row scratch holds");
-        MUSER_CUDA_TRY(ctx, launch_rms_rows_sequential(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
-        if (x_dtype == MUSER_DTYPE_F32)
-            nvfp4_norm_quantize_kernel<true><<<tokens_pad, 256, 0, stream>>>(x, tokens, (uint32_t)n_in, kt, isi, norm_weight, inv, packed, scales);
-        else
-            nvfp4_norm_quantize_kernel<false><<<tokens_pad, 256, 0, stream>>>(x, tokens, (uint32_t)n_in, kt, isi, norm_weight, inv, packed, scales);
-        MUSER_CUDA_TRY(ctx, cudaGetLastError());
+        if (tokens > kNormSegmentRows) {
+            MUSER_CUDA_TRY(ctx, launch_rms_rows_sequential(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
+            const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
+            MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(256), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, (const float *)inv,
+                                           packed, scales));
+            return MUSER_CUDA_OK;
+        }
+        const bool keep = n_in <= 12288; // rows of up to 48 KB of squares stay in shared memory, longer ones are read again
+        const size_t smem = keep ? (size_t)n_in * sizeof(float) : 0;
+        const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_norm_quantize_kernel<true> : nvfp4_norm_quantize_kernel<false>;
+        MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, smem));
+        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(kNormThreads), smem, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps,
+                                       (uint32_t)keep, packed, scales));
         return MUSER_CUDA_OK;
     }
     const uint64_t total = (uint64_t)tokens_pad * kt * 4;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (x_dtype == MUSER_DTYPE_F32)
-        nvfp4_quantize_kernel<true><<<blocks, 256, 0, stream>>>(x, tokens, tokens_pad, (uint32_t)n_in, kt, isi, packed, scales);
-    else
-        nvfp4_quantize_kernel<false><<<blocks, 256, 0, stream>>>(x, tokens, tokens_pad, (uint32_t)n_in, kt, isi, packed, scales);
-    MUSER_CUDA_TRY(ctx, cudaGetLastError());
+    const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_quantize_kernel<true> : nvfp4_quantize_kernel<false>;
+    MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(blocks), dim3(256), 0, stream, x, tokens, tokens_pad, (uint32_t)n_in, kt, isi, packed, scales));
     return MUSER_CUDA_OK;
 }
 

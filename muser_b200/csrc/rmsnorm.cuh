@@ -7,15 +7,17 @@
 
 namespace muser {
 
-// Eight consecutive activations of one row as f32 (the row starts 16-byte aligned and i8 counts groups of eight).
+// Eight consecutive activations of one row (which an earlier kernel may just have written) as f32 (the row starts 16-byte aligned and i8 counts groups of eight).
 template <bool XF32>
 __device__ __forceinline__ void load8(const void *row, uint32_t i8, float (&v)[8]) {
     if constexpr (XF32) {
-        const float4 *p = reinterpret_cast<const float4 *>(row) + 2 * (size_t)i8;
-        const float4 a = __ldg(p), b = __ldg(p + 1);
-        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        const uint4 *p = reinterpret_cast<const uint4 *>(row) + 2 * (size_t)i8;
+        const uint4 a = ld_fresh(p), b = ld_fresh(p + 1);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
     } else {
-        const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(row) + i8);
+        const uint4 raw = ld_fresh(reinterpret_cast<const uint4 *>(row) + i8);
         const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

@@ -291,6 +291,36 @@ def test_fused_input_rmsnorm(gpu, x_dtype):
     assert H.rel_l2(y.cpu().numpy(), O.silu_mul(gate, upv)) <= 2 * REL_L2_TOL  # f16 boundaries of both factors can flip
 
 
+@pytest.mark.parametrize("n_in", [64, 1088, 5120, 12352])
+@pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
+def test_fused_norm_adds_the_squares_front_to_back(gpu, n_in, x_dtype):
+    """The sum of squares is the reference's chain of additions to the last bit whatever the row looks like, so codes
+    and scales are the CPU lane's bytes: rows whose sums tie at every step, cross many binades, shrink, are zero, hold
+    one huge or one infinite value; lengths with empty and short segments, and rows too long to keep."""
+    op, ctx, k = gpu
+    g = torch.Generator().manual_seed(n_in)
+    x = torch.randn((11, n_in), generator=g)
+    x[1] = 1.0                                             # sums that are whole numbers: no rounding, then
+    x[2] = 1.0 + torch.arange(n_in).remainder(3) * 0.0078125  # ties as the sum's last place grows past the squares' bits
+    x[3] = torch.exp2(torch.linspace(-40, 20, n_in)).float()  # a binade every few values
+    x[4] = x[3].flip(0)
+    x[5] = 0.0
+    x[6, 3:] = 0.0
+    x[7] *= 1e-18                                          # squares in f32's subnormal range
+    x[8, n_in // 2] = 1e15
+    x[9, n_in // 3] = float("inf")
+    x = x.to(x_dtype)
+    nw = 1.0 + 0.1 * torch.randn(n_in, generator=g)
+    isi, eps = 41.5, 1e-6
+    xn = O.rms_norm_mul(x.float().numpy(), eps, nw.numpy())
+    want_p, want_s = O.quantize_nvfp4_activation(xn, isi)
+    got_p, got_s = k.quantize_nvfp4_activation(x.cuda(), isi, norm_weight=nw.cuda(), norm_eps=eps)
+    ctx.sync_status()
+    rows = [r for r in range(11) if r != 9]  # (an infinite row normalizes to zeros and a NaN, whose sign no reference defines)
+    assert np.array_equal(got_p.cpu().numpy()[rows], want_p[rows])
+    assert np.array_equal(op.unswizzle_scales(got_s, 11, n_in).cpu().numpy(), want_s)
+
+
 def test_nvfp4_tensor_parallel_shards(gpu):
     op, ctx, k = gpu
     from muser_b200 import synth
