@@ -235,7 +235,7 @@ muser_cuda_status muser_cuda_ctx_create(int device, size_t workspace_bytes, muse
     if (e == cudaSuccess) e = cudaMalloc(&ctx->gemv_partial, ctx->gemv_partial_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->gemv_counters, ctx->gemv_counter_slots * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMemset(ctx->gemv_counters, 0, ctx->gemv_counter_slots * sizeof(unsigned int));
-    ctx->tc_scratch_bytes = (size_t)64 * 32768 * 2 + (size_t)64 * 2048 * 2 + 4096; // f16 rows + sub-block sums, 64 tokens
+    ctx->tc_scratch_bytes = (size_t)64 * 32768 * 4 + (size_t)128 * 64 * 36; // prepared activations of the batched K-quant kernels: 64 tokens, f16 head + remainder, sums, scales
     if (e == cudaSuccess) e = cudaMalloc(&ctx->tc_scratch, ctx->tc_scratch_bytes);
     ctx->norm_scratch_bytes = (size_t)64 * 32768 * sizeof(float); // 64 tokens x the widest row
     if (e == cudaSuccess) e = cudaMalloc(&ctx->norm_scratch, ctx->norm_scratch_bytes);
@@ -435,7 +435,7 @@ muser_cuda_status muser_cuda_quantized_matmul_group(muser_cuda_ctx *c, const mus
             return fail(ctx, MUSER_CUDA_BAD_ARG, "the projections of a group share one input, so they must share the fused input norm");
     }
     MUSER_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    const cudaError_t de = launch_kquant_decode(ctx, w, nullptr, n_items, x, x_dtype, y, yd, tokens, e, (cudaStream_t)stream);
+    const cudaError_t de = launch_kquant_group(ctx, w, n_items, x, x_dtype, y, yd, tokens, e, (cudaStream_t)stream);
     if (de != cudaErrorNotSupported) {
         MUSER_CUDA_TRY(ctx, de);
         return MUSER_CUDA_OK;

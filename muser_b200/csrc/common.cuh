@@ -206,6 +206,10 @@ muser_cuda_status launch_kquant_matmul(Ctx *, const Weight *w, const Weight *w_u
                                        cudaStream_t);
 cudaError_t launch_kquant_tc(Ctx *, const Weight *w, const void *x, uint32_t x_dtype, void *y, uint32_t y_dtype,
                              uint32_t tokens, const Epilogue &, cudaStream_t);
+cudaError_t launch_kquant_group(Ctx *, const Weight *const *w, uint32_t n_jobs, const void *x, uint32_t x_dtype, void *const *y, const uint32_t *y_dtype,
+                                uint32_t tokens, const Epilogue *ep, cudaStream_t);
+cudaError_t launch_kquant_mma(Ctx *, const Weight *const *w, const Weight *w_up, uint32_t n_jobs, const void *x, uint32_t x_dtype, void *const *y,
+                              const uint32_t *y_dtype, uint32_t tokens, const Epilogue *ep, bool clamp, cudaStream_t);
 muser_cuda_status decode_autotune(Ctx *, const Weight *const *w, const Weight *w_up, uint32_t n_jobs, uint32_t max_tokens, cudaStream_t);
 cudaError_t launch_kquant_decode(Ctx *, const Weight *const *w, const Weight *w_up, uint32_t n_jobs, const void *x,
                                  uint32_t x_dtype, void *const *y, const uint32_t *y_dtype, uint32_t tokens,

@@ -1214,21 +1214,58 @@ muser_cuda_status decode_autotune(Ctx *ctx, const Weight *const *w, const Weight
 }
 
 // ------------------------------------------------------------------------------------ dispatch
-// Which kernel serves a K-quant call (bf16 or f32 activations alike): up to 16 tokens the decode kernel above; from
-// 17 tokens the tcgen05 kernel (kquant_tc.cu) when the weight has enough 128-row blocks to fill the GPU and the token
-// count fits its columns (64, or 32 for f32 activations, which travel as f16 head + remainder pairs); everything else
-// in chunks of 16 tokens through the decode kernel.  The thresholds can be moved through muser_cuda_tuning_set.
+// Which kernel serves a K-quant call (1 to 64 tokens).  Up to 12 tokens the decode kernel above; from 13 one of the two
+// batched kernels.  Of the batched kernels the one on the warp-level instructions (kquant_mma.cu) has the
+// smaller fixed part and pads token columns to 8, the tcgen05 one (kquant_tc.cu, to 16, 32 or 64; Q4_K and Q6_K) the
+// cheaper column: see takes_tcgen05.  At 13 to 16 tokens the decode kernel's integer products are bound by their scale
+// arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 40, 5120 x 27648 Q6_K 68 -> 43, 5120 x 5120 21 -> 15,
+// 1024 x 5120 18.5 -> 12); at 9 to 12 the two are even (40 / 40, 55 / 43, 17 / 15, but 8192 x 5120 17 / 20), below it wins.
+// The decode kernel also keeps
+//   - K shards up to 16 tokens, whose partial sums must carry the same bits with and without the all-reduce fused in,
+//   - calls under a forced launch plan (MUSER_TUNE_DECODE_*), and shapes the batched kernels refuse.
+static bool takes_mma(const Ctx *ctx, const Weight *w, uint32_t tokens) {
+    if (tokens < 13 || ctx->dec_warps || ctx->dec_ksplit || ctx->dec_ring || ctx->dec_wsplit) return false;
+    return tokens > 16 || w->shard.axis != MUSER_SHARD_K || w->shard.world <= 1;
+}
+
+// The tcgen05 kernel for large Q4_K weights at token counts that fill its columns (us, tcgen05 / warp-level: 27648 x 5120
+// 44 / 46 at 32 tokens, 61 / 70 at 64, 55 / 61 at 32 in f32, which take two columns each; 61 / 56 at 48; 13824 x 5120 37 / 40
+// at 64; 8192 x 5120 22 / 22 and 33 / 31; 5120 x 5120 19 / 17 and 29 / 23).  Q6_K: 63 / 52 at 32 and 78 / 76 at 64 for
+// 5120 x 27648.  A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves.
+static bool takes_tcgen05(const Weight *w, uint32_t tokens, bool two_columns, uint32_t tc_from) {
+    if (tc_from < 17) return true;
+    const uint32_t cols = two_columns ? 2 * tokens : tokens;
+    return w->dtype == MUSER_DTYPE_Q4_K && (uint64_t)w->row_tiles * w->nsb > 12000 && (cols <= 32 || cols > 48);
+}
+
+// Up to four projections of one input (or a fused gate/up pair), 1..64 tokens.
+static cudaError_t launch_kquant_batch(Ctx *ctx, const Weight *const *w, const Weight *w_up, uint32_t n_jobs, const void *x, uint32_t x_dtype,
+                                       void *const *y, const uint32_t *y_dtype, uint32_t tokens, const Epilogue *ep, bool clamp, cudaStream_t stream) {
+    if (takes_mma(ctx, w[0], tokens)) {
+        const cudaError_t e = launch_kquant_mma(ctx, w, w_up, n_jobs, x, x_dtype, y, y_dtype, tokens, ep, clamp, stream);
+        if (e != cudaErrorNotSupported) return e;
+    }
+    if (tokens <= 16) return launch_kquant_decode(ctx, w, w_up, n_jobs, x, x_dtype, y, y_dtype, tokens, ep, stream);
+    return cudaErrorNotSupported;
+}
+
+cudaError_t launch_kquant_group(Ctx *ctx, const Weight *const *w, uint32_t n_jobs, const void *x, uint32_t x_dtype, void *const *y, const uint32_t *y_dtype,
+                                uint32_t tokens, const Epilogue *ep, cudaStream_t stream) {
+    return launch_kquant_batch(ctx, w, nullptr, n_jobs, x, x_dtype, y, y_dtype, tokens, ep, false, stream);
+}
+
 muser_cuda_status launch_kquant_matmul(Ctx *ctx, const Weight *w, const Weight *w_up, const void *x, uint32_t x_dtype,
                                        void *y, uint32_t y_dtype, uint32_t tokens, const Epilogue &ep,
                                        cudaStream_t stream) {
     const bool q6 = w->dtype == MUSER_DTYPE_Q6_K, xf32 = x_dtype == MUSER_DTYPE_F32;
     const uint32_t tc_from = ctx->tc_min_tokens[q6 ? 1 : 0]; // above 64: switched off
+    // (the calls that take activations in f16's range, larger magnitudes clamped, whichever kernel serves them)
     const bool tc_fits = !w_up && w->dtype != MUSER_DTYPE_Q5_K && tokens >= tc_from && tokens <= (xf32 ? 32u : 64u) && w->n_out >= ctx->tc_min_rows;
-    if (tc_fits) {
+    if (tc_fits && takes_tcgen05(w, tokens, xf32 || ep.norm_weight, tc_from)) {
         const void *xin = x;
         uint32_t xin_dtype = x_dtype;
         if (ep.norm_weight) {
-            // the tensor-core kernel reads its activations through TMA, so the fused input norm runs as a pass of its
+            // the tcgen05 kernel reads its activations through TMA, so the fused input norm runs as a pass of its
             // own into the context's scratch rows (f32), which the projection then reads instead of x
             const size_t need = (size_t)tokens * w->n_in * sizeof(float);
             if (need > ctx->norm_scratch_bytes) return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: tokens x n_in exceeds the context's norm scratch");
@@ -1267,14 +1304,19 @@ muser_cuda_status launch_kquant_matmul(Ctx *ctx, const Weight *w, const Weight *
         return muser_cuda_all_reduce(reinterpret_cast<muser_cuda_ctx *>(ctx), y, count, y_dtype, stream);
     }
     const size_t xb = xf32 ? 4 : 2, yb = y_dtype == MUSER_DTYPE_BF16 ? 2 : 4;
-    for (uint32_t t0 = 0; t0 < tokens; t0 += 16) {
-        const uint32_t n = std::min(16u, tokens - t0);
+    uint32_t chunk = takes_mma(ctx, w, tokens) ? 64 : 16;
+    for (uint32_t t0 = 0, n; t0 < tokens; t0 += n) {
+        n = std::min(chunk, tokens - t0);
         Epilogue e = ep;
         if (e.row_scale) e.row_scale += t0;
         if (e.residual) e.residual = reinterpret_cast<const uint8_t *>(e.residual) + (size_t)t0 * w->n_out * yb;
         void *yc = reinterpret_cast<uint8_t *>(y) + (size_t)t0 * w->n_out * yb;
-        const cudaError_t de = launch_kquant_decode(ctx, &w, w_up, 1, reinterpret_cast<const uint8_t *>(x) + (size_t)t0 * w->n_in * xb,
-                                                    x_dtype, &yc, &y_dtype, n, &e, stream);
+        const cudaError_t de = launch_kquant_batch(ctx, &w, w_up, 1, reinterpret_cast<const uint8_t *>(x) + (size_t)t0 * w->n_in * xb,
+                                                   x_dtype, &yc, &y_dtype, n, &e, tc_fits, stream);
+        if (de == cudaErrorNotSupported && n > 16) { // a shape the batched kernel refuses: again, in the decode kernel's steps
+            chunk = 16, n = 0;
+            continue;
+        }
         if (de == cudaErrorNotSupported) return fail(ctx, MUSER_CUDA_BAD_SHAPE, "this shape does not fit the decode kernel");
         MUSER_CUDA_TRY(ctx, de);
     }

@@ -314,6 +314,35 @@ def test_every_launch_plan_of_the_decode_kernel(gpu, dtype):
         w.free()
 
 
+@pytest.mark.parametrize("dtype", [O.Q4_K, O.Q5_K, O.Q6_K])
+@pytest.mark.parametrize("tokens", [13, 16, 17, 24, 33, 48, 49, 64])
+def test_batched_kernel_at_its_edges(gpu, dtype, tokens):
+    """The batched kernel at the edges of its token groups, on row counts that end inside a tile, a quad and a CTA, on
+    few and many K tiles (one CTA and clusters), bf16 and f32 inputs, magnitudes far from one.  Its operands are exact
+    (f32 inputs to 22 bits) and its sums are f32 over at most 12 x 256 inputs: 2^-22 per addition at worst, some 1e-6 of
+    the result's norm; Q6_K beyond 16 tokens rounds operands to 11 bits, at most 2^-12 each."""
+    op, ctx, k = gpu
+    tol = 3e-4 if dtype == O.Q6_K and tokens > 16 else 3e-6
+    for n_in, n_out in ((256, 5), (1024, 203), (3072, 1030)):
+        raw = H.lcg_weights(dtype, n_out, n_in // 256, seed=n_out + tokens)
+        w = op.Weight(ctx, op.TensorView(raw, dtype, n_in, n_out))
+        deq = O.dequant_blocks(dtype, raw).reshape(n_out, n_in).astype(np.float64)
+        for x_dtype, scale in ((torch.bfloat16, 1.0), (torch.float32, 1.0), (torch.bfloat16, 2.0 ** -90), (torch.float32, 2.0 ** 12)):
+            x = (torch.from_numpy(H.lcg_activations(tokens * n_in, seed=tokens).reshape(tokens, n_in)) * scale).to(x_dtype)
+            y = torch.full((tokens, n_out), float("nan"), dtype=torch.float32, device="cuda")
+            k.encode_quantized_matmul(w, x.cuda(), y, tokens)
+            ctx.sync_status()
+            want = x.double().numpy() @ deq.T
+            assert H.rel_l2(y.cpu().numpy().astype(np.float64) / scale, want / scale) <= tol, (n_in, n_out, x_dtype, scale)
+        if tokens == 16:  # a NaN and an infinity poison their tokens and no other; a zero token stays zero
+            x = torch.from_numpy(H.lcg_activations(tokens * n_in, seed=1).reshape(tokens, n_in)).clone()
+            x[2, 7], x[5, 100], x[9] = float("nan"), float("inf"), 0.0
+            k.encode_quantized_matmul(w, x.cuda(), y, tokens)
+            got = y.cpu().numpy()
+            assert np.isnan(got[[2, 5]]).all() and (got[9] == 0).all() and np.isfinite(np.delete(got, [2, 5], 0)).all()
+        w.free()
+
+
 def test_grouped_projections_in_one_launch(gpu):
     """q | k | v of one hidden state in one launch (Q4_K, Q4_K and Q6_K rows of different counts), each with its own
     output dtype and epilogue, with and without the shared fused input norm: against the CPU lane and against the
