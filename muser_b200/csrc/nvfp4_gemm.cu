@@ -74,6 +74,8 @@ struct GemmArgs {
     float q_isi;        // the next projection's input_scale_inv
     uint32_t q_kt;      // n_out / 64
     uint32_t group_m;   // token tiles per raster group (tile_coords)
+    uint32_t a_bytes;   // of a stage's activation box: 128 bytes per token row
+    uint32_t ksplit;    // SPLIT form: CTAs of a cluster that share one tile's K
     // GROUP form: up to four projections of the same activations in one launch; weight-row tiles are numbered through
     // all of them (projection p owns tiles grp_tile0[p] .. grp_tile0[p + 1] - 1)
     uint32_t grp_tile0[5];
@@ -216,6 +218,24 @@ __device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T 
     }
 }
 
+// SPLIT form: f32 sums of a tile as [row][256 columns + padding] in shared memory.
+constexpr uint32_t kRedPitch = BN + 4;
+static_assert((uint32_t)BM * kRedPitch * 4 <= (uint32_t)(kStages * kStageBytes), "the slices' sums exceed the stage ring");
+__device__ __forceinline__ void split_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t split_map(uint32_t cta_addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float4 split_load(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
 // Persistent: CTA b takes output tiles b, b + gridDim.x, ...; tile index -> (n tile, m tile) with m fastest, so the
 // CTAs that run side by side share one weight tile (read from HBM once, from L2 afterwards).
 //
@@ -231,7 +251,9 @@ __device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T 
 // GROUP: several projections that read the same quantized activations (q | k | v) share one launch: their weight-row
 // tiles form one tile space, so the small ones fill the SMs that a launch of their own would leave idle.  Plain
 // outputs only (no fused tail, row scale or residual).
-template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false>
+// SPLIT: the slabs of one output tile are cut between the CTAs of a cluster (gemm_ksplit()): each leaves its f32 sums in
+// its shared memory, and all of them add the slices up in slice order, every CTA finishing a share of the tile's outputs.
+template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, bool SPLIT = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_b3,
@@ -249,6 +271,13 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t m_tiles = (g.tokens + BM - 1) / BM, n_tiles_total = g.n_tiles * m_tiles;
+    // This CTA's tiles and, of each, its slabs.  (Macros, so that the other forms compile as if SPLIT did not exist: with
+    // variables in their place the roles' lambdas kept them in registers and every form's slab took 10 % longer.)
+#define GEMM_SLICE (SPLIT ? blockIdx.x % g.ksplit : 0u)
+#define GEMM_TILE_FIRST (SPLIT ? blockIdx.x / g.ksplit : blockIdx.x)
+#define GEMM_TILE_STEP (SPLIT ? n_tiles_total : gridDim.x)
+#define GEMM_KT_FIRST (SPLIT ? g.k_tiles * GEMM_SLICE / g.ksplit : 0u)
+#define GEMM_KT_END (SPLIT ? g.k_tiles * (GEMM_SLICE + 1) / g.ksplit : g.k_tiles)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -301,7 +330,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             auto sf_bytes = [&](uint32_t kt) { return min(4u, g.kt64 - 4 * kt) * 512; };
             auto load_weights = [&](uint32_t kt, uint32_t s) {
                 const uint32_t st = base + s * kStageBytes, full = bar_full + 8 * s;
-                mbar_expect_tx_elect(full, kABytes + kBBytes + 3 * sf_bytes(kt));
+                mbar_expect_tx_elect(full, g.a_bytes + kBBytes + 3 * sf_bytes(kt));
                 if constexpr (DUAL) {
                     tma_load_2d_elect(st + kABytes, &map_b, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
                     tma_load_2d_elect(st + kABytes + kBBytes / 2, &map_b2, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
@@ -317,14 +346,14 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 bulk_load_elect(st + kABytes + kBBytes, sfa + (size_t)kt * kSfaBytes, sf_bytes(kt), full);
             };
             // weights are constants: the first stages' are on their way before the kernel that makes the activations is done
-            locate(blockIdx.x);
-            const uint32_t ahead = min((uint32_t)kStages, g.k_tiles);
-            for (uint32_t kt = 0; kt < ahead; ++kt) load_weights(kt, kt);
+            locate(GEMM_TILE_FIRST);
+            const uint32_t ahead = min((uint32_t)kStages, GEMM_KT_END - GEMM_KT_FIRST);
+            for (uint32_t i = 0; i < ahead; ++i) load_weights(GEMM_KT_FIRST + i, i);
             pdl_wait();
             pdl_release(); // (behind the wait: what starts early starts when the kernel before this one is complete)
-            for (uint32_t tile = blockIdx.x; tile < n_tiles_total && ok; tile += gridDim.x) {
+            for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total && ok; tile += GEMM_TILE_STEP) {
                 locate(tile);
-                for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
+                for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
                     const uint32_t s = it % kStages, round = it / kStages;
                     PROF_BEGIN if (round > 0) ok = mbar_wait_warp(bar_empty + 8 * s, (round - 1) & 1, abort_flag); PROF_END(0)
                     if (!ok) break;
@@ -356,14 +385,14 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
             uint32_t it = 0, local = 0;
             bool ok = true; PROF_DECL
-            for (uint32_t tile = blockIdx.x; tile < n_tiles_total && ok; tile += gridDim.x, ++local) {
+            for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total && ok; tile += GEMM_TILE_STEP, ++local) {
                 // the accumulator is free again once the epilogue warps have read the previous tile out of it
                 if (local > 0) {
                     PROF_BEGIN ok = mbar_wait_warp(bar_acc_empty, (local - 1) & 1, abort_flag); PROF_END(0)
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
-                for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
+                for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
                     const uint32_t s = it % kStages, round = it / kStages;
                     PROF_BEGIN ok = mbar_wait_warp(bar_full + 8 * s, round & 1, abort_flag); PROF_END(1)
                     if (!ok) break;
@@ -381,7 +410,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         tmem_cp_scales_elect(sf + 4 * kb, scale_desc(sfa + 512 * kb));
                         tmem_cp_scales_elect(sf + 16 + 8 * kb, scale_desc(sfb + 512 * kb));
                         tmem_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
-                        mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, (kt | kb) != 0);
+                        mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, ((kt - GEMM_KT_FIRST) | kb) != 0);
                     }
                     mma_commit_elect(bar_empty + 8 * s); // the stage may be overwritten once these MMAs have read it
                 }
@@ -406,7 +435,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         constexpr uint32_t kOutCols = DUAL ? BN / 2 : BN, kPartCols = kOutCols / 4, kStrips = kPartCols / 32;
         uint32_t local = 0;
         pdl_wait(); // the residual and row scales come from, and the outputs may still be read by, earlier kernels
-        for (uint32_t tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++local) {
+        for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total; tile += GEMM_TILE_STEP, ++local) {
             uint32_t tile_m, tile_n;
             tile_coords(tile, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
             uint32_t n_out = g.n_out; // (of this tile's projection)
@@ -457,6 +486,18 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
+            if constexpr (SPLIT) {
+                // (every stage has been consumed: the ring is scratch now)
+                if (tok < g.tokens) {
+                    float4 *row = reinterpret_cast<float4 *>(aligned + ((quad * 32 + lane) * kRedPitch + col0) * 4);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const uint32_t *v = &r[i >> 3][4 * (i & 7)];
+                        row[i] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
+                    }
+                }
+                continue;
+            }
             if constexpr (QOUT) {
                 // rows of the last 128-token block that hold no token get zero scale bytes: the next GEMM reads the
                 // block's whole scale chunk (their codes come from TMA's zero fill)
@@ -524,12 +565,55 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     }
+    if constexpr (SPLIT) {
+        split_barrier();
+        pdl_wait(); // (every warp stores here)
+        uint32_t tile_m, tile_n;
+        tile_coords(GEMM_TILE_FIRST, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
+        const uint32_t rows = min((uint32_t)BM, g.tokens - tile_m * BM);
+        // one 32-column strip of one row at a time
+        for (uint32_t e = GEMM_SLICE * blockDim.x + threadIdx.x; e < rows * (BN / 32); e += g.ksplit * blockDim.x) {
+            const uint32_t row = e / (BN / 32), c0 = (e % (BN / 32)) * 32, tok = tile_m * BM + row, n0 = tile_n * BN + c0;
+            if (n0 >= g.n_out) continue;
+            float v[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+            for (uint32_t p = 0; p < g.ksplit; ++p) {
+                const uint32_t at = split_map(base + (row * kRedPitch + c0) * 4, p);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float4 q = split_load(at + 16 * i);
+                    v[4 * i] += q.x, v[4 * i + 1] += q.y, v[4 * i + 2] += q.z, v[4 * i + 3] += q.w;
+                }
+            }
+            const float rs = g.row_scale ? g.row_scale[tok] : 1.0f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], g.scale2), g.inv_input_scale) * rs;
+            const size_t o = (size_t)tok * g.n_out + n0;
+            const uint32_t valid = min(32u, g.n_out - n0);
+            const bool vec_ok = (g.n_out & 7) == 0;
+            if (g.y_dtype == MUSER_DTYPE_F32)
+                store_strip<float>(v, reinterpret_cast<float *>(g.y) + o, g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
+            else if (g.y_dtype == MUSER_DTYPE_BF16)
+                store_strip<__nv_bfloat16>(v, reinterpret_cast<__nv_bfloat16 *>(g.y) + o,
+                                           g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
+            else
+                store_strip<__half>(v, reinterpret_cast<__half *>(g.y) + o, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
+        }
+        split_barrier(); // no CTA leaves while another may read its sums
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
 }
+
+#undef GEMM_SLICE
+#undef GEMM_TILE_FIRST
+#undef GEMM_TILE_STEP
+#undef GEMM_KT_FIRST
+#undef GEMM_KT_END
 
 // ------------------------------------------------------------------------------------------ paired CTAs
 // The same GEMM on pairs of SMs (tcgen05 cta_group::2): a cluster of two CTAs owns a 256-token x 256-row output tile,
@@ -1095,11 +1179,49 @@ void nvfp4_free_tensor_map(Weight *w) {
     w->tmap_half = nullptr;
 }
 
+// Token rows of an activation box.  A single token tile that is not full fetches whole 8-row swizzle atoms of its tokens
+// only; the stage's other rows hold whatever was there (any byte is a pair of finite E2M1 codes) and belong to outputs
+// that nobody stores (gate/up + quantize at 16 tokens: 36 -> 32 us).
+static uint32_t box_tokens(uint32_t tokens) { return std::min<uint32_t>(BM, (tokens + 7) / 8 * 8); }
+
+// CTAs that share the K of one output tile.  A slab takes a CTA 0.45 us, so a long K over few tiles leaves most SMs idle:
+// 5120 x 27648 has 20 tiles of 108 slabs per 128 tokens.  Split where the row is at least 48 slabs long and all tiles
+// with all their slices are on the GPU at once (clusters stay inside a GPC), eight slabs a slice at least.  The rule looks
+// at the weight and the token count alone, so that a call gives the same bits whoever makes it; weights it splits are
+// launched one by one from a group, and the fused gate/up form, whose weights are wider than long, never splits.
+// 5120 x 27648 (us, whole -> split): 48 -> 23 at 16 tokens, 52 -> 37 at 200, 52 -> 39 at 384; 509 tokens are 80 tiles, whole.
+static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
+    const uint32_t k_tiles = (uint32_t)((w->n_in + BK - 1) / BK), tiles = (uint32_t)(w->n_out_pad / BN) * ((tokens + BM - 1) / BM);
+    if (k_tiles < 48 || tiles * 2 > (uint32_t)ctx->sm_count || ctx->device < 0 || ctx->device >= kMaxDevices) return 1;
+    struct Room { int n[9] = {}; };
+    static PerDevice<Room> rooms; // clusters of n CTAs the device holds at once, asked once
+    std::lock_guard<std::mutex> lock(rooms.mu);
+    Room &room = rooms.slot[ctx->device];
+    if (!room.n[1]) {
+        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, true>;
+        if (ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes) != cudaSuccess) return 1;
+        Room found;
+        for (int n = 2; n <= 8; ++n) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = n, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3(n * 64), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kSmemBytes, cfg.attrs = attr, cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&found.n[n], kernel, &cfg) != cudaSuccess) return 1;
+        }
+        found.n[1] = 1;
+        room = found;
+    }
+    for (uint32_t ks = 8; ks >= 2; --ks)
+        if (tiles <= (uint32_t)room.n[ks] && k_tiles / ks >= 8) return ks;
+    return 1;
+}
+
 muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_packed, const uint8_t *x_scales, void *y,
                                     uint32_t y_dtype, uint32_t tokens, const Epilogue &ep, cudaStream_t stream,
                                     const Weight *w_up, const NvFp4Out *qout) {
     CUtensorMap map_a;
-    if (!make_map(&map_a, x_packed, tokens, w->n_in / 2, BM))
+    if (!make_map(&map_a, x_packed, tokens, w->n_in / 2, ctx->nvfp4_pair ? BM : box_tokens(tokens)))
         return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the activations");
     GemmArgs g;
     g.a_scales = x_scales;
@@ -1112,6 +1234,8 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     g.residual = ep.residual;
     g.status = ctx->dev_status;
     g.tokens = tokens;
+    g.a_bytes = (ctx->nvfp4_pair ? BM : box_tokens(tokens)) * (BK / 2);
+    g.ksplit = 1;
     g.n_out = (uint32_t)w->n_out;
     g.k_tiles = (uint32_t)((w->n_in + BK - 1) / BK);
     g.kt64 = (uint32_t)(w->n_in / 64);
@@ -1179,6 +1303,22 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
         return MUSER_CUDA_OK;
     }
     const uint32_t tiles = g.n_tiles * m_blocks;
+    const uint32_t ks = w_up || tail ? 1 : gemm_ksplit(ctx, w, tokens);
+    if (ks > 1) {
+        g.ksplit = ks;
+        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, true>;
+        MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes));
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = ks, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(tiles * ks), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kSmemBytes, cfg.stream = stream;
+        cfg.attrs = attr, cfg.numAttrs = 2;
+        MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, map_a, mb, mb, mb, mb, g));
+        return MUSER_CUDA_OK;
+    }
     const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
     // (the attribute is per device: set where the launch happens, with the launching context's device current)
     const void *kfn = w_up ? reinterpret_cast<const void *>(nvfp4_gemm_kernel<true, false>)
@@ -1202,14 +1342,25 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
 // Up to four projections of the same quantized activations in one launch (GROUP form of the kernel).
 muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uint32_t n, const uint8_t *x_packed, const uint8_t *x_scales,
                                           void *const *ys, uint32_t y_dtype, uint32_t tokens, cudaStream_t stream) {
+    bool split = false;
+    for (uint32_t p = 0; p < n; ++p) split = split || gemm_ksplit(ctx, ws[p], tokens) > 1;
+    if (split) {
+        for (uint32_t p = 0; p < n; ++p) {
+            const muser_cuda_status st = launch_nvfp4_gemm(ctx, ws[p], x_packed, x_scales, ys[p], y_dtype, tokens, Epilogue{}, stream);
+            if (st != MUSER_CUDA_OK) return st;
+        }
+        return MUSER_CUDA_OK;
+    }
     const Weight *w0 = ws[0];
     CUtensorMap map_a;
-    if (!make_map(&map_a, x_packed, tokens, w0->n_in / 2, BM))
+    if (!make_map(&map_a, x_packed, tokens, w0->n_in / 2, box_tokens(tokens)))
         return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the activations");
     GemmArgs g = {};
     g.a_scales = x_scales;
     g.status = ctx->dev_status;
     g.tokens = tokens;
+    g.a_bytes = box_tokens(tokens) * (BK / 2);
+    g.ksplit = 1;
     g.k_tiles = (uint32_t)((w0->n_in + BK - 1) / BK);
     g.kt64 = (uint32_t)(w0->n_in / 64);
     g.y_dtype = y_dtype;

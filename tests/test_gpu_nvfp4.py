@@ -291,6 +291,38 @@ def test_fused_input_rmsnorm(gpu, x_dtype):
     assert H.rel_l2(y.cpu().numpy(), O.silu_mul(gate, upv)) <= 2 * REL_L2_TOL  # f16 boundaries of both factors can flip
 
 
+@pytest.mark.parametrize("n_out, n_in", [(37, 12288), (300, 12864), (520, 27648)])
+@pytest.mark.parametrize("tokens", [1, 77, 128, 131])
+def test_long_rows_split_between_the_ctas_of_a_cluster(gpu, n_out, n_in, tokens):
+    """Long rows over few tiles: slices of whole and ragged slabs, partial token and row tiles, every output type, the
+    residual and the row scale, against exact products (the sums are f32: some 1e-6 of their norm, f16 and bf16 round to
+    2^-12 and 2^-9), the same bits from a repeated call and from a group."""
+    op, ctx, k = gpu
+    from muser_b200 import synth
+    packed, scales, scale2 = make_weight(op, ctx, n_out, n_in, seed=n_in)
+    x = synth.normal_activations(tokens, n_in, seed=7)
+    isi = synth.activation_input_scale_inv(x)
+    w = op.Weight(ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, scale2, isi))
+    xp, xs = synth.quantize_nvfp4(x.float(), isi)
+    want = torch.from_numpy(O.dequant_nvfp4(xp.numpy(), xs.numpy(), 1.0).astype(np.float64) @ O.dequant_nvfp4(packed, scales, scale2).astype(np.float64).T / isi)
+    q = k.quantize_nvfp4_activation(x.cuda(), isi)
+    res, rs = torch.randn((tokens, n_out)), torch.linspace(0.5, 2.0, tokens)
+    for dtype, tol in ((torch.float32, 3e-6), (torch.float16, 3e-4), (torch.bfloat16, 3e-3)):
+        r = res.to(dtype)
+        for kw, ref in (({}, want), (dict(residual=r.cuda(), row_scale=rs.cuda()), want * rs[:, None] + r.double())):
+            y, again = (torch.full((tokens, n_out), float("nan"), dtype=dtype, device="cuda") for _ in range(2))
+            k.encode_nvfp4_prequant(w, *q, y, tokens, **kw)
+            k.encode_nvfp4_prequant(w, *q, again, tokens, **kw)
+            assert torch.equal(y, again)
+            assert H.rel_l2(y.double().cpu().numpy(), ref.numpy()) <= tol, (dtype, kw.keys())
+        k.encode_nvfp4_prequant(w, *q, y, tokens)
+        pair = [torch.zeros_like(y), torch.zeros_like(y)]
+        k.encode_nvfp4_group_prequant([w, w], *q, pair, tokens)
+        assert torch.equal(pair[0], y) and torch.equal(pair[1], y)
+    ctx.sync_status()
+    w.free()
+
+
 @pytest.mark.parametrize("n_in", [64, 1088, 5120, 12352])
 @pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
 def test_fused_norm_adds_the_squares_front_to_back(gpu, n_in, x_dtype):
