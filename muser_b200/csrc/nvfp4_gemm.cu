@@ -163,13 +163,13 @@ __device__ __forceinline__ void store_16_wide(const float *v, T *y, const uint32
     }
     st_32b(y, o);
 }
-// One 32-column strip of one accumulator row: scale, fuse, convert, store (16-byte stores when the row allows).
-template <typename T>
-__device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T *res, uint32_t valid, bool vec_ok) {
+// One strip of 32 (or 8) columns of one accumulator row: scale, fuse, convert, store (16-byte stores when the row allows).
+template <typename T, int N = 32>
+__device__ __forceinline__ void store_strip(const float (&v)[N], T *y, const T *res, uint32_t valid, bool vec_ok) {
     if constexpr (sizeof(T) == 4) {
-        if (vec_ok && valid == 32) {
+        if (vec_ok && valid == N) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
+            for (int i = 0; i < N; i += 4) {
                 float4 q = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 if (res) {
                     const float4 r = *reinterpret_cast<const float4 *>(res + i);
@@ -180,7 +180,7 @@ __device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T 
             return;
         }
 #pragma unroll
-        for (uint32_t i = 0; i < 32; ++i) // (unrolled with a predicate: a run-time index would push v[] out of registers)
+        for (uint32_t i = 0; i < N; ++i) // (unrolled with a predicate: a run-time index would push v[] out of registers)
             if (i < valid) y[i] = v[i] + (res ? res[i] : 0.0f);
     } else {
         auto to_f = [](T h) { if constexpr (std::is_same<T, __half>::value) return __half2float(h); else return __bfloat162float(h); };
@@ -193,9 +193,9 @@ __device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T 
                 return *reinterpret_cast<const uint32_t *>(&h);
             }
         };
-        if (vec_ok && valid == 32) {
+        if (vec_ok && valid == N) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
+            for (int i = 0; i < N; i += 8) {
                 float f[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) f[k] = v[i + k];
@@ -210,7 +210,7 @@ __device__ __forceinline__ void store_strip(const float (&v)[32], T *y, const T 
             return;
         }
 #pragma unroll
-        for (uint32_t i = 0; i < 32; ++i) {
+        for (uint32_t i = 0; i < N; ++i) {
             if (i >= valid) continue;
             const float f = v[i] + (res ? to_f(res[i]) : 0.0f);
             if constexpr (std::is_same<T, __half>::value) y[i] = __float2half_rn(f); else y[i] = __float2bfloat16_rn(f);
@@ -571,34 +571,30 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         uint32_t tile_m, tile_n;
         tile_coords(GEMM_TILE_FIRST, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
         const uint32_t rows = min((uint32_t)BM, g.tokens - tile_m * BM);
-        // one 32-column strip of one row at a time
-        for (uint32_t e = GEMM_SLICE * blockDim.x + threadIdx.x; e < rows * (BN / 32); e += g.ksplit * blockDim.x) {
-            const uint32_t row = e / (BN / 32), c0 = (e % (BN / 32)) * 32, tok = tile_m * BM + row, n0 = tile_n * BN + c0;
+        // eight columns of one row at a time: neighbouring lanes read and store neighbouring pieces
+        for (uint32_t e = GEMM_SLICE * blockDim.x + threadIdx.x; e < rows * (BN / 8); e += g.ksplit * blockDim.x) {
+            const uint32_t row = e / (BN / 8), c0 = (e % (BN / 8)) * 8, tok = tile_m * BM + row, n0 = tile_n * BN + c0;
             if (n0 >= g.n_out) continue;
-            float v[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+            float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
             for (uint32_t p = 0; p < g.ksplit; ++p) {
                 const uint32_t at = split_map(base + (row * kRedPitch + c0) * 4, p);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float4 q = split_load(at + 16 * i);
-                    v[4 * i] += q.x, v[4 * i + 1] += q.y, v[4 * i + 2] += q.z, v[4 * i + 3] += q.w;
-                }
+                const float4 q0 = split_load(at), q1 = split_load(at + 16);
+                v[0] += q0.x, v[1] += q0.y, v[2] += q0.z, v[3] += q0.w, v[4] += q1.x, v[5] += q1.y, v[6] += q1.z, v[7] += q1.w;
             }
             const float rs = g.row_scale ? g.row_scale[tok] : 1.0f;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], g.scale2), g.inv_input_scale) * rs;
+            for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], g.scale2), g.inv_input_scale) * rs;
             const size_t o = (size_t)tok * g.n_out + n0;
-            const uint32_t valid = min(32u, g.n_out - n0);
+            const uint32_t valid = min(8u, g.n_out - n0);
             const bool vec_ok = (g.n_out & 7) == 0;
             if (g.y_dtype == MUSER_DTYPE_F32)
-                store_strip<float>(v, reinterpret_cast<float *>(g.y) + o, g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
+                store_strip<float, 8>(v, reinterpret_cast<float *>(g.y) + o, g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
             else if (g.y_dtype == MUSER_DTYPE_BF16)
-                store_strip<__nv_bfloat16>(v, reinterpret_cast<__nv_bfloat16 *>(g.y) + o,
-                                           g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
+                store_strip<__nv_bfloat16, 8>(v, reinterpret_cast<__nv_bfloat16 *>(g.y) + o,
+                                              g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
             else
-                store_strip<__half>(v, reinterpret_cast<__half *>(g.y) + o, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
+                store_strip<__half, 8>(v, reinterpret_cast<__half *>(g.y) + o, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
         }
         split_barrier(); // no CTA leaves while another may read its sums
     }
@@ -1189,7 +1185,7 @@ static uint32_t box_tokens(uint32_t tokens) { return std::min<uint32_t>(BM, (tok
 // with all their slices are on the GPU at once (clusters stay inside a GPC), eight slabs a slice at least.  The rule looks
 // at the weight and the token count alone, so that a call gives the same bits whoever makes it; weights it splits are
 // launched one by one from a group, and the fused gate/up form, whose weights are wider than long, never splits.
-// 5120 x 27648 (us, whole -> split): 48 -> 23 at 16 tokens, 52 -> 37 at 200, 52 -> 39 at 384; 509 tokens are 80 tiles, whole.
+// 5120 x 27648 (us, whole -> split): 48 -> 20 at 16 tokens, 52 -> 29 at 128, 52 -> 34 at 384; 509 tokens are 80 tiles, whole.
 static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
     const uint32_t k_tiles = (uint32_t)((w->n_in + BK - 1) / BK), tiles = (uint32_t)(w->n_out_pad / BN) * ((tokens + BM - 1) / BM);
     if (k_tiles < 48 || tiles * 2 > (uint32_t)ctx->sm_count || ctx->device < 0 || ctx->device >= kMaxDevices) return 1;
