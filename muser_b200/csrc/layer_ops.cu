@@ -12,6 +12,15 @@
 
 namespace muser {
 
+// These kernels are a few microseconds of latency between two projections.  Each lets its successor launch as soon as it
+// has its own inputs' go-ahead (pdl_release behind pdl_wait): the projection that follows sets up and starts its weight
+// copies under it.  They work in place, and a successor may sit on an SM whose L1 holds a line from before the update, so
+// rows are read past L1 (ld_fresh; the rows of two blocks may share a line).
+__device__ __forceinline__ float4 ld_row(const float4 *p) {
+    const uint4 v = ld_fresh(reinterpret_cast<const uint4 *>(p));
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+
 // Sum over the block of one value per thread; `red` holds 33 floats; every thread gets the total.
 __device__ __forceinline__ float block_sum(float v, float *red) {
 #pragma unroll
@@ -31,25 +40,26 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
 }
 
 // One block per token row.  n % 4 == 0; rows 16-byte aligned.
-__global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *__restrict__ hidden, const float *__restrict__ src, float *__restrict__ output,
+__global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, const float *src, float *output,
                                                                  const float *__restrict__ w1, const float *__restrict__ w2, uint32_t n, float eps1,
                                                                  float eps2) {
     __shared__ float red[33];
     pdl_wait();
+    pdl_release();
     const uint32_t n4 = n / 4;
     float4 *h4 = reinterpret_cast<float4 *>(hidden + (size_t)blockIdx.x * n);
     const float4 *s4 = reinterpret_cast<const float4 *>(src + (size_t)blockIdx.x * n);
     const float4 *w14 = reinterpret_cast<const float4 *>(w1), *w24 = reinterpret_cast<const float4 *>(w2);
     float ss = 0.0f;
     for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x) {
-        const float4 v = s4[i];
+        const float4 v = ld_row(s4 + i);
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
     const float inv_src = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(ss, red), (float)n) + eps1));
     float sh = 0.0f;
     for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x) {
-        const float4 s = s4[i], w = w14[i];
-        float4 h = h4[i];
+        const float4 s = ld_row(s4 + i), w = w14[i];
+        float4 h = ld_row(h4 + i);
         h.x += s.x * inv_src * w.x, h.y += s.y * inv_src * w.y, h.z += s.z * inv_src * w.z, h.w += s.w * inv_src * w.w;
         h4[i] = h;
         sh += h.x * h.x + h.y * h.y + h.z * h.z + h.w * h.w;
@@ -58,17 +68,18 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *__restri
     const float inv_h = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(sh, red), (float)n) + eps2));
     float4 *o4 = reinterpret_cast<float4 *>(output + (size_t)blockIdx.x * n);
     for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x) { // this thread re-reads what it wrote itself
-        const float4 h = h4[i], w = w24[i];
+        const float4 h = ld_row(h4 + i), w = w24[i];
         o4[i] = make_float4(h.x * inv_h * w.x, h.y * inv_h * w.y, h.z * inv_h * w.z, h.w * inv_h * w.w);
     }
 }
 
 // x[i] *= 1 / (1 + exp(-gate[i])), four at a time.
-__global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *__restrict__ x, const float *__restrict__ gate, size_t n4) {
+__global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *x, const float *gate, size_t n4) {
     pdl_wait();
+    pdl_release();
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
-        float4 v = reinterpret_cast<float4 *>(x)[i];
-        const float4 g = reinterpret_cast<const float4 *>(gate)[i];
+        float4 v = ld_row(reinterpret_cast<const float4 *>(x) + i);
+        const float4 g = ld_row(reinterpret_cast<const float4 *>(gate) + i);
         v.x *= __fdiv_rn(1.0f, 1.0f + expf(-g.x)), v.y *= __fdiv_rn(1.0f, 1.0f + expf(-g.y));
         v.z *= __fdiv_rn(1.0f, 1.0f + expf(-g.z)), v.w *= __fdiv_rn(1.0f, 1.0f + expf(-g.w));
         reinterpret_cast<float4 *>(x)[i] = v;
@@ -76,9 +87,10 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *__restrict__ x
 }
 
 // One warp per (token, head): x <- x * 1/sqrt(mean(x^2) + eps) * w, head_dim % 4 == 0, head_dim <= 1024.
-__global__ void __launch_bounds__(256) head_rms_norm_kernel(float *__restrict__ x, const float *__restrict__ w, float eps, uint32_t heads_total,
+__global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const float *__restrict__ w, float eps, uint32_t heads_total,
                                                             uint32_t head_dim) {
     pdl_wait();
+    pdl_release();
     const uint32_t head = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (head >= heads_total) return;
     float4 *row = reinterpret_cast<float4 *>(x + (size_t)head * head_dim);
@@ -86,14 +98,14 @@ __global__ void __launch_bounds__(256) head_rms_norm_kernel(float *__restrict__ 
     const uint32_t n4 = head_dim / 4;
     float ss = 0.0f;
     for (uint32_t i = lane; i < n4; i += 32) {
-        const float4 v = row[i];
+        const float4 v = ld_row(row + i);
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(ss, (float)head_dim) + eps));
     for (uint32_t i = lane; i < n4; i += 32) {
-        const float4 v = row[i], ww = w4[i];
+        const float4 v = ld_row(row + i), ww = w4[i];
         row[i] = make_float4(v.x * inv * ww.x, v.y * inv * ww.y, v.z * inv * ww.z, v.w * inv * ww.w);
     }
 }
