@@ -50,27 +50,53 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, 
     float4 *h4 = reinterpret_cast<float4 *>(hidden + (size_t)blockIdx.x * n);
     const float4 *s4 = reinterpret_cast<const float4 *>(src + (size_t)blockIdx.x * n);
     const float4 *w14 = reinterpret_cast<const float4 *>(w1), *w24 = reinterpret_cast<const float4 *>(w2);
+    // The row's first kHeld pieces per thread (8192 values a block of 512) stay in registers from one fetch: reading them
+    // again for each of the three passes was two more trips to L2 in a kernel that is nothing but such trips.
+    constexpr uint32_t kHeld = 4;
+    float4 s[kHeld], h[kHeld];
     float ss = 0.0f;
-    for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x) {
+#pragma unroll
+    for (uint32_t k = 0; k < kHeld; ++k) {
+        const uint32_t i = threadIdx.x + k * blockDim.x;
+        s[k] = h[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < n4) s[k] = ld_row(s4 + i), h[k] = ld_row(h4 + i);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kHeld; ++k) ss += s[k].x * s[k].x + s[k].y * s[k].y + s[k].z * s[k].z + s[k].w * s[k].w;
+    for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) {
         const float4 v = ld_row(s4 + i);
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
     const float inv_src = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(ss, red), (float)n) + eps1));
     float sh = 0.0f;
-    for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x) {
-        const float4 s = ld_row(s4 + i), w = w14[i];
-        float4 h = ld_row(h4 + i);
-        h.x += s.x * inv_src * w.x, h.y += s.y * inv_src * w.y, h.z += s.z * inv_src * w.z, h.w += s.w * inv_src * w.w;
-        h4[i] = h;
-        sh += h.x * h.x + h.y * h.y + h.z * h.z + h.w * h.w;
+    auto tail = [&](uint32_t i, const float4 &sv, float4 &hv) {
+        const float4 w = w14[i];
+        hv.x += sv.x * inv_src * w.x, hv.y += sv.y * inv_src * w.y, hv.z += sv.z * inv_src * w.z, hv.w += sv.w * inv_src * w.w;
+        h4[i] = hv;
+        sh += hv.x * hv.x + hv.y * hv.y + hv.z * hv.z + hv.w * hv.w;
+    };
+#pragma unroll
+    for (uint32_t k = 0; k < kHeld; ++k) {
+        const uint32_t i = threadIdx.x + k * blockDim.x;
+        if (i < n4) tail(i, s[k], h[k]);
+    }
+    for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) {
+        float4 hv = ld_row(h4 + i);
+        tail(i, ld_row(s4 + i), hv);
     }
     if (!output) return;
     const float inv_h = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(sh, red), (float)n) + eps2));
     float4 *o4 = reinterpret_cast<float4 *>(output + (size_t)blockIdx.x * n);
-    for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x) { // this thread re-reads what it wrote itself
-        const float4 h = ld_row(h4 + i), w = w24[i];
-        o4[i] = make_float4(h.x * inv_h * w.x, h.y * inv_h * w.y, h.z * inv_h * w.z, h.w * inv_h * w.w);
+    auto out = [&](uint32_t i, const float4 &hv) {
+        const float4 w = w24[i];
+        o4[i] = make_float4(hv.x * inv_h * w.x, hv.y * inv_h * w.y, hv.z * inv_h * w.z, hv.w * inv_h * w.w);
+    };
+#pragma unroll
+    for (uint32_t k = 0; k < kHeld; ++k) {
+        const uint32_t i = threadIdx.x + k * blockDim.x;
+        if (i < n4) out(i, h[k]);
     }
+    for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) out(i, ld_row(h4 + i)); // (this thread's own)
 }
 
 // x[i] *= 1 / (1 + exp(-gate[i])), four at a time.
