@@ -13,6 +13,9 @@
 // quantized once into the context workspace by a kernel of their own; the contraction runs on the int8 tensor pipe.
 #include <cuda_fp8.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 
 namespace muser {
@@ -94,6 +97,7 @@ __device__ __forceinline__ void e4m3_q9(uint32_t codes, int (&q9)[4]) {
 __device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return (&v.x)[i]; } // compile-time i only
 
 constexpr int kA16Warps = 8;
+constexpr int a16_ctas_per_sm(int pairs) { return pairs == 1 ? 3 : 2; } // what the registers allow
 
 // A warp contracts one 256-value block of 16 weight rows with 2 * PAIRS tokens at a time.  The codes come as they lie in
 // memory: lane (g, t) loads 16 bytes of row g (and of row g + 8) of each 128-value chunk, which are the two 16-groups
@@ -107,12 +111,12 @@ constexpr int kA16Warps = 8;
 // shared memory, meet at a named barrier, and every (row, token) sum is continued front to back by one thread, so the
 // order of the additions is the reference's whatever ksplit is.
 //
-// Two tokens: 27648 x 5120 151 -> 35 us, 5120 x 27648 222 -> 58, 1024 x 5120 23 -> 6.5, a layer's seven calls 699 -> 167
+// Two tokens: 27648 x 5120 151 -> 30 us, 5120 x 27648 222 -> 40, 1024 x 5120 23 -> 6, a layer's seven calls 699 -> 137
 // (bound by instruction issue; the weights' bytes take 12 us each for the large ones).  The earlier form, one warp per
 // row with eight scalar multiply-adds per lane and a 64-bit shuffle tree per token and block, had about five times the
 // instructions per weight.
-template <int PAIRS>
-__global__ void __launch_bounds__(kA16Warps * 32, 2) nvfp4_a16_kernel(const __grid_constant__ A16Args a) {
+template <int PAIRS, int CTAS>
+__global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const __grid_constant__ A16Args a) {
     __shared__ float contrib[2][kA16Warps][2 * PAIRS * 16];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t slot = warp / a.ksplit, part = warp % a.ksplit, slots = kA16Warps / a.ksplit;
@@ -237,14 +241,20 @@ __global__ void __launch_bounds__(kA16Warps * 32, 2) nvfp4_a16_kernel(const __gr
     }
 }
 
-// Warps per row tile: the split with the fewest rounds of (CTAs on the GPU) x (blocks in turn), two CTAs an SM.  Few
-// rows (attn_k: 64 tiles) want all eight warps on one tile, 27648 rows of 20 blocks four (15 rounds against 20 and 18).
-static uint32_t a16_ksplit(uint32_t row_tiles, uint32_t blocks, int sm_count) {
-    uint32_t best = 1, best_rounds = ~0u;
+// Warps per row tile.  A block costs a warp about 500 cycles of its scheduler (mostly the byte-and-logic pipe, which takes
+// an instruction every two cycles) and no less than 2500 from end to end, so a split is worth the rounds of CTAs over the
+// GPU times the blocks in turn times the longer of the two.  Few rows (attn_k: 64 tiles) want all eight warps on a tile;
+// so do 5120 x 27648 (320 CTAs at once against 160, one to an SM).
+static uint32_t a16_ksplit(uint32_t row_tiles, uint32_t blocks, uint32_t tokens, int sm_count) {
+    const int per_sm = a16_ctas_per_sm(tokens <= 2 ? 1 : 2);
+    const double issue = 500.0 + 70.0 * std::min(tokens, 16u);
+    uint32_t best = 1;
+    double best_cost = 1e300;
     for (uint32_t ks = 1; ks <= kA16Warps; ks *= 2) {
         const uint32_t ctas = (row_tiles + kA16Warps / ks - 1) / (kA16Warps / ks);
-        const uint32_t rounds = (ctas + 2 * sm_count - 1) / (2 * sm_count) * ((blocks + ks - 1) / ks);
-        if (rounds < best_rounds) best = ks, best_rounds = rounds;
+        const double rounds = std::ceil((double)ctas / (per_sm * sm_count)), busy = std::min<double>(per_sm, std::ceil((double)ctas / sm_count));
+        const double cost = rounds * std::ceil((double)blocks / ks) * std::max(busy * kA16Warps / 4 * issue, 2000.0 + issue);
+        if (cost < best_cost * 0.999) best = ks, best_cost = cost;
     }
     return best;
 }
@@ -267,12 +277,15 @@ muser_cuda_status launch_nvfp4_a16(Ctx *ctx, const Weight *w, const void *x, uin
     a.scale2 = w->scale2;
     a.n_out = (uint32_t)w->n_out, a.n_in = (uint32_t)w->n_in, a.kt = (uint32_t)((w->n_in + 63) / 64), a.tokens = tokens, a.y_dtype = y_dtype;
     a.row_tiles = (a.n_out + 127) / 128 * 8;
-    a.ksplit = a16_ksplit(a.row_tiles, a.n_in / 256, ctx->sm_count);
+    a.ksplit = a16_ksplit(a.row_tiles, a.n_in / 256, tokens, ctx->sm_count);
     const dim3 grid((a.row_tiles * a.ksplit + kA16Warps - 1) / kA16Warps), threads(kA16Warps * 32);
-    if (tokens <= 2) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<1>, grid, threads, 0, stream, a));
-    else if (tokens <= 4) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<2>, grid, threads, 0, stream, a));
-    else if (tokens <= 8) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<4>, grid, threads, 0, stream, a));
-    else MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<8>, grid, threads, 0, stream, a));
+    // three CTAs an SM cost the kernel for two tokens a third of its registers: only where there are as many
+    // (1024 x 5120: 5.8 us with 2 an SM, 7.3 with 3; 5120 x 27648: 56 and 40)
+    if (tokens <= 2 && grid.x > 2 * (unsigned)ctx->sm_count) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<1, 3>, grid, threads, 0, stream, a));
+    else if (tokens <= 2) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<1, 2>, grid, threads, 0, stream, a));
+    else if (tokens <= 4) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<2, 2>, grid, threads, 0, stream, a));
+    else if (tokens <= 8) MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<4, 2>, grid, threads, 0, stream, a));
+    else MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_a16_kernel<8, 2>, grid, threads, 0, stream, a));
     return MUSER_CUDA_OK;
 }
 
