@@ -119,8 +119,73 @@ __global__ void __launch_bounds__(32) rms_rows_sequential_kernel(const void *x, 
     if (my_row < tokens) inv_rms[my_row] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)n_in), eps)));
 }
 
+// The same chains for few rows, where one warp that fetches, unpacks, squares and adds takes 11 cycles an input: here the
+// first warp's lanes only read squares and add (four cycles an addition is the floor, 11 us for 5120 values), and the
+// block's other seven warps fetch, square and lay the squares out for it, 256 inputs of 32 rows ahead.  From some
+// thousands of rows the shared-memory traffic costs more than the latency saved (us with the quantizer behind it,
+// 5120 values: 2048 rows 51 -> 42, 4096 even, 32768 rows 245 against 320).
+constexpr int kRmsThreads = 256, kRmsRows = 32, kRmsChunk = 256;
+constexpr int kRmsPitch = kRmsRows + 1;                                     // float4 per four inputs: rows side by side, padded
+constexpr int kRmsBuffer = kRmsChunk / 4 * kRmsPitch;                       // float4 of one buffer
+constexpr size_t kRmsSmem = 2 * kRmsBuffer * sizeof(float4);
+template <bool XF32>
+__global__ void __launch_bounds__(kRmsThreads) rms_rows_staged_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms) {
+    extern __shared__ float4 rms_squares[]; // two buffers
+    pdl_wait();
+    pdl_release();
+    const uint32_t row0 = blockIdx.x * kRmsRows, steps = (n_in + kRmsChunk - 1) / kRmsChunk;
+    // warps 1 .. 7: pieces of eight inputs, neighbouring lanes along a row; all of a thread's loads before the first is used
+    constexpr uint32_t kPieces = kRmsRows * (kRmsChunk / 8), kLoaders = kRmsThreads - 32, kPer = (kPieces + kLoaders - 1) / kLoaders;
+    auto stage = [&](uint32_t step, float4 *buf) {
+        float v[kPer][8];
+#pragma unroll
+        for (uint32_t n = 0; n < kPer; ++n) {
+            const uint32_t p = threadIdx.x - 32 + n * kLoaders, r = p / (kRmsChunk / 8), i8 = step * (kRmsChunk / 8) + p % (kRmsChunk / 8);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[n][k] = 0.0f; // zeros add nothing to the chain
+            if (p < kPieces && row0 + r < tokens && i8 < n_in / 8)
+                load8<XF32>(XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)(row0 + r) * n_in)
+                                 : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)(row0 + r) * n_in), i8, v[n]);
+        }
+#pragma unroll
+        for (uint32_t n = 0; n < kPer; ++n) {
+            const uint32_t p = threadIdx.x - 32 + n * kLoaders, r = p / (kRmsChunk / 8), j = p % (kRmsChunk / 8);
+            if (p >= kPieces) break;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[n][k] = __fmul_rn(v[n][k], v[n][k]);
+            buf[(2 * j) * kRmsPitch + r] = make_float4(v[n][0], v[n][1], v[n][2], v[n][3]);
+            buf[(2 * j + 1) * kRmsPitch + r] = make_float4(v[n][4], v[n][5], v[n][6], v[n][7]);
+        }
+    };
+    float ss = 0.0f;
+    if (threadIdx.x >= 32) stage(0, rms_squares);
+    for (uint32_t step = 0; step < steps; ++step) {
+        __syncthreads(); // this step's squares are there, and the other buffer has been read
+        if (threadIdx.x >= 32) {
+            if (step + 1 < steps) stage(step + 1, rms_squares + ((step + 1) & 1) * kRmsBuffer);
+        } else {
+            const float4 *cur = rms_squares + (step & 1) * kRmsBuffer + threadIdx.x;
+#pragma unroll 32
+            for (int q = 0; q < kRmsChunk / 4; ++q) {
+                const float4 v = cur[q * kRmsPitch];
+                ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, v.x), v.y), v.z), v.w);
+            }
+        }
+    }
+    if (threadIdx.x < 32 && row0 + threadIdx.x < tokens)
+        inv_rms[row0 + threadIdx.x] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)n_in), eps)));
+}
+
+constexpr uint32_t kRmsStagedRows = 4096;
+
 static cudaError_t launch_rms_rows_sequential(Ctx *ctx, const void *x, uint32_t x_dtype, uint32_t tokens, uint32_t n_in, float eps,
                                               float *inv_rms, cudaStream_t stream) {
+    if (tokens <= kRmsStagedRows) {
+        const auto kernel = x_dtype == MUSER_DTYPE_F32 ? rms_rows_staged_kernel<true> : rms_rows_staged_kernel<false>;
+        const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kRmsSmem);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(kernel, dim3((tokens + kRmsRows - 1) / kRmsRows), dim3(kRmsThreads), kRmsSmem, stream, x, tokens, n_in, eps, inv_rms);
+    }
     const unsigned blocks = (tokens + 31) / 32;
     const bool f32 = x_dtype == MUSER_DTYPE_F32;
     const size_t smem = (size_t)2 * 32 * ((f32 ? 64 : 32) + 1) * sizeof(uint4);
@@ -276,9 +341,9 @@ __global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, inv, packed, scales);
 }
 
-// The same behind rms_rows_sequential_kernel, whose 32 chains a warp do less work per row than the segments above and
-// take 30 us however few the rows: the better form from about 1500 rows of 5120 (20.5 ns a row for the kernel above,
-// 7.6 for these two; 2048 rows 50 us either way).
+// The same behind a kernel that runs the chains as chains, which does less work per row than the segments above but takes
+// their length in latency: the better form from 1537 rows (us, segments / chains with quantizer, 5120 values: 15 / 19 at 16
+// rows, 28 / 36 at 1024, 43 / 42 at 2048) and for rows of up to 3072 values (1024 values: 11 / 6 at 16 rows, 15 / 8 at 1024).
 template <bool XF32>
 __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
                                                                     const float *__restrict__ norm_w, const float *inv_rms, uint8_t *packed,
@@ -290,7 +355,7 @@ __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
 }
-constexpr uint32_t kNormSegmentRows = 1536; // up to here the segmented kernel
+constexpr uint32_t kNormSegmentRows = 1536, kNormSegmentMin = 3073; // up to so many rows of at least so many values: the segmented kernel
 
 // Plain rows: out[t][k] = (x[t][k] * inv_rms_t) * w[k] in f32, for the kernels that read their activations as they go.
 template <bool XF32>
@@ -334,7 +399,7 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
     if (norm_weight) {
         float *inv = ctx->inv_rms;
         if (!inv || tokens > ctx->inv_rms_rows) return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: more rows than the context's per-row scratch holds");
-        if (tokens > kNormSegmentRows) {
+        if (tokens > kNormSegmentRows || n_in < kNormSegmentMin) {
             MUSER_CUDA_TRY(ctx, launch_rms_rows_sequential(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
             const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
             MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(256), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, (const float *)inv,
