@@ -1304,7 +1304,9 @@ muser_cuda_status launch_kquant_matmul(Ctx *ctx, const Weight *w, const Weight *
         return muser_cuda_all_reduce(reinterpret_cast<muser_cuda_ctx *>(ctx), y, count, y_dtype, stream);
     }
     const size_t xb = xf32 ? 4 : 2, yb = y_dtype == MUSER_DTYPE_BF16 ? 2 : 4;
-    uint32_t chunk = takes_mma(ctx, w, tokens) ? 64 : 16;
+    // (the batched kernel rounds Q6_K operands beyond 16 tokens, as the tcgen05 kernel does for the calls it may serve; the
+    // other Q6_K calls keep exact operands, 16 tokens at a time)
+    uint32_t chunk = takes_mma(ctx, w, tokens) && (tc_fits || !q6) ? 64 : 16;
     for (uint32_t t0 = 0, n; t0 < tokens; t0 += n) {
         n = std::min(chunk, tokens - t0);
         Epilogue e = ep;
