@@ -130,10 +130,12 @@ MUSER_CUDA_API const char *muser_cuda_last_error(const muser_cuda_ctx *ctx);
 MUSER_CUDA_API muser_cuda_status muser_cuda_sync_status(muser_cuda_ctx *ctx, void *stream);
 
 /* No counterpart in the reference (its kernel choice is compiled in, src/metal/encode/qkv.rs:425-449).  Which kernel
- * serves a K-quant call depends on the token count: up to 16 tokens the decode kernel, from 17 the tcgen05 skinny
- * kernel where the weight is large enough.  The thresholds and the decode kernel's launch plan can be moved, e.g. to
- * force one kernel in a test.  A TC_MIN_TOKENS value above 64 switches the tensor-core skinny kernel off. */
-#define MUSER_TUNE_TC_MIN_TOKENS_Q4_K 1u /* Q4_K calls with at least this many tokens take the tcgen05 kernel (default 17) */
+ * serves a K-quant call depends on the token count: up to 12 tokens the decode kernel, from 13 the batched kernel on
+ * warp-level products, or from 17 the tcgen05 skinny kernel for large Q4_K weights at token counts that fill its
+ * columns.  The thresholds and the decode kernel's launch plan can be moved, e.g. to force one kernel in a test.  A
+ * TC_MIN_TOKENS value below 17 asks for the tcgen05 kernel wherever it can serve, one above 64 switches it off; a forced
+ * launch plan keeps calls of up to 16 tokens with the decode kernel. */
+#define MUSER_TUNE_TC_MIN_TOKENS_Q4_K 1u /* from how many tokens Q4_K calls may take the tcgen05 kernel (default 17) */
 #define MUSER_TUNE_TC_MIN_TOKENS_Q6_K 2u /* likewise for Q6_K (default 17) */
 #define MUSER_TUNE_TC_MIN_ROWS 3u        /* ... if the weight has at least this many output rows (default 1024) */
 #define MUSER_TUNE_DECODE_WARPS 8u       /* decode kernel: warps per CTA, even (0: from its cost model) */

@@ -35,10 +35,10 @@ struct Ctx {
     size_t gemv_partial_bytes = 0;
     unsigned int *gemv_counters = nullptr; // one arrival counter per 16-row tile, zero between launches
     uint32_t gemv_counter_slots = 0;
-    void *tc_scratch = nullptr;            // f16 activations + sub-block sums of the tensor-core K-quant kernel
+    void *tc_scratch = nullptr;            // f16 activations + sub-block sums of the batched K-quant kernels
     size_t tc_scratch_bytes = 0;
-    uint32_t tc_min_tokens[2] = {17, 17};  // from how many tokens Q4_K / Q6_K calls take that kernel (tuning knobs,
-    uint32_t tc_min_rows = 1024;           // and from how many output rows); fewer tokens take the decode kernel
+    uint32_t tc_min_tokens[2] = {17, 17};  // from how many tokens Q4_K / Q6_K calls may take the tcgen05 kernel (tuning knobs,
+    uint32_t tc_min_rows = 1024;           // and from how many output rows); the rule is beside takes_tcgen05() in kquant_decode.cu
     uint32_t dec_warps = 0, dec_ksplit = 0, dec_ring = 0, dec_wsplit = 0;
     uint32_t dec_last_plan[4] = {0, 0, 0, 0}; // (warps, ksplit, wsplit, ring) of the decode kernel's latest launch on this context // decode kernel plan overrides (0: from its cost model)
     float *norm_scratch = nullptr;         // normalized rows for the skinny K-quant kernel (fused input norm)
