@@ -1218,8 +1218,8 @@ muser_cuda_status decode_autotune(Ctx *ctx, const Weight *const *w, const Weight
 // batched kernels.  Of the batched kernels the one on the warp-level instructions (kquant_mma.cu) has the
 // smaller fixed part and pads token columns to 8, the tcgen05 one (kquant_tc.cu, to 16, 32 or 64; Q4_K and Q6_K) the
 // cheaper column: see takes_tcgen05.  At 13 to 16 tokens the decode kernel's integer products are bound by their scale
-// arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 40, 5120 x 27648 Q6_K 68 -> 43, 5120 x 5120 21 -> 15,
-// 1024 x 5120 18.5 -> 12); at 9 to 12 the two are even (40 / 40, 55 / 43, 17 / 15, but 8192 x 5120 17 / 20), below it wins.
+// arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 35, 5120 x 27648 Q6_K 68 -> 42, 5120 x 5120 21 -> 14,
+// 1024 x 5120 18.5 -> 10); at 9 to 12 the two are even (40 / 40, 55 / 43, 17 / 15, but 8192 x 5120 17 / 20), below it wins.
 // The decode kernel also keeps
 //   - K shards up to 16 tokens, whose partial sums must carry the same bits with and without the all-reduce fused in,
 //   - calls under a forced launch plan (MUSER_TUNE_DECODE_*), and shapes the batched kernels refuse.

@@ -534,7 +534,7 @@ cudaError_t cluster_room(int device, int sm_count, ClusterRoom *out) {
 }
 
 // Warps per CTA (= row tiles), K slices per cluster and ring depth.  A warp's tile costs about `tile` cycles of its
-// scheduler (issue or tensor pipe, whichever is longer) and takes at least 1500 + tile from end to end; the plan with the
+// scheduler and takes at least 1500 + 1.1 tile from end to end; the plan with the
 // fewest (rounds over the GPU) x (tiles that share a scheduler) x (columns in turn) wins, the meeting of the slices
 // counted as 2500 cycles.
 MmaPlan mma_plan(const uint32_t *tiles, uint32_t n_jobs, bool dual, uint32_t nsb, uint32_t blob_bytes, uint32_t tile_slot, uint32_t red_tokens,
@@ -555,7 +555,7 @@ MmaPlan mma_plan(const uint32_t *tiles, uint32_t n_jobs, bool dual, uint32_t nsb
                 if (slots < 1.0) continue;
                 const double rounds = std::ceil(groups / slots);
                 const double ctas = std::min<double>(per_sm, std::ceil((double)groups / room.n[ks]));
-                const double column = std::max(ctas * w / 4.0 * tile, 1500.0 + tile);
+                const double column = std::max(ctas * w / 4.0 * tile, 1500.0 + 1.1 * tile);
                 const double cost = rounds * (std::ceil((double)nsb / ks) * column + (ks > 1 ? 2500.0 : 800.0));
                 if (cost < best_cost * 0.999) best_cost = cost, best = {w, ks, stages};
             }
@@ -617,8 +617,9 @@ cudaError_t mma_run(Ctx *ctx, MmaArgs &a, const uint32_t *tiles, bool dual, bool
             set.next = (set.next + 1) % 16;
             c.nsb = a.nsb, c.n_jobs = a.n_jobs, c.slot = a.tile_slot, c.dual = dual;
             for (uint32_t i = 0; i < a.n_jobs; ++i) c.tiles[i] = tiles[i];
-            const double issue = !q6 ? 450.0 + 40.0 * NG : NG <= 2 ? 600.0 + 110.0 * NG : 600.0 + 40.0 * NG, pipe = 8.3 * 17 * NG * PLANES;
-            c.plan = mma_plan(tiles, a.n_jobs, dual, a.nsb, B::kBytes, a.tile_slot, NG * 8, room, std::max(issue, pipe * 1.3));
+            // cycles of a scheduler per tile, fitted to 27648 x 5120 (Q4_K) and 5120 x 27648 (Q6_K) at 8 to 64 tokens
+            const double tile = (q6 ? 1050.0 : 950.0) + (q6 && NG <= 2 ? 190.0 : 30.0) * NG + 130.0 * NG * PLANES;
+            c.plan = mma_plan(tiles, a.n_jobs, dual, a.nsb, B::kBytes, a.tile_slot, NG * 8, room, tile);
             hit = &c;
         }
         p = hit->plan;
