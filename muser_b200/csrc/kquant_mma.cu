@@ -23,9 +23,10 @@
 // (a full and an empty barrier each).  K is cut between the CTAs of a cluster; the slices meet through distributed shared
 // memory and are added in slice order, every CTA finishing its share of the outputs.
 //
-// What bounds it: the schedulers.  A tile costs a warp about 450 instructions besides its products (half of them on the
-// byte-and-logic pipe, which takes one every two cycles), and m16n8k16 itself takes the tensor pipe 8.3 cycles: at 64
-// tokens (1130 cycles a tile) the products are the longer half.  Figures beside takes_mma() in kquant_decode.cu.
+// What bounds it: no one unit.  A tile costs a warp about 450 instructions besides its products; at 16 tokens of
+// 27648 x 5120 the issue slots are 44 % used, the byte-and-logic pipe 37 %, the tensor pipe 23 %, with three warps a
+// scheduler in chains of unpack, product and scale.  m16n8k16 takes the tensor pipe 8.3 cycles: from 48 tokens the
+// products are the largest part.  Figures beside takes_mma() in kquant_decode.cu.
 #include <algorithm>
 #include <cmath>
 
@@ -38,7 +39,7 @@ namespace muser {
 
 constexpr int kMmaMaxJobs = 4, kMmaMaxSplit = 8;
 // Warps on an SM, one of every CTA's being its producer, at 128 registers a thread.  (24 warps of 80 registers were no
-// faster up to 16 tokens: 27648 x 5120 at 16 tokens 41.7 us against 40.2; the schedulers are busy, not waiting.)
+// faster: 27648 x 5120 at 16 tokens 41.7 us against 40.2 under the same plan.)
 constexpr int kMmaWarps = 16;
 
 struct MmaJob {
