@@ -121,10 +121,10 @@ __global__ void __launch_bounds__(32) rms_rows_sequential_kernel(const void *x, 
 
 // The same chains for few rows, where one warp that fetches, unpacks, squares and adds takes 11 cycles an input: here the
 // first warp's lanes only read squares and add (four cycles an addition is the floor, 11 us for 5120 values), and the
-// block's other seven warps fetch, square and lay the squares out for it, 256 inputs of 32 rows ahead.  From some
-// thousands of rows the shared-memory traffic costs more than the latency saved (us with the quantizer behind it,
-// 5120 values: 2048 rows 51 -> 42, 4096 even, 32768 rows 245 against 320).
-constexpr int kRmsThreads = 256, kRmsRows = 32, kRmsChunk = 256;
+// block's other seven warps fetch, square and lay the squares out for it, 256 inputs of 16 rows ahead (of 32 rows the
+// seven could not keep up: 2048 rows 41 us, 37 with 16).  From some thousands of rows the shared-memory traffic costs more
+// than the latency saved (us with the quantizer behind it, 5120 values: 2048 rows 51 -> 37, 4096 rows 46 against about 50).
+constexpr int kRmsThreads = 256, kRmsRows = 16, kRmsChunk = 256;
 constexpr int kRmsPitch = kRmsRows + 1;                                     // float4 per four inputs: rows side by side, padded
 constexpr int kRmsBuffer = kRmsChunk / 4 * kRmsPitch;                       // float4 of one buffer
 constexpr size_t kRmsSmem = 2 * kRmsBuffer * sizeof(float4);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kRmsThreads) rms_rows_staged_kernel(const void
         if (threadIdx.x >= 32) {
             if (step + 1 < steps) stage(step + 1, rms_squares + ((step + 1) & 1) * kRmsBuffer);
         } else {
-            const float4 *cur = rms_squares + (step & 1) * kRmsBuffer + threadIdx.x;
+            const float4 *cur = rms_squares + (step & 1) * kRmsBuffer + min(threadIdx.x, kRmsRows - 1u); // (lanes without a row repeat the last)
 #pragma unroll 32
             for (int q = 0; q < kRmsChunk / 4; ++q) {
                 const float4 v = cur[q * kRmsPitch];
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kRmsThreads) rms_rows_staged_kernel(const void
             }
         }
     }
-    if (threadIdx.x < 32 && row0 + threadIdx.x < tokens)
+    if (threadIdx.x < kRmsRows && row0 + threadIdx.x < tokens)
         inv_rms[row0 + threadIdx.x] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)n_in), eps)));
 }
 
@@ -342,8 +342,9 @@ __global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const
 }
 
 // The same behind a kernel that runs the chains as chains, which does less work per row than the segments above but takes
-// their length in latency: the better form from 1537 rows (us, segments / chains with quantizer, 5120 values: 15 / 19 at 16
-// rows, 28 / 36 at 1024, 43 / 42 at 2048) and for rows of up to 3072 values (1024 values: 11 / 6 at 16 rows, 15 / 8 at 1024).
+// their length in latency: the better form from 449 rows (us, segments / chains with quantizer, 5120 values: 15 / 17 at 16
+// rows, 19 / 19 at 512, 40 / 33 at 1536, 43 / 37 at 2048; 3136 values: 20 / 13 at 448 rows) and for rows of up to 4096 values
+// (1024 values: 11 / 6 at 16 rows, 15 / 7 at 1024).
 template <bool XF32>
 __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
                                                                     const float *__restrict__ norm_w, const float *inv_rms, uint8_t *packed,
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
 }
-constexpr uint32_t kNormSegmentRows = 1536, kNormSegmentMin = 3073; // up to so many rows of at least so many values: the segmented kernel
+constexpr uint32_t kNormSegmentRows = 448, kNormSegmentMin = 4097; // up to so many rows of at least so many values: the segmented kernel
 
 // Plain rows: out[t][k] = (x[t][k] * inv_rms_t) * w[k] in f32, for the kernels that read their activations as they go.
 template <bool XF32>

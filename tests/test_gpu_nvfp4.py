@@ -347,7 +347,7 @@ def test_fused_norm_adds_the_squares_front_to_back(gpu, n_in, x_dtype):
     xn = O.rms_norm_mul(x.float().numpy(), eps, nw.numpy())
     want_p, want_s = O.quantize_nvfp4_activation(xn, isi)
     rows = [r for r in range(11) if r != 9]  # (an infinite row normalizes to zeros and a NaN, whose sign no reference defines)
-    for copies in (1, 150, 400) if n_in <= 5120 else (1,):  # the same rows among few, more than 1536 and more than 4096
+    for copies in (1, 150, 400) if n_in <= 5120 else (1,):  # the same rows among few, some thousand and more than 4096
         many = x.cuda().repeat(copies, 1)
         got_p, got_s = k.quantize_nvfp4_activation(many, isi, norm_weight=nw.cuda(), norm_eps=eps)
         ctx.sync_status()
