@@ -27,7 +27,7 @@ def _newest(paths) -> float:
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     srcs = [CSRC / s for s in SOURCES]
-    deps = list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "muser_cuda.h"]
+    deps = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [PKG.parent / "include" / "muser_cuda.h"]
     if not force and LIB.exists() and LIB.stat().st_mtime >= _newest(srcs + deps):
         return LIB
     objdir = CSRC / "build"

@@ -17,6 +17,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "nvfp4_a16_exchange.h"
 
 namespace muser {
 
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const _
     const uint32_t tile_row = (rt / 8) * 128 + 4 * (rt % 8);
     auto row_of = [&](uint32_t m) { return tile_row + 32 * (m & 3) + (m >> 2); };
     if (rt >= a.row_tiles || tile_row >= a.n_out) return; // whole slots leave; barriers are per slot
-    const uint32_t blocks = a.n_in / 256;
+    const uint32_t blocks = a.n_in / 256, steps = (blocks + a.ksplit - 1) / a.ksplit;
     const uint8_t *code0 = a.packed + (size_t)row_of(g) * (a.n_in / 2) + 16 * t, *code1 = a.packed + (size_t)row_of(g + 8) * (a.n_in / 2) + 16 * t;
     auto scale_ptr = [&](uint32_t row) {
         return a.scales + (size_t)(row / 128) * ((size_t)a.kt * 512) + (row % 32) * 16 + ((row % 128) / 32) * 4 + (t & 1) * 512;
@@ -159,8 +160,8 @@ __global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const _
         for (int i = 0; i < PAIRS; ++i) total[i] = 0.0f;
         uint32_t step = 0;
         for (uint32_t b0 = 0; b0 < blocks; b0 += a.ksplit, ++step) {
-            const uint32_t b = b0 + part;
-            float *mine = contrib[step & 1][warp];
+            const uint32_t b = b0 + part, buffer = a16_buffer(t0 / (2 * PAIRS), steps, step);
+            float *mine = contrib[buffer][warp];
             if (b < blocks) {
                 cur = nxt;
                 if (b + a.ksplit < blocks) fetch(b + a.ksplit, nxt);
@@ -219,13 +220,12 @@ __global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const _
                 }
             }
             asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(a.ksplit * 32) : "memory");
-            // (two buffers in turn: a warp writes a buffer again only behind the next step's barrier)
             const uint32_t n_here = min(a.ksplit, blocks - b0);
 #pragma unroll
             for (int i = 0; i < PAIRS; ++i) {
                 const uint32_t e = part * 32 + lane + (uint32_t)i * a.ksplit * 32;
                 if (e < 32u * PAIRS)
-                    for (uint32_t s = 0; s < n_here; ++s) total[i] = __fmaf_rn(1.0f, contrib[step & 1][slot * a.ksplit + s][e], total[i]);
+                    for (uint32_t s = 0; s < n_here; ++s) total[i] = __fmaf_rn(1.0f, contrib[buffer][slot * a.ksplit + s][e], total[i]);
             }
         }
 #pragma unroll

@@ -407,7 +407,9 @@ def test_weight_only_lane_is_bit_identical(gpu, golden):
     """A weight without input_scale_inv takes the reference's weight-only lane (int8 activations per 256, exact
     integer contraction, f16 result).  First the reference's own fixture (7 tokens x 11 rows x 256 inputs: its Q8
     codes, scales and expected f16 bits were produced by the reference's Python), then larger shapes with several
-    blocks, negative block scales, bf16 and f32 activations, against the CPU lane: equal bits everywhere."""
+    blocks, negative block scales, bf16 and f32 activations, against the CPU lane: equal bits everywhere.  The last
+    shapes go through every form of the kernel (up to 2, 4, 8 and 16 tokens a pass, two and three CTAs an SM) and through
+    several passes of an odd and an even number of steps, each call twice."""
     op, ctx, k = gpu
     wp, ws, s2 = golden["a16_w_packed"], golden["a16_w_scales"], float(golden["a16_scale2"])
     x16 = torch.from_numpy(golden["a16_activation_f16_bits"].view(np.float16).astype(np.float32))
@@ -417,8 +419,12 @@ def test_weight_only_lane_is_bit_identical(gpu, golden):
     ctx.sync_status()
     assert np.array_equal(y.cpu().numpy().view(np.uint16), golden["a16_expected_f16_bits"])
     w.free()
-    for n_out, n_in, tokens, x_dtype in ((300, 1024, 19, torch.bfloat16), (37, 2560, 8, torch.float32), (130, 256, 1, torch.float32)):
-        packed, scales, scale2 = make_weight(op, ctx, n_out, n_in, seed=n_out, negative_scales=True)
+    for n_out, n_in, tokens, x_dtype in ((300, 1024, 19, torch.bfloat16), (37, 2560, 8, torch.float32), (130, 256, 1, torch.float32),
+                                         (1024, 5120, 17, torch.bfloat16), (520, 5120, 33, torch.float32), (1024, 5120, 64, torch.bfloat16),
+                                         (200, 4096, 40, torch.bfloat16), (520, 5120, 2, torch.bfloat16), (520, 5120, 4, torch.float32),
+                                         (4800, 27648, 2, torch.bfloat16)):
+        packed, scales, scale2 = make_weight(op, ctx, min(n_out, 1024), n_in, seed=n_out, negative_scales=True)
+        packed, scales = np.resize(packed, (n_out, n_in // 2)), np.resize(scales, (n_out, n_in // 16))  # (many rows: the first again)
         w = op.Weight(ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, scale2, None))
         x = (torch.from_numpy(H.lcg_activations(tokens * n_in, seed=tokens).reshape(tokens, n_in)) * 3.0).to(x_dtype)
         x[0, :256] = 0.0   # a block of zeros is skipped
@@ -427,6 +433,9 @@ def test_weight_only_lane_is_bit_identical(gpu, golden):
         k.encode_nvfp4_matmul(w, x.cuda(), y, tokens)
         ctx.sync_status()
         assert np.array_equal(y.cpu().numpy().view(np.uint32), want.astype(np.float32).view(np.uint32)), (n_out, n_in, tokens)
+        again = torch.empty_like(y)
+        k.encode_nvfp4_matmul(w, x.cuda(), again, tokens)
+        assert torch.equal(again, y), (n_out, n_in, tokens)
         w.free()
 
 
