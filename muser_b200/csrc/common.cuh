@@ -206,6 +206,7 @@ muser_cuda_status launch_kquant_matmul(Ctx *, const Weight *w, const Weight *w_u
                                        cudaStream_t);
 cudaError_t launch_kquant_tc(Ctx *, const Weight *w, const void *x, uint32_t x_dtype, void *y, uint32_t y_dtype,
                              uint32_t tokens, const Epilogue &, cudaStream_t);
+bool kquant_tc_holds(const Weight *w, uint32_t tokens, bool two_columns);
 cudaError_t launch_kquant_group(Ctx *, const Weight *const *w, uint32_t n_jobs, const void *x, uint32_t x_dtype, void *const *y, const uint32_t *y_dtype,
                                 uint32_t tokens, const Epilogue *ep, cudaStream_t);
 cudaError_t launch_kquant_mma(Ctx *, const Weight *const *w, const Weight *w_up, uint32_t n_jobs, const void *x, uint32_t x_dtype, void *const *y,

@@ -1259,29 +1259,32 @@ muser_cuda_status launch_kquant_matmul(Ctx *ctx, const Weight *w, const Weight *
                                        cudaStream_t stream) {
     const bool q6 = w->dtype == MUSER_DTYPE_Q6_K, xf32 = x_dtype == MUSER_DTYPE_F32;
     const uint32_t tc_from = ctx->tc_min_tokens[q6 ? 1 : 0]; // above 64: switched off
-    // (the calls that take activations in f16's range, larger magnitudes clamped, whichever kernel serves them)
-    const bool tc_fits = !w_up && w->dtype != MUSER_DTYPE_Q5_K && tokens >= tc_from && tokens <= (xf32 ? 32u : 64u) && w->n_out >= ctx->tc_min_rows;
-    if (tc_fits && takes_tcgen05(w, tokens, xf32 || ep.norm_weight, tc_from)) {
+    // The calls that the tcgen05 kernel can serve take activations in f16's range, larger magnitudes clamped, and Q6_K
+    // operands rounded to 11 bits, whichever of the batched kernels serves them; all others keep exact operands and have no
+    // limit.  (Rows behind a fused norm are f32, two columns a token, whatever x is.)
+    const bool two_columns = xf32 || ep.norm_weight;
+    const bool tc_kind = !w_up && w->dtype != MUSER_DTYPE_Q5_K && tokens >= tc_from && w->n_out >= ctx->tc_min_rows;
+    const bool tc_fits = tc_kind && kquant_tc_holds(w, tokens, two_columns);
+    // (the fused norm's limit at these token counts, whichever kernel serves the call)
+    if (tc_kind && ep.norm_weight && tokens <= (xf32 ? 32u : 64u) && (size_t)tokens * w->n_in * sizeof(float) > ctx->norm_scratch_bytes)
+        return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: tokens x n_in exceeds the context's norm scratch");
+    if (tc_fits && takes_tcgen05(w, tokens, two_columns, tc_from)) {
         const void *xin = x;
         uint32_t xin_dtype = x_dtype;
         if (ep.norm_weight) {
             // the tcgen05 kernel reads its activations through TMA, so the fused input norm runs as a pass of its
             // own into the context's scratch rows (f32), which the projection then reads instead of x
-            const size_t need = (size_t)tokens * w->n_in * sizeof(float);
-            if (need > ctx->norm_scratch_bytes) return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: tokens x n_in exceeds the context's norm scratch");
             muser_cuda_status st = launch_rmsnorm_rows(ctx, x, x_dtype, tokens, w->n_in, ep.norm_weight, ep.norm_eps, ctx->norm_scratch, stream);
             if (st != MUSER_CUDA_OK) return st;
             xin = ctx->norm_scratch;
             xin_dtype = MUSER_DTYPE_F32;
         }
-        if (xin_dtype != MUSER_DTYPE_F32 || tokens <= 32) {
-            Epilogue tail = ep;
-            tail.norm_weight = nullptr;
-            const cudaError_t te = launch_kquant_tc(ctx, w, xin, xin_dtype, y, y_dtype, tokens, tail, stream);
-            if (te != cudaErrorNotSupported) {
-                MUSER_CUDA_TRY(ctx, te);
-                return MUSER_CUDA_OK;
-            }
+        Epilogue tail = ep;
+        tail.norm_weight = nullptr;
+        const cudaError_t te = launch_kquant_tc(ctx, w, xin, xin_dtype, y, y_dtype, tokens, tail, stream);
+        if (te != cudaErrorNotSupported) {
+            MUSER_CUDA_TRY(ctx, te);
+            return MUSER_CUDA_OK;
         }
     }
     if (ep.all_reduce) {
@@ -1304,8 +1307,7 @@ muser_cuda_status launch_kquant_matmul(Ctx *ctx, const Weight *w, const Weight *
         return muser_cuda_all_reduce(reinterpret_cast<muser_cuda_ctx *>(ctx), y, count, y_dtype, stream);
     }
     const size_t xb = xf32 ? 4 : 2, yb = y_dtype == MUSER_DTYPE_BF16 ? 2 : 4;
-    // (the batched kernel rounds Q6_K operands beyond 16 tokens, as the tcgen05 kernel does for the calls it may serve; the
-    // other Q6_K calls keep exact operands, 16 tokens at a time)
+    // (the batched kernel rounds Q6_K operands beyond 16 tokens; Q6_K calls that keep exact ones go 16 tokens at a time)
     uint32_t chunk = takes_mma(ctx, w, tokens) && (tc_fits || !q6) ? 64 : 16;
     for (uint32_t t0 = 0, n; t0 < tokens; t0 += n) {
         n = std::min(chunk, tokens - t0);

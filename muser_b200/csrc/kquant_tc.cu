@@ -864,16 +864,37 @@ static cudaError_t tc_launch(const CUtensorMap &mx, const CUtensorMap &mxs, cons
     return launch_pdl(kquant_tc_kernel<DT, N>, dim3(grid), dim3(S::kThreads), S::kBytes, stream, mx, mxs, a);
 }
 
+// The prepared activations of a call: `n` token columns (f32 activations take two each, f16 head + remainder) of f16
+// values, then their sub-block sums.
+struct TcPrepared {
+    uint32_t n;
+    size_t sums_at, bytes;
+};
+static TcPrepared tc_prepared(const Weight *w, uint32_t cols) {
+    const uint32_t n = cols <= 16 ? 16 : (cols <= 32 ? 32 : 64);
+    const size_t xh_bytes = (size_t)n * w->nsb * 256 * sizeof(__half), xs_bytes = (size_t)n * w->nsb * 16 * sizeof(__half);
+    const size_t xs_off = (xh_bytes + 1023) & ~(size_t)1023;
+    return TcPrepared{n, xs_off, xs_off + xs_bytes};
+}
+
+// Whether the kernel can serve so many tokens: 64 columns, of rows of 32768 inputs at most (fewer columns: longer rows).
+// The limit is the kernel's own and not the scratch's size, because it decides which calls take clamped activations and
+// rounded Q6_K operands.
+bool kquant_tc_holds(const Weight *w, uint32_t tokens, bool two_columns) {
+    constexpr size_t kMaxPrepared = (size_t)64 * 32768 * 2 + (size_t)64 * 2048 * 2 + 4096;
+    const uint32_t cols = two_columns ? 2 * tokens : tokens;
+    return cols <= 64 && tc_prepared(w, cols).bytes <= kMaxPrepared;
+}
+
 // cudaErrorNotSupported: this shape is not served here (the caller falls back to the other kernels).
 cudaError_t launch_kquant_tc(Ctx *ctx, const Weight *w, const void *x, uint32_t x_dtype, void *y, uint32_t y_dtype,
                              uint32_t tokens, const Epilogue &ep, cudaStream_t stream) {
     const bool xf32 = x_dtype == MUSER_DTYPE_F32;
-    const uint32_t cols = xf32 ? 2 * tokens : tokens; // f32 activations take two columns each (f16 head + remainder)
-    if (cols > 64 || !ctx->tc_scratch) return cudaErrorNotSupported;
-    const uint32_t n = cols <= 16 ? 16 : (cols <= 32 ? 32 : 64);
-    const size_t xh_bytes = (size_t)n * w->nsb * 256 * sizeof(__half), xs_bytes = (size_t)n * w->nsb * 16 * sizeof(__half);
-    const size_t xs_off = (xh_bytes + 1023) & ~(size_t)1023;
-    if (xs_off + xs_bytes > ctx->tc_scratch_bytes) return cudaErrorNotSupported;
+    if (!kquant_tc_holds(w, tokens, xf32)) return cudaErrorNotSupported;
+    const TcPrepared prep = tc_prepared(w, xf32 ? 2 * tokens : tokens);
+    if (!ctx->tc_scratch || prep.bytes > ctx->tc_scratch_bytes) return cudaErrorNotSupported;
+    const uint32_t n = prep.n;
+    const size_t xs_off = prep.sums_at;
     __half *xh = reinterpret_cast<__half *>(ctx->tc_scratch);
     __half *xs = reinterpret_cast<__half *>(reinterpret_cast<uint8_t *>(ctx->tc_scratch) + xs_off);
     const dim3 pgrid(w->nsb, n);

@@ -346,6 +346,42 @@ def test_batched_kernel_at_its_edges(gpu, dtype, tokens):
         w.free()
 
 
+@pytest.mark.parametrize("dtype", [O.Q4_K, O.Q6_K])
+@pytest.mark.parametrize("n_in, tokens, x_dtype, norm", [(3072, 33, torch.bfloat16, True), (3072, 48, torch.bfloat16, True), (3072, 64, torch.bfloat16, True),
+                                                         (33024, 64, torch.bfloat16, False), (33024, 32, torch.float32, False)])
+def test_calls_that_the_tcgen05_kernel_cannot_hold_keep_range_and_precision(gpu, dtype, n_in, tokens, x_dtype, norm):
+    """More than 64 columns (the rows behind a fused norm are f32 and take two each) and rows of more than 32768 inputs at
+    64 columns: magnitudes beyond f16's range are not cut, and Q6_K operands stay exact.  Bounds as at the batched kernel's
+    edges: f32 sums for Q4_K; Q6_K goes 16 tokens at a time, the last few through the decode kernel (inputs to 2^-15 of
+    their tile's largest), where operands rounded to 11 bits show 1.1e-4."""
+    op, ctx, k = gpu
+    n_out, eps = 1030, 1e-6
+    raw = H.lcg_weights(dtype, n_out, n_in // 256, seed=n_in + tokens)
+    w = op.Weight(ctx, op.TensorView(raw, dtype, n_in, n_out))
+    deq = O.dequant_blocks(dtype, raw).reshape(n_out, n_in).astype(np.float64)
+    x = torch.from_numpy(H.lcg_activations(tokens * n_in, seed=tokens).reshape(tokens, n_in)).clone()
+    nw = torch.linspace(0.5, 1.5, n_in)
+    if norm:
+        nw[17] = 3.0e6
+    else:
+        x[0, 5], x[tokens - 1, 700] = 3.0e5, -1.0e6
+    x = x.to(x_dtype)
+    want = x.double().numpy()
+    if norm:
+        want = want / np.sqrt((want ** 2).mean(1, keepdims=True) + eps) * nw.double().numpy()
+    assert np.abs(want).max() > 1.0e5
+    want = want @ deq.T
+    y = torch.full((tokens, n_out), float("nan"), dtype=torch.float32, device="cuda")
+    k.encode_quantized_matmul(w, x.cuda(), y, tokens, **(dict(norm_weight=nw.cuda(), norm_eps=eps) if norm else {}))
+    ctx.sync_status()
+    plain = np.ones(tokens, dtype=bool)  # tokens without a large magnitude, on their own: the large ones would hide them
+    if not norm:
+        plain[[0, tokens - 1]] = False
+    got, tol = y.cpu().numpy().astype(np.float64), 3e-6 if dtype == O.Q4_K else 8e-5
+    assert H.rel_l2(got, want) <= tol and H.rel_l2(got[plain], want[plain]) <= tol
+    w.free()
+
+
 def test_grouped_projections_in_one_launch(gpu):
     """q | k | v of one hidden state in one launch (Q4_K, Q4_K and Q6_K rows of different counts), each with its own
     output dtype and epilogue, with and without the shared fused input norm: against the CPU lane and against the
