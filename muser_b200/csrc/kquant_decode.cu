@@ -1241,7 +1241,9 @@ static bool takes_tcgen05(const Weight *w, uint32_t tokens, bool two_columns, ui
 // Up to four projections of one input (or a fused gate/up pair), 1..64 tokens.
 static cudaError_t launch_kquant_batch(Ctx *ctx, const Weight *const *w, const Weight *w_up, uint32_t n_jobs, const void *x, uint32_t x_dtype,
                                        void *const *y, const uint32_t *y_dtype, uint32_t tokens, const Epilogue *ep, bool clamp, cudaStream_t stream) {
-    if (takes_mma(ctx, w[0], tokens)) {
+    bool mma = true;
+    for (uint32_t i = 0; i < n_jobs; ++i) mma = mma && takes_mma(ctx, w[i], tokens);
+    if (mma) {
         const cudaError_t e = launch_kquant_mma(ctx, w, w_up, n_jobs, x, x_dtype, y, y_dtype, tokens, ep, clamp, stream);
         if (e != cudaErrorNotSupported) return e;
     }

@@ -382,6 +382,29 @@ def test_calls_that_the_tcgen05_kernel_cannot_hold_keep_range_and_precision(gpu,
     w.free()
 
 
+def test_a_k_shard_anywhere_in_a_group_keeps_the_decode_kernel(gpu):
+    """K shards of up to 16 tokens stay with the decode kernel, whose partial sums are the same bits as with the
+    all-reduce fused in; in a group that holds for the whole launch, whichever of its weights is the shard."""
+    op, ctx, k = gpu
+    plain = op.Weight(ctx, op.TensorView(H.lcg_weights(O.Q4_K, 200, 4, seed=1), O.Q4_K, 1024, 200))
+    raw = H.lcg_weights(O.Q4_K, 300, 8, seed=2)
+    shard = op.Weight(ctx, op.TensorView(raw, O.Q4_K, 2048, 300), shard=(0, 2, op.SHARD_K))
+    x = torch.from_numpy(H.lcg_activations(16 * 1024, seed=3).reshape(16, 1024)).cuda()
+    y = [torch.empty((16, n), device="cuda") for n in (200, 300)]
+    try:
+        ctx.tuning_set(op.TUNE_DECODE_WARPS, 2)  # a plan that the cost model would not choose
+        k.encode_quantized_matmul(plain, x, y[0], 16)
+    finally:
+        ctx.tuning_set(op.TUNE_DECODE_WARPS, 0)
+    forced = k.last_decode_plan()
+    k.encode_quantized_matmul_group([plain, shard], x, y, 16)
+    ctx.sync_status()
+    assert k.last_decode_plan() != forced
+    want = x.double().cpu().numpy() @ O.dequant_blocks(O.Q4_K, raw).reshape(300, 2048)[:, :1024].astype(np.float64).T
+    assert H.rel_l2(y[1].cpu().numpy(), want) <= REL_L2_TOL
+    plain.free(), shard.free()
+
+
 def test_grouped_projections_in_one_launch(gpu):
     """q | k | v of one hidden state in one launch (Q4_K, Q4_K and Q6_K rows of different counts), each with its own
     output dtype and epilogue, with and without the shared fused input norm: against the CPU lane and against the
