@@ -328,14 +328,13 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1) kquant_mma_kernel(const __g
             issued = i + 1;
             if (++s == a.stages) s = 0, phase ^= 1;
         }
-        if (!ok) {
-            if (lane == 0) {
-                *abort_flag = 1;
-                atomicExch(a.status + 1, 311);
-            }
-            // let the copies in flight land before the shared memory is used for anything else
-            for (uint32_t i = issued > a.stages ? issued - a.stages : 0; i < issued; ++i) mbar_wait_alone(full + 8 * (i % a.stages), (i / a.stages) & 1);
+        if (!ok && lane == 0) {
+            *abort_flag = 1;
+            atomicExch(a.status + 1, 311);
         }
+        // The copies in flight land before the shared memory is used for anything else, also when a consumer gave up
+        // after the last copy was issued (otherwise the consumers have waited for them anyway).
+        for (uint32_t i = issued > a.stages ? issued - a.stages : 0; i < issued; ++i) mbar_wait_alone(full + 8 * (i % a.stages), (i / a.stages) & 1);
     } else {
         // ---------------------------------------------------------------- one row tile per warp
         pdl_wait(); // the epilogue reads and writes what earlier kernels may still use
@@ -361,7 +360,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1) kquant_mma_kernel(const __g
         }
     }
     // ---------------------------------------------------------------- the K slices meet, and out
-    __syncthreads(); // every stage has been read (and on the failure path every copy has landed): the ring becomes scratch
+    __syncthreads(); // every stage has been read, or given up, and every copy has landed: the ring becomes scratch
     const uint32_t rows_cta = W * 16, row_pitch = rows_cta + 4; // (pitch: conflict-free stores)
     float *red = reinterpret_cast<float *>(smem);               // [token][row of the CTA]
     if (warp < W) {
