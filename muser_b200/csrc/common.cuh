@@ -112,18 +112,18 @@ extern thread_local std::string g_create_error;
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Loads of what the kernel before this one wrote, kept behind pdl_wait(): __ldg and loads through const __restrict__
-// pointers count as reads of constant memory, which the compiler may move across it.
+// Loads of what an earlier kernel may have written, kept behind pdl_wait(), which makes its writes visible to every load
+// that follows: __ldg and loads through const __restrict__ pointers count as reads of constant memory, which the compiler
+// may move across it and the hardware may serve from a line fetched before.  The norm weights of a call count too (a caller
+// may make them on the stream); the weight images do not (repacking synchronizes).
 __device__ __forceinline__ uint4 ld_after_wait(const uint4 *p) {
     uint4 v;
     asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
-// The same from L2, past the SM's L1: for kernels that may have been launched while a kernel two back was still running
-// (its reads of the buffer's former contents could sit in L1).
-__device__ __forceinline__ uint4 ld_fresh(const uint4 *p) {
-    uint4 v;
-    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+__device__ __forceinline__ float4 ld_after_wait(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ float ld_after_wait(const float *p) {

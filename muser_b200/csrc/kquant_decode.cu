@@ -153,11 +153,11 @@ __device__ __forceinline__ void stage(const DecArgs &a, uint32_t sb_first, uint3
         const uint32_t tile = task / a.tokens, tok = task % a.tokens;
         const int64_t k = (int64_t)(sb_first + tile) * 256 - (int64_t)a.k_off + 8 * lane;
         if ((uint64_t)k < a.n_in) { // a negative k wraps to a huge value
-            if (a.x_f32) load8<true, true>(reinterpret_cast<const float *>(a.x) + (size_t)tok * a.n_in + k, 0, v);
-            else load8<false, true>(reinterpret_cast<const __nv_bfloat16 *>(a.x) + (size_t)tok * a.n_in + k, 0, v);
+            if (a.x_f32) load8<true>(reinterpret_cast<const float *>(a.x) + (size_t)tok * a.n_in + k, 0, v);
+            else load8<false>(reinterpret_cast<const __nv_bfloat16 *>(a.x) + (size_t)tok * a.n_in + k, 0, v);
             if (a.norm_weight) { // (x * 1/rms) * weight, in that order
                 const float rs = inv_rms[tok];
-                const float4 w0 = __ldg(reinterpret_cast<const float4 *>(a.norm_weight + k)), w1 = __ldg(reinterpret_cast<const float4 *>(a.norm_weight + k) + 1);
+                const float4 w0 = ld_after_wait(reinterpret_cast<const float4 *>(a.norm_weight + k)), w1 = ld_after_wait(reinterpret_cast<const float4 *>(a.norm_weight + k) + 1);
                 const float nw[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], rs), nw[i]);
@@ -543,8 +543,8 @@ __device__ __forceinline__ void run(const DecArgs &a, const DecJob &jb, uint32_t
     __shared__ float norm_red[33];
     if (a.norm_weight) { // every CTA needs the whole row's mean square, whatever its K slice
         for (uint32_t tok = 0; tok < a.tokens; ++tok) {
-            const float r = a.x_f32 ? block_inv_rms<true, true>(reinterpret_cast<const float *>(a.x) + (size_t)tok * a.n_in, a.n_in, a.norm_eps, norm_red)
-                                    : block_inv_rms<false, true>(reinterpret_cast<const __nv_bfloat16 *>(a.x) + (size_t)tok * a.n_in, a.n_in, a.norm_eps, norm_red);
+            const float r = a.x_f32 ? block_inv_rms<true>(reinterpret_cast<const float *>(a.x) + (size_t)tok * a.n_in, a.n_in, a.norm_eps, norm_red)
+                                    : block_inv_rms<false>(reinterpret_cast<const __nv_bfloat16 *>(a.x) + (size_t)tok * a.n_in, a.n_in, a.norm_eps, norm_red);
             if (threadIdx.x == 0) inv_rms[tok] = r;
         }
         __syncthreads();

@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1) kquant_mma_kernel(const __g
 // row's mean square, which costs less than a pass of its own.
 template <int NG, int PLANES, bool XF32>
 __global__ void __launch_bounds__(256) kquant_mma_prepare_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t k_off, uint32_t nsb,
-                                                                 uint32_t clamp, const float *__restrict__ norm_weight, float norm_eps,
+                                                                 uint32_t clamp, const float *norm_weight, float norm_eps,
                                                                  uint8_t *blobs) {
     using B = MmaBlob<NG, PLANES>;
     __shared__ float red[33];
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(256) kquant_mma_prepare_kernel(const void *x, 
     if (tok < tokens && k >= 0 && k < (int64_t)n_in) {
         load8<XF32>(row, (uint32_t)(k / 8), v);
         if (norm_weight) {
-            const float4 w0 = __ldg(reinterpret_cast<const float4 *>(norm_weight + k)), w1 = __ldg(reinterpret_cast<const float4 *>(norm_weight + k) + 1);
+            const float4 w0 = ld_after_wait(reinterpret_cast<const float4 *>(norm_weight + k)), w1 = ld_after_wait(reinterpret_cast<const float4 *>(norm_weight + k) + 1);
             const float nw[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], inv_rms), nw[i]);

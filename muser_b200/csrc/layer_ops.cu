@@ -14,12 +14,7 @@ namespace muser {
 
 // These kernels are a few microseconds of latency between two projections.  Each lets its successor launch as soon as it
 // has its own inputs' go-ahead (pdl_release behind pdl_wait): the projection that follows sets up and starts its weight
-// copies under it.  They work in place, and a successor may sit on an SM whose L1 holds a line from before the update, so
-// rows are read past L1 (ld_fresh; the rows of two blocks may share a line).
-__device__ __forceinline__ float4 ld_row(const float4 *p) {
-    const uint4 v = ld_fresh(reinterpret_cast<const uint4 *>(p));
-    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
-}
+// copies under it.  They work in place: rows are read behind the wait (ld_after_wait).
 
 // Sum over the block of one value per thread; `red` holds 33 floats; every thread gets the total.
 __device__ __forceinline__ float block_sum(float v, float *red) {
@@ -59,12 +54,12 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, 
     for (uint32_t k = 0; k < kHeld; ++k) {
         const uint32_t i = threadIdx.x + k * blockDim.x;
         s[k] = h[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (i < n4) s[k] = ld_row(s4 + i), h[k] = ld_row(h4 + i);
+        if (i < n4) s[k] = ld_after_wait(s4 + i), h[k] = ld_after_wait(h4 + i);
     }
 #pragma unroll
     for (uint32_t k = 0; k < kHeld; ++k) ss += s[k].x * s[k].x + s[k].y * s[k].y + s[k].z * s[k].z + s[k].w * s[k].w;
     for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) {
-        const float4 v = ld_row(s4 + i);
+        const float4 v = ld_after_wait(s4 + i);
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
     const float inv_src = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(ss, red), (float)n) + eps1));
@@ -81,8 +76,8 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, 
         if (i < n4) tail(i, s[k], h[k]);
     }
     for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) {
-        float4 hv = ld_row(h4 + i);
-        tail(i, ld_row(s4 + i), hv);
+        float4 hv = ld_after_wait(h4 + i);
+        tail(i, ld_after_wait(s4 + i), hv);
     }
     if (!output) return;
     const float inv_h = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(sh, red), (float)n) + eps2));
@@ -96,7 +91,7 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, 
         const uint32_t i = threadIdx.x + k * blockDim.x;
         if (i < n4) out(i, h[k]);
     }
-    for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) out(i, ld_row(h4 + i)); // (this thread's own)
+    for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) out(i, ld_after_wait(h4 + i)); // (this thread's own)
 }
 
 // x[i] *= 1 / (1 + exp(-gate[i])), four at a time.
@@ -104,8 +99,8 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *x, const float
     pdl_wait();
     pdl_release();
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
-        float4 v = ld_row(reinterpret_cast<const float4 *>(x) + i);
-        const float4 g = ld_row(reinterpret_cast<const float4 *>(gate) + i);
+        float4 v = ld_after_wait(reinterpret_cast<const float4 *>(x) + i);
+        const float4 g = ld_after_wait(reinterpret_cast<const float4 *>(gate) + i);
         v.x *= __fdiv_rn(1.0f, 1.0f + expf(-g.x)), v.y *= __fdiv_rn(1.0f, 1.0f + expf(-g.y));
         v.z *= __fdiv_rn(1.0f, 1.0f + expf(-g.z)), v.w *= __fdiv_rn(1.0f, 1.0f + expf(-g.w));
         reinterpret_cast<float4 *>(x)[i] = v;
@@ -124,14 +119,14 @@ __global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const floa
     const uint32_t n4 = head_dim / 4;
     float ss = 0.0f;
     for (uint32_t i = lane; i < n4; i += 32) {
-        const float4 v = ld_row(row + i);
+        const float4 v = ld_after_wait(row + i);
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(ss, (float)head_dim) + eps));
     for (uint32_t i = lane; i < n4; i += 32) {
-        const float4 v = ld_row(row + i), ww = w4[i];
+        const float4 v = ld_after_wait(row + i), ww = w4[i];
         row[i] = make_float4(v.x * inv * ww.x, v.y * inv * ww.y, v.z * inv * ww.z, v.w * inv * ww.w);
     }
 }

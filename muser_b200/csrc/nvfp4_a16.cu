@@ -149,8 +149,7 @@ __global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const _
     Block cur, nxt;
     if (part < blocks) fetch(part, nxt);
     pdl_wait(); // the int8 activations come from the kernel before this one; weights are constants
-    // (released behind the wait, so that whatever starts early starts when the kernel before THIS one is complete: no
-    // line of a buffer that is about to be rewritten can enter an SM's L1 after its launch)
+    // (released behind the wait: what starts early finds the kernel before THIS one complete and takes no room from it)
     pdl_release();
     for (uint32_t t0 = 0; t0 < a.tokens; t0 += 2 * PAIRS) {
         if (t0 > 0 && part < blocks) fetch(part, nxt);

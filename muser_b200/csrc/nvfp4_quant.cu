@@ -198,7 +198,7 @@ static cudaError_t launch_rms_rows_sequential(Ctx *ctx, const void *x, uint32_t 
 // (x * inv_rms) * w of one row, quantized group by group by the whole block; rows past `tokens` only clear their scales.
 template <bool XF32>
 __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
-                                                  const float *__restrict__ norm_w, float inv, uint8_t *packed, uint8_t *scales) {
+                                                  const float *norm_w, float inv, uint8_t *packed, uint8_t *scales) {
     const uint32_t groups_pad = kt * 4;
     for (uint32_t g0 = 0; g0 < groups_pad; g0 += blockDim.x) { // blockDim % 4 == 0: quads stay together
         const uint32_t grp = g0 + threadIdx.x;
@@ -210,7 +210,7 @@ __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, 
             const float4 *wp = reinterpret_cast<const float4 *>(norm_w + grp * 16);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float4 w = __ldg(wp + i);
+                const float4 w = ld_after_wait(wp + i);
                 const float *src = i < 2 ? a + 4 * i : b + 4 * (i - 2);
                 r[4 * i] = __fmul_rn(__fmul_rn(src[0], inv), w.x);
                 r[4 * i + 1] = __fmul_rn(__fmul_rn(src[1], inv), w.y);
@@ -238,7 +238,7 @@ __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, 
 constexpr int kNormThreads = 128;
 template <bool XF32>
 __global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
-                                                                           const float *__restrict__ norm_w, float eps, uint32_t keep, uint8_t *packed,
+                                                                           const float *norm_w, float eps, uint32_t keep, uint8_t *packed,
                                                                            uint8_t *scales) {
     extern __shared__ float4 norm_squares[]; // n_in squares, if they fit
     __shared__ float warp_sum[kNormThreads / 32];
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const
 // (1024 values: 11 / 6 at 16 rows, 15 / 7 at 1024).
 template <bool XF32>
 __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
-                                                                    const float *__restrict__ norm_w, const float *inv_rms, uint8_t *packed,
+                                                                    const float *norm_w, const float *inv_rms, uint8_t *packed,
                                                                     uint8_t *scales) {
     pdl_wait();
     pdl_release();

@@ -8,23 +8,17 @@
 namespace muser {
 
 // Eight consecutive activations of one row (which an earlier kernel may just have written) as f32 (the row starts 16-byte
-// aligned and i8 counts groups of eight).  L1: keep the line, for the decode kernel, whose CTAs read a row twice (from L2
-// both times, eight tokens through a layer took 2 us longer).
-template <bool L1>
-__device__ __forceinline__ uint4 load8_piece(const uint4 *p) {
-    if constexpr (L1) return __ldg(p);
-    else return ld_fresh(p);
-}
-template <bool XF32, bool L1 = false>
+// aligned and i8 counts groups of eight).
+template <bool XF32>
 __device__ __forceinline__ void load8(const void *row, uint32_t i8, float (&v)[8]) {
     if constexpr (XF32) {
         const uint4 *p = reinterpret_cast<const uint4 *>(row) + 2 * (size_t)i8;
-        const uint4 a = load8_piece<L1>(p), b = load8_piece<L1>(p + 1);
+        const uint4 a = ld_after_wait(p), b = ld_after_wait(p + 1);
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
     } else {
-        const uint4 raw = load8_piece<L1>(reinterpret_cast<const uint4 *>(row) + i8);
+        const uint4 raw = ld_after_wait(reinterpret_cast<const uint4 *>(row) + i8);
         const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -36,12 +30,12 @@ __device__ __forceinline__ void load8(const void *row, uint32_t i8, float (&v)[8
 
 // 1/sqrt(mean(x^2) + eps) of one row of n values (n % 8 == 0), computed by the whole block; `red` holds 33 floats
 // of shared memory.  Every thread of the block must call it, and all get the result.
-template <bool XF32, bool L1 = false>
+template <bool XF32>
 __device__ __forceinline__ float block_inv_rms(const void *row, uint32_t n, float eps, float *red) {
     float ss = 0.0f;
     for (uint32_t i = threadIdx.x; i < n / 8; i += blockDim.x) {
         float v[8];
-        load8<XF32, L1>(row, i, v);
+        load8<XF32>(row, i, v);
 #pragma unroll
         for (int k = 0; k < 8; ++k) ss = fmaf(v[k], v[k], ss);
     }
