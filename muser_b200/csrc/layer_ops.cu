@@ -12,9 +12,11 @@
 
 namespace muser {
 
-// These kernels are a few microseconds of latency between two projections.  Each lets its successor launch as soon as it
-// has its own inputs' go-ahead (pdl_release behind pdl_wait): the projection that follows sets up and starts its weight
-// copies under it.  They work in place: rows are read behind the wait (ld_after_wait).
+// These kernels are a few microseconds of latency between two projections.  Up to one block an SM (decode: a row per token)
+// each lets its successor launch as soon as it has its own inputs' go-ahead (`early`: pdl_release behind pdl_wait): the
+// projection that follows sets up and starts its weight copies under it.  Larger grids do not: the successor's blocks only
+// took the slots of their own later ones (head norm, gate and tail of 512 rows of 2048, us: 12.6 with the release, 10.6
+// without; of 16 rows of 5120: 6.0 and 6.9).  They work in place: rows are read behind the wait (ld_after_wait).
 
 // Sum over the block of one value per thread; `red` holds 33 floats; every thread gets the total.
 __device__ __forceinline__ float block_sum(float v, float *red) {
@@ -35,20 +37,23 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
 }
 
 // One block per token row.  n % 4 == 0; rows 16-byte aligned.
+// HELD: the row's first kHeld pieces per thread (8192 values a block of 512) stay in registers from one fetch: reading them
+// again for each of the three passes is two more trips to L2 in a kernel that, with one block an SM, is nothing but such
+// trips (16 rows of 5120 values: 2.8 us against 3.8).  The registers leave an SM room for one block, so more rows read again
+// and have their trips covered by other blocks (512 rows of 2048: 7.2 us held, 5.7 read again).
+template <bool HELD>
 __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, const float *src, float *output,
                                                                  const float *__restrict__ w1, const float *__restrict__ w2, uint32_t n, float eps1,
                                                                  float eps2) {
     __shared__ float red[33];
     pdl_wait();
-    pdl_release();
+    if constexpr (HELD) pdl_release();
     const uint32_t n4 = n / 4;
     float4 *h4 = reinterpret_cast<float4 *>(hidden + (size_t)blockIdx.x * n);
     const float4 *s4 = reinterpret_cast<const float4 *>(src + (size_t)blockIdx.x * n);
     const float4 *w14 = reinterpret_cast<const float4 *>(w1), *w24 = reinterpret_cast<const float4 *>(w2);
-    // The row's first kHeld pieces per thread (8192 values a block of 512) stay in registers from one fetch: reading them
-    // again for each of the three passes was two more trips to L2 in a kernel that is nothing but such trips.
-    constexpr uint32_t kHeld = 4;
-    float4 s[kHeld], h[kHeld];
+    constexpr uint32_t kHeld = HELD ? 4 : 0;
+    float4 s[kHeld + 1], h[kHeld + 1];
     float ss = 0.0f;
 #pragma unroll
     for (uint32_t k = 0; k < kHeld; ++k) {
@@ -95,9 +100,9 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, 
 }
 
 // x[i] *= 1 / (1 + exp(-gate[i])), four at a time.
-__global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *x, const float *gate, size_t n4) {
+__global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *x, const float *gate, size_t n4, bool early) {
     pdl_wait();
-    pdl_release();
+    if (early) pdl_release();
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
         float4 v = ld_after_wait(reinterpret_cast<const float4 *>(x) + i);
         const float4 g = ld_after_wait(reinterpret_cast<const float4 *>(gate) + i);
@@ -109,9 +114,9 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *x, const float
 
 // One warp per (token, head): x <- x * 1/sqrt(mean(x^2) + eps) * w, head_dim % 4 == 0, head_dim <= 1024.
 __global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const float *__restrict__ w, float eps, uint32_t heads_total,
-                                                            uint32_t head_dim) {
+                                                            uint32_t head_dim, bool early) {
     pdl_wait();
-    pdl_release();
+    if (early) pdl_release();
     const uint32_t head = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (head >= heads_total) return;
     float4 *row = reinterpret_cast<float4 *>(x + (size_t)head * head_dim);
@@ -134,21 +139,23 @@ __global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const floa
 muser_cuda_status launch_norm_residual_norm(Ctx *ctx, float *hidden, const float *src, float *output, const float *w1, const float *w2,
                                             uint32_t tokens, uint32_t n, float eps1, float eps2, cudaStream_t stream) {
     const unsigned threads = n / 4 >= 512 ? 512 : n / 4 >= 256 ? 256 : 128;
-    MUSER_CUDA_TRY(ctx, launch_pdl(norm_residual_norm_kernel, dim3(tokens), dim3(threads), 0, stream, hidden, src, output, w1, w2, n, eps1, eps2));
+    const auto kernel = tokens <= (uint32_t)ctx->sm_count ? norm_residual_norm_kernel<true> : norm_residual_norm_kernel<false>;
+    MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens), dim3(threads), 0, stream, hidden, src, output, w1, w2, n, eps1, eps2));
     return MUSER_CUDA_OK;
 }
 
 muser_cuda_status launch_sigmoid_gate(Ctx *ctx, float *x, const float *gate, size_t count, cudaStream_t stream) {
     const size_t n4 = count / 4;
     const unsigned blocks = (unsigned)std::min<size_t>((n4 + 255) / 256, (size_t)ctx->sm_count * 8);
-    MUSER_CUDA_TRY(ctx, launch_pdl(sigmoid_gate_kernel, dim3(blocks), dim3(256), 0, stream, x, gate, n4));
+    MUSER_CUDA_TRY(ctx, launch_pdl(sigmoid_gate_kernel, dim3(blocks), dim3(256), 0, stream, x, gate, n4, blocks <= (unsigned)ctx->sm_count));
     return MUSER_CUDA_OK;
 }
 
 muser_cuda_status launch_head_rms_norm(Ctx *ctx, float *x, const float *w, float eps, uint32_t tokens, uint32_t heads, uint32_t head_dim,
                                        cudaStream_t stream) {
     const uint32_t total = tokens * heads;
-    MUSER_CUDA_TRY(ctx, launch_pdl(head_rms_norm_kernel, dim3((total + 7) / 8), dim3(256), 0, stream, x, w, eps, total, head_dim));
+    const uint32_t blocks = (total + 7) / 8;
+    MUSER_CUDA_TRY(ctx, launch_pdl(head_rms_norm_kernel, dim3(blocks), dim3(256), 0, stream, x, w, eps, total, head_dim, blocks <= (uint32_t)ctx->sm_count));
     return MUSER_CUDA_OK;
 }
 
