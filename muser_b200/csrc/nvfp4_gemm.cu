@@ -83,6 +83,7 @@ struct GemmArgs {
     void *grp_y[4];
     uint32_t grp_n_out[4];
     float grp_scale2[4];
+    uint32_t grp_slices[4]; // SLICED form: slices that a projection's K is summed in
 };
 
 // Output tile number -> (token tile, weight-row tile).  Tiles are numbered group by group: a group is `group_m` token
@@ -253,12 +254,17 @@ __device__ __forceinline__ float4 split_load(uint32_t addr) {
 // outputs only (no fused tail, row scale or residual).
 // SPLIT: the slabs of one output tile are cut between the CTAs of a cluster (gemm_ksplit()): each leaves its f32 sums in
 // its shared memory, and all of them add the slices up in slice order, every CTA finishing a share of the tile's outputs.
+// SLICED (SPLIT with GROUP): a group that holds weights which SPLIT cuts when they are called alone.  Tiles are whole, but
+// the accumulator starts anew with every slice of such a weight and the epilogue adds the slices up as SPLIT does: the bits
+// of the single call in the group's one launch.  (Launched one by one the group took up to twice as long: 12288 + 1024 +
+// 1024 rows of 12288 inputs at 200 tokens 31 -> 62 us.)
 template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, bool SPLIT = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_b3,
                   const __grid_constant__ CUtensorMap map_b4, const GemmArgs g) {
     constexpr uint32_t kTileRows = DUAL ? BN / 2 : BN; // output columns (weight rows) per tile
+    constexpr bool CLUSTER = SPLIT && !GROUP, SLICED = SPLIT && GROUP;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // swizzled tiles need 1024-byte alignment
     uint8_t *aligned = smem_raw + (base - smem_u32(smem_raw));
@@ -271,13 +277,13 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t m_tiles = (g.tokens + BM - 1) / BM, n_tiles_total = g.n_tiles * m_tiles;
-    // This CTA's tiles and, of each, its slabs.  (Macros, so that the other forms compile as if SPLIT did not exist: with
+    // This CTA's tiles and, of each, its slabs.  (Macros, so that the other forms compile as if CLUSTER did not exist: with
     // variables in their place the roles' lambdas kept them in registers and every form's slab took 10 % longer.)
-#define GEMM_SLICE (SPLIT ? blockIdx.x % g.ksplit : 0u)
-#define GEMM_TILE_FIRST (SPLIT ? blockIdx.x / g.ksplit : blockIdx.x)
-#define GEMM_TILE_STEP (SPLIT ? n_tiles_total : gridDim.x)
-#define GEMM_KT_FIRST (SPLIT ? g.k_tiles * GEMM_SLICE / g.ksplit : 0u)
-#define GEMM_KT_END (SPLIT ? g.k_tiles * (GEMM_SLICE + 1) / g.ksplit : g.k_tiles)
+#define GEMM_SLICE (CLUSTER ? blockIdx.x % g.ksplit : 0u)
+#define GEMM_TILE_FIRST (CLUSTER ? blockIdx.x / g.ksplit : blockIdx.x)
+#define GEMM_TILE_STEP (CLUSTER ? n_tiles_total : gridDim.x)
+#define GEMM_KT_FIRST (CLUSTER ? g.k_tiles * GEMM_SLICE / g.ksplit : 0u)
+#define GEMM_KT_END (CLUSTER ? g.k_tiles * (GEMM_SLICE + 1) / g.ksplit : g.k_tiles)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -392,7 +398,22 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
+                uint32_t slices = 1, slice = 0, slice_first = 0; // SLICED only
+                if constexpr (SLICED) {
+                    uint32_t tile_m, tile_n;
+                    tile_coords(tile, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
+                    slices = g.grp_slices[(tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3])];
+                }
                 for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
+                    if constexpr (SLICED) {
+                        if (kt == g.k_tiles * (slice + 1) / slices) { // (never true at the last slice's end, where the loop ends)
+                            mma_commit_elect(bar_acc_full);
+                            PROF_BEGIN ok = mbar_wait_warp(bar_acc_empty, local & 1, abort_flag); PROF_END(0)
+                            if (!ok) break;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            ++local, ++slice, slice_first = kt;
+                        }
+                    }
                     const uint32_t s = it % kStages, round = it / kStages;
                     PROF_BEGIN ok = mbar_wait_warp(bar_full + 8 * s, round & 1, abort_flag); PROF_END(1)
                     if (!ok) break;
@@ -410,7 +431,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         tmem_cp_scales_elect(sf + 4 * kb, scale_desc(sfa + 512 * kb));
                         tmem_cp_scales_elect(sf + 16 + 8 * kb, scale_desc(sfb + 512 * kb));
                         tmem_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
-                        mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, ((kt - GEMM_KT_FIRST) | kb) != 0);
+                        mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, ((kt - (SLICED ? slice_first : GEMM_KT_FIRST)) | kb) != 0);
                     }
                     mma_commit_elect(bar_empty + 8 * s); // the stage may be overwritten once these MMAs have read it
                 }
@@ -441,10 +462,12 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             uint32_t n_out = g.n_out; // (of this tile's projection)
             void *y_out = g.y;
             float scale2 = g.scale2;
+            uint32_t slices = 1; // SLICED only
             if constexpr (GROUP) {
                 const uint32_t p = (tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3]);
                 tile_n -= g.grp_tile0[p];
                 n_out = g.grp_n_out[p], y_out = g.grp_y[p], scale2 = g.grp_scale2[p];
+                if constexpr (SLICED) slices = g.grp_slices[p];
             }
             const uint32_t tok = tile_m * BM + quad * 32 + lane, col0 = part * kPartCols, out0 = tile_n * kOutCols + col0;
             const bool live = tok < g.tokens && out0 < n_out;
@@ -463,7 +486,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 if (wide_res) asm volatile("prefetch.global.L2 [%0];" ::"l"(res_at + 64));
             }
             // (with a sleep between the polls: sixteen polling warps cost the SM power that the products could use)
-            const bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64));
+            bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64));
             if (!ok) {
                 if (lane == 0) {
                     *abort_flag = 1;
@@ -483,10 +506,43 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             for (uint32_t s = 0; s < 2; ++s) // fused form: strip 0 is gate columns, strip 1 the same columns of up
                 tmem_ld32(lane_base + col0 + s * (DUAL ? kOutCols : 32), r[s]);
             tmem_ld_wait();
+            if constexpr (SLICED) {
+                if (slices > 1) { // (as SPLIT adds: from zero, in slice order)
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) r[i >> 5][i & 31] = __float_as_uint(0.0f + __uint_as_float(r[i >> 5][i & 31]));
+                }
+                for (uint32_t slice = 1; slice < slices; ++slice) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
+                    ++local;
+                    ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int c = 0; c < 64; c += 8) { // (eight columns at a time: the sums so far fill the registers)
+                        uint32_t v[8];
+                        tmem_ld8(lane_base + col0 + c, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            uint32_t &sum = r[(c + i) >> 5][(c + i) & 31];
+                            sum = __float_as_uint(__uint_as_float(sum) + __uint_as_float(v[i]));
+                        }
+                    }
+                }
+                if (!ok) {
+                    if (lane == 0) {
+                        *abort_flag = 1;
+                        atomicCAS(g.status + 1, 0, 103);
+                    }
+                    break;
+                }
+            }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
-            if constexpr (SPLIT) {
+            if constexpr (CLUSTER) {
                 // (every stage has been consumed: the ring is scratch now)
                 if (tok < g.tokens) {
                     float4 *row = reinterpret_cast<float4 *>(aligned + ((quad * 32 + lane) * kRedPitch + col0) * 4);
@@ -565,7 +621,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     }
-    if constexpr (SPLIT) {
+    if constexpr (CLUSTER) {
         split_barrier();
         pdl_wait(); // (every warp stores here)
         uint32_t tile_m, tile_n;
@@ -1338,15 +1394,6 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
 // Up to four projections of the same quantized activations in one launch (GROUP form of the kernel).
 muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uint32_t n, const uint8_t *x_packed, const uint8_t *x_scales,
                                           void *const *ys, uint32_t y_dtype, uint32_t tokens, cudaStream_t stream) {
-    bool split = false;
-    for (uint32_t p = 0; p < n; ++p) split = split || gemm_ksplit(ctx, ws[p], tokens) > 1;
-    if (split) {
-        for (uint32_t p = 0; p < n; ++p) {
-            const muser_cuda_status st = launch_nvfp4_gemm(ctx, ws[p], x_packed, x_scales, ys[p], y_dtype, tokens, Epilogue{}, stream);
-            if (st != MUSER_CUDA_OK) return st;
-        }
-        return MUSER_CUDA_OK;
-    }
     const Weight *w0 = ws[0];
     CUtensorMap map_a;
     if (!make_map(&map_a, x_packed, tokens, w0->n_in / 2, box_tokens(tokens)))
@@ -1363,6 +1410,7 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     g.out_scale = 1.0f;
     g.inv_input_scale = 1.0f / w0->input_scale_inv;
     uint32_t tiles_n = 0;
+    bool sliced = false;
     for (uint32_t p = 0; p < 4; ++p) {
         g.grp_tile0[p] = tiles_n;
         if (p >= n) continue;
@@ -1370,6 +1418,8 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
         g.grp_y[p] = ys[p];
         g.grp_n_out[p] = (uint32_t)ws[p]->n_out;
         g.grp_scale2[p] = ws[p]->scale2;
+        g.grp_slices[p] = ctx->nvfp4_pair ? 1 : gemm_ksplit(ctx, ws[p], tokens); // (the paired kernel, which serves single calls then, never splits)
+        sliced = sliced || g.grp_slices[p] > 1;
         tiles_n += (uint32_t)(ws[p]->n_out_pad / BN);
     }
     g.grp_tile0[4] = tiles_n;
@@ -1386,9 +1436,9 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     for (uint32_t p = 0; p < 4; ++p) maps[p] = reinterpret_cast<const CUtensorMap *>(ws[p < n ? p : 0]->tmap_cache);
     const uint32_t tiles = tiles_n * ((tokens + BM - 1) / BM);
     const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
-    const void *kfn = reinterpret_cast<const void *>(nvfp4_gemm_kernel<false, false, false, true>);
-    MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(kfn, ctx->device, kSmemBytes));
-    MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, false, false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, *maps[0], *maps[1], *maps[2], *maps[3], g));
+    const auto kernel = sliced ? nvfp4_gemm_kernel<false, false, false, true, true> : nvfp4_gemm_kernel<false, false, false, true>;
+    MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes));
+    MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, *maps[0], *maps[1], *maps[2], *maps[3], g));
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
     return MUSER_CUDA_OK;
 }
