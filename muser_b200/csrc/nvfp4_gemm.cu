@@ -141,28 +141,54 @@ __device__ __forceinline__ void st_32b(void *p, const uint32_t (&r)[8]) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
-// Sixteen neighbouring 16-bit outputs in one 32-byte store (a lane's row is its own: narrower stores write half
-// sectors), with the residual, fetched the same way, added in f32.
-template <typename T>
-__device__ __forceinline__ void store_16_wide(const float *v, T *y, const uint32_t *res) {
-    uint32_t o[8];
+// 64 neighbouring bytes of outputs, 16 f32 or 32 16-bit ones, in 32-byte stores where the row's pieces are whole sectors
+// (`wide`; a lane's row is its own: narrower stores write half sectors) and in 16-byte stores otherwise, with the residual,
+// fetched the same way (ld_64), added in f32.
+__device__ __forceinline__ void ld_64(const void *p, bool wide, uint32_t (&r)[2][8]) {
+    const uint8_t *at = reinterpret_cast<const uint8_t *>(p);
+    if (wide) {
+        ld_32b(at, r[0]), ld_32b(at + 32, r[1]);
+        return;
+    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        float a = v[2 * i], b = v[2 * i + 1];
-        if constexpr (std::is_same<T, __half>::value) {
-            if (res) {
-                const float2 r = __half22float2(*reinterpret_cast<const __half2 *>(res + i));
-                a += r.x, b += r.y;
+    for (int i = 0; i < 4; ++i) {
+        const uint4 v = ld_after_wait(reinterpret_cast<const uint4 *>(at) + i);
+        uint32_t *o = &r[i >> 1][4 * (i & 1)];
+        o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void st_64(const float *v, T *y, bool has_res, const uint32_t (&res)[2][8], bool wide) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t w = res[h][i];
+            if constexpr (sizeof(T) == 4) {
+                o[i] = __float_as_uint(has_res ? v[8 * h + i] + __uint_as_float(w) : v[8 * h + i]);
+            } else {
+                float a = v[16 * h + 2 * i], b = v[16 * h + 2 * i + 1];
+                if constexpr (std::is_same<T, __half>::value) {
+                    const float2 r = __half22float2(*reinterpret_cast<const __half2 *>(&w));
+                    if (has_res) a += r.x, b += r.y;
+                    const __half2 packed = __floats2half2_rn(a, b);
+                    o[i] = *reinterpret_cast<const uint32_t *>(&packed);
+                } else {
+                    if (has_res) a += __uint_as_float(w << 16), b += __uint_as_float(w & 0xFFFF0000u);
+                    const __nv_bfloat162 packed = __floats2bfloat162_rn(a, b);
+                    o[i] = *reinterpret_cast<const uint32_t *>(&packed);
+                }
             }
-            const __half2 h = __floats2half2_rn(a, b);
-            o[i] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+        uint8_t *at = reinterpret_cast<uint8_t *>(y) + 32 * h;
+        if (wide) {
+            st_32b(at, o);
         } else {
-            if (res) a += __uint_as_float(res[i] << 16), b += __uint_as_float(res[i] & 0xFFFF0000u);
-            const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-            o[i] = *reinterpret_cast<const uint32_t *>(&h);
+            reinterpret_cast<uint4 *>(at)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            reinterpret_cast<uint4 *>(at)[1] = make_uint4(o[4], o[5], o[6], o[7]);
         }
     }
-    st_32b(y, o);
 }
 // One strip of 32 (or 8) columns of one accumulator row: scale, fuse, convert, store (16-byte stores when the row allows).
 template <typename T, int N = 32>
@@ -471,19 +497,22 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             const uint32_t tok = tile_m * BM + quad * 32 + lane, col0 = part * kPartCols, out0 = tile_n * kOutCols + col0;
             const bool live = tok < g.tokens && out0 < n_out;
-            // 16-bit rows whose 16-value pieces are whole 32-byte sectors
-            const bool wide = live && g.y_dtype != MUSER_DTYPE_F32 && (n_out & 15) == 0 && out0 + kPartCols <= n_out &&
-                              ((reinterpret_cast<uintptr_t>(y_out) | reinterpret_cast<uintptr_t>(g.residual)) & 31) == 0;
-            // the residual is fetched while the products still run: the first strip's to registers, the second's to L2
+            // rows whose pieces lie on 16 bytes, and on whole 32-byte sectors
+            const bool is_f32 = g.y_dtype == MUSER_DTYPE_F32;
+            const uint32_t align = (uint32_t)(reinterpret_cast<uintptr_t>(y_out) | reinterpret_cast<uintptr_t>(g.residual));
+            const bool vec_ok = (n_out & 7) == 0 && (align & 15) == 0, vec = vec_ok && live && out0 + kPartCols <= n_out;
+            const bool wide = (align & 31) == 0 && (is_f32 || (n_out & 15) == 0);
+            // the residual is fetched while the products still run: its first 64 bytes to registers, the others to L2
             uint32_t res[2][8];
-            const bool wide_res = !DUAL && !GROUP && wide && g.residual;
-            const uint8_t *res_at = reinterpret_cast<const uint8_t *>(g.residual) + ((size_t)tok * n_out + out0) * 2;
-            auto load_res = [&](uint32_t s) {
-                if (wide_res) ld_32b(res_at + 64 * s, res[0]), ld_32b(res_at + 64 * s + 32, res[1]);
+            const bool vec_res = !DUAL && !GROUP && vec && g.residual;
+            const uint8_t *res_at = reinterpret_cast<const uint8_t *>(g.residual) + ((size_t)tok * n_out + out0) * (is_f32 ? 4 : 2);
+            auto load_res = [&](uint32_t piece) {
+                if (vec_res) ld_64(res_at + 64 * piece, wide, res);
             };
             if constexpr (!DUAL && !GROUP) {
                 load_res(0);
-                if (wide_res) asm volatile("prefetch.global.L2 [%0];" ::"l"(res_at + 64));
+                if (vec_res)
+                    for (uint32_t at = 64; at < kPartCols * (is_f32 ? 4 : 2); at += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(res_at + at));
             }
             // (with a sleep between the polls: sixteen polling warps cost the SM power that the products could use)
             bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64));
@@ -496,7 +525,6 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float rs = (g.row_scale && tok < g.tokens) ? g.row_scale[tok] : 1.0f;
-            const bool vec_ok = (n_out & 7) == 0;
             const uint32_t lane_base = tmem + ((quad * 32) << 16);
             // All of this warp's part of the accumulator goes to registers first (64 values a thread) and the
             // accumulator is handed back at once: the MMA warp cannot start the next tile before that, so nothing
@@ -582,7 +610,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 const uint32_t n0 = out0 + 32 * s;
                 if (tok >= g.tokens || n0 >= n_out) continue;
                 if constexpr (!DUAL && !GROUP) {
-                    if (s > 0) load_res(s);
+                    if (s > 0) load_res(is_f32 ? 2 * s : s);
                 }
                 const size_t o = (size_t)tok * n_out + n0;
                 const uint32_t valid = min(32u, n_out - n0);
@@ -598,26 +626,21 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     v[i] *= rs;
                     if constexpr (TAIL) v[i] = logit_tail(v[i], g.out_scale, g.softcap);
                 }
-                if (g.y_dtype == MUSER_DTYPE_F32) {
-                    store_strip<float>(v, reinterpret_cast<float *>(y_out) + o,
-                                       g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
-                } else if (g.y_dtype == MUSER_DTYPE_BF16) {
-                    __nv_bfloat16 *y = reinterpret_cast<__nv_bfloat16 *>(y_out) + o;
-                    if (wide) {
-                        store_16_wide(v, y, wide_res ? res[0] : nullptr);
-                        store_16_wide(v + 16, y + 16, wide_res ? res[1] : nullptr);
+                auto store = [&](auto *y) {
+                    using T = std::remove_pointer_t<decltype(y)>;
+                    if (!vec) {
+                        store_strip<T>(v, y + o, g.residual ? reinterpret_cast<const T *>(g.residual) + o : nullptr, valid, vec_ok);
+                    } else if constexpr (sizeof(T) == 4) {
+                        st_64(v, y + o, vec_res, res, wide);
+                        if constexpr (!DUAL && !GROUP) load_res(2 * s + 1);
+                        st_64(v + 16, y + o + 16, vec_res, res, wide);
                     } else {
-                        store_strip<__nv_bfloat16>(v, y, g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
+                        st_64(v, y + o, vec_res, res, wide);
                     }
-                } else {
-                    __half *y = reinterpret_cast<__half *>(y_out) + o;
-                    if (wide) {
-                        store_16_wide(v, y, wide_res ? res[0] : nullptr);
-                        store_16_wide(v + 16, y + 16, wide_res ? res[1] : nullptr);
-                    } else {
-                        store_strip<__half>(v, y, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
-                    }
-                }
+                };
+                if (is_f32) store(reinterpret_cast<float *>(y_out));
+                else if (g.y_dtype == MUSER_DTYPE_BF16) store(reinterpret_cast<__nv_bfloat16 *>(y_out));
+                else store(reinterpret_cast<__half *>(y_out));
             }
         }
     }
@@ -643,7 +666,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], g.scale2), g.inv_input_scale) * rs;
             const size_t o = (size_t)tok * g.n_out + n0;
             const uint32_t valid = min(8u, g.n_out - n0);
-            const bool vec_ok = (g.n_out & 7) == 0;
+            const bool vec_ok = (g.n_out & 7) == 0 && ((reinterpret_cast<uintptr_t>(g.y) | reinterpret_cast<uintptr_t>(g.residual)) & 15) == 0;
             if (g.y_dtype == MUSER_DTYPE_F32)
                 store_strip<float, 8>(v, reinterpret_cast<float *>(g.y) + o, g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
             else if (g.y_dtype == MUSER_DTYPE_BF16)
@@ -956,7 +979,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tok = (2 * tile_m + rank) * BM + quad * 32 + lane;
             const float rs = (g.row_scale && tok < g.tokens) ? g.row_scale[tok] : 1.0f;
-            const bool vec_ok = (g.n_out & 7) == 0;
+            const bool vec_ok = (g.n_out & 7) == 0 && ((reinterpret_cast<uintptr_t>(g.y) | reinterpret_cast<uintptr_t>(g.residual)) & 15) == 0;
             const uint32_t lane_base = tmem + ((quad * 32) << 16), col0 = part * kPartCols;
             uint32_t r[4][32]; // as in the single-CTA kernel: everything to registers, then the accumulator goes back
 #pragma unroll

@@ -323,6 +323,72 @@ def test_long_rows_split_between_the_ctas_of_a_cluster(gpu, n_out, n_in, tokens)
     w.free()
 
 
+@pytest.mark.parametrize("shapes, tokens", [((9600, 300, 37), 131), ((300, 9600), 250), ((700, 37, 300, 256), 16)])
+def test_groups_of_long_rows_sum_in_the_single_calls_slices(gpu, shapes, tokens):
+    """A group of long rows is one launch of whole tiles, some of its weights summed in the slices that the single call
+    splits them into, in different numbers of slices, beside weights that are never split: equal bits."""
+    op, ctx, k = gpu
+    from muser_b200 import synth
+    n_in = 12352  # (49 slabs, the last one short)
+    x = synth.normal_activations(tokens, n_in, seed=11)
+    isi = synth.activation_input_scale_inv(x)
+    ws = []
+    for i, n_out in enumerate(shapes):
+        packed, scales, scale2 = make_weight(op, ctx, min(n_out, 700), n_in, seed=40 + i, negative_scales=(i == 0))
+        packed, scales = np.resize(packed, (n_out, n_in // 2)), np.resize(scales, (n_out, n_in // 16))
+        ws.append(op.Weight(ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, scale2, isi)))
+    q = k.quantize_nvfp4_activation(x.cuda(), isi)
+    for dt in (torch.float32, torch.bfloat16):
+        alone, grouped = ([torch.full((tokens, n), float("nan"), dtype=dt, device="cuda") for n in shapes] for _ in range(2))
+        for w, y in zip(ws, alone):
+            k.encode_nvfp4_prequant(w, *q, y, tokens)
+        k.encode_nvfp4_group_prequant(ws, *q, grouped, tokens)
+        ctx.sync_status()
+        bits = torch.int32 if dt == torch.float32 else torch.int16
+        for a, b in zip(alone, grouped):
+            assert not torch.isnan(a).any() and torch.equal(a.view(bits), b.view(bits))
+    for w in ws:
+        w.free()
+
+
+@pytest.mark.parametrize("n_out", [37, 40, 264, 304, 512])
+@pytest.mark.parametrize("dtype, tol", [(torch.float32, 3e-6), (torch.float16, 3e-4), (torch.bfloat16, 3e-3)])
+def test_outputs_and_residuals_at_any_alignment(gpu, n_out, dtype, tol):
+    """Rows of whole 32-byte sectors, of 16-byte pieces and of neither, full and partial tiles, outputs and residuals that
+    start on a sector, in the middle of one, and (the residual) off any vector: values and no byte beyond, against exact
+    products (f32 sums: some 1e-6 of the norm; f16 and bf16 round to 2^-12 and 2^-9)."""
+    op, ctx, k = gpu
+    from muser_b200 import synth
+    n_in, tokens = 512, 130
+    packed, scales, scale2 = make_weight(op, ctx, n_out, n_in, seed=n_out)
+    x = synth.normal_activations(tokens, n_in, seed=5)
+    isi = synth.activation_input_scale_inv(x)
+    w = op.Weight(ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, scale2, isi))
+    xp, xs = synth.quantize_nvfp4(x.float(), isi)
+    want = torch.from_numpy(O.dequant_nvfp4(xp.numpy(), xs.numpy(), 1.0).astype(np.float64) @ O.dequant_nvfp4(packed, scales, scale2).astype(np.float64).T / isi)
+    q = k.quantize_nvfp4_activation(x.cuda(), isi)
+    count, size = tokens * n_out, dtype.itemsize
+    values = torch.randn(count).to(dtype)
+
+    def at(offset, fill=None):  # a [tokens][n_out] tensor that starts `offset` bytes behind an aligned address
+        whole = torch.full((count + 64,), 7.0, dtype=dtype, device="cuda")
+        part = whole[offset // size: offset // size + count].view(tokens, n_out)
+        if fill is not None:
+            part.copy_(fill.view(tokens, n_out))
+        return whole, part
+
+    for y_off, res_off in ((0, None), (16, None), (0, 0), (16, 0), (0, 16), (16, 16), (0, size)):
+        whole, y = at(y_off)
+        res = None if res_off is None else at(res_off, values)[1]
+        k.encode_nvfp4_prequant(w, *q, y, tokens, residual=res)
+        ctx.sync_status()
+        ref = want if res is None else want + values.double().view(tokens, n_out)
+        assert H.rel_l2(y.double().cpu().numpy(), ref.numpy()) <= tol, (y_off, res_off)
+        rest = torch.cat([whole[: y_off // size], whole[y_off // size + count:]])
+        assert (rest == 7.0).all(), (y_off, res_off)
+    w.free()
+
+
 @pytest.mark.parametrize("n_in", [64, 1088, 5120, 12352])
 @pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
 def test_fused_norm_adds_the_squares_front_to_back(gpu, n_in, x_dtype):
