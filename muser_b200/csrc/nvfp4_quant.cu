@@ -176,11 +176,18 @@ __global__ void __launch_bounds__(kRmsThreads) rms_rows_staged_kernel(const void
         inv_rms[row0 + threadIdx.x] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)n_in), eps)));
 }
 
+// Up to so many rows of bf16.  f32 rows carry twice the bytes per value and the crew falls behind the chains earlier
+// (norm + quantize, us, staged / one warp per 32 chains: 2048 values 28 / 30 at 4096 rows; 5120 values 48 / 59 at 2048,
+// 73 / 66 at 3072; 8192 values 77 / 86 at 1536, 98 / 92 at 2048; 27648 values 234 / 282 at 1536, 339 / 305 at 2048).
 constexpr uint32_t kRmsStagedRows = 4096;
+static uint32_t rms_staged_rows(uint32_t x_dtype, uint32_t n_in) {
+    if (x_dtype != MUSER_DTYPE_F32 || n_in <= 2048) return kRmsStagedRows;
+    return n_in <= 5120 ? 2048 : 1536;
+}
 
 static cudaError_t launch_rms_rows_sequential(Ctx *ctx, const void *x, uint32_t x_dtype, uint32_t tokens, uint32_t n_in, float eps,
                                               float *inv_rms, cudaStream_t stream) {
-    if (tokens <= kRmsStagedRows) {
+    if (tokens <= rms_staged_rows(x_dtype, n_in)) {
         const auto kernel = x_dtype == MUSER_DTYPE_F32 ? rms_rows_staged_kernel<true> : rms_rows_staged_kernel<false>;
         const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kRmsSmem);
         if (e != cudaSuccess) return e;
