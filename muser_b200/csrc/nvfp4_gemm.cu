@@ -282,8 +282,7 @@ __device__ __forceinline__ float4 split_load(uint32_t addr) {
 // its shared memory, and all of them add the slices up in slice order, every CTA finishing a share of the tile's outputs.
 // SLICED (SPLIT with GROUP): a group that holds weights which SPLIT cuts when they are called alone.  Tiles are whole, but
 // the accumulator starts anew with every slice of such a weight and the epilogue adds the slices up as SPLIT does: the bits
-// of the single call in the group's one launch.  (Launched one by one the group took up to twice as long: 12288 + 1024 +
-// 1024 rows of 12288 inputs at 200 tokens 31 -> 62 us.)
+// of the single call in the group's one launch (where that is the faster way: group_in_one_launch).
 template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, bool SPLIT = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -424,20 +423,21 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
-                uint32_t slices = 1, slice = 0, slice_first = 0; // SLICED only
+                uint32_t slices = 1, slice = 0, slice_first = 0, slice_end = 0; // SLICED only
                 if constexpr (SLICED) {
                     uint32_t tile_m, tile_n;
                     tile_coords(tile, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
                     slices = g.grp_slices[(tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3])];
+                    slice_end = g.k_tiles / slices; // (kept: a division a slab took the issuing warp longer than the slab's products)
                 }
                 for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
                     if constexpr (SLICED) {
-                        if (kt == g.k_tiles * (slice + 1) / slices) { // (never true at the last slice's end, where the loop ends)
+                        if (kt == slice_end) { // (never true at the last slice's end, where the loop ends)
                             mma_commit_elect(bar_acc_full);
                             PROF_BEGIN ok = mbar_wait_warp(bar_acc_empty, local & 1, abort_flag); PROF_END(0)
                             if (!ok) break;
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            ++local, ++slice, slice_first = kt;
+                            ++local, ++slice, slice_first = kt, slice_end = g.k_tiles * (slice + 1) / slices;
                         }
                     }
                     const uint32_t s = it % kStages, round = it / kStages;
@@ -544,16 +544,16 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     __syncwarp();
                     if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
                     ++local;
-                    ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64));
+                    ok = mbar_wait_warp(bar_acc_full, local & 1, abort_flag); // (no sleep: the tensor pipe stands still from here on)
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                    for (int c = 0; c < 64; c += 8) { // (eight columns at a time: the sums so far fill the registers)
-                        uint32_t v[8];
-                        tmem_ld8(lane_base + col0 + c, v);
+                    for (int c = 0; c < 64; c += 16) { // (sixteen columns at a time: the sums so far fill the registers)
+                        uint32_t v[16];
+                        tmem_ld16(lane_base + col0 + c, v);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
+                        for (int i = 0; i < 16; ++i) {
                             uint32_t &sum = r[(c + i) >> 5][(c + i) & 31];
                             sum = __float_as_uint(__uint_as_float(sum) + __uint_as_float(v[i]));
                         }
@@ -1414,10 +1414,49 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     return MUSER_CUDA_OK;
 }
 
+// A group that holds weights which are split when they are called alone: one launch of whole tiles (SLICED), or each of
+// those weights in a launch of its own and the rest in one?  In us: a slab of a tile 0.43 or the weights' bytes at 6.5 TB/s,
+// a launch about 4, a change of slices 0.5, the meeting of the slices 0.6 and 0.075 per token row of a tile.  Measured, one
+// launch / apart: 3 x 1024 rows of 27648 inputs 53 / 40 at 16 tokens, 54 / 54 at 100, 55 / 64 at 200; 2048 + 512 + 512 of
+// 12288 27 / 25 at 8, 26 / 29 at 16, 28 / 51 at 128; 12288 + 1024 + 1024 of 12288 28 / 36 at 8, 31 / 63 at 256.  (Not split
+// at all, with other bits than the single calls': 50, 51, 52; 25, 25, 27; 28, 32.)
+static bool group_in_one_launch(const uint32_t *slices, const Weight *const *ws, uint32_t n, uint32_t tokens, int sm_count) {
+    const uint32_t m_tiles = (tokens + BM - 1) / BM;
+    const double k_tiles = (double)((ws[0]->n_in + BK - 1) / BK), rows = std::min<uint32_t>(tokens, BM);
+    const auto bytes_us = [&](uint32_t tiles) { return (double)tiles / m_tiles * BN * ws[0]->n_in * 0.5625 / 6.5e6; };
+    const auto whole_us = [&](uint32_t tiles) { return tiles ? std::max(std::ceil((double)tiles / sm_count) * k_tiles * 0.43, bytes_us(tiles)) + 4.0 : 0.0; };
+    uint32_t all = 0, unsplit = 0, most = 1;
+    double apart = 0.0;
+    for (uint32_t p = 0; p < n; ++p) {
+        const uint32_t tiles = (uint32_t)(ws[p]->n_out_pad / BN) * m_tiles;
+        all += tiles, most = std::max(most, slices[p]);
+        if (slices[p] > 1) apart += std::max(std::ceil(k_tiles / slices[p]) * 0.43, bytes_us(tiles)) + 4.6 + 0.075 * rows;
+        else unsplit += tiles;
+    }
+    return whole_us(all) + (most - 1) * 0.5 <= apart + whole_us(unsplit);
+}
+
 // Up to four projections of the same quantized activations in one launch (GROUP form of the kernel).
 muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uint32_t n, const uint8_t *x_packed, const uint8_t *x_scales,
                                           void *const *ys, uint32_t y_dtype, uint32_t tokens, cudaStream_t stream) {
     const Weight *w0 = ws[0];
+    uint32_t slices[4] = {1, 1, 1, 1}; // (the paired kernel, which serves single calls where it is on, never splits)
+    bool sliced = false;
+    for (uint32_t p = 0; p < n && !ctx->nvfp4_pair; ++p) slices[p] = gemm_ksplit(ctx, ws[p], tokens), sliced = sliced || slices[p] > 1;
+    if (sliced && !group_in_one_launch(slices, ws, n, tokens, ctx->sm_count)) {
+        const Weight *rest[4];
+        void *rest_y[4];
+        uint32_t n_rest = 0;
+        for (uint32_t p = 0; p < n; ++p) {
+            if (slices[p] == 1) {
+                rest[n_rest] = ws[p], rest_y[n_rest++] = ys[p];
+                continue;
+            }
+            const muser_cuda_status st = launch_nvfp4_gemm(ctx, ws[p], x_packed, x_scales, ys[p], y_dtype, tokens, Epilogue{}, stream);
+            if (st != MUSER_CUDA_OK) return st;
+        }
+        return n_rest ? launch_nvfp4_gemm_group(ctx, rest, n_rest, x_packed, x_scales, rest_y, y_dtype, tokens, stream) : MUSER_CUDA_OK;
+    }
     CUtensorMap map_a;
     if (!make_map(&map_a, x_packed, tokens, w0->n_in / 2, box_tokens(tokens)))
         return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the activations");
@@ -1433,7 +1472,6 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     g.out_scale = 1.0f;
     g.inv_input_scale = 1.0f / w0->input_scale_inv;
     uint32_t tiles_n = 0;
-    bool sliced = false;
     for (uint32_t p = 0; p < 4; ++p) {
         g.grp_tile0[p] = tiles_n;
         if (p >= n) continue;
@@ -1441,8 +1479,7 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
         g.grp_y[p] = ys[p];
         g.grp_n_out[p] = (uint32_t)ws[p]->n_out;
         g.grp_scale2[p] = ws[p]->scale2;
-        g.grp_slices[p] = ctx->nvfp4_pair ? 1 : gemm_ksplit(ctx, ws[p], tokens); // (the paired kernel, which serves single calls then, never splits)
-        sliced = sliced || g.grp_slices[p] > 1;
+        g.grp_slices[p] = slices[p];
         tiles_n += (uint32_t)(ws[p]->n_out_pad / BN);
     }
     g.grp_tile0[4] = tiles_n;
