@@ -502,7 +502,9 @@ struct MmaPlan {
 };
 
 // How many clusters of n CTAs (one CTA an SM) the device holds at once: a cluster stays inside one GPC, so sizes that do
-// not divide a GPC's SMs leave some idle (a B200: 74, 45, 33, 26, 22, 15, 15 for two to eight).  Asked once per device.
+// not divide a GPC's SMs leave some idle (a B200: 74, 45, 33, 26, 22, 15, 15 for two to eight).  Asked once per device
+// and kept whatever the answer, so that the process's calls agree: a device that cannot say holds no clusters (its error is
+// taken off: a launch without clusters reports errors of its own).
 struct ClusterRoom {
     int n[kMmaMaxSplit + 1] = {};
 };
@@ -525,7 +527,10 @@ cudaError_t cluster_room(int device, int sm_count, ClusterRoom *out) {
             cfg.attrs = attr, cfg.numAttrs = 1;
             e = cudaOccupancyMaxActiveClusters(&found.n[n], fn, &cfg);
         }
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            found = ClusterRoom{};
+        }
         found.n[1] = sm_count;
         r = found;
     }

@@ -15,6 +15,8 @@
 // stops issuing work, waits (bounded) for its own copies in flight, frees its tensor memory and returns.
 #include <cuda.h>
 
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "common.cuh"
@@ -1260,32 +1262,41 @@ void nvfp4_free_tensor_map(Weight *w) {
 static uint32_t box_tokens(uint32_t tokens) { return std::min<uint32_t>(BM, (tokens + 7) / 8 * 8); }
 
 // CTAs that share the K of one output tile.  A slab takes a CTA 0.45 us, so a long K over few tiles leaves most SMs idle:
-// 5120 x 27648 has 20 tiles of 108 slabs per 128 tokens.  Split where the row is at least 48 slabs long and all tiles
-// with all their slices are on the GPU at once (clusters stay inside a GPC), eight slabs a slice at least.  The rule looks
-// at the weight and the token count alone, so that a call gives the same bits whoever makes it; weights it splits are
-// launched one by one from a group, and the fused gate/up form, whose weights are wider than long, never splits.
-// 5120 x 27648 (us, whole -> split): 48 -> 20 at 16 tokens, 52 -> 29 at 128, 52 -> 34 at 384; 509 tokens are 80 tiles, whole.
+// 5120 x 27648 has 20 tiles of 108 slabs per 128 tokens.  Split where all tiles with all their slices are on the GPU at once
+// (clusters stay inside a GPC) and a slice keeps eight slabs.  Rows below 48 slabs are left whole: measured are 108 slabs
+// (us, whole -> split: 48 -> 20 at 16 tokens, 52 -> 29 at 128, 52 -> 34 at 384; 509 tokens are 80 tiles, whole) and rows of
+// 48 (1024 x 12288 24 -> 10 at 16 tokens, 28 -> 17 at 128), not shorter ones.
+// What the bits of a result depend on: the number of slices, i.e. the weight's rows and row length, the token count and the
+// device (its SMs, and how many clusters of a size it holds).  Calls with a logit scale or soft cap, the fused gate/up form
+// and contexts that use the paired kernel never split; a group gives the bits of the single calls.
+struct SplitRoom {
+    bool asked = false;
+    int n[9] = {}; // clusters of n CTAs the device holds at once
+};
 static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
     const uint32_t k_tiles = (uint32_t)((w->n_in + BK - 1) / BK), tiles = (uint32_t)(w->n_out_pad / BN) * ((tokens + BM - 1) / BM);
     if (k_tiles < 48 || tiles * 2 > (uint32_t)ctx->sm_count || ctx->device < 0 || ctx->device >= kMaxDevices) return 1;
-    struct Room { int n[9] = {}; };
-    static PerDevice<Room> rooms; // clusters of n CTAs the device holds at once, asked once
+    static PerDevice<SplitRoom> rooms;
     std::lock_guard<std::mutex> lock(rooms.mu);
-    Room &room = rooms.slot[ctx->device];
-    if (!room.n[1]) {
+    SplitRoom &room = rooms.slot[ctx->device];
+    if (!room.asked) {
+        // Asked once and kept whatever the answer, so that the process's calls agree: a device that cannot say holds no
+        // clusters.  (Its error is taken off: whole tiles need no clusters, and the launch reports errors of its own.)
+        room.asked = true;
         const auto kernel = nvfp4_gemm_kernel<false, false, false, false, true>;
-        if (ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes) != cudaSuccess) return 1;
-        Room found;
-        for (int n = 2; n <= 8; ++n) {
+        cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes);
+        for (int n = 2; n <= 8 && e == cudaSuccess; ++n) {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = n, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
             cfg.gridDim = dim3(n * 64), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kSmemBytes, cfg.attrs = attr, cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&found.n[n], kernel, &cfg) != cudaSuccess) return 1;
+            e = cudaOccupancyMaxActiveClusters(&room.n[n], kernel, &cfg);
         }
-        found.n[1] = 1;
-        room = found;
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            for (int &n : room.n) n = 0;
+        }
     }
     for (uint32_t ks = 8; ks >= 2; --ks)
         if (tiles <= (uint32_t)room.n[ks] && k_tiles / ks >= 8) return ks;
