@@ -88,10 +88,10 @@ def test_matmul_matches_cpu_lane(gpu, dtype, x_dtype):
 
 @pytest.mark.parametrize("dtype", [O.Q4_K, O.Q6_K])
 def test_activations_beyond_the_f16_range(gpu, dtype):
-    """bf16 and f32 activations can exceed f16's range (|x| > 65504).  The decode kernel (up to 16 tokens, and longer
-    batches on weights below the tcgen05 kernel's row threshold) scales every 256-input tile by its own maximum, so
-    such inputs cost nothing; the tcgen05 kernel (17-64 tokens) takes activations as f16 and clamps them: the stated
-    range limit of that kernel, checked here so that it stays a clamp and never becomes inf or NaN."""
+    """bf16 and f32 activations can exceed f16's range (|x| > 65504).  The decode and the batched kernel scale every
+    256-input tile by its own maximum, so such inputs cost nothing; the tcgen05 kernel takes activations as f16 and
+    clamps them, and so do the calls (17-64 tokens, enough rows) that it can serve, whichever kernel does: a stated range
+    limit, checked here so that it stays a clamp and never becomes inf or NaN."""
     from muser_b200._lib import TUNE_TC_MIN_ROWS
     op, ctx, k = gpu
     n_in, n_out = 1024, 1100
@@ -104,22 +104,35 @@ def test_activations_beyond_the_f16_range(gpu, dtype):
             x[0, 5], x[tokens - 1, 700], x[0, 300] = 3.0e5, -1.0e6, 7.0e4
             x = x.to(x_dtype)
             want = O.matmul(ow, x.float().numpy(), threads=4)
+            for warps in (10, 0):  # every token count through the decode kernel, then from 13 tokens the batched one
+                y = torch.full((tokens, n_out), float("nan"), dtype=torch.float32, device="cuda")
+                try:
+                    ctx.tuning_set(TUNE_TC_MIN_ROWS, 1 << 30)
+                    ctx.tuning_set(op.TUNE_DECODE_WARPS, warps)
+                    k.encode_quantized_matmul(w, x.cuda(), y, tokens)
+                    ctx.sync_status()
+                finally:
+                    ctx.tuning_set(TUNE_TC_MIN_ROWS, 1024)
+                    ctx.tuning_set(op.TUNE_DECODE_WARPS, 0)
+                assert warps == 0 or k.last_decode_plan()[0] == warps
+                assert H.rel_l2(y.cpu().numpy(), want) <= REL_L2_TOL, (x_dtype, tokens, warps, H.rel_l2(y.cpu().numpy(), want))
+        # the tcgen05 kernel, then the batched one, on the same 24 tokens: finite, and equal to the CPU lane on the
+        # clamped activations
+        tokens, key = 24, op.TUNE_TC_MIN_TOKENS_Q4_K if dtype == O.Q4_K else op.TUNE_TC_MIN_TOKENS_Q6_K
+        outputs = []
+        for threshold in (16, 17):
             y = torch.full((tokens, n_out), float("nan"), dtype=torch.float32, device="cuda")
             try:
-                ctx.tuning_set(TUNE_TC_MIN_ROWS, 1 << 30)  # every token count through the decode kernel
+                ctx.tuning_set(key, threshold)
                 k.encode_quantized_matmul(w, x.cuda(), y, tokens)
                 ctx.sync_status()
             finally:
-                ctx.tuning_set(TUNE_TC_MIN_ROWS, 1024)
-            assert H.rel_l2(y.cpu().numpy(), want) <= REL_L2_TOL, (x_dtype, tokens, H.rel_l2(y.cpu().numpy(), want))
-        # the tcgen05 kernel on the same 24 tokens: finite, and equal to the CPU lane on the clamped activations
-        tokens = 24
-        y = torch.full((tokens, n_out), float("nan"), dtype=torch.float32, device="cuda")
-        k.encode_quantized_matmul(w, x.cuda(), y, tokens)
-        ctx.sync_status()
-        assert torch.isfinite(y).all()
-        want_clamped = O.matmul(ow, x.float().clamp(-65504.0, 65504.0).numpy(), threads=4)
-        assert H.rel_l2(y.cpu().numpy(), want_clamped) <= REL_L2_TOL, (x_dtype, H.rel_l2(y.cpu().numpy(), want_clamped))
+                ctx.tuning_set(key, 17)
+            assert torch.isfinite(y).all()
+            want_clamped = O.matmul(ow, x.float().clamp(-65504.0, 65504.0).numpy(), threads=4)
+            assert H.rel_l2(y.cpu().numpy(), want_clamped) <= REL_L2_TOL, (x_dtype, threshold, H.rel_l2(y.cpu().numpy(), want_clamped))
+            outputs.append(y)
+        assert not torch.equal(*outputs)  # two kernels, two orders of summation
     w.free()
 
 
@@ -160,8 +173,8 @@ def test_fused_gate_up_silu(gpu, dtype):
 @pytest.mark.parametrize("x_dtype", [torch.bfloat16, torch.float32])
 def test_fused_input_rmsnorm(gpu, dtype, x_dtype):
     """rms_norm_mul (reference.rs:59-80) fused in front of the projection: the decode kernel norms while it stages
-    the activations (bf16, few tokens), the skinny kernel behind a pass of its own; both against the CPU lane's
-    norm followed by weights::matmul."""
+    the activations (few tokens), the batched kernel while it prepares them; both against the CPU lane's norm followed
+    by weights::matmul."""
     op, ctx, k = gpu
     n_in, n_out, eps = 1024, 37, 1e-6
     raw = H.lcg_weights(dtype, n_out, 4, seed=31)
@@ -192,8 +205,9 @@ def test_fused_input_rmsnorm(gpu, dtype, x_dtype):
 @pytest.mark.parametrize("x_dtype", [torch.bfloat16, torch.float32])
 def test_tensor_core_skinny_kernel(gpu, dtype, x_dtype):
     """The tcgen05 kernel (exact integer f16 operands, per-super-block drain) forced for every token count it serves,
-    on shapes with a short last row block, one to many K slices, and the fused row scale / residual; then the same
-    calls with that kernel switched off, which sends them through the decode kernel in chunks of 16 tokens."""
+    on shapes with a short last row block, one to many K slices, the fused row scale / residual and the input norm; then
+    the same calls with that kernel switched off and a decode plan forced, which sends them through the decode kernel in
+    chunks of 16 tokens."""
     op, ctx, k = gpu
     key = op.TUNE_TC_MIN_TOKENS_Q4_K if dtype == O.Q4_K else op.TUNE_TC_MIN_TOKENS_Q6_K
     shapes = [(512, 13, 2), (1024, 37, 4), (2048, 300, 8)]
@@ -201,6 +215,7 @@ def test_tensor_core_skinny_kernel(gpu, dtype, x_dtype):
         ctx.tuning_set(op.TUNE_TC_MIN_ROWS, 1)
         for threshold in (1, 65):
             ctx.tuning_set(key, threshold)
+            ctx.tuning_set(op.TUNE_DECODE_WARPS, 10 if threshold == 65 else 0)
             for n_in, n_out, blocks in shapes:
                 raw = H.lcg_weights(dtype, n_out, blocks, seed=n_out + dtype)
                 w = op.Weight(ctx, op.TensorView(raw, dtype, n_in, n_out))
@@ -212,6 +227,12 @@ def test_tensor_core_skinny_kernel(gpu, dtype, x_dtype):
                     ctx.sync_status()
                     err = H.rel_l2(y.cpu().numpy(), want)
                     assert err <= REL_L2_TOL, (threshold, n_in, n_out, tokens, err)
+                    assert threshold == 1 or k.last_decode_plan()[0] == 10
+                nw, xn = torch.linspace(0.5, 1.5, n_in), x[:20]
+                want = O.matmul(O.TensorView(raw, dtype, n_in, n_out), O.rms_norm_mul(xn.float().numpy(), 1e-6, nw.numpy()), threads=O.host_threads())
+                y = torch.full((20, n_out), float("nan"), dtype=torch.float32, device="cuda")
+                k.encode_quantized_matmul(w, xn.contiguous().cuda(), y, 20, norm_weight=nw.cuda(), norm_eps=1e-6)
+                assert H.rel_l2(y.cpu().numpy(), want) <= REL_L2_TOL, (threshold, n_in, n_out)
                 rs = torch.linspace(0.5, 2.0, 5, device="cuda")
                 res = torch.randn((5, n_out), device="cuda")
                 x = torch.from_numpy(H.lcg_activations(5 * n_in, seed=3).reshape(5, n_in)).to(x_dtype)
@@ -224,6 +245,7 @@ def test_tensor_core_skinny_kernel(gpu, dtype, x_dtype):
         ctx.tuning_set(op.TUNE_TC_MIN_TOKENS_Q4_K, 17)
         ctx.tuning_set(op.TUNE_TC_MIN_TOKENS_Q6_K, 17)
         ctx.tuning_set(op.TUNE_TC_MIN_ROWS, 1024)
+        ctx.tuning_set(op.TUNE_DECODE_WARPS, 0)
     ctx.sync_status()
 
 
@@ -465,7 +487,8 @@ def test_grouped_projections_in_one_launch(gpu):
 
 def test_measured_launch_plans_keep_the_results(gpu):
     """muser_cuda_decode_autotune replaces the cost model's launch plans with measured ones for a group, a single
-    projection and a fused gate/up pair: results stay within tolerance of the CPU lane and repeat bit for bit."""
+    projection and a fused gate/up pair: results stay within tolerance of the CPU lane and repeat bit for bit (16 tokens:
+    the batched kernel, which has no such plans; the decode kernel's at 13 to 16 serve K shards and the LM head)."""
     op, ctx, k = gpu
     n_in = 2048
     shapes = [(O.Q4_K, 1100), (O.Q6_K, 260)]
@@ -532,7 +555,7 @@ def test_config1_full_size_q4k_gemv(gpu):
 @pytest.mark.parametrize("name", ["ffn_gate", "ffn_down"])
 def test_layer_shapes_every_kernel_sampled_rows_and_determinism(gpu, name):
     """The layer's two big projections at full size, one token count per kernel variant and split-K regime (decode
-    kernel with one to four token groups, tcgen05 kernel at 32 / 64 columns): 96 sampled output rows against the CPU
+    kernel with one to three token groups, batched kernel, tcgen05 kernel at 32 / 64 columns of the Q4_K weight): 96 sampled output rows against the CPU
     lane, and bit-identical results when the same call runs twice (the K slices are summed in a fixed order)."""
     op, ctx, k = gpu
     from muser_b200 import synth
@@ -582,9 +605,11 @@ def test_lm_head_tail_and_selected_rows(gpu, dtype):
     raw = H.lcg_weights(dtype, n_out, n_in // 256, seed=55)
     ow = O.TensorView(raw, dtype, n_in, n_out)
     w = op.Weight(ctx, op.TensorView(raw, dtype, n_in, n_out))
+    key = op.TUNE_TC_MIN_TOKENS_Q6_K if dtype == O.Q6_K else op.TUNE_TC_MIN_TOKENS_Q4_K
     ctx.tuning_set(op.TUNE_TC_MIN_ROWS, 1)
     try:
-        for tokens in (1, 3, 7, 20):  # decode kernel (one and two token groups), tcgen05 kernel
+        for tokens, threshold in ((1, 17), (3, 17), (7, 17), (20, 17), (20, 16)):  # decode kernel (one and two token groups), batched, tcgen05 (Q5_K: batched)
+            ctx.tuning_set(key, threshold)
             x = torch.from_numpy(H.lcg_activations(tokens * n_in, seed=tokens).reshape(tokens, n_in)).to(torch.bfloat16)
             plain = O.matmul(ow, x.float().numpy())
             scale = float(15.0 / plain.std())  # scaled logits of std 15 against a cap of 30: both regimes of the tanh occur
@@ -597,6 +622,7 @@ def test_lm_head_tail_and_selected_rows(gpu, dtype):
             assert H.rel_l2(y.cpu().numpy(), O.logit_tail(plain, scale, 0.0)) <= REL_L2_TOL
     finally:
         ctx.tuning_set(op.TUNE_TC_MIN_ROWS, 1024)
+        ctx.tuning_set(key, 17)
     rows = np.array([299, 0, 17, 17, 128, 255, 16], dtype=np.int32)
     for x_dtype in (torch.bfloat16, torch.float32):
         x = torch.from_numpy(H.lcg_activations(11 * n_in, seed=9).reshape(11, n_in)).to(x_dtype)
