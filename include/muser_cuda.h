@@ -205,7 +205,8 @@ MUSER_CUDA_API muser_cuda_status muser_cuda_quantized_matmul_group(muser_cuda_ct
  * plan (warps per CTA, how K is split between CTAs and between the warps of a CTA) comes from a cost model; this
  * call measures the model's best candidates for one projection or one group (`weights`, as they will be passed to
  * muser_cuda_quantized_matmul / _group; `w_up` non-NULL for the fused gate/up form of weights[0]) at 1 .. max_tokens
- * tokens and remembers the fastest for this device, for every later call on the same geometry in this process.
+ * tokens and remembers the fastest for this device, for every later call on the same geometry in this process that the
+ * decode kernel serves: up to 12 tokens all of them, at 13 to 16 K shards and muser_cuda_lm_head_argmax.
  * Every candidate is timed as a CUDA graph of back-to-back launches over temporary copies of the weight images (so
  * that they stream from HBM).  Optional load-time work: it allocates scratch (up to ~350 MB), synchronizes
  * `stream`, runs on a stream of its own, and frees the scratch. */
@@ -291,8 +292,8 @@ MUSER_CUDA_API muser_cuda_status muser_cuda_nvfp4_matmul_prequant(muser_cuda_ctx
 /* The NVFP4 form of muser_cuda_quantized_matmul_group (MetalKernels::encode_quantized_decode_group,
  * src/metal/encode/qkv.rs:414-449: q | k | v on the same activations in one dispatch): 2..4 NVFP4 weights with the same
  * n_in and the same input_scale_inv, the activations quantized earlier, one launch whose output tiles run through
- * all of them, so the small projections fill the SMs that a launch of their own would leave idle.  Every output is
- * bit-identical to what muser_cuda_nvfp4_matmul_prequant gives for that weight.  Plain outputs (no epilogue), all of
+ * all of them, so the small projections fill the SMs that a launch of their own would leave idle (rows of more than
+ * 12000 inputs may take several launches where those are faster).  Every output is bit-identical to what muser_cuda_nvfp4_matmul_prequant gives for that weight.  Plain outputs (no epilogue), all of
  * y_dtype, outputs[i] [tokens][n_out of weights[i]]. */
 MUSER_CUDA_API muser_cuda_status muser_cuda_nvfp4_matmul_group_prequant(muser_cuda_ctx *ctx, const muser_cuda_weight *const *weights,
                                                          uint32_t n_weights, const uint8_t *x_packed,

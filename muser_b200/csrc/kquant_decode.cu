@@ -1156,7 +1156,7 @@ muser_cuda_status decode_autotune(Ctx *ctx, const Weight *const *w, const Weight
         for (uint32_t i = 0; i < n_jobs; ++i) wc[i] = &shadow[(size_t)c * (n_jobs + 1) + i];
         return launch_kquant_decode(ctx, wc, w_up ? &shadow[(size_t)c * (n_jobs + 1) + n_jobs] : nullptr, n_jobs, x, MUSER_DTYPE_BF16, ys, yd, tokens, eps, side);
     };
-    static const uint32_t kTokenSteps[] = {1, 2, 4, 8, 12, 16};
+    static const uint32_t kTokenSteps[] = {1, 2, 4, 8, 12, 16}; // (16: K shards and the LM head)
     std::vector<DecCandidate> cands;
     muser_cuda_status st = MUSER_CUDA_OK;
     for (uint32_t tokens : kTokenSteps) {
@@ -1219,8 +1219,9 @@ muser_cuda_status decode_autotune(Ctx *ctx, const Weight *const *w, const Weight
 // smaller fixed part and pads token columns to 8, the tcgen05 one (kquant_tc.cu, to 16, 32 or 64; Q4_K and Q6_K) the
 // cheaper column: see takes_tcgen05.  At 13 to 16 tokens the decode kernel's integer products are bound by their scale
 // arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 35, 5120 x 27648 Q6_K 68 -> 42, 5120 x 5120 21 -> 14,
-// 1024 x 5120 18.5 -> 10); at 9 to 12 the two are even (40 / 40, 55 / 43, 17 / 15, but 8192 x 5120 17 / 20), below it wins.
-// The decode kernel also keeps
+// 1024 x 5120 18.5 -> 10).  At 9 to 12 it depends on the weight (40 / 40, 55 / 43 for the long Q6_K rows, 17 / 15, but
+// 8192 x 5120 17 / 20), which one line for all of them does not follow; below it wins (27648 x 5120 at 8: 27 / 34).
+// The decode kernel also keeps, and its forms for 13 to 16 tokens (fused gate/up among them) are there for,
 //   - K shards up to 16 tokens, whose partial sums must carry the same bits with and without the all-reduce fused in,
 //   - calls under a forced launch plan (MUSER_TUNE_DECODE_*), and shapes the batched kernels refuse.
 static bool takes_mma(const Ctx *ctx, const Weight *w, uint32_t tokens) {
@@ -1231,7 +1232,8 @@ static bool takes_mma(const Ctx *ctx, const Weight *w, uint32_t tokens) {
 // The tcgen05 kernel for large Q4_K weights at token counts that fill its columns (us, tcgen05 / warp-level: 27648 x 5120
 // 44 / 46 at 32 tokens, 61 / 70 at 64, 55 / 61 at 32 in f32, which take two columns each; 61 / 56 at 48; 13824 x 5120 37 / 40
 // at 64; 8192 x 5120 22 / 22 and 33 / 31; 5120 x 5120 19 / 17 and 29 / 23).  Q6_K: 63 / 52 at 32 and 78 / 76 at 64 for
-// 5120 x 27648.  A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves.
+// 5120 x 27648.  A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves, which is
+// what its Q6_K form is kept for: the caller's choice of range and rounding against another kernel's.
 static bool takes_tcgen05(const Weight *w, uint32_t tokens, bool two_columns, uint32_t tc_from) {
     if (tc_from < 17) return true;
     const uint32_t cols = two_columns ? 2 * tokens : tokens;
