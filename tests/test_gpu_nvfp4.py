@@ -323,10 +323,11 @@ def test_long_rows_split_between_the_ctas_of_a_cluster(gpu, n_out, n_in, tokens)
     w.free()
 
 
-@pytest.mark.parametrize("shapes, tokens", [((9600, 300, 37), 131), ((300, 9600), 250), ((700, 37, 300, 256), 16)])
+@pytest.mark.parametrize("shapes, tokens", [((9600, 300, 37), 131), ((300, 9600), 250), ((700, 37, 300, 256), 16), ((300, 37, 37888), 9)])
 def test_groups_of_long_rows_sum_in_the_single_calls_slices(gpu, shapes, tokens):
     """A group of long rows is one launch of whole tiles, some of its weights summed in the slices that the single call
-    splits them into, in different numbers of slices, beside weights that are never split: equal bits."""
+    splits them into, in different numbers of slices, beside weights that are never split: equal bits.  (The last group is
+    launched in parts: one launch would take a round of tiles more.)"""
     op, ctx, k = gpu
     from muser_b200 import synth
     n_in = 12352  # (49 slabs, the last one short)
@@ -389,7 +390,7 @@ def test_outputs_and_residuals_at_any_alignment(gpu, n_out, dtype, tol):
     w.free()
 
 
-@pytest.mark.parametrize("n_in", [64, 1088, 5120, 12352])
+@pytest.mark.parametrize("n_in", [64, 1088, 5120, 12288, 12352])
 @pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
 def test_fused_norm_adds_the_squares_front_to_back(gpu, n_in, x_dtype):
     """The sum of squares is the reference's chain of additions to the last bit whatever the row looks like, so codes
