@@ -241,7 +241,7 @@ __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, 
 // prefix sum; then one warp walks the 128 segments, checks for each that S was in the guessed binade before and is
 // after (else it adds that segment's squares one by one: about one segment per power of two that the sum passes), and
 // ends with exactly the chain's sum.  Up to 500 rows of 5120 values: 31 us for the chain kernel and 3 to 5 for a quantizer
-// behind it -> about 12 (a layer at 16 tokens 202 -> 145 us, together with the launches that follow one another closer).
+// behind it -> 15 to 19 (a layer at 16 tokens 202 -> 145 us, together with the launches that follow one another closer).
 constexpr int kNormThreads = 128;
 template <bool XF32>
 __global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
@@ -252,9 +252,12 @@ __global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const
     __shared__ uint2 seg_add[kNormThreads];
     __shared__ uint32_t seg_binade[kNormThreads]; // exponent field the additions hold for, 0: one by one
     __shared__ float inv_rms;
+    const uint32_t row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    // the norm weights are read last, from L2 if they are asked for now (between two layers' weights they go to memory)
+    if (row < tokens)
+        for (uint32_t i = 32 * tid; i < n_in; i += 32 * kNormThreads) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + i));
     pdl_wait();
     pdl_release();
-    const uint32_t row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     float inv = 0.0f;
@@ -351,14 +354,17 @@ __global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const
 // The same behind a kernel that runs the chains as chains, which does less work per row than the segments above but takes
 // their length in latency: the better form from 449 rows (us, segments / chains with quantizer, 5120 values: 15 / 17 at 16
 // rows, 19 / 19 at 512, 40 / 33 at 1536, 43 / 37 at 2048; 3136 values: 20 / 13 at 448 rows) and for rows of up to 4096 values
-// (1024 values: 11 / 6 at 16 rows, 15 / 7 at 1024).
+// (1024 values: 11 / 6 at 16 rows, 15 / 7 at 1024; on either side of the line, chains of 4096 values 13.8 at 16 rows and 15.1
+// at 448, segments of 4160 14.8 and 17.1; on either side of the other, 27648 values, 63 at 448 rows and 87 at 449).
 template <bool XF32>
 __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
                                                                     const float *norm_w, const float *inv_rms, uint8_t *packed,
                                                                     uint8_t *scales) {
+    const uint32_t row = blockIdx.x;
+    if (row == 0) // (as above)
+        for (uint32_t i = 32 * threadIdx.x; i < n_in; i += 32 * 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + i));
     pdl_wait();
     pdl_release();
-    const uint32_t row = blockIdx.x;
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
