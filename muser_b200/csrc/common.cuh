@@ -58,7 +58,7 @@ struct Ctx {
     unsigned int *amax_flags = nullptr;
     uint32_t host_direct_output = 2;           // host-group entry: 2 one copy per output on the copy stream (beside the next launches), 1 a kernel
                                                // stores the outputs into mapped host buffers, 0 one copy per output on the launches' stream
-    uint32_t nvfp4_pair = 0;                   // NVFP4 GEMM on pairs of SMs (cta_group::2): 0 off, 1 on
+    uint32_t nvfp4_pair = 2;                   // NVFP4 GEMM on pairs of SMs (cta_group::2): 0 never, 1 always, 2 where they are faster
     uint32_t nvfp4_group_m = 0;                // NVFP4 GEMM: token tiles per raster group, 0 = automatic
     uint32_t oneshot_max_bytes = 1536u << 10;  // all-reduce payloads up to this size take the one-shot peer exchange
     std::string last_error;
@@ -86,7 +86,8 @@ struct Weight {
     bool has_input_scale_inv = false;
     uint64_t image_bytes = 0;
     void *tmap_cache = nullptr; // CUtensorMap of `packed` with 256-row boxes, built at repack time
-    void *tmap_half = nullptr;  // the same image with 128-row boxes (fused gate/up form)
+    void *tmap_half = nullptr;  // the same image with 128-row boxes (fused gate/up form, pairs of SMs)
+    void *tmap_scales = nullptr; // of `scales`, one slab of a 128-row block per box (pairs of SMs)
 };
 
 inline muser_cuda_status fail(Ctx *ctx, muser_cuda_status st, const std::string &msg) {

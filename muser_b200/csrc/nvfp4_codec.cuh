@@ -21,7 +21,7 @@ __device__ __forceinline__ uint32_t e2m1_word(const float (&q)[8]) {
     return w;
 }
 
-// Quantizes one group of 16 values: writes its 8 code bytes and returns its E4M3 scale code.
+// Quantizes one group of 16 values: its 8 code bytes (as two words, or written), and its E4M3 scale code as the result.
 //
 // The reference compares m = |r| * isi with scale * {0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5} by > and >= in turn.  Those
 // products are exact (a 4-bit and a 3-bit significand), the bounds are the midpoints between neighbouring E2M1 values
@@ -32,7 +32,7 @@ __device__ __forceinline__ uint32_t e2m1_word(const float (&q)[8]) {
 // reciprocal (tests/test_nvfp4_codec_cpu.py runs every scale against the floats around every bound).  The chain (seven
 // multiplies, compares and adds a value) bounded both quantizer kernels and the GEMM epilogue that quantizes: quantize
 // of 32768 x 5120 237 -> 117 us (the memory alone: 66), behind the norm 334 -> 227, gate/up + quantize 6.14 -> 4.82 ms.
-__device__ __forceinline__ uint32_t quantize_group(const float (&r)[16], float isi, uint8_t *codes) {
+__device__ __forceinline__ uint32_t quantize_group(const float (&r)[16], float isi, uint32_t &codes_lo, uint32_t &codes_hi) {
     __half2 h[8], top = __floats2half2_rn(0.0f, 0.0f);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -69,7 +69,13 @@ __device__ __forceinline__ uint32_t quantize_group(const float (&r)[16], float i
         const float q1 = __fmaf_rn(__fmaf_rn(-q0, scale, m[i]), inv, q0);
         q[i >> 3][i & 7] = __uint_as_float(__float_as_uint(q1) | (__float_as_uint(v[i]) & 0x80000000u));
     }
-    *reinterpret_cast<uint2 *>(codes) = make_uint2(e2m1_word(q[0]), e2m1_word(q[1]));
+    codes_lo = e2m1_word(q[0]), codes_hi = e2m1_word(q[1]);
+    return scale_code;
+}
+__device__ __forceinline__ uint32_t quantize_group(const float (&r)[16], float isi, uint8_t *codes) {
+    uint32_t lo, hi;
+    const uint32_t scale_code = quantize_group(r, isi, lo, hi);
+    *reinterpret_cast<uint2 *>(codes) = make_uint2(lo, hi);
     return scale_code;
 }
 

@@ -265,6 +265,125 @@ __device__ __forceinline__ float4 split_load(uint32_t addr) {
     return v;
 }
 
+// PAIR form: a cluster of two CTAs owns a 256-token x 256-row tile (tcgen05 cta_group::2).  Each CTA holds 128 of the tokens
+// (their activations, their accumulator) and HALF of the weight rows of every slab; the pair's tensor cores read both halves.
+constexpr int kPStages = 5;
+constexpr int kPBBytes = (BN / 2) * BK / 2; // 16 KiB: this CTA's half of the pair's 256 weight rows
+constexpr int kPStageBytes = kABytes + kPBBytes + kSfaBytes + kSfbBytes;
+constexpr int kOutPiece = 32 * 64;           // an epilogue warp's staging buffer: 32 rows of 64 bytes
+constexpr int kPSmemBytes = kPStages * kPStageBytes + kEpiWarps * kOutPiece + 1024 + 256;
+static_assert(kPSmemBytes <= 227 * 1024, "stage ring exceeds the shared memory of one CTA");
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t cta_addr, uint32_t rank) { // shared::cta address -> that CTA's window
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Staging buffer (64-byte rows, 64-byte swizzle) -> a box of the output; columns and rows past its end are not written.
+__device__ __forceinline__ void tma_store_2d_elect(const CUtensorMap *map, uint32_t src, int x, int y) {
+    asm volatile("{\n\t" MUSER_ELECT_PRED
+                 "@e cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];\n\t@e cp.async.bulk.commit_group;\n\t}"
+                 ::"l"(map), "r"(x), "r"(y), "r"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void store_buffer_free() { // the warp's last store has read its buffer
+    asm volatile("{\n\t" MUSER_ELECT_PRED "@e cp.async.bulk.wait_group.read 0;\n\t}" ::: "memory");
+    __syncwarp();
+}
+__device__ __forceinline__ uint4 lds_16(uint32_t at) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_16(uint32_t at, const uint32_t (&v)[4]) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster_elect(uint32_t cluster_addr) {
+    asm volatile("{\n\t" MUSER_ELECT_PRED "@e mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// mbar_wait_warp for barriers that the other CTA of the pair arrives on.
+__device__ __forceinline__ bool mbar_wait_pair_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    bool ok = false;
+    for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        ok = done;
+        if ((i & 1023u) == 1023u && *abort_flag) break;
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ void tma_load_2d_pair_elect(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile("{\n\t" MUSER_ELECT_PRED
+                 "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void pair_commit_elect(uint32_t cluster_addr) {
+    asm volatile("{\n\t" MUSER_ELECT_PRED "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void pair_cp_scales_elect(uint32_t tmem_addr, uint64_t desc) {
+    asm volatile("{\n\t" MUSER_ELECT_PRED "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n\t}" ::"r"(tmem_addr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void pair_mma_nvf4_elect(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                    uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t" MUSER_ELECT_PRED
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
+        : "memory");
+}
+
+// A whole slab's twelve scale copies, four products and the commit behind ONE election: with an elect.sync each and a loop
+// around them the issuing warp took 1080 cycles a slab, unrolled 740, so about 460, and the products take 512.  Chunks of
+// 512 bytes follow one another in shared memory: four of the activations, then four of either half of the weight rows.  The
+// role is entered by a branch that does not tell the compiler that its warp runs converged: told so, as the other roles are
+// (they issue their loads in 128 cycles instead of 304, and the single CTAs' slabs are 10 % shorter), it takes 923 cycles to
+// issue these seventeen instructions.
+#define PAIR_CP(COL, CHUNK)                                                                                                  \
+    "add.u32 t, %4, " #COL ";\n\tadd.u32 v, %5, " #CHUNK " * 32;\n\tmov.b64 d, {v, %8};\n\t"                                     \
+    "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [t], d;\n\t"
+#define PAIR_MMA(KB, SFA, SFB, P)                                                                                            \
+    "add.u32 v, %1, 2 * " #KB ";\n\tmov.b64 a, {v, %9};\n\tadd.u32 v, %2, 2 * " #KB ";\n\tmov.b64 b, {v, %9};\n\t"              \
+    "add.u32 t, %4, " #SFA ";\n\tadd.u32 u, %4, " #SFB ";\n\t"                                                                 \
+    "@e tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a, b, %3, [t], [u], " P ";\n\t"
+__device__ __forceinline__ void pair_slab_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales,
+                                                uint32_t accumulate, uint32_t empty) {
+    // (shared-memory addresses lie below 256 KB: the low words of operand_desc() and scale_desc() are address / 16 and constants)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 t, u, v;\n\t.reg .b64 a, b, d;\n\t" MUSER_ELECT_PRED
+        "setp.ne.b32 p, %6, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
+        PAIR_CP(0, 0) PAIR_CP(16, 4) PAIR_CP(20, 8) PAIR_CP(4, 1) PAIR_CP(24, 5) PAIR_CP(28, 9)
+        PAIR_CP(8, 2) PAIR_CP(32, 6) PAIR_CP(36, 10) PAIR_CP(12, 3) PAIR_CP(40, 7) PAIR_CP(44, 11)
+        PAIR_MMA(0, 0, 16, "p") PAIR_MMA(1, 4, 24, "q") PAIR_MMA(2, 8, 32, "q") PAIR_MMA(3, 12, 40, "q")
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t}"
+        ::"r"(tmem_d), "r"((a >> 4) | (1u << 16)), "r"((b >> 4) | (1u << 16)), "r"(idesc), "r"(sf), "r"(scales >> 4), "r"(accumulate), "r"(empty),
+          "n"((128 >> 4) | (1 << 14)), "n"((1024 >> 4) | (1 << 14) | (2 << 29))
+        : "memory");
+}
+
+// Tensor maps of a launch beside the activations': the weights (one, gate and up, or a group's), and for PAIR the outputs, the
+// residual and all scales
+// (tiled loads with the pair's qualifier run a little faster than untiled bulk copies: 560 against 594 cycles per 32 KB).
+struct GemmMaps {
+    CUtensorMap b[4], a_scales, b_scales[4], y[4], residual;
+};
+
 // Persistent: CTA b takes output tiles b, b + gridDim.x, ...; tile index -> (n tile, m tile) with m fastest, so the
 // CTAs that run side by side share one weight tile (read from HBM once, from L2 afterwards).
 //
@@ -285,74 +404,90 @@ __device__ __forceinline__ float4 split_load(uint32_t addr) {
 // SLICED (SPLIT with GROUP): a group that holds weights which SPLIT cuts when they are called alone.  Tiles are whole, but
 // the accumulator starts anew with every slice of such a weight and the epilogue adds the slices up as SPLIT does: the bits
 // of the single call in the group's one launch (where that is the faster way: group_in_one_launch).
-template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, bool SPLIT = false>
+// PAIR: pairs of SMs on 256-token tiles (above).  Each CTA's loads report to its own barrier; the second CTA (rank 1) passes
+// "landed" on with an arrival on the leader's barrier of that stage (loads that report to the other CTA's barrier themselves
+// take 1600 cycles per 32 KB instead of 560); the leader issues the scale copies and the products for both and commits to
+// both CTAs' barriers.
+template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, bool SPLIT = false, bool PAIR = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_b3,
-                  const __grid_constant__ CUtensorMap map_b4, const GemmArgs g) {
+nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ GemmMaps maps, const GemmArgs g) {
     constexpr uint32_t kTileRows = DUAL ? BN / 2 : BN; // output columns (weight rows) per tile
     constexpr bool CLUSTER = SPLIT && !GROUP, SLICED = SPLIT && GROUP;
+    constexpr uint32_t kStages = PAIR ? kPStages : muser::kStages, kStageBytes = PAIR ? kPStageBytes : muser::kStageBytes;
+    constexpr uint32_t kBBytes = PAIR ? kPBBytes : muser::kBBytes;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // swizzled tiles need 1024-byte alignment
     uint8_t *aligned = smem_raw + (base - smem_u32(smem_raw));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(aligned + kStages * kStageBytes);
+    const uint32_t out_base = base + kStages * kStageBytes; // PAIR: the epilogue warps' staging buffers
+    uint64_t *bars = reinterpret_cast<uint64_t *>(aligned + kStages * kStageBytes + (PAIR ? kEpiWarps * kOutPiece : 0));
     const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kStages);
     const uint32_t bar_acc_full = smem_u32(bars + 2 * kStages), bar_acc_empty = smem_u32(bars + 2 * kStages + 1);
-    const uint32_t bar_sf_full = smem_u32(bars + 2 * kStages + 2), bar_sf_empty = smem_u32(bars + 2 * kStages + 2 + kSfBufs);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 2 + 2 * kSfBufs);
+    const uint32_t bar_res = smem_u32(bars + 2 * kStages + 2); // PAIR: one per epilogue warp, "the residual has landed"
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kStages + 2 + (PAIR ? kEpiWarps : 0));
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t m_tiles = (g.tokens + BM - 1) / BM, n_tiles_total = g.n_tiles * m_tiles;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31; // (told to be the same in the whole warp)
+    const uint32_t m_tiles = (g.tokens + (PAIR ? 2 : 1) * BM - 1) / ((PAIR ? 2 : 1) * BM), n_tiles_total = g.n_tiles * m_tiles;
+    const uint32_t rank = PAIR ? cluster_rank() : 0u;
     // This CTA's tiles and, of each, its slabs.  (Macros, so that the other forms compile as if CLUSTER did not exist: with
     // variables in their place the roles' lambdas kept them in registers and every form's slab took 10 % longer.)
 #define GEMM_SLICE (CLUSTER ? blockIdx.x % g.ksplit : 0u)
-#define GEMM_TILE_FIRST (CLUSTER ? blockIdx.x / g.ksplit : blockIdx.x)
-#define GEMM_TILE_STEP (CLUSTER ? n_tiles_total : gridDim.x)
+#define GEMM_TILE_FIRST (CLUSTER ? blockIdx.x / g.ksplit : PAIR ? blockIdx.x >> 1 : blockIdx.x)
+#define GEMM_TILE_STEP (CLUSTER ? n_tiles_total : PAIR ? gridDim.x >> 1 : gridDim.x)
 #define GEMM_KT_FIRST (CLUSTER ? g.k_tiles * GEMM_SLICE / g.ksplit : 0u)
 #define GEMM_KT_END (CLUSTER ? g.k_tiles * (GEMM_SLICE + 1) / g.ksplit : g.k_tiles)
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            mbar_init(bar_full + 8 * s, 1);
+        for (uint32_t s = 0; s < kStages; ++s) {
+            mbar_init(bar_full + 8 * s, PAIR && rank == 0 ? 2 : 1); // the leader's: its own copies and the other CTA's "landed"
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_acc_full, 1);
-        mbar_init(bar_acc_empty, kEpiWarps); // one arrival per epilogue warp
-        for (int b = 0; b < (int)kSfBufs; ++b) {
-            mbar_init(bar_sf_full + 8 * b, 1);
-            mbar_init(bar_sf_empty + 8 * b, 1);
-        }
+        mbar_init(bar_acc_empty, (PAIR ? 2 : 1) * kEpiWarps); // one arrival per epilogue warp (of the pair, in the leader)
+        if constexpr (PAIR)
+            for (int e = 0; e < kEpiWarps; ++e) mbar_init(bar_res + 8 * e, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
+    if constexpr (PAIR) { // one warp of each CTA takes part in the paired allocation, and both CTAs' barriers exist before anything reports to them
+        __syncthreads();
+        cluster_barrier();
+        if (warp == 1) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
+    } else if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer (whole warp; one elected lane issues)
         {
             uint32_t it = 0, issued = 0; // k slabs issued so far, over all tiles
+            uint32_t stage = 0, phase = 1; // PAIR: of slab `it`
             bool ok = true; PROF_DECL
+            const uint32_t peer_empty = PAIR ? map_to_rank(bar_empty, 1) : 0u;
+            const CUtensorMap *ms = nullptr; // PAIR: the scales of `mb`
             uint32_t tile_m, tile_n;
             const uint8_t *sfa, *sfb0, *sfb1;
             const CUtensorMap *mb;
             auto locate = [&](uint32_t tile) {
                 tile_coords(tile, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
                 const uint8_t *b_scales = g.b_scales;
-                mb = &map_b;
+                mb = &maps.b[0];
+                if constexpr (PAIR) ms = &maps.b_scales[0];
                 if constexpr (GROUP) {
                     const uint32_t p = (tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3]);
                     tile_n -= g.grp_tile0[p];
                     b_scales = g.grp_b_scales[p];
-                    mb = p == 0 ? &map_b : p == 1 ? &map_b2 : p == 2 ? &map_b3 : &map_b4;
+                    mb = &maps.b[p];
+                    if constexpr (PAIR) ms = &maps.b_scales[p];
                 }
                 sfa = g.a_scales + (size_t)tile_m * g.kt64 * 512;
                 sfb0 = b_scales + (size_t)(DUAL ? tile_n : 2 * tile_n) * g.kt64 * 512;
@@ -363,10 +498,20 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             auto sf_bytes = [&](uint32_t kt) { return min(4u, g.kt64 - 4 * kt) * 512; };
             auto load_weights = [&](uint32_t kt, uint32_t s) {
                 const uint32_t st = base + s * kStageBytes, full = bar_full + 8 * s;
+                if constexpr (PAIR) { // (scale rows of 8-byte elements; what lies past a row's or the tensor's end arrives as zeros)
+                    mbar_expect_tx_elect(full, g.a_bytes + kBBytes + kSfaBytes + kSfbBytes);
+                    // the leader holds the tile's first 128 weight rows (the gate rows of the fused form), the other CTA the rest (up)
+                    const CUtensorMap *half = DUAL ? &maps.b[rank] : mb;
+                    tma_load_2d_pair_elect(st + kABytes, half, (int)(kt * (BK / 2)), (int)(DUAL ? tile_n * kTileRows : tile_n * BN + rank * (BN / 2)), full);
+                    const uint32_t sfb = st + kABytes + kBBytes + kSfaBytes, x = kt * (4 * 512 / 8);
+                    tma_load_2d_pair_elect(sfb, ms, (int)x, (int)(DUAL ? tile_n : 2 * tile_n), full);
+                    tma_load_2d_pair_elect(sfb + 2048, DUAL ? &maps.b_scales[1] : ms, (int)x, (int)(DUAL ? tile_n : 2 * tile_n + 1), full);
+                    return;
+                }
                 mbar_expect_tx_elect(full, g.a_bytes + kBBytes + 3 * sf_bytes(kt));
                 if constexpr (DUAL) {
-                    tma_load_2d_elect(st + kABytes, &map_b, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
-                    tma_load_2d_elect(st + kABytes + kBBytes / 2, &map_b2, (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
+                    tma_load_2d_elect(st + kABytes, &maps.b[0], (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
+                    tma_load_2d_elect(st + kABytes + kBBytes / 2, &maps.b[1], (int)(kt * (BK / 2)), (int)(tile_n * kTileRows), full);
                 } else {
                     tma_load_2d_elect(st + kABytes, mb, (int)(kt * (BK / 2)), (int)(tile_n * BN), full);
                 }
@@ -375,27 +520,40 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             };
             auto load_activations = [&](uint32_t kt, uint32_t s) {
                 const uint32_t st = base + s * kStageBytes, full = bar_full + 8 * s;
+                if constexpr (PAIR) {
+                    tma_load_2d_pair_elect(st, &map_a, (int)(kt * (BK / 2)), (int)((2 * tile_m + rank) * BM), full);
+                    tma_load_2d_pair_elect(st + kABytes + kBBytes, &maps.a_scales, (int)(kt * (4 * 512 / 8)), (int)(2 * tile_m + rank), full);
+                    return;
+                }
                 tma_load_2d_elect(st, &map_a, (int)(kt * (BK / 2)), (int)(tile_m * BM), full);
                 bulk_load_elect(st + kABytes + kBBytes, sfa + (size_t)kt * kSfaBytes, sf_bytes(kt), full);
             };
             // weights are constants: the first stages' are on their way before the kernel that makes the activations is done
             locate(GEMM_TILE_FIRST);
-            const uint32_t ahead = min((uint32_t)kStages, GEMM_KT_END - GEMM_KT_FIRST);
+            const uint32_t ahead = min(kStages, GEMM_KT_END - GEMM_KT_FIRST);
             for (uint32_t i = 0; i < ahead; ++i) load_weights(GEMM_KT_FIRST + i, i);
             pdl_wait();
             pdl_release(); // (behind the wait: what starts early starts when the kernel before this one is complete)
             for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total && ok; tile += GEMM_TILE_STEP) {
                 locate(tile);
                 for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
-                    const uint32_t s = it % kStages, round = it / kStages;
-                    PROF_BEGIN if (round > 0) ok = mbar_wait_warp(bar_empty + 8 * s, (round - 1) & 1, abort_flag); PROF_END(0)
+                    const uint32_t s = PAIR ? stage : it % kStages, round = it / kStages;
+                    PROF_BEGIN if (PAIR) { if (it >= kStages) ok = mbar_wait_warp(bar_empty + 8 * s, phase, abort_flag); } else if (round > 0) ok = mbar_wait_warp(bar_empty + 8 * s, (round - 1) & 1, abort_flag); PROF_END(0)
                     if (!ok) break;
+                    if (PAIR && rank == 0 && it >= kStages) mbar_arrive_cluster_elect(peer_empty + 8 * s); // (a second commit a slab costs the tensor pipe 30 cycles)
                     if (it >= ahead) load_weights(kt, s);
                     load_activations(kt, s);
                     issued = it + 1;
+                    if (PAIR && ++stage == kStages) stage = 0, phase ^= 1;
                 }
             }
             if (lane == 0) { PROF_FLUSH(0) }
+            if constexpr (PAIR) { // the last commits have reached this CTA's barriers before it may leave
+                for (uint32_t k = issued > kStages ? issued - kStages : 0; k < issued && ok; ++k) {
+                    ok = mbar_wait_warp(bar_empty + 8 * (k % kStages), (k / kStages) & 1, abort_flag);
+                    if (ok && rank == 0) mbar_arrive_cluster_elect(peer_empty + 8 * (k % kStages));
+                }
+            }
             if (!ok) {
                 if (lane == 0) {
                     *abort_flag = 1;
@@ -411,17 +569,32 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
             }
         }
-    } else if (warp == 1) {
+    } else if (PAIR && warp == 1 && rank) {
+        // ---------------------------------------------------------------- the other CTA of a pair: "my stage has landed"
+        const uint32_t leader_full = map_to_rank(bar_full, 0);
+        const uint32_t slabs = GEMM_TILE_FIRST < n_tiles_total ? ((n_tiles_total - GEMM_TILE_FIRST - 1) / (GEMM_TILE_STEP) + 1) * g.k_tiles : 0;
+        bool ok = true;
+        for (uint32_t it = 0; it < slabs && ok; ++it) {
+            const uint32_t s = it % kStages;
+            ok = mbar_wait_warp(bar_full + 8 * s, (it / kStages) & 1, abort_flag);
+            if (ok) mbar_arrive_cluster_elect(leader_full + 8 * s);
+        }
+        if (!ok && lane == 0) {
+            *abort_flag = 1;
+            atomicCAS(g.status + 1, 0, 116);
+        }
+    } else if ((PAIR ? threadIdx.x >> 5 : (uint32_t)warp) == 1) { // (see pair_slab_elect)
         // ---------------------------------------------------------------- MMA issuer (whole warp; one elected lane issues)
         {
             // kind::mxf4nvf4: A and B E2M1 (format 1), K-major, UE4M3 scales, N >> 3 at bit 17, M >> 4 at bit 24
-            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            uint32_t it = 0, local = 0;
+            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(((PAIR ? 2 : 1) * BM) >> 4) << 24);
+            const uint32_t peer_acc_full = PAIR ? map_to_rank(bar_acc_full, 1) : 0u;
+            uint32_t it = 0, local = 0, stage = 0, phase = 0;
             bool ok = true; PROF_DECL
             for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total && ok; tile += GEMM_TILE_STEP, ++local) {
                 // the accumulator is free again once the epilogue warps have read the previous tile out of it
                 if (local > 0) {
-                    PROF_BEGIN ok = mbar_wait_warp(bar_acc_empty, (local - 1) & 1, abort_flag); PROF_END(0)
+                    PROF_BEGIN ok = PAIR ? mbar_wait_pair_warp(bar_acc_empty, (local - 1) & 1, abort_flag) : mbar_wait_warp(bar_acc_empty, (local - 1) & 1, abort_flag); PROF_END(0)
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
@@ -432,6 +605,32 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     slices = g.grp_slices[(tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3])];
                     slice_end = g.k_tiles / slices; // (kept: a division a slab took the issuing warp longer than the slab's products)
                 }
+                if constexpr (PAIR) {
+                    // A pair's copies run beside the products only when the slab's are issued together in front of them
+                    // (512 cycles per slab in isolation, the four products' own time; three in front of each product 642).
+                    for (uint32_t kt = 0; kt < g.k_tiles; ++kt) {
+                        ok = mbar_wait_pair_warp(bar_full + 8 * stage, phase, abort_flag);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t st = base + stage * kStageBytes, sf = tmem + kSfCol + stage * kSfBufCols;
+                        const uint32_t sfa = st + kABytes + kBBytes, sfb = sfa + kSfaBytes;
+                        if (g.kt64 - 4 * kt >= 4) {
+                            pair_slab_elect(tmem, st, st + kABytes, idesc, sf, sfa, kt != 0, bar_empty + 8 * stage);
+                        } else { // the ragged end of a row
+                            const uint64_t da = operand_desc(st), db = operand_desc(st + kABytes);
+                            const uint32_t nkb = g.kt64 - 4 * kt;
+                            for (uint32_t kb = 0; kb < nkb; ++kb) {
+                                pair_cp_scales_elect(sf + 4 * kb, scale_desc(sfa + 512 * kb));
+                                pair_cp_scales_elect(sf + 16 + 8 * kb, scale_desc(sfb + 512 * kb));
+                                pair_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
+                            }
+                            for (uint32_t kb = 0; kb < nkb; ++kb)
+                                pair_mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, (kt | kb) != 0);
+                            pair_commit_elect(bar_empty + 8 * stage);
+                        }
+                        if (++stage == kStages) stage = 0, phase ^= 1;
+                    }
+                } else
                 for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
                     if constexpr (SLICED) {
                         if (kt == slice_end) { // (never true at the last slice's end, where the loop ends)
@@ -463,7 +662,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     }
                     mma_commit_elect(bar_empty + 8 * s); // the stage may be overwritten once these MMAs have read it
                 }
-                if (ok) mma_commit_elect(bar_acc_full);
+                if (ok) {
+                    if constexpr (PAIR) pair_commit_elect(bar_acc_full), pair_commit_elect(peer_acc_full);
+                    else mma_commit_elect(bar_acc_full);
+                }
             }
             if (lane == 0) { PROF_FLUSH(1) }
             if (!ok && lane == 0) {
@@ -482,7 +684,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const uint32_t quad = warp & 3;                 // the 32 accumulator lanes this warp may read
         const uint32_t part = (uint32_t)(warp - 2) >> 2; // which quarter of the output columns
         constexpr uint32_t kOutCols = DUAL ? BN / 2 : BN, kPartCols = kOutCols / 4, kStrips = kPartCols / 32;
-        uint32_t local = 0;
+        const uint32_t leader_acc_empty = PAIR ? map_to_rank(bar_acc_empty, 0) : 0u;
+        uint32_t local = 0, res_phase = 0;
         pdl_wait(); // the residual and row scales come from, and the outputs may still be read by, earlier kernels
         for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total; tile += GEMM_TILE_STEP, ++local) {
             uint32_t tile_m, tile_n;
@@ -490,14 +693,14 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             uint32_t n_out = g.n_out; // (of this tile's projection)
             void *y_out = g.y;
             float scale2 = g.scale2;
-            uint32_t slices = 1; // SLICED only
+            uint32_t slices = 1, grp = 0; // SLICED, GROUP only
             if constexpr (GROUP) {
-                const uint32_t p = (tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3]);
+                const uint32_t p = grp = (tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3]);
                 tile_n -= g.grp_tile0[p];
                 n_out = g.grp_n_out[p], y_out = g.grp_y[p], scale2 = g.grp_scale2[p];
                 if constexpr (SLICED) slices = g.grp_slices[p];
             }
-            const uint32_t tok = tile_m * BM + quad * 32 + lane, col0 = part * kPartCols, out0 = tile_n * kOutCols + col0;
+            const uint32_t tok = (PAIR ? 2 * tile_m + rank : tile_m) * BM + quad * 32 + lane, col0 = part * kPartCols, out0 = tile_n * kOutCols + col0;
             const bool live = tok < g.tokens && out0 < n_out;
             // rows whose pieces lie on 16 bytes, and on whole 32-byte sectors
             const bool is_f32 = g.y_dtype == MUSER_DTYPE_F32;
@@ -506,23 +709,39 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const bool wide = (align & 31) == 0 && (is_f32 || (n_out & 15) == 0);
             // the residual is fetched while the products still run: its first 64 bytes to registers, the others to L2
             uint32_t res[2][8];
-            const bool vec_res = !DUAL && !GROUP && vec && g.residual;
+            const bool vec_res = !PAIR && !DUAL && !GROUP && vec && g.residual;
             const uint8_t *res_at = reinterpret_cast<const uint8_t *>(g.residual) + ((size_t)tok * n_out + out0) * (is_f32 ? 4 : 2);
             auto load_res = [&](uint32_t piece) {
                 if (vec_res) ld_64(res_at + 64 * piece, wide, res);
             };
-            if constexpr (!DUAL && !GROUP) {
+            // PAIR: outputs leave (and the residual comes) through the warp's staging buffer, 64 bytes of 32 rows at a time.  Stored
+            // straight from the registers, a row per lane, a tile's outputs kept the load/store pipe for 4000 cycles, behind
+            // which the copies and products of the next tile could not be issued.
+            const uint32_t buf = out_base + (uint32_t)(warp - 2) * kOutPiece, row0 = tok - lane;
+            const CUtensorMap *map_y = &maps.y[0];
+            if constexpr (PAIR && GROUP) map_y = &maps.y[grp];
+            const bool staged_res = PAIR && !DUAL && !GROUP && g.residual;
+            auto fetch_piece = [&](uint32_t n0) { // (warp-uniform)
+                mbar_expect_tx_elect(bar_res + 8 * (warp - 2), kOutPiece);
+                tma_load_2d_elect(buf, &maps.residual, (int)n0, (int)row0, bar_res + 8 * (warp - 2));
+            };
+            if constexpr (PAIR && !QOUT) {
+                store_buffer_free();
+                if (staged_res && row0 < g.tokens && out0 < n_out) fetch_piece(out0);
+            }
+            if constexpr (!PAIR && !DUAL && !GROUP) {
                 load_res(0);
                 if (vec_res)
                     for (uint32_t at = 64; at < kPartCols * (is_f32 ? 4 : 2); at += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(res_at + at));
             }
             // (with a sleep between the polls: sixteen polling warps cost the SM power that the products could use)
-            bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64));
+            bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, PAIR ? 20 : 64));
             if (!ok) {
                 if (lane == 0) {
                     *abort_flag = 1;
                     atomicCAS(g.status + 1, 0, 103);
                 }
+                if (staged_res && row0 < g.tokens && out0 < n_out) mbar_wait_alone(bar_res + 8 * (warp - 2), res_phase); // (it is in flight)
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -571,7 +790,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
+            if (lane == 0) {
+                if constexpr (PAIR) mbar_arrive_cluster(leader_acc_empty);
+                else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
+            }
             if constexpr (CLUSTER) {
                 // (every stage has been consumed: the ring is scratch now)
                 if (tok < g.tokens) {
@@ -587,7 +809,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             if constexpr (QOUT) {
                 // rows of the last 128-token block that hold no token get zero scale bytes: the next GEMM reads the
                 // block's whole scale chunk (their codes come from TMA's zero fill)
-                if (out0 < n_out) {
+                if (out0 < n_out && (!PAIR || (2 * tile_m + rank) * BM < g.tokens)) { // (the plane ends with the last block that holds a token)
                     uint32_t q_scales = 0; // the two scale bytes of this thread's 32 outputs
                     if (tok < g.tokens) {
                         float v[32];
@@ -598,13 +820,96 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                             v[i] = __fdiv_rn(gate, 1.0f + expf(-gate)) * up;
                         }
                         uint8_t *codes = g.q_packed + (size_t)tok * (n_out / 2) + out0 / 2;
+                        const bool vec_codes = (reinterpret_cast<uintptr_t>(g.q_packed) & 15) == 0; // (rows are whole 32 bytes)
                         float(&lo)[16] = *reinterpret_cast<float(*)[16]>(&v[0]);
                         float(&hi)[16] = *reinterpret_cast<float(*)[16]>(&v[16]);
-                        q_scales = quantize_group(lo, g.q_isi, codes);
-                        q_scales |= quantize_group(hi, g.q_isi, codes + 8) << 8;
+                        uint4 packed;
+                        q_scales = quantize_group(lo, g.q_isi, packed.x, packed.y);
+                        q_scales |= quantize_group(hi, g.q_isi, packed.z, packed.w) << 8;
+                        if (vec_codes) {
+                            *reinterpret_cast<uint4 *>(codes) = packed;
+                        } else {
+                            *reinterpret_cast<uint2 *>(codes) = make_uint2(packed.x, packed.y);
+                            *reinterpret_cast<uint2 *>(codes + 8) = make_uint2(packed.z, packed.w);
+                        }
                     }
                     *reinterpret_cast<uint16_t *>(g.q_scales + swizzled_scale_offset(tok, out0 / 16, g.q_kt)) = (uint16_t)q_scales;
                 }
+                continue;
+            }
+            if constexpr (PAIR) {
+                auto leave = [&](auto type) {
+                    using T = decltype(type);
+                    constexpr int kCols = 64 / sizeof(T), kChunk = 16 / sizeof(T), kPieces = kPartCols / kCols;
+#pragma unroll
+                    for (int piece = 0; piece < kPieces; ++piece) {
+                        const uint32_t n0 = out0 + piece * kCols;
+                        if (row0 >= g.tokens || n0 >= n_out) break; // (the whole warp's)
+                        if (piece > 0) {
+                            store_buffer_free();
+                            if (staged_res) fetch_piece(n0);
+                        }
+                        if (staged_res) {
+                            if (!mbar_wait_warp(bar_res + 8 * (warp - 2), res_phase, abort_flag)) {
+                                if (lane == 0) {
+                                    *abort_flag = 1;
+                                    atomicCAS(g.status + 1, 0, 105);
+                                }
+                                ok = false;
+                                break;
+                            }
+                            res_phase ^= 1;
+                        }
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            float v[kChunk];
+#pragma unroll
+                            for (int i = 0; i < kChunk; ++i) {
+                                const int at = piece * kCols + c * kChunk + i;
+                                v[i] = __fmul_rn(__fmul_rn(__uint_as_float(r[at >> 5][at & 31]), scale2), g.inv_input_scale);
+                                if constexpr (DUAL) {
+                                    const float gate = __half2float(__float2half_rn(v[i]));
+                                    const float up = __half2float(__float2half_rn(__fmul_rn(__fmul_rn(__uint_as_float(r[1][at & 31]), g.scale2_up), g.inv_input_scale)));
+                                    v[i] = __fdiv_rn(gate, 1.0f + expf(-gate)) * up; // silu_fast, quant/helpers.rs:72
+                                }
+                                v[i] *= rs;
+                                if constexpr (TAIL) v[i] = logit_tail(v[i], g.out_scale, g.softcap);
+                            }
+                            const uint32_t at = buf + lane * 64 + ((c ^ ((lane >> 1) & 3)) * 16);
+                            uint32_t o[4], w[4] = {0, 0, 0, 0};
+                            if (staged_res) {
+                                const uint4 q = lds_16(at);
+                                w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+                            }
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                if constexpr (sizeof(T) == 4) {
+                                    o[i] = __float_as_uint(staged_res ? v[i] + __uint_as_float(w[i]) : v[i]);
+                                } else {
+                                    float a = v[2 * i], b = v[2 * i + 1];
+                                    if constexpr (std::is_same<T, __half>::value) {
+                                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[i]));
+                                        if (staged_res) a += f.x, b += f.y;
+                                        const __half2 packed = __floats2half2_rn(a, b);
+                                        o[i] = *reinterpret_cast<const uint32_t *>(&packed);
+                                    } else {
+                                        if (staged_res) a += __uint_as_float(w[i] << 16), b += __uint_as_float(w[i] & 0xFFFF0000u);
+                                        const __nv_bfloat162 packed = __floats2bfloat162_rn(a, b);
+                                        o[i] = *reinterpret_cast<const uint32_t *>(&packed);
+                                    }
+                                }
+                            }
+                            sts_16(at, o);
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                        tma_store_2d_elect(map_y, buf, (int)n0, (int)row0);
+                    }
+                };
+                if (is_f32) leave(float{});
+                else if (g.y_dtype == MUSER_DTYPE_BF16) leave(__nv_bfloat16{});
+                else leave(__half{});
+                if (!ok) break;
                 continue;
             }
 #pragma unroll
@@ -646,6 +951,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     }
+    if constexpr (PAIR && !QOUT) // the stores are done with the staging buffers
+        if (warp >= 2) asm volatile("{\n\t" MUSER_ELECT_PRED "@e cp.async.bulk.wait_group 0;\n\t}" ::: "memory");
     if constexpr (CLUSTER) {
         split_barrier();
         pdl_wait(); // (every warp stores here)
@@ -681,7 +988,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) {
+    if constexpr (PAIR) {
+        cluster_barrier(); // nothing of the pair is in flight towards this CTA any more
+        if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    } else if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
 }
@@ -691,348 +1001,6 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #undef GEMM_TILE_STEP
 #undef GEMM_KT_FIRST
 #undef GEMM_KT_END
-
-// ------------------------------------------------------------------------------------------ paired CTAs
-// The same GEMM on pairs of SMs (tcgen05 cta_group::2): a cluster of two CTAs owns a 256-token x 256-row output tile,
-// each CTA holding 128 of the tokens (its own accumulator, 128 lanes x 256 columns) and HALF of the weight rows of
-// every K slab; the tensor cores of the pair read both halves.  Per slab a CTA therefore fetches 16 KiB of
-// activations + 16 KiB of weights (+ 6 KiB of scale factors) for the same 128 x 256 x 256 of work that costs the
-// single-CTA kernel 48 + 6 KiB: the L2-to-SM traffic, which bounds that kernel, drops by 30 %.
-//
-// Roles as above, with the pair's hand-offs made of plain cluster instructions (no multicast of any kind):
-//   - every CTA loads its own operands (TMA, own mbarrier);
-//   - the follower (cluster rank 1) has one thread that waits for each of its stages to land and then arrives on the
-//     leader's barrier of that stage (mbarrier.arrive on the mapped address), so one wait in the leader covers the pair;
-//   - the leader (rank 0) issues the scale copies and the MMAs for both CTAs; "stage consumed" and "accumulator
-//     complete" are committed twice, once to its own barrier and once to the follower's;
-//   - the follower's epilogue warps hand the accumulator back by arriving on the leader's barrier.
-// All waits are bounded as in the single-CTA kernel; both CTAs meet at a cluster barrier before they free tensor
-// memory and leave, so no arrival can reach a CTA that is gone.
-constexpr int kPStages = 5;
-constexpr int kPBBytes = (BN / 2) * BK / 2; // 16 KiB: this CTA's half of the pair's 256 weight rows
-constexpr int kPStageBytes = kABytes + kPBBytes + kSfaBytes + kSfbBytes;
-constexpr int kPSmemBytes = kPStages * kPStageBytes + 1024 + 256;
-static_assert(kPSmemBytes <= 227 * 1024, "stage ring exceeds the shared memory of one CTA");
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t cta_addr, uint32_t rank) { // shared::cta address -> that CTA's window
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// mbar_wait for barriers that the other CTA of the pair arrives on.
-__device__ __forceinline__ bool mbar_wait_pair(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}"
-            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
-        if ((i & 1023u) == 1023u && *abort_flag) return false;
-    }
-    return false;
-}
-__device__ __forceinline__ void pair_commit(uint32_t cluster_addr) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void pair_cp_scales(uint32_t tmem_addr, uint64_t desc) {
-    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_addr), "l"(desc) : "memory");
-}
-__device__ __forceinline__ void pair_mma_nvf4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                              uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
-        : "memory");
-}
-
-__device__ __forceinline__ bool mbar_wait_pair_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, mbar_wait_pair(bar, parity, abort_flag));
-}
-__device__ __forceinline__ void mbar_arrive_cluster_elect(uint32_t cluster_addr) {
-    asm volatile("{\n\t" MUSER_ELECT_PRED "@e mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n\t}" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void pair_commit_elect(uint32_t cluster_addr) {
-    asm volatile("{\n\t" MUSER_ELECT_PRED "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void pair_cp_scales_elect(uint32_t tmem_addr, uint64_t desc) {
-    asm volatile("{\n\t" MUSER_ELECT_PRED "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n\t}" ::"r"(tmem_addr), "l"(desc) : "memory");
-}
-__device__ __forceinline__ void pair_mma_nvf4_elect(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                    uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t" MUSER_ELECT_PRED
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
-        : "memory");
-}
-
-template <bool DUAL, bool TAIL>
-__global__ void __launch_bounds__(352, 1)
-nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const __grid_constant__ CUtensorMap map_b2, const GemmArgs g) {
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t *aligned = smem_raw + (base - smem_u32(smem_raw));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(aligned + kPStages * kPStageBytes);
-    const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kPStages);
-    const uint32_t bar_acc_full = smem_u32(bars + 2 * kPStages), bar_acc_empty = smem_u32(bars + 2 * kPStages + 1);
-    const uint32_t bar_sf_full = smem_u32(bars + 2 * kPStages + 2), bar_sf_empty = smem_u32(bars + 2 * kPStages + 2 + kSfBufs);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kPStages + 2 + 2 * kSfBufs);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank(), leader = rank == 0;
-    const uint32_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const uint32_t m_blocks = (g.tokens + BM - 1) / BM;            // 128-token blocks (the rows of the scale image)
-    const uint32_t m_tiles = (m_blocks + 1) / 2, n_tiles_total = g.n_tiles * m_tiles;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kPStages; ++s) {
-            mbar_init(bar_full + 8 * s, leader ? 2 : 1); // leader: its own copies and the follower's "landed"
-            mbar_init(bar_empty + 8 * s, 1);
-        }
-        mbar_init(bar_acc_full, 1);
-        mbar_init(bar_acc_empty, 16); // one arrival per epilogue warp of the pair (used in the leader)
-        for (int b = 0; b < (int)kSfBufs; ++b) {
-            mbar_init(bar_sf_full + 8 * b, 1);
-            mbar_init(bar_sf_empty + 8 * b, 1);
-        }
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    __syncthreads();
-    cluster_barrier(); // both CTAs' barriers exist before anything arrives on them
-    if (warp == 1) {   // one warp of EACH CTA of the pair takes part in the paired allocation
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
-
-    if (warp == 0) {
-        // ---------------------------------------------------------------- producer (both CTAs; whole warp, one elected lane issues)
-        {
-            uint32_t it = 0, issued = 0;
-            bool ok = true; PROF_DECL
-            for (uint32_t tile = pair; tile < n_tiles_total && ok; tile += pairs) {
-                const uint32_t tile_m = tile % m_tiles, tile_n = tile / m_tiles;
-                const uint32_t m_block = 2 * tile_m + rank;
-                // a follower whose 128 tokens do not exist reads zero-filled activation boxes; its scale chunks
-                // come from block 0 so that the copy stays inside the scale image (the products are zero anyway)
-                const uint8_t *sfa = g.a_scales + (size_t)(m_block < m_blocks ? m_block : 0) * g.kt64 * 512;
-                const uint8_t *sfb0 = g.b_scales + (size_t)(DUAL ? tile_n : 2 * tile_n) * g.kt64 * 512;
-                const uint8_t *sfb1 = DUAL ? g.b2_scales + (size_t)tile_n * g.kt64 * 512 : sfb0 + (size_t)g.kt64 * 512;
-                // this CTA's half of the weight rows: the leader takes rows 0..127 of the tile (the gate rows of the
-                // fused form), the follower rows 128..255 (the up rows)
-                const CUtensorMap *mb = (DUAL && rank) ? &map_b2 : &map_b;
-                const int b_row = DUAL ? (int)(tile_n * (BN / 2)) : (int)(tile_n * BN + rank * (BN / 2));
-                for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
-                    const uint32_t s = it % kPStages, round = it / kPStages;
-                    PROF_BEGIN if (round > 0) ok = mbar_wait_pair_warp(bar_empty + 8 * s, (round - 1) & 1, abort_flag); PROF_END(0)
-                    if (!ok) break;
-                    const uint32_t st = base + s * kPStageBytes;
-                    const uint32_t full = bar_full + 8 * s;
-                    const uint32_t nkb = min(4u, g.kt64 - 4 * kt), sf_bytes = nkb * 512;
-                    mbar_expect_tx_elect(full, kABytes + kPBBytes + 3 * sf_bytes);
-                    tma_load_2d_elect(st, &map_a, (int)(kt * (BK / 2)), (int)(m_block * BM), full);
-                    tma_load_2d_elect(st + kABytes, mb, (int)(kt * (BK / 2)), b_row, full);
-                    bulk_load_elect(st + kABytes + kPBBytes, sfa + (size_t)kt * kSfaBytes, sf_bytes, full);
-                    bulk_load_elect(st + kABytes + kPBBytes + kSfaBytes, sfb0 + (size_t)kt * 2048, sf_bytes, full);
-                    bulk_load_elect(st + kABytes + kPBBytes + kSfaBytes + 2048, sfb1 + (size_t)kt * 2048, sf_bytes, full);
-                    issued = it + 1;
-                }
-            }
-            if (lane == 0) { PROF_FLUSH(0) }
-            if (!ok) {
-                if (lane == 0) {
-                    *abort_flag = 1;
-                    atomicCAS(g.status + 1, 0, 111);
-                }
-                // let the copies already in flight land before the CTA's shared memory goes away (bounded: the
-                // leader's phases also need the follower's arrival)
-                const uint32_t first = issued > (uint32_t)kPStages ? issued - kPStages : 0;
-                for (uint32_t k = first; k < issued; ++k) mbar_wait_alone(bar_full + 8 * (k % kPStages), (k / kPStages) & 1);
-            }
-        }
-    } else if (warp == 1) {
-        if (leader) {
-            // ---------------------------------------------------------------- MMA issuer (leader, for the pair; whole warp)
-            // M = 256 (128 rows in each CTA), N = 256: N >> 3 at bit 17, M >> 4 at bit 24
-            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
-            const uint32_t peer_empty = map_to_rank(bar_empty, 1), peer_acc_full = map_to_rank(bar_acc_full, 1);
-            uint32_t it = 0, local = 0;
-            bool ok = true; PROF_DECL
-            for (uint32_t tile = pair; tile < n_tiles_total && ok; tile += pairs, ++local) {
-                if (local > 0) {
-                    PROF_BEGIN ok = mbar_wait_pair_warp(bar_acc_empty, (local - 1) & 1, abort_flag); PROF_END(0)
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                }
-                for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
-                    const uint32_t s = it % kPStages, round = it / kPStages;
-                    PROF_BEGIN ok = mbar_wait_pair_warp(bar_full + 8 * s, round & 1, abort_flag); PROF_END(1)
-                    if (!ok) break;
-                    const uint32_t st = base + s * kPStageBytes;
-                    const uint64_t da = operand_desc(st), db = operand_desc(st + kABytes);
-                    const uint32_t nkb = min(4u, g.kt64 - 4 * kt);
-                    const uint32_t buf = it % kSfBufs, sf = tmem + kSfCol + buf * kSfBufCols;
-                    PROF_BEGIN ok = mbar_wait_warp(bar_sf_full + 8 * buf, (it / kSfBufs) & 1, abort_flag); PROF_END(2)
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (uint32_t kb = 0; kb < nkb; ++kb)
-                        pair_mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, (kt | kb) != 0);
-                    pair_commit_elect(bar_sf_empty + 8 * buf);
-                    pair_commit_elect(bar_empty + 8 * s);   // both CTAs may overwrite the stage once these MMAs have read it
-                    pair_commit_elect(peer_empty + 8 * s);
-                }
-                if (ok) {
-                    pair_commit_elect(bar_acc_full);
-                    pair_commit_elect(peer_acc_full);
-                }
-            }
-            if (lane == 0) { PROF_FLUSH(1) }
-            if (!ok && lane == 0) {
-                *abort_flag = 1;
-                atomicCAS(g.status + 1, 0, 112);
-            }
-        } else {
-            // ---------------------------------------------------------------- follower: "my stage has landed"
-            const uint32_t leader_full = map_to_rank(bar_full, 0);
-            uint32_t it = 0;
-            bool ok = true; PROF_DECL
-            for (uint32_t tile = pair; tile < n_tiles_total && ok; tile += pairs) {
-                for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
-                    const uint32_t s = it % kPStages, round = it / kPStages;
-                    PROF_BEGIN ok = mbar_wait_warp(bar_full + 8 * s, round & 1, abort_flag); PROF_END(0)
-                    if (!ok) break;
-                    mbar_arrive_cluster_elect(leader_full + 8 * s);
-                }
-            }
-            if (lane == 0) { PROF_FLUSH(3) }
-            if (!ok && lane == 0) {
-                *abort_flag = 1;
-                atomicCAS(g.status + 1, 0, 116);
-            }
-        }
-    } else if (warp == 10) {
-        // ---------------------------------------------------------------- scale copier (leader, for the pair)
-        if (leader) { // whole warp
-            uint32_t it = 0;
-            bool ok = true; PROF_DECL
-            for (uint32_t tile = pair; tile < n_tiles_total && ok; tile += pairs) {
-                for (uint32_t kt = 0; kt < g.k_tiles; ++kt, ++it) {
-                    const uint32_t s = it % kPStages, round = it / kPStages, buf = it % kSfBufs;
-                    PROF_BEGIN ok = mbar_wait_pair_warp(bar_full + 8 * s, round & 1, abort_flag); PROF_END(0)
-                    PROF_BEGIN if (ok && it >= kSfBufs) ok = mbar_wait_warp(bar_sf_empty + 8 * buf, ((it / kSfBufs) - 1) & 1, abort_flag); PROF_END(1)
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t st = base + s * kPStageBytes, sfa = st + kABytes + kPBBytes, sfb = sfa + kSfaBytes;
-                    const uint32_t sf = tmem + kSfCol + buf * kSfBufCols, nkb = min(4u, g.kt64 - 4 * kt);
-                    for (uint32_t kb = 0; kb < nkb; ++kb) { // each CTA copies from its own shared memory into its own tensor memory
-                        pair_cp_scales_elect(sf + 4 * kb, scale_desc(sfa + 512 * kb));
-                        pair_cp_scales_elect(sf + 16 + 8 * kb, scale_desc(sfb + 512 * kb));
-                        pair_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
-                    }
-                    pair_commit_elect(bar_sf_full + 8 * buf);
-                }
-            }
-            if (lane == 0) { PROF_FLUSH(2) }
-            if (!ok && lane == 0) {
-                *abort_flag = 1;
-                atomicCAS(g.status + 1, 0, 115);
-            }
-        }
-    } else {
-        // ---------------------------------------------------------------- epilogue (warps 2..9 of both CTAs)
-        const uint32_t quad = warp & 3;
-        const uint32_t part = (uint32_t)(warp - 2) >> 2;
-        constexpr uint32_t kOutCols = DUAL ? BN / 2 : BN, kPartCols = kOutCols / 2;
-        const uint32_t leader_acc_empty = map_to_rank(bar_acc_empty, 0);
-        uint32_t local = 0;
-        for (uint32_t tile = pair; tile < n_tiles_total; tile += pairs, ++local) {
-            const uint32_t tile_m = tile % m_tiles, tile_n = tile / m_tiles;
-            const bool ok = __all_sync(0xffffffffu, mbar_wait_pair(bar_acc_full, local & 1, abort_flag));
-            if (!ok) {
-                if (lane == 0) {
-                    *abort_flag = 1;
-                    atomicCAS(g.status + 1, 0, 113);
-                }
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tok = (2 * tile_m + rank) * BM + quad * 32 + lane;
-            const float rs = (g.row_scale && tok < g.tokens) ? g.row_scale[tok] : 1.0f;
-            const bool vec_ok = (g.n_out & 7) == 0 && ((reinterpret_cast<uintptr_t>(g.y) | reinterpret_cast<uintptr_t>(g.residual)) & 15) == 0;
-            const uint32_t lane_base = tmem + ((quad * 32) << 16), col0 = part * kPartCols;
-            uint32_t r[4][32]; // as in the single-CTA kernel: everything to registers, then the accumulator goes back
-#pragma unroll
-            for (uint32_t s = 0; s < 4; ++s)
-                tmem_ld32(lane_base + col0 + (DUAL ? (s & 1) * 32 + (s >> 1) * kOutCols : 32 * s), r[s]);
-            tmem_ld_wait();
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
-#pragma unroll
-            for (uint32_t s = 0; s < kPartCols / 32; ++s) {
-                const uint32_t c0 = col0 + 32 * s;
-                uint32_t(&cur)[32] = r[s];
-                uint32_t(&r_up)[32] = r[DUAL ? 2 + s : s];
-                const uint32_t n0 = tile_n * kOutCols + c0;
-                if (tok < g.tokens && n0 < g.n_out) {
-                    const size_t o = (size_t)tok * g.n_out + n0;
-                    const uint32_t valid = min(32u, g.n_out - n0);
-                    float v[32];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        v[i] = __fmul_rn(__fmul_rn(__uint_as_float(cur[i]), g.scale2), g.inv_input_scale);
-                        if constexpr (DUAL) {
-                            const float gate = __half2float(__float2half_rn(v[i]));
-                            const float up = __half2float(__float2half_rn(
-                                __fmul_rn(__fmul_rn(__uint_as_float(r_up[i]), g.scale2_up), g.inv_input_scale)));
-                            v[i] = __fdiv_rn(gate, 1.0f + expf(-gate)) * up;
-                        }
-                        v[i] *= rs;
-                        if constexpr (TAIL) v[i] = logit_tail(v[i], g.out_scale, g.softcap);
-                    }
-                    if (g.y_dtype == MUSER_DTYPE_F32)
-                        store_strip<float>(v, reinterpret_cast<float *>(g.y) + o,
-                                           g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
-                    else if (g.y_dtype == MUSER_DTYPE_BF16)
-                        store_strip<__nv_bfloat16>(v, reinterpret_cast<__nv_bfloat16 *>(g.y) + o,
-                                                   g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
-                    else
-                        store_strip<__half>(v, reinterpret_cast<__half *>(g.y) + o,
-                                            g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
-                }
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    cluster_barrier(); // nothing of the pair is in flight towards this CTA any more
-    if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
-}
 
 // Tensor-pipe ceiling for this instruction: every SM issues `iters` x 4 block-scaled FP4 MMAs (128 x 256 x 64 each)
 // on whatever its shared and tensor memory hold, with no loads, no scale copies and no epilogue.  The time of this
@@ -1232,28 +1200,51 @@ bool tma_make_map(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t row
 static bool make_map(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t row_bytes, uint32_t box_rows) {
     return tma_make_map(map, ptr, rows, row_bytes, box_rows, 128);
 }
+// A swizzled scale plane as one row of 8-byte elements per 128 operand rows; box = one slab's chunks (2048 bytes, zero fill).
+static bool make_scale_map(CUtensorMap *map, const void *ptr, uint64_t blocks, uint64_t kt64) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[2] = {kt64 * 64, blocks}, strides[1] = {kt64 * 512};
+    cuuint32_t box[2] = {256, 1}, elem[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void *>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// [tokens][n_out] outputs or residuals in boxes of 32 rows x 64 bytes, and whether they can be reached so.
+static bool pair_rows_fit(const void *y, const void *residual, uint64_t n_out, uint32_t y_dtype) {
+    return aligned16(y) && aligned16(residual) && n_out * (y_dtype == MUSER_DTYPE_F32 ? 4 : 2) % 16 == 0;
+}
+static bool make_out_map(CUtensorMap *map, const void *ptr, uint64_t tokens, uint64_t n_out, uint32_t y_dtype) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    const uint32_t size = y_dtype == MUSER_DTYPE_F32 ? 4 : 2;
+    cuuint64_t dims[2] = {n_out, tokens}, strides[1] = {n_out * size};
+    cuuint32_t box[2] = {64 / size, 32}, elem[2] = {1, 1};
+    return fn(map, size == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(ptr), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 muser_cuda_status nvfp4_build_tensor_map(Ctx *ctx, Weight *w) {
-    CUtensorMap *m = new CUtensorMap;
-    if (!make_map(m, w->packed, w->n_out_pad, w->n_in / 2, BN)) {
-        delete m;
-        return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the weight image");
+    struct Form {
+        void **slot;
+        bool scales;
+        uint32_t box_rows;
+    };
+    const Form forms[3] = {{&w->tmap_cache, false, BN}, {&w->tmap_half, false, BN / 2}, {&w->tmap_scales, true, 1}};
+    for (const Form &f : forms) {
+        CUtensorMap *m = new CUtensorMap;
+        *f.slot = m; // (freed with the weight)
+        if (!(f.scales ? make_scale_map(m, w->scales, w->n_out_pad / 128, w->n_in / 64) : make_map(m, w->packed, w->n_out_pad, w->n_in / 2, f.box_rows)))
+            return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the weight image");
     }
-    w->tmap_cache = m;
-    CUtensorMap *half = new CUtensorMap; // 128-row boxes, for the fused gate/up form
-    if (!make_map(half, w->packed, w->n_out_pad, w->n_in / 2, BN / 2)) {
-        delete half;
-        return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the weight image (128-row boxes)");
-    }
-    w->tmap_half = half;
     return MUSER_CUDA_OK;
 }
 
 void nvfp4_free_tensor_map(Weight *w) {
     delete reinterpret_cast<CUtensorMap *>(w->tmap_cache);
     delete reinterpret_cast<CUtensorMap *>(w->tmap_half);
-    w->tmap_cache = nullptr;
-    w->tmap_half = nullptr;
+    delete reinterpret_cast<CUtensorMap *>(w->tmap_scales);
+    w->tmap_cache = w->tmap_half = w->tmap_scales = nullptr;
 }
 
 // Token rows of an activation box.  A single token tile that is not full fetches whole 8-row swizzle atoms of its tokens
@@ -1303,11 +1294,80 @@ static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
     return 1;
 }
 
+// ------------------------------------------------------------------------------------------ paired CTAs
+// Clusters of two that the device holds at once, asked once and kept (a device that cannot say holds none).
+static uint32_t pair_room(Ctx *ctx) {
+    struct Room { int n = -1; };
+    static PerDevice<Room> rooms;
+    if (ctx->device < 0 || ctx->device >= kMaxDevices) return 0;
+    std::lock_guard<std::mutex> lock(rooms.mu);
+    Room &room = rooms.slot[ctx->device];
+    if (room.n < 0) {
+        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, false, true>;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(2 * 64), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kPSmemBytes, cfg.attrs = attr, cfg.numAttrs = 1;
+        cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kPSmemBytes);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&room.n, kernel, &cfg);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            room.n = 0;
+        }
+    }
+    return (uint32_t)std::max(0, std::min(room.n, ctx->sm_count / 2));
+}
+// Pairs of SMs or single CTAs for `n_tiles` weight-row tiles of `m_blocks` 128-token blocks?  The same bits either way.  A
+// round of pairs takes 0.86 to 0.93 of a round of single CTAs (us, single / pairs at 2048 tokens: 5120 x 5120 32.3 / 27.7,
+// 7168 x 5120 in a group 37.7 / 32.4, 5120 x 27648 138 / 120, gate/up 237 / 220), but an odd block of tokens is half of a
+// pair's tile (gate/up at 384 tokens, five rounds against six: 55 / 60).
+static bool takes_pairs(Ctx *ctx, uint32_t n_tiles, uint32_t m_blocks) {
+    if (ctx->nvfp4_pair != 2) return ctx->nvfp4_pair == 1;
+    const uint32_t room = pair_room(ctx);
+    if (!room) return false;
+    const uint64_t pair_rounds = ((uint64_t)n_tiles * ((m_blocks + 1) / 2) + room - 1) / room;
+    const uint64_t single_rounds = ((uint64_t)n_tiles * m_blocks + ctx->sm_count - 1) / ctx->sm_count;
+    return pair_rounds * 9 <= single_rounds * 10;
+}
+template <bool DUAL, bool TAIL, bool QOUT, bool GROUP>
+static cudaError_t launch_pairs(Ctx *ctx, const CUtensorMap &map_a, const GemmMaps &maps, const GemmArgs &g, cudaStream_t stream) {
+    const auto kernel = nvfp4_gemm_kernel<DUAL, TAIL, QOUT, GROUP, false, true>;
+    const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kPSmemBytes);
+    if (e != cudaSuccess) return e;
+    const uint32_t room = pair_room(ctx);
+    if (!room) return cudaErrorNotSupported;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(2 * std::min(room, g.n_tiles * ((g.tokens + 2 * BM - 1) / (2 * BM))));
+    cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kPSmemBytes, cfg.stream = stream, cfg.attrs = attr, cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, map_a, maps, g);
+}
+
+// Token tiles (of 128, or of 256 where pairs take them) per raster group: about 32 MB of activations, at least 8 x 128 tokens.
+static uint32_t raster_group(Ctx *ctx, const Weight *w, uint32_t m_blocks, bool pair) {
+    const uint64_t tile_bytes = (uint64_t)BM * (w->n_in / 2 + w->n_in / 16);
+    uint32_t gm = (uint32_t)std::max<uint64_t>(8, (32ull << 20) / std::max<uint64_t>(1, tile_bytes));
+    if (ctx->nvfp4_group_m) gm = ctx->nvfp4_group_m;
+    gm = std::max<uint32_t>(1, std::min<uint32_t>(gm, m_blocks));
+    return pair ? (gm + 1) / 2 : gm;
+}
+
 muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_packed, const uint8_t *x_scales, void *y,
                                     uint32_t y_dtype, uint32_t tokens, const Epilogue &ep, cudaStream_t stream,
                                     const Weight *w_up, const NvFp4Out *qout) {
+    const uint32_t m_blocks = (tokens + BM - 1) / BM, n_tiles = w_up ? (uint32_t)((w->n_out + BN / 2 - 1) / (BN / 2)) : (uint32_t)(w->n_out_pad / BN);
+    const bool tail = ep.out_scale != 1.0f || ep.softcap > 0.0f;
+    const uint32_t ks = w_up || tail || ctx->nvfp4_pair == 1 ? 1 : gemm_ksplit(ctx, w, tokens);
+    const bool pair = ks == 1 && takes_pairs(ctx, n_tiles, m_blocks) && (qout || pair_rows_fit(y, ep.residual, w->n_out, y_dtype));
+    const uint32_t a_rows = pair ? BM : box_tokens(tokens);
     CUtensorMap map_a;
-    if (!make_map(&map_a, x_packed, tokens, w->n_in / 2, ctx->nvfp4_pair ? BM : box_tokens(tokens)))
+    GemmMaps maps;
+    if (!make_map(&map_a, x_packed, tokens, w->n_in / 2, a_rows) || (pair && !make_scale_map(&maps.a_scales, x_scales, m_blocks, w->n_in / 64)))
         return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the activations");
     GemmArgs g;
     g.a_scales = x_scales;
@@ -1320,7 +1380,7 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     g.residual = ep.residual;
     g.status = ctx->dev_status;
     g.tokens = tokens;
-    g.a_bytes = (ctx->nvfp4_pair ? BM : box_tokens(tokens)) * (BK / 2);
+    g.a_bytes = a_rows * (BK / 2);
     g.ksplit = 1;
     g.n_out = (uint32_t)w->n_out;
     g.k_tiles = (uint32_t)((w->n_in + BK - 1) / BK);
@@ -1329,67 +1389,28 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     g.scale2 = w->scale2;
     g.scale2_up = w_up ? w_up->scale2 : 0.0f;
     g.inv_input_scale = 1.0f / w->input_scale_inv;
-    g.n_tiles = w_up ? (uint32_t)((w->n_out + BN / 2 - 1) / (BN / 2)) : (uint32_t)(w->n_out_pad / BN);
+    g.n_tiles = n_tiles;
     g.q_packed = qout ? qout->packed : nullptr;
     g.q_scales = qout ? qout->scales : nullptr;
     g.q_isi = qout ? qout->input_scale_inv : 0.0f;
     g.q_kt = (uint32_t)(w->n_out / 64);
-    {   // raster groups of about 32 MB of activations (at least 8 token tiles)
-        const uint64_t tile_bytes = (uint64_t)BM * (w->n_in / 2 + w->n_in / 16);
-        uint32_t gm = (uint32_t)std::max<uint64_t>(8, (32ull << 20) / std::max<uint64_t>(1, tile_bytes));
-        if (ctx->nvfp4_group_m) gm = ctx->nvfp4_group_m;
-        g.group_m = std::max<uint32_t>(1, std::min<uint32_t>(gm, (tokens + BM - 1) / BM));
-    }
+    g.group_m = raster_group(ctx, w, m_blocks, pair);
     if (qout && (!w_up || w->n_out % 64)) return fail(ctx, MUSER_CUDA_BAD_SHAPE, "quantized outputs come from the fused gate/up form, with n_out % 64 == 0");
-    const CUtensorMap &mb = *reinterpret_cast<const CUtensorMap *>(w_up ? w->tmap_half : w->tmap_cache);
-    const CUtensorMap &mb2 = w_up ? *reinterpret_cast<const CUtensorMap *>(w_up->tmap_half) : mb;
-    const bool tail = ep.out_scale != 1.0f || ep.softcap > 0.0f;
-    const uint32_t m_blocks = (tokens + BM - 1) / BM;
-    // Pairs of SMs on 256-token tiles are opt-in: the pair halves the operand traffic per SM, but this GEMM is bound
-    // by the scale-factor copies into tensor memory, which a pair does not reduce, and the pair's hand-offs cost more
-    // than its traffic saves (ffn_gate at 2048 tokens: 2.4 against 2.8 PFLOP/s).
-    const bool pair = ctx->nvfp4_pair == 1 && !qout;
+    // (the fused form's boxes hold 128 rows of either weight, a pair's the 128 rows of one CTA)
+    maps.b[0] = *reinterpret_cast<const CUtensorMap *>(w_up || pair ? w->tmap_half : w->tmap_cache);
+    if (w_up) maps.b[1] = *reinterpret_cast<const CUtensorMap *>(w_up->tmap_half);
     if (pair) {
-        struct PairLimit { int n[3] = {0, 0, 0}; };
-        static PerDevice<PairLimit> max_pairs; // co-resident clusters of two, asked once per device and kernel
-        const void *kfn = w_up ? reinterpret_cast<const void *>(nvfp4_gemm_pair_kernel<true, false>)
-                          : tail ? reinterpret_cast<const void *>(nvfp4_gemm_pair_kernel<false, true>)
-                                 : reinterpret_cast<const void *>(nvfp4_gemm_pair_kernel<false, false>);
-        MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(kfn, ctx->device, kPSmemBytes));
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-        cfg.blockDim = dim3(352), cfg.dynamicSmemBytes = kPSmemBytes, cfg.stream = stream, cfg.attrs = attr, cfg.numAttrs = 1;
-        int cached;
-        {
-            std::lock_guard<std::mutex> lock(max_pairs.mu);
-            int &slot = max_pairs.slot[ctx->device].n[w_up ? 1 : tail ? 2 : 0];
-            if (slot == 0) {
-                cfg.gridDim = dim3(2 * (ctx->sm_count / 2));
-                int n = 0;
-                MUSER_CUDA_TRY(ctx, cudaOccupancyMaxActiveClusters(&n, kfn, &cfg));
-                if (n < 1) return fail(ctx, MUSER_CUDA_ERROR, "no cluster of two CTAs of the paired NVFP4 GEMM fits on this device");
-                slot = n;
-            }
-            cached = slot;
-        }
-        const uint32_t pair_tiles = g.n_tiles * ((m_blocks + 1) / 2);
-        const uint32_t pairs = std::min<uint32_t>(pair_tiles, std::min<uint32_t>((uint32_t)cached, (uint32_t)ctx->sm_count / 2));
-        cfg.gridDim = dim3(2 * pairs);
-        // every CTA of a pair fetches 128 weight rows per slab: the maps with 128-row boxes, in both forms
-        const CUtensorMap &half = *reinterpret_cast<const CUtensorMap *>(w->tmap_half);
-        const CUtensorMap &half_up = w_up ? *reinterpret_cast<const CUtensorMap *>(w_up->tmap_half) : half;
-        if (w_up)
-            MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel<true, false>, map_a, half, half_up, g));
-        else if (tail)
-            MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel<false, true>, map_a, half, half_up, g));
-        else
-            MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel<false, false>, map_a, half, half_up, g));
+        maps.b_scales[0] = *reinterpret_cast<const CUtensorMap *>(w->tmap_scales);
+        if (w_up) maps.b_scales[1] = *reinterpret_cast<const CUtensorMap *>(w_up->tmap_scales);
+        if (!qout && (!make_out_map(&maps.y[0], y, tokens, w->n_out, y_dtype) || (ep.residual && !make_out_map(&maps.residual, ep.residual, tokens, w->n_out, y_dtype))))
+            return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the outputs");
+        MUSER_CUDA_TRY(ctx, qout   ? (launch_pairs<true, false, true, false>(ctx, map_a, maps, g, stream))
+                            : w_up ? (launch_pairs<true, false, false, false>(ctx, map_a, maps, g, stream)) // (the fused FFN form has no tail)
+                            : tail ? (launch_pairs<false, true, false, false>(ctx, map_a, maps, g, stream))
+                                   : (launch_pairs<false, false, false, false>(ctx, map_a, maps, g, stream)));
         return MUSER_CUDA_OK;
     }
     const uint32_t tiles = g.n_tiles * m_blocks;
-    const uint32_t ks = w_up || tail ? 1 : gemm_ksplit(ctx, w, tokens);
     if (ks > 1) {
         g.ksplit = ks;
         const auto kernel = nvfp4_gemm_kernel<false, false, false, false, true>;
@@ -1402,7 +1423,7 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
         attr[1].val.clusterDim.x = ks, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         cfg.gridDim = dim3(tiles * ks), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kSmemBytes, cfg.stream = stream;
         cfg.attrs = attr, cfg.numAttrs = 2;
-        MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, map_a, mb, mb, mb, mb, g));
+        MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, map_a, maps, g));
         return MUSER_CUDA_OK;
     }
     const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
@@ -1414,13 +1435,13 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     if (qout) {
         const void *qfn = reinterpret_cast<const void *>(nvfp4_gemm_kernel<true, false, true>);
         MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(qfn, ctx->device, kSmemBytes));
-        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<true, false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g));
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<true, false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, maps, g));
     } else if (w_up)
-        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<true, false>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g)); // (the fused FFN form has no tail)
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<true, false>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, maps, g)); // (the fused FFN form has no tail)
     else if (tail)
-        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g));
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, true>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, maps, g));
     else
-        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, false>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, mb, mb2, mb, mb, g));
+        MUSER_CUDA_TRY(ctx, launch_pdl(nvfp4_gemm_kernel<false, false>, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, maps, g));
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
     return MUSER_CUDA_OK;
 }
@@ -1453,7 +1474,7 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     const Weight *w0 = ws[0];
     uint32_t slices[4] = {1, 1, 1, 1}; // (the paired kernel, which serves single calls where it is on, never splits)
     bool sliced = false;
-    for (uint32_t p = 0; p < n && !ctx->nvfp4_pair; ++p) slices[p] = gemm_ksplit(ctx, ws[p], tokens), sliced = sliced || slices[p] > 1;
+    for (uint32_t p = 0; p < n && ctx->nvfp4_pair != 1; ++p) slices[p] = gemm_ksplit(ctx, ws[p], tokens), sliced = sliced || slices[p] > 1;
     if (sliced && !group_in_one_launch(slices, ws, n, tokens, ctx->sm_count)) {
         const Weight *rest[4];
         void *rest_y[4];
@@ -1468,22 +1489,33 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
         }
         return n_rest ? launch_nvfp4_gemm_group(ctx, rest, n_rest, x_packed, x_scales, rest_y, y_dtype, tokens, stream) : MUSER_CUDA_OK;
     }
+    const uint32_t m_blocks = (tokens + BM - 1) / BM;
+    uint32_t tiles_n = 0;
+    for (uint32_t p = 0; p < n; ++p) tiles_n += (uint32_t)(ws[p]->n_out_pad / BN);
+    bool pair = !sliced && takes_pairs(ctx, tiles_n, m_blocks);
+    for (uint32_t p = 0; p < n; ++p) pair = pair && pair_rows_fit(ys[p], nullptr, ws[p]->n_out, y_dtype);
+    const uint32_t a_rows = pair ? BM : box_tokens(tokens);
     CUtensorMap map_a;
-    if (!make_map(&map_a, x_packed, tokens, w0->n_in / 2, box_tokens(tokens)))
+    GemmMaps maps;
+    if (!make_map(&map_a, x_packed, tokens, w0->n_in / 2, a_rows) || (pair && !make_scale_map(&maps.a_scales, x_scales, m_blocks, w0->n_in / 64)))
         return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the activations");
     GemmArgs g = {};
     g.a_scales = x_scales;
     g.status = ctx->dev_status;
     g.tokens = tokens;
-    g.a_bytes = box_tokens(tokens) * (BK / 2);
+    g.a_bytes = a_rows * (BK / 2);
     g.ksplit = 1;
     g.k_tiles = (uint32_t)((w0->n_in + BK - 1) / BK);
     g.kt64 = (uint32_t)(w0->n_in / 64);
     g.y_dtype = y_dtype;
     g.out_scale = 1.0f;
     g.inv_input_scale = 1.0f / w0->input_scale_inv;
-    uint32_t tiles_n = 0;
+    tiles_n = 0;
     for (uint32_t p = 0; p < 4; ++p) {
+        maps.b[p] = *reinterpret_cast<const CUtensorMap *>(pair ? ws[p < n ? p : 0]->tmap_half : ws[p < n ? p : 0]->tmap_cache);
+        if (pair) maps.b_scales[p] = *reinterpret_cast<const CUtensorMap *>(ws[p < n ? p : 0]->tmap_scales);
+        if (pair && p < n && !make_out_map(&maps.y[p], ys[p], tokens, ws[p]->n_out, y_dtype))
+            return fail(ctx, MUSER_CUDA_ERROR, "cuTensorMapEncodeTiled failed for the outputs");
         g.grp_tile0[p] = tiles_n;
         if (p >= n) continue;
         g.grp_b_scales[p] = ws[p]->scales;
@@ -1497,19 +1529,16 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     for (uint32_t p = n; p < 4; ++p) g.grp_tile0[p] = tiles_n; // no tile falls into a projection that is not there
     g.n_tiles = tiles_n;
     g.n_out = g.grp_n_out[0], g.y = g.grp_y[0], g.scale2 = g.grp_scale2[0], g.b_scales = g.grp_b_scales[0];
-    {
-        const uint64_t tile_bytes = (uint64_t)BM * (w0->n_in / 2 + w0->n_in / 16);
-        uint32_t gm = (uint32_t)std::max<uint64_t>(8, (32ull << 20) / std::max<uint64_t>(1, tile_bytes));
-        if (ctx->nvfp4_group_m) gm = ctx->nvfp4_group_m;
-        g.group_m = std::max<uint32_t>(1, std::min<uint32_t>(gm, (tokens + BM - 1) / BM));
+    g.group_m = raster_group(ctx, w0, m_blocks, pair);
+    if (pair) {
+        MUSER_CUDA_TRY(ctx, (launch_pairs<false, false, false, true>(ctx, map_a, maps, g, stream)));
+        return MUSER_CUDA_OK;
     }
-    const CUtensorMap *maps[4];
-    for (uint32_t p = 0; p < 4; ++p) maps[p] = reinterpret_cast<const CUtensorMap *>(ws[p < n ? p : 0]->tmap_cache);
-    const uint32_t tiles = tiles_n * ((tokens + BM - 1) / BM);
+    const uint32_t tiles = tiles_n * m_blocks;
     const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
     const auto kernel = sliced ? nvfp4_gemm_kernel<false, false, false, true, true> : nvfp4_gemm_kernel<false, false, false, true>;
     MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes));
-    MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, *maps[0], *maps[1], *maps[2], *maps[3], g));
+    MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, maps, g));
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
     return MUSER_CUDA_OK;
 }

@@ -595,3 +595,47 @@ def test_grouped_projections_equal_the_single_calls(gpu, shapes, n_in, tokens):
         k.encode_nvfp4_group_prequant([ws[0], w_isi], xp, xs, [grouped[0], y], tokens)
     with pytest.raises(op.MuserCudaError):
         k.encode_nvfp4_group_prequant([ws[0]], xp, xs, [grouped[0]], tokens)
+
+
+@pytest.mark.parametrize("n_in", [64, 320, 1088, 5120])
+@pytest.mark.parametrize("tokens", [1, 97, 129, 385, 640])
+def test_paired_forms_equal_the_single_sm_forms(gpu, n_in, tokens):
+    """Pairs of SMs against single CTAs, bit for bit: a group of projections of different row counts (one past a tile's
+    end, one a tile, one with an odd 128-row block), the SwiGLU that leaves quantized, residuals of each type through the
+    staging buffers, in place as well, and rows that are not whole 16 bytes (which pairs do not take); a row shorter than a
+    slab, ragged slabs, an odd 128-token block and less than one."""
+    from muser_b200 import synth
+    from muser_b200._lib import TUNE_NVFP4_PAIR
+    op, ctx, k = gpu
+    x = synth.normal_activations(tokens, n_in, seed=21)
+    isi = synth.activation_input_scale_inv(x)
+    ws = []
+    for i, n_out in enumerate((296, 256, 384, 300)):
+        packed, scales, scale2 = make_weight(op, ctx, n_out, n_in, seed=40 + i)
+        ws.append(op.Weight(ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, scale2, isi)))
+    xp, xs = k.quantize_nvfp4_activation(x.cuda(), isi)
+    out = {}
+    try:
+        for mode in (0, 1):
+            ctx.tuning_set(TUNE_NVFP4_PAIR, mode)
+            got = []
+            for dt in (torch.float32, torch.float16, torch.bfloat16):
+                ys = [torch.full((tokens, w.n_out), float("nan"), dtype=dt, device="cuda") for w in ws]
+                k.encode_nvfp4_group_prequant(ws[:3], xp, xs, ys[:3], tokens)
+                g = torch.Generator("cuda").manual_seed(7)
+                res = torch.randn((tokens, ws[0].n_out), device="cuda", generator=g).to(dt)
+                y_res, in_place = torch.empty_like(res), res.clone()
+                k.encode_nvfp4_prequant(ws[0], xp, xs, y_res, tokens, residual=res)
+                k.encode_nvfp4_prequant(ws[0], xp, xs, in_place, tokens, residual=in_place)
+                k.encode_nvfp4_prequant(ws[3], xp, xs, ys[3], tokens)
+                assert torch.equal(y_res, in_place)
+                got += ys + [y_res]
+            got += list(k.encode_nvfp4_ffn_gate_up_silu_requant(ws[2], ws[2], xp, xs, tokens, 3.0))
+            ctx.sync_status()
+            out[mode] = [y.cpu() for y in got]
+    finally:
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 0)
+    for i, (a, b) in enumerate(zip(out[0], out[1])):
+        assert torch.equal(a, b), f"output {i} differs between the two forms"
+    for w in ws:
+        w.free()
