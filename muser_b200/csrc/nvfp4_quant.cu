@@ -202,6 +202,126 @@ static cudaError_t launch_rms_rows_sequential(Ctx *ctx, const void *x, uint32_t 
     return launch_pdl(f32 ? rms_rows_sequential_kernel<true> : rms_rows_sequential_kernel<false>, dim3(blocks), dim3(32), smem, stream, x, tokens, n_in, eps, inv_rms);
 }
 
+// ---- the chain without its latency ----------------------------------------------------------------------------------
+// A chain of n dependent additions takes 4 cycles each at best.  A block cuts the row into one segment per thread.  While
+// the running sum S stays inside one binade, adding a square moves S's bit pattern by a whole number of units that
+// depends on the square and, for a tie, on whether the pattern is even; so a whole segment acts on the pattern as
+// "add `even` if it is even, `odd` if it is odd", and two chains of the segment's own squares, from the bottom of the binade
+// and from one unit above it, give the two numbers.  The binade is guessed from a parallel prefix sum.  Segments of one
+// binade that follow one another in a warp are composed by a scan; one warp then walks the warps' runs, checks for each
+// that S was in the guessed binade before and is after (S never falls, so it was in between), and adds the squares of a
+// segment that fails one by one: one or two per power of two that the sum passes.  The sum that results is the chain's.
+constexpr int kChainThreads = 1024; // most threads of a block, one segment each
+struct ChainShared {
+    uint2 add[kChainThreads];      // per thread: its run's units up to and with its segment, from an even and an odd pattern
+    uint32_t binade[kChainThreads]; // exponent field that the segment's additions hold for, kNoBinade: one by one
+    uint32_t starts[32];           // per warp: the lanes that begin a run
+    float warp_sum[32];
+    float inv_rms;
+};
+constexpr uint32_t kNoBinade = 256;
+__device__ __forceinline__ uint2 chain_compose(uint2 first, uint2 then) {
+    return make_uint2(first.x + ((first.x & 1) ? then.y : then.x), first.y + ((first.y & 1) ? then.x : then.y)); // (odd + odd: even)
+}
+// 1 / sqrt(mean(x^2) + eps) of one row of n_in <= 8 K blockDim values, for every thread of the block.
+template <bool XF32, int K>
+__device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, float eps, ChainShared &sh) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5, n8 = n_in / 8;
+    float v[K][8];
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[i][k] = 0.0f; // (zeros leave any sum as it is)
+        if (tid * K + i < n8) load8<XF32>(xr, tid * K + i, v[i]);
+    }
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[i][k] = __fmul_rn(v[i][k], v[i][k]), sum += v[i][k];
+    float after = sum; // of the segments up to and including this one
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, after, o);
+        if (lane >= (uint32_t)o) after += up;
+    }
+    float before = __shfl_up_sync(0xffffffffu, after, 1);
+    if (lane == 0) before = 0.0f;
+    if (lane == 31) sh.warp_sum[warp] = after;
+    __syncthreads();
+    float carry = 0.0f;
+    for (uint32_t w = 0; w < warp; ++w) carry += sh.warp_sum[w];
+    before += carry, after += carry;
+    uint32_t binade = __float_as_uint(before) >> 23; // (sums of squares: no sign; infinities and NaN are 255)
+    if (binade != __float_as_uint(after) >> 23 || binade == 255) binade = kNoBinade;
+    uint2 add = make_uint2(0, 0);
+    if (binade != kNoBinade) {
+        const uint32_t bottom = binade << 23;
+        float even = __uint_as_float(bottom), odd = __uint_as_float(bottom + 1);
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) even = __fadd_rn(even, v[i][k]), odd = __fadd_rn(odd, v[i][k]);
+        add = make_uint2(__float_as_uint(even) - bottom, __float_as_uint(odd) - (bottom + 1));
+    }
+    const uint32_t left = __shfl_up_sync(0xffffffffu, binade, 1);
+    const uint32_t starts = __ballot_sync(0xffffffffu, lane == 0 || binade != left || binade == kNoBinade);
+    const uint32_t start = 31 - __clz(starts & (0xffffffffu >> (31 - lane))); // of this lane's run
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint2 l = make_uint2(__shfl_up_sync(0xffffffffu, add.x, o), __shfl_up_sync(0xffffffffu, add.y, o));
+        if (lane >= start + o) add = chain_compose(l, add);
+    }
+    sh.add[tid] = add, sh.binade[tid] = binade;
+    if (lane == 0) sh.starts[warp] = starts;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t s = 0; // the running sum's bit pattern, the same in every lane
+        const auto step = [&](uint32_t e, uint32_t even, uint32_t odd) {
+            const uint32_t next = s + ((s & 1) ? odd : even);
+            const bool holds = (s >> 23) == e && (next >> 23) == e;
+            if (holds) s = next;
+            return holds;
+        };
+        // what there is to know of a warp that is one run, a warp per lane
+        const uint32_t w_starts = lane < warps ? sh.starts[lane] : 0u, w_last = min(lane, warps - 1) * 32 + 31;
+        const uint32_t w_binade = sh.binade[w_last];
+        const uint2 w_add = sh.add[w_last];
+        for (uint32_t w = 0; w < warps; ++w) {
+            uint32_t runs = __shfl_sync(0xffffffffu, w_starts, w);
+            const uint32_t e = __shfl_sync(0xffffffffu, w_binade, w), x = __shfl_sync(0xffffffffu, w_add.x, w), y = __shfl_sync(0xffffffffu, w_add.y, w);
+            if (runs == 1 && step(e, x, y)) continue;
+            const uint2 my_add = sh.add[w * 32 + lane];
+            const uint32_t my_binade = sh.binade[w * 32 + lane];
+            for (uint32_t pos = 0; pos < 32;) {
+                const uint32_t rest = runs & ~(0xffffffffu >> (31 - pos)); // starts behind `pos`
+                const uint32_t end = rest ? __ffs(rest) - 1 : 32;
+                const uint32_t re = __shfl_sync(0xffffffffu, my_binade, end - 1);
+                const uint32_t rx = __shfl_sync(0xffffffffu, my_add.x, end - 1), ry = __shfl_sync(0xffffffffu, my_add.y, end - 1);
+                if (((runs >> pos) & 1) && step(re, rx, ry)) {
+                    pos = end;
+                    continue;
+                }
+                float t = __uint_as_float(s);
+#pragma unroll
+                for (int i = 0; i < K; ++i) {
+                    const uint32_t i8 = (w * 32 + pos) * K + i;
+                    float q[8];
+                    if (i8 >= n8) break;
+                    load8<XF32>(xr, i8, q);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) t = __fadd_rn(t, __fmul_rn(q[k], q[k]));
+                }
+                s = __float_as_uint(t);
+                ++pos;
+            }
+        }
+        if (lane == 0) sh.inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(__uint_as_float(s), (float)n_in), eps)));
+    }
+    __syncthreads();
+    return sh.inv_rms;
+}
+
 // (x * inv_rms) * w of one row, quantized group by group by the whole block; rows past `tokens` only clear their scales.
 template <bool XF32>
 __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
@@ -230,146 +350,48 @@ __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, 
     }
 }
 
-// The same quantizer behind a fused input RMSNorm (reference.rs:59-80): one block per token row adds the row's squares as
-// rms_norm does, FRONT TO BACK in f32 with one rounding per step (why that order: rms_rows_sequential_kernel), and
-// quantizes (x * inv_rms) * w group by group.
-//
-// A chain of n dependent additions takes 4 cycles each at best.  It is cut into 128 segments, one per thread.  While the
-// running sum S stays inside one binade, adding s moves S up by a whole number of units u of its last place:
-// s / u rounded to nearest, where a tie goes by the parity of S / u.  So a segment acts on S's bit pattern as "add c0 if S is
-// even, c1 if odd", which its thread can work out without S, given the binade.  The binade is guessed from a parallel
-// prefix sum; then one warp walks the 128 segments, checks for each that S was in the guessed binade before and is
-// after (else it adds that segment's squares one by one: about one segment per power of two that the sum passes), and
-// ends with exactly the chain's sum.  Up to 500 rows of 5120 values: 31 us for the chain kernel and 3 to 5 for a quantizer
-// behind it -> 15 to 19 (a layer at 16 tokens 202 -> 145 us, together with the launches that follow one another closer).
-constexpr int kNormThreads = 128;
-template <bool XF32>
-__global__ void __launch_bounds__(kNormThreads) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
-                                                                           const float *norm_w, float eps, uint32_t keep, uint8_t *packed,
-                                                                           uint8_t *scales) {
-    extern __shared__ float4 norm_squares[]; // n_in squares, if they fit
-    __shared__ float warp_sum[kNormThreads / 32];
-    __shared__ uint2 seg_add[kNormThreads];
-    __shared__ uint32_t seg_binade[kNormThreads]; // exponent field the additions hold for, 0: one by one
-    __shared__ float inv_rms;
-    const uint32_t row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+// The same quantizer behind a fused input RMSNorm (reference.rs:59-80): one block per token row takes the row's factor
+// (chain_inv_rms) and quantizes (x * inv_rms) * w group by group.
+template <bool XF32, int K>
+__global__ void __launch_bounds__(kChainThreads) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
+                                                                            const float *norm_w, float eps, uint8_t *packed, uint8_t *scales) {
+    __shared__ ChainShared sh;
+    const uint32_t row = blockIdx.x;
     // the norm weights are read last, from L2 if they are asked for now (between two layers' weights they go to memory)
-    if (row < tokens)
-        for (uint32_t i = 32 * tid; i < n_in; i += 32 * kNormThreads) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + i));
+    if (row < min(tokens, 16u))
+        for (uint32_t i = 32 * threadIdx.x; i < n_in; i += 32 * blockDim.x) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + i));
     pdl_wait();
     pdl_release();
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
-    float inv = 0.0f;
-    if (row < tokens) { // (uniform over the block)
-        const uint32_t len8 = (n_in / 8 + kNormThreads - 1) / kNormThreads; // eights per segment
-        const uint32_t first8 = min(tid * len8, n_in / 8), end8 = min(first8 + len8, n_in / 8);
-        float sum = 0.0f;
-        for (uint32_t i = first8; i < end8; ++i) {
-            float v[8];
-            load8<XF32>(xr, i, v);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(v[k], v[k]), sum += v[k];
-            if (keep) {
-                norm_squares[2 * i] = make_float4(v[0], v[1], v[2], v[3]);
-                norm_squares[2 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
-            }
-        }
-        auto squares = [&](uint32_t i, float (&v)[8]) {
-            if (keep) {
-                const float4 p = norm_squares[2 * i], q = norm_squares[2 * i + 1];
-                v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = p.w, v[4] = q.x, v[5] = q.y, v[6] = q.z, v[7] = q.w;
-            } else {
-                load8<XF32>(xr, i, v);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(v[k], v[k]);
-            }
-        };
-        float before = sum; // sum of the segments up to and including this one, then without it
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float up = __shfl_up_sync(0xffffffffu, before, o);
-            if (lane >= (uint32_t)o) before += up;
-        }
-        if (lane == 31) warp_sum[tid >> 5] = before;
-        __syncthreads();
-        float carry = 0.0f;
-        for (uint32_t w = 0; w < (tid >> 5); ++w) carry += warp_sum[w];
-        const float after = carry + before;
-        before = __shfl_up_sync(0xffffffffu, before, 1);
-        before = lane ? carry + before : carry;
-        const uint32_t binade = __float_as_uint(before) >> 23; // (sums of squares: no sign; infinities and NaN are 255)
-        uint32_t add0 = 0, add1 = 1; // additions to an even and, counted from 1, to an odd pattern
-        const bool guess = binade == (__float_as_uint(after) >> 23) && binade >= 24 && binade < 255;
-        if (guess) {
-            const float per_unit = __uint_as_float((277 - binade) << 23); // 1 / u = 2^(150 - binade)
-            for (uint32_t i = first8; i < end8; ++i) {
-                float v[8];
-                squares(i, v);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float units = v[k] * per_unit, whole = floorf(units), rest = units - whole; // all exact
-                    const uint32_t q = (uint32_t)whole, up = rest > 0.5f, tie = rest == 0.5f;
-                    add0 += q, add1 += q;
-                    add0 += up | (tie & add0), add1 += up | (tie & add1); // (bit 0 of tie & add: odd)
-                }
-            }
-        }
-        seg_add[tid] = make_uint2(add0, add1 - 1);
-        seg_binade[tid] = guess ? binade : 0;
-        __syncthreads();
-        if (tid < 32) {
-            uint32_t s = 0; // the running sum's bit pattern, the same in every lane
-            for (uint32_t base = 0; base < kNormThreads; base += 32) {
-                const uint2 my_add = seg_add[base + lane];
-                const uint32_t my_binade = seg_binade[base + lane];
-#pragma unroll 8
-                for (uint32_t j = 0; j < 32; ++j) {
-                    const uint32_t a0 = __shfl_sync(0xffffffffu, my_add.x, j), a1 = __shfl_sync(0xffffffffu, my_add.y, j);
-                    const uint32_t e = __shfl_sync(0xffffffffu, my_binade, j);
-                    const uint32_t next = s + ((s & 1) ? a1 : a0);
-                    if (e && (s >> 23) == e && (next >> 23) == e) {
-                        s = next;
-                    } else {
-                        const uint32_t f = min((base + j) * len8, n_in / 8), l = min(f + len8, n_in / 8);
-                        float t = __uint_as_float(s);
-                        for (uint32_t i = f; i < l; ++i) {
-                            float v[8];
-                            squares(i, v);
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) t = __fadd_rn(t, v[k]);
-                        }
-                        s = __float_as_uint(t);
-                    }
-                }
-            }
-            if (lane == 0) inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(__uint_as_float(s), (float)n_in), eps)));
-        }
-        __syncthreads();
-        inv = inv_rms;
-    }
+    const float inv = row < tokens ? chain_inv_rms<XF32, K>(xr, n_in, eps, sh) : 0.0f; // (uniform over the block)
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, inv, packed, scales);
 }
 
-// The same behind a kernel that runs the chains as chains, which does less work per row than the segments above but takes
-// their length in latency: the better form from 449 rows (us, segments / chains with quantizer, 5120 values: 15 / 17 at 16
-// rows, 19 / 19 at 512, 40 / 33 at 1536, 43 / 37 at 2048; 3136 values: 20 / 13 at 448 rows) and for rows of up to 4096 values
-// (1024 values: 11 / 6 at 16 rows, 15 / 7 at 1024; on either side of the line, chains of 4096 values 13.8 at 16 rows and 15.1
-// at 448, segments of 4160 14.8 and 17.1; on either side of the other, 27648 values, 63 at 448 rows and 87 at 449).
+// The quantizer behind a kernel that leaves the rows' factors in memory (chain_eights).
 template <bool XF32>
 __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
                                                                     const float *norm_w, const float *inv_rms, uint8_t *packed,
                                                                     uint8_t *scales) {
     const uint32_t row = blockIdx.x;
-    if (row == 0) // (as above)
-        for (uint32_t i = 32 * threadIdx.x; i < n_in; i += 32 * 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + i));
     pdl_wait();
     pdl_release();
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
 }
-constexpr uint32_t kNormSegmentRows = 448, kNormSegmentMin = 4097; // up to so many rows of at least so many values: the segmented kernel
+
+// Eights a thread holds in the kernel above, 0: the chains run as chains in a kernel of their own, which take their length
+// in latency but less work per row.  us with bf16 rows, chains and quantizer (or, below 449 rows, segments whose additions one
+// warp composed one after another) / this kernel: 5120 values 14.6 / 8.1 at 16 rows, 18.7 / 11.1 at 512, 28.4 / 13.9 at 1024,
+// 35.7 / 29.2 at 2048, 45 / 43 at 4096; 3136 values 12.0 / 6.9, 13.1 / 9.6, 18.2 / 12.4, 21.6 / 19.1, 27.5 / 36; 2048 values
+// 8.3 / 6.3 at 16, 11.6 / 9.3 at 1024, 14.4 / 14.4 at 2048; 1024 values 5.4 / 5.8 at 16; 8192 values 46 / 23 at 1024, 46 / 55
+// at 2048; 27648 values 33 / 14 at 16, 135 / 86 at 1024, 153 / 173 at 2048.  Two eights or four (5120 values): 8.1 / 9.3 at 16
+// rows, 10.0 / 10.3 at 300, 18 / 11 at 512.
+static uint32_t chain_eights(uint32_t tokens, uint32_t n_in) {
+    if (n_in < 1536 || n_in > 32 * kChainThreads || tokens > (n_in >= 3072 && n_in <= 6144 ? 2048u : 1024u)) return 0;
+    return tokens <= 448 && n_in <= 16 * kChainThreads ? 2 : 4;
+}
 
 // Plain rows: out[t][k] = (x[t][k] * inv_rms_t) * w[k] in f32, for the kernels that read their activations as they go.
 template <bool XF32>
@@ -413,19 +435,19 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
     if (norm_weight) {
         float *inv = ctx->inv_rms;
         if (!inv || tokens > ctx->inv_rms_rows) return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: more rows than the context's per-row scratch holds");
-        if (tokens > kNormSegmentRows || n_in < kNormSegmentMin) {
+        const uint32_t eights = chain_eights(tokens, (uint32_t)n_in);
+        const bool f32 = x_dtype == MUSER_DTYPE_F32;
+        if (!eights) {
             MUSER_CUDA_TRY(ctx, launch_rms_rows_sequential(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
-            const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
+            const auto kernel = f32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
             MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(256), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, (const float *)inv,
                                            packed, scales));
             return MUSER_CUDA_OK;
         }
-        const bool keep = n_in <= 12288; // rows of up to 48 KB of squares stay in shared memory, longer ones are read again
-        const size_t smem = keep ? (size_t)n_in * sizeof(float) : 0;
-        const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_norm_quantize_kernel<true> : nvfp4_norm_quantize_kernel<false>;
-        MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, smem));
-        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(kNormThreads), smem, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps,
-                                       (uint32_t)keep, packed, scales));
+        const auto kernel = eights == 2 ? (f32 ? nvfp4_norm_quantize_kernel<true, 2> : nvfp4_norm_quantize_kernel<false, 2>)
+                                        : (f32 ? nvfp4_norm_quantize_kernel<true, 4> : nvfp4_norm_quantize_kernel<false, 4>);
+        const uint32_t threads = ((uint32_t)((n_in / 8 + eights - 1) / eights) + 31) / 32 * 32;
+        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(threads), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps, packed, scales));
         return MUSER_CUDA_OK;
     }
     const uint64_t total = (uint64_t)tokens_pad * kt * 4;
