@@ -492,7 +492,7 @@ template <int DT, int NG, bool DUAL, bool AMAX = false, bool PUSH = false>
 __device__ __forceinline__ void run(const DecArgs &a, const DecJob &jb, uint32_t group, uint32_t slice, uint4 *dyn, float *inv_rms) {
     using Regs = typename RegsOf<DT>::type;
     constexpr int kBytes = Fmt<DT>::kTileBytes, kImages = DUAL ? 2 : 1, TOK = 4 * NG;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), warps = blockDim.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t sb_first = a.nsb * slice / a.ksplit, sb_last = a.nsb * (slice + 1) / a.ksplit, n_tiles = sb_last - sb_first;
     const uint32_t ring_n = a.ring, ring_mask = a.ring - 1, ring_shift = a.ring == 4 ? 2 : 1;

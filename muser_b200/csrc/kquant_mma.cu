@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1) kquant_mma_kernel(const __g
     __shared__ int abort_word;
     volatile int *abort_flag = &abort_word;
     const uint32_t full = smem_u32(bars), empty = full + 64;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = a.warps;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, W = a.warps;
     const uint32_t rank = blockIdx.x % a.ksplit, group = blockIdx.x / a.ksplit;
     uint32_t ji = 0;
 #pragma unroll

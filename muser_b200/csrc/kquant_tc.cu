@@ -360,7 +360,7 @@ kquant_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     float2 *hdr = reinterpret_cast<float2 *>(aligned + S::kOffHdr);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStagesA; ++s) {
             mbar_init(bar_full_a + 8 * s, 4); // the four 32-row quarters of the stage
