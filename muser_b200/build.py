@@ -4,12 +4,14 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libmuser_cuda.so"
+CALL = PKG / "_call.so"  # the Python binding's per-call half (csrc/host_call.c)
 SOURCES = ["api.cu", "repack.cu", "kquant_decode.cu", "kquant_tc.cu", "kquant_mma.cu", "nvfp4_quant.cu", "nvfp4_gemm.cu", "nvfp4_static.cu", "nvfp4_a16.cu", "collective.cu", "layer_ops.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -25,7 +27,19 @@ def _newest(paths) -> float:
     return max(p.stat().st_mtime for p in paths)
 
 
+def build_call(force: bool = False) -> Path:
+    src = CSRC / "host_call.c"
+    if not force and CALL.exists() and CALL.stat().st_mtime >= _newest([src, PKG.parent / "include" / "muser_cuda.h"]):
+        return CALL
+    cmd = [os.environ.get("CC", "gcc"), "-shared", "-fPIC", "-O2", "-Wall", "-Wno-unused-parameter", "-I" + sysconfig.get_paths()["include"], str(src), "-o", str(CALL), "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("gcc failed for host_call.c:\n" + r.stderr[-4000:])
+    return CALL
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
+    build_call(force)
     srcs = [CSRC / s for s in SOURCES]
     deps = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [PKG.parent / "include" / "muser_cuda.h"]
     if not force and LIB.exists() and LIB.stat().st_mtime >= _newest(srcs + deps):

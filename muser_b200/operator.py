@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
-from . import _lib
+from . import _call, _lib
 from ._lib import (BF16, F16, F32, NVFP4, Q4_K, Q6_K, SHARD_K, SHARD_NONE, SHARD_ROWS, TUNE_DECODE_KSPLIT, TUNE_DECODE_RING,
                    TUNE_DECODE_WARPS, TUNE_DECODE_WSPLIT, TUNE_TC_MIN_ROWS, TUNE_TC_MIN_TOKENS_Q4_K, TUNE_TC_MIN_TOKENS_Q6_K, MuserCudaError)
 
@@ -31,6 +31,10 @@ _TORCH_DTYPE = {torch.float32: F32, torch.bfloat16: BF16, torch.float16: F16}
 
 def _stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
+
+
+# the calls that a decode step makes go through csrc/host_call.c
+_call.bind(str(_lib.LIB_PATH), _TORCH_DTYPE, torch.float32, torch._C._cuda_getCurrentRawStream, _stream_ptr, MuserCudaError, C.ArgumentError)
 
 
 @dataclass
@@ -191,26 +195,17 @@ class CudaKernels:
                                 softcap=0.0, all_reduce=False) -> None:
         """y[t][r] = dot(W_r, x_t) for K-quant weights; input [tokens][n_in] f32|bf16, output [tokens][n_out] f32|bf16.
         all_reduce: the weight is a K shard; the call also sums the output over the context's communicator."""
-        ep = _epilogue(row_scale, residual, norm_weight, norm_eps, out_scale, softcap, all_reduce)
-        self.ctx.check(_L.muser_cuda_quantized_matmul(
-            self.ctx._h, weights._h, input.data_ptr(), _TORCH_DTYPE[input.dtype], output.data_ptr(),
-            _TORCH_DTYPE[output.dtype], tokens, C.byref(ep) if ep else None, _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.quantized_matmul(ctx, ctx.device, weights, input, output, tokens, row_scale, residual, norm_weight, norm_eps,
+                                         out_scale, softcap, all_reduce))
         self.launches += 2 if all_reduce else 1
 
     def encode_quantized_matmul_group(self, weights, input: torch.Tensor, outputs, tokens: int, epilogues=None) -> None:
         """Up to four K-quant projections of the same `input` in one launch (q | k | v, or gate | up), the counterpart
         of the reference's one-barrier-interval dispatch (decode.rs:5569-5598).  `epilogues`: per projection a dict of
         encode_quantized_matmul's keyword arguments, or None."""
-        n = len(weights)
-        items = (_lib.GroupItem * n)()
-        keep = []
-        for i, (w, y) in enumerate(zip(weights, outputs)):
-            ep = _epilogue(**(epilogues[i] or {})) if epilogues else None
-            keep.append(ep)
-            items[i].w, items[i].y, items[i].y_dtype, items[i].reserved = w._h.value, y.data_ptr(), _TORCH_DTYPE[y.dtype], 0
-            items[i].epilogue = C.pointer(ep) if ep is not None else None
-        self.ctx.check(_L.muser_cuda_quantized_matmul_group(
-            self.ctx._h, items, n, input.data_ptr(), _TORCH_DTYPE[input.dtype], tokens, _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.quantized_matmul_group(ctx, ctx.device, weights, input, outputs, tokens, epilogues))
         self.launches += 1
 
     def last_decode_plan(self) -> tuple:
@@ -256,30 +251,27 @@ class CudaKernels:
         """hidden += rms_norm(src, eps1) * weight1 in place; output = rms_norm(hidden, eps2) * weight2 when given
         (rmsnorm_batch_tail.metal:147-200; reference.rs:466-490).  f32 [tokens][n]."""
         tokens, n = src.shape
-        self.ctx.check(_L.muser_cuda_fused_norm_residual_rms_norm(
-            self.ctx._h, hidden.data_ptr(), src.data_ptr(), output.data_ptr() if output is not None else None, weight1.data_ptr(),
-            weight2.data_ptr() if weight2 is not None else None, tokens, n, C.c_float(eps1), C.c_float(eps2), _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.norm_residual_norm(ctx, ctx.device, hidden, src, output, weight1, weight2, tokens, n, eps1, eps2))
         self.launches += 1
 
     def encode_sigmoid_gate(self, x: torch.Tensor, gate: torch.Tensor) -> None:
         """x *= sigmoid(gate) in place (reference.rs:447-455)."""
-        self.ctx.check(_L.muser_cuda_sigmoid_gate(self.ctx._h, x.data_ptr(), gate.data_ptr(), x.numel(), _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.sigmoid_gate(ctx, ctx.device, x, gate, x.numel()))
         self.launches += 1
 
     def encode_head_rms_norm(self, x: torch.Tensor, weight: torch.Tensor, eps: float, heads: int) -> None:
         """Per-head rms_norm_mul of x [tokens][heads * head_dim] in place (reference.rs:384-393)."""
-        tokens = x.shape[0]
-        self.ctx.check(_L.muser_cuda_head_rms_norm(self.ctx._h, x.data_ptr(), weight.data_ptr(), C.c_float(eps), tokens, heads,
-                                                   x.shape[1] // heads, _stream_ptr(self.ctx.device)))
+        ctx, shape = self.ctx, x.shape
+        ctx.check(_call.head_rms_norm(ctx, ctx.device, x, weight, eps, shape[0], heads, shape[1] // heads))
         self.launches += 1
 
     def encode_ffn_gate_up_silu(self, gate_w: Weight, up_w: Weight, input: torch.Tensor, output: torch.Tensor,
                                 tokens: int, norm_weight=None, norm_eps=0.0) -> None:
         """output[t][j] = silu(gate_j . x_t) * (up_j . x_t); K-quant (tokens <= 16) or NVFP4 weights."""
-        ep = _epilogue(None, None, norm_weight, norm_eps)
-        self.ctx.check(_L.muser_cuda_ffn_gate_up_silu(
-            self.ctx._h, gate_w._h, up_w._h, input.data_ptr(), _TORCH_DTYPE[input.dtype], output.data_ptr(),
-            _TORCH_DTYPE[output.dtype], tokens, C.byref(ep) if ep else None, _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.gate_up_silu(ctx, ctx.device, gate_w, up_w, input, output, tokens, norm_weight, norm_eps))
         self.launches += 2 if gate_w.dtype == NVFP4 else 1
 
     def encode_nvfp4_ffn_gate_up_silu_requant(self, gate_w: Weight, up_w: Weight, packed: torch.Tensor, scales: torch.Tensor,
@@ -292,9 +284,8 @@ class CudaKernels:
             out_packed = torch.empty((tokens, n_out // 2), dtype=torch.uint8, device=packed.device)
         if out_scales is None:
             out_scales = torch.empty(_L.muser_cuda_nvfp4_swizzled_scale_bytes(tokens, n_out), dtype=torch.uint8, device=packed.device)
-        self.ctx.check(_L.muser_cuda_nvfp4_ffn_gate_up_silu_requant(
-            self.ctx._h, gate_w._h, up_w._h, packed.data_ptr(), scales.data_ptr(), tokens, C.c_float(out_input_scale_inv),
-            out_packed.data_ptr(), out_scales.data_ptr(), _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.nvfp4_gate_up_requant(ctx, ctx.device, gate_w, up_w, packed, scales, tokens, out_input_scale_inv, out_packed, out_scales))
         self.launches += 1
         return out_packed, out_scales
 
@@ -316,14 +307,8 @@ class CudaKernels:
             scales = torch.empty((_L.muser_cuda_nvfp4_swizzled_scale_bytes(tokens, n_in),), dtype=torch.uint8, device=dev)
         else:
             packed, scales = out
-        if norm_weight is not None:
-            self.ctx.check(_L.muser_cuda_rmsnorm_quantize_nvfp4_activation(
-                self.ctx._h, input.data_ptr(), _TORCH_DTYPE[input.dtype], tokens, n_in, norm_weight.data_ptr(),
-                float(norm_eps), input_scale_inv, packed.data_ptr(), scales.data_ptr(), _stream_ptr(self.ctx.device)))
-        else:
-            self.ctx.check(_L.muser_cuda_quantize_nvfp4_activation(
-                self.ctx._h, input.data_ptr(), _TORCH_DTYPE[input.dtype], tokens, n_in, input_scale_inv, packed.data_ptr(),
-                scales.data_ptr(), _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.quantize_activation(ctx, ctx.device, input, tokens, n_in, input_scale_inv, norm_weight, norm_eps, packed, scales))
         self.launches += 1
         return packed, scales
 
@@ -331,29 +316,21 @@ class CudaKernels:
                             row_scale=None, residual=None, norm_weight=None, norm_eps=0.0, out_scale=1.0,
                             softcap=0.0) -> None:
         """W4A4 lane: quantizes `input` with the weight's input_scale_inv, then the block-scaled GEMM."""
-        ep = _epilogue(row_scale, residual, norm_weight, norm_eps, out_scale, softcap)
-        self.ctx.check(_L.muser_cuda_nvfp4_matmul(
-            self.ctx._h, weights._h, input.data_ptr(), _TORCH_DTYPE[input.dtype], output.data_ptr(),
-            _TORCH_DTYPE[output.dtype], columns, C.byref(ep) if ep else None, _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.nvfp4_matmul(ctx, ctx.device, weights, input, output, columns, row_scale, residual, norm_weight, norm_eps, out_scale, softcap))
         self.launches += 2
 
     def encode_nvfp4_prequant(self, weights: Weight, packed: torch.Tensor, scales: torch.Tensor, output: torch.Tensor,
                               columns: int, row_scale=None, residual=None) -> None:
-        ep = _epilogue(row_scale, residual)
-        self.ctx.check(_L.muser_cuda_nvfp4_matmul_prequant(
-            self.ctx._h, weights._h, packed.data_ptr(), scales.data_ptr(), output.data_ptr(),
-            _TORCH_DTYPE[output.dtype], columns, C.byref(ep) if ep else None, _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.nvfp4_prequant(ctx, ctx.device, weights, packed, scales, output, columns, row_scale, residual))
         self.launches += 1
 
     def encode_nvfp4_group_prequant(self, weights, packed: torch.Tensor, scales: torch.Tensor, outputs, columns: int) -> None:
         """muser_cuda_nvfp4_matmul_group_prequant: 2..4 NVFP4 projections of the same quantized activations (q | k | v)
         in one launch; every output carries the bits encode_nvfp4_prequant gives for its weight."""
-        n = len(weights)
-        ws = (C.c_void_p * n)(*[w._h.value for w in weights])
-        ys = (C.c_void_p * n)(*[y.data_ptr() for y in outputs])
-        self.ctx.check(_L.muser_cuda_nvfp4_matmul_group_prequant(
-            self.ctx._h, ws, n, packed.data_ptr(), scales.data_ptr(), ys, _TORCH_DTYPE[outputs[0].dtype], columns,
-            _stream_ptr(self.ctx.device)))
+        ctx = self.ctx
+        ctx.check(_call.nvfp4_group_prequant(ctx, ctx.device, weights, packed, scales, outputs, columns))
         self.launches += 1
 
 

@@ -1,0 +1,75 @@
+"""The per-call binding (csrc/host_call.c) on the CPU: what it hands to the library and what it refuses.  The library's own
+argument checks come first, so a call with a freed handle ends in them without a GPU."""
+import ctypes as C
+import types
+
+import pytest
+import torch
+
+from muser_b200 import _call, _lib, operator as op
+
+
+@pytest.fixture
+def kern():
+    def bind(raw, slow):
+        _call.bind(str(_lib.LIB_PATH), op._TORCH_DTYPE, torch.float32, raw, slow, op.MuserCudaError, C.ArgumentError)
+    bind(lambda device: 0, lambda device: 0)
+    ctx = op.Context.__new__(op.Context)
+    ctx.device, ctx._h = 0, None
+    yield op.CudaKernels(ctx), types.SimpleNamespace(_h=None, dtype=op.Q4_K, n_out=16)
+    bind(torch._C._cuda_getCurrentRawStream, op._stream_ptr)
+
+
+def test_arguments_are_refused_as_before(kern):
+    k, w = kern
+    x, y = torch.zeros((2, 256)), torch.zeros((2, 16))
+    calls = {
+        "matmul": lambda **kw: k.encode_quantized_matmul(w, kw.pop("x", x), y, kw.pop("tokens", 2), **kw),
+        "group": lambda **kw: k.encode_quantized_matmul_group([w, w], kw.pop("x", x), [y, y], kw.pop("tokens", 2), epilogues=[None, kw]),
+        "nvfp4": lambda **kw: k.encode_nvfp4_matmul(w, kw.pop("x", x), y, kw.pop("tokens", 2), **kw),
+        "gate_up": lambda **kw: k.encode_ffn_gate_up_silu(w, w, kw.pop("x", x), y, kw.pop("tokens", 2), **kw),
+    }
+    for name, call in calls.items():
+        with pytest.raises(op.MuserCudaError) as e:
+            call(norm_weight=torch.ones(256), norm_eps=1e-5)
+        assert e.value.status_name == "BAD_ARG", name  # (no context: the library's first check)
+        with pytest.raises(op.MuserCudaError, match="norm_weight must be f32"):
+            call(norm_weight=torch.ones(256, dtype=torch.float64))
+        with pytest.raises(KeyError):
+            call(x=x.to(torch.int32))
+        for tokens in (2.0, "2", None):
+            with pytest.raises(C.ArgumentError):
+                call(tokens=tokens)
+        with pytest.raises(TypeError):
+            call(no_such_argument=1)
+    with pytest.raises(IndexError):
+        k.encode_quantized_matmul_group([w, w], x, [y, y], 2, epilogues=[None])
+    for n in (1, 5, 40):  # (lists longer than the library takes)
+        with pytest.raises(op.MuserCudaError):
+            k.encode_quantized_matmul_group([w] * n, x, [y] * n, 2)
+        with pytest.raises(op.MuserCudaError):
+            k.encode_nvfp4_group_prequant([w] * n, x, x, [y] * n, 2)
+    with pytest.raises(IndexError):
+        k.encode_nvfp4_group_prequant([w], x, x, [y, y], 2)
+    with pytest.raises(C.ArgumentError):
+        k.quantize_nvfp4_activation(x, "1.0", out=(x, x))
+    with pytest.raises(op.MuserCudaError):
+        k.quantize_nvfp4_activation(x, 1, norm_weight=torch.ones(256), norm_eps=1e-5, out=(x, x))
+    for call in (lambda: k.encode_sigmoid_gate(x, x), lambda: k.encode_head_rms_norm(x, y, 1e-5, 2), lambda: k.encode_nvfp4_prequant(w, x, x, y, 2, residual=y),
+                 lambda: k.encode_fused_norm_residual_rms_norm(x, x, x[0], 1e-5),
+                 lambda: k.encode_nvfp4_ffn_gate_up_silu_requant(w, w, x, x, 2, 1.0, out_packed=x, out_scales=x)):
+        with pytest.raises(op.MuserCudaError):
+            call()
+    assert k.launches == 0
+
+
+def test_the_stream_is_asked_for_on_every_call(kern):
+    k, w = kern
+    asked = []
+    _call.bind(str(_lib.LIB_PATH), op._TORCH_DTYPE, torch.float32, lambda d: asked.append(d) or 0, lambda d: asked.append(d) or 0, op.MuserCudaError, C.ArgumentError)
+    x = torch.zeros((2, 256))
+    for device in (0, 3):
+        k.ctx.device = device
+        with pytest.raises(op.MuserCudaError):
+            k.encode_sigmoid_gate(x, x)
+    assert asked == [0, 3]
