@@ -285,7 +285,7 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t cta_addr, uint32_t rank
     return r;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Staging buffer (64-byte rows, 64-byte swizzle) -> a box of the output; columns and rows past its end are not written.
 __device__ __forceinline__ void tma_store_2d_elect(const CUtensorMap *map, uint32_t src, int x, int y) {
@@ -307,7 +307,7 @@ __device__ __forceinline__ void sts_16(uint32_t at, const uint32_t (&v)[4]) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster_elect(uint32_t cluster_addr) {
-    asm volatile("{\n\t" MUSER_ELECT_PRED "@e mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(cluster_addr) : "memory");
+    asm volatile("{\n\t" MUSER_ELECT_PRED "@e mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n\t}" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -350,32 +350,46 @@ __device__ __forceinline__ void pair_mma_nvf4_elect(uint32_t tmem_d, uint64_t de
 }
 
 // A whole slab's twelve scale copies, four products and the commit behind ONE election: with an elect.sync each and a loop
-// around them the issuing warp took 1080 cycles a slab, unrolled 740, so about 460, and the products take 512.  Chunks of
+// around them the issuing warp took 1080 cycles a slab, unrolled 740, so about 400, and the products take 512.  Chunks of
 // 512 bytes follow one another in shared memory: four of the activations, then four of either half of the weight rows.  The
 // role is entered by a branch that does not tell the compiler that its warp runs converged: told so, as the other roles are
 // (they issue their loads in 128 cycles instead of 304, and the single CTAs' slabs are 10 % shorter), it takes 923 cycles to
 // issue these seventeen instructions.
 #define PAIR_CP(COL, CHUNK)                                                                                                  \
-    "add.u32 t, %4, " #COL ";\n\tadd.u32 v, %5, " #CHUNK " * 32;\n\tmov.b64 d, {v, %8};\n\t"                                     \
+    "add.u32 t, %4, " #COL ";\n\tadd.u32 v, %5, " #CHUNK " * 32;\n\tmov.b64 d, {v, %7};\n\t"                                     \
     "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [t], d;\n\t"
 #define PAIR_MMA(KB, SFA, SFB, P)                                                                                            \
-    "add.u32 v, %1, 2 * " #KB ";\n\tmov.b64 a, {v, %9};\n\tadd.u32 v, %2, 2 * " #KB ";\n\tmov.b64 b, {v, %9};\n\t"              \
+    "add.u32 v, %1, 2 * " #KB ";\n\tmov.b64 a, {v, %8};\n\tadd.u32 v, %2, 2 * " #KB ";\n\tmov.b64 b, {v, %8};\n\t"              \
     "add.u32 t, %4, " #SFA ";\n\tadd.u32 u, %4, " #SFB ";\n\t"                                                                 \
     "@e tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a, b, %3, [t], [u], " P ";\n\t"
-__device__ __forceinline__ void pair_slab_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales,
-                                                uint32_t accumulate, uint32_t empty) {
-    // (shared-memory addresses lie below 256 KB: the low words of operand_desc() and scale_desc() are address / 16 and constants)
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b32 t, u, v;\n\t.reg .b64 a, b, d;\n\t" MUSER_ELECT_PRED
-        "setp.ne.b32 p, %6, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
-        PAIR_CP(0, 0) PAIR_CP(16, 4) PAIR_CP(20, 8) PAIR_CP(4, 1) PAIR_CP(24, 5) PAIR_CP(28, 9)
-        PAIR_CP(8, 2) PAIR_CP(32, 6) PAIR_CP(36, 10) PAIR_CP(12, 3) PAIR_CP(40, 7) PAIR_CP(44, 11)
-        PAIR_MMA(0, 0, 16, "p") PAIR_MMA(1, 4, 24, "q") PAIR_MMA(2, 8, 32, "q") PAIR_MMA(3, 12, 40, "q")
-        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t}"
-        ::"r"(tmem_d), "r"((a >> 4) | (1u << 16)), "r"((b >> 4) | (1u << 16)), "r"(idesc), "r"(sf), "r"(scales >> 4), "r"(accumulate), "r"(empty),
-          "n"((128 >> 4) | (1 << 14)), "n"((1024 >> 4) | (1 << 14) | (2 << 29))
-        : "memory");
+#define PAIR_HEAD "{\n\t.reg .pred q;\n\t.reg .b32 t, u, v;\n\t.reg .b64 a, b, d;\n\t" MUSER_ELECT_PRED "setp.eq.b32 q, 0, 0;\n\t"
+#define PAIR_CPS                                                                                     \
+    PAIR_CP(0, 0) PAIR_CP(16, 4) PAIR_CP(20, 8) PAIR_CP(4, 1) PAIR_CP(24, 5) PAIR_CP(28, 9)          \
+    PAIR_CP(8, 2) PAIR_CP(32, 6) PAIR_CP(36, 10) PAIR_CP(12, 3) PAIR_CP(40, 7) PAIR_CP(44, 11)
+#define PAIR_MMAS(FIRST)                                                                             \
+    PAIR_MMA(0, 0, 16, FIRST) PAIR_MMA(1, 4, 24, "q") PAIR_MMA(2, 8, 32, "q") PAIR_MMA(3, 12, 40, "q") \
+    "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+// (shared-memory addresses lie below 256 KB: the low words of operand_desc() and scale_desc() are address / 16 and constants)
+#define PAIR_ARGS                                                                                                          \
+    ::"r"(tmem_d), "r"((a >> 4) | (1u << 16)), "r"((b >> 4) | (1u << 16)), "r"(idesc), "r"(sf), "r"(scales >> 4),         \
+        "r"(empty), "n"((128 >> 4) | (1 << 14)), "n"((1024 >> 4) | (1 << 14) | (2 << 29))                         \
+        : "memory"
+__device__ __forceinline__ void pair_slab_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty) {
+    asm volatile(PAIR_HEAD PAIR_CPS PAIR_MMAS("q") PAIR_ARGS);
 }
+// A tile's first slab in two parts: its copies, and the products that start the accumulator anew.
+__device__ __forceinline__ void pair_first_copies_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty) {
+    asm volatile(PAIR_HEAD PAIR_CPS "}" PAIR_ARGS);
+}
+__device__ __forceinline__ void pair_first_products_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty) {
+    asm volatile(PAIR_HEAD PAIR_MMAS("!q") PAIR_ARGS);
+}
+#undef PAIR_CP
+#undef PAIR_MMA
+#undef PAIR_HEAD
+#undef PAIR_CPS
+#undef PAIR_MMAS
+#undef PAIR_ARGS
 
 // Tensor maps of a launch beside the activations': the weights (one, gate and up, or a group's), and for PAIR the outputs, the
 // residual and all scales
@@ -583,18 +597,88 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             *abort_flag = 1;
             atomicCAS(g.status + 1, 0, 116);
         }
-    } else if ((PAIR ? threadIdx.x >> 5 : (uint32_t)warp) == 1) { // (see pair_slab_elect)
+    } else if (PAIR && (threadIdx.x >> 5) == 1) { // (see pair_slab_elect)
+        // ---------------------------------------------------------------- MMA issuer of a pair (whole warp; one elected lane issues)
+        // A pair's copies run beside the products only when the slab's are issued together in front of them (512 cycles per
+        // slab in isolation, the four products' own time; three in front of each product 642).  The loop over a tile's slabs
+        // holds nothing that it could do without: with the first slab's and the last one's cases inside it a slab took 545
+        // cycles, and 30 more with one more flag to look at; now the products' 512 (gate/up at 2048 tokens 234 -> 220 us).
+        // What is left is the change of tiles, about 1800 cycles from the last slab's issue to the next tile's first.
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+        const uint32_t peer_acc_full = map_to_rank(bar_acc_full, 1), whole_slabs = g.kt64 / 4;
+        uint32_t local = 0, stage = 0, phase = 0;
+        bool ok = true;
+        auto landed = [&] {
+            ok = mbar_wait_pair_warp(bar_full + 8 * stage, phase, abort_flag);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            return ok;
+        };
+        auto drained = [&] { // the epilogue warps of both CTAs have read the previous tile
+            if (local == 0) return true;
+            ok = mbar_wait_pair_warp(bar_acc_empty, (local - 1) & 1, abort_flag);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            return ok;
+        };
+        auto next_stage = [&] {
+            if (++stage == kStages) stage = 0, phase ^= 1;
+        };
+#define PAIR_STAGE base + stage * kStageBytes, base + stage * kStageBytes + kABytes
+#define PAIR_SCALES tmem + kSfCol + stage * kSfBufCols, base + stage * kStageBytes + kABytes + kBBytes
+        auto ragged = [&](bool fresh) { // the end of a row
+            const uint32_t st = base + stage * kStageBytes, sf = tmem + kSfCol + stage * kSfBufCols, sfa = st + kABytes + kBBytes, sfb = sfa + kSfaBytes;
+            const uint64_t da = operand_desc(st), db = operand_desc(st + kABytes);
+            for (uint32_t kb = 0; kb < g.kt64 % 4; ++kb) {
+                pair_cp_scales_elect(sf + 4 * kb, scale_desc(sfa + 512 * kb));
+                pair_cp_scales_elect(sf + 16 + 8 * kb, scale_desc(sfb + 512 * kb));
+                pair_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
+            }
+            for (uint32_t kb = 0; kb < g.kt64 % 4; ++kb)
+                pair_mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, !fresh || kb != 0);
+            pair_commit_elect(bar_empty + 8 * stage);
+            next_stage();
+        };
+        for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total; tile += GEMM_TILE_STEP, ++local) {
+            if (!landed()) break;
+            if (whole_slabs) {
+                // the first copies go into the tensor pipe's queue behind the last tile's products, before the accumulator is free
+                pair_first_copies_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, 0);
+                if (!drained()) break;
+                pair_first_products_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, bar_empty + 8 * stage);
+                next_stage();
+            } else {
+                if (!drained()) break;
+                ragged(true);
+            }
+            for (uint32_t i = 1; i < whole_slabs; ++i) {
+                if (!landed()) break;
+                pair_slab_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, bar_empty + 8 * stage);
+                next_stage();
+            }
+            if (!ok) break;
+            if (whole_slabs && g.kt64 % 4) {
+                if (!landed()) break;
+                ragged(false);
+            }
+            pair_commit_elect(bar_acc_full);
+            pair_commit_elect(peer_acc_full);
+        }
+#undef PAIR_STAGE
+#undef PAIR_SCALES
+        if (!ok && lane == 0) {
+            *abort_flag = 1;
+            atomicExch(g.status + 1, 102);
+        }
+    } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (whole warp; one elected lane issues)
         {
             // kind::mxf4nvf4: A and B E2M1 (format 1), K-major, UE4M3 scales, N >> 3 at bit 17, M >> 4 at bit 24
-            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(((PAIR ? 2 : 1) * BM) >> 4) << 24);
-            const uint32_t peer_acc_full = PAIR ? map_to_rank(bar_acc_full, 1) : 0u;
-            uint32_t it = 0, local = 0, stage = 0, phase = 0;
+            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+            uint32_t it = 0, local = 0;
             bool ok = true; PROF_DECL
             for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total && ok; tile += GEMM_TILE_STEP, ++local) {
                 // the accumulator is free again once the epilogue warps have read the previous tile out of it
                 if (local > 0) {
-                    PROF_BEGIN ok = PAIR ? mbar_wait_pair_warp(bar_acc_empty, (local - 1) & 1, abort_flag) : mbar_wait_warp(bar_acc_empty, (local - 1) & 1, abort_flag); PROF_END(0)
+                    PROF_BEGIN ok = mbar_wait_warp(bar_acc_empty, (local - 1) & 1, abort_flag); PROF_END(0)
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
@@ -605,32 +689,6 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     slices = g.grp_slices[(tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3])];
                     slice_end = g.k_tiles / slices; // (kept: a division a slab took the issuing warp longer than the slab's products)
                 }
-                if constexpr (PAIR) {
-                    // A pair's copies run beside the products only when the slab's are issued together in front of them
-                    // (512 cycles per slab in isolation, the four products' own time; three in front of each product 642).
-                    for (uint32_t kt = 0; kt < g.k_tiles; ++kt) {
-                        ok = mbar_wait_pair_warp(bar_full + 8 * stage, phase, abort_flag);
-                        if (!ok) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint32_t st = base + stage * kStageBytes, sf = tmem + kSfCol + stage * kSfBufCols;
-                        const uint32_t sfa = st + kABytes + kBBytes, sfb = sfa + kSfaBytes;
-                        if (g.kt64 - 4 * kt >= 4) {
-                            pair_slab_elect(tmem, st, st + kABytes, idesc, sf, sfa, kt != 0, bar_empty + 8 * stage);
-                        } else { // the ragged end of a row
-                            const uint64_t da = operand_desc(st), db = operand_desc(st + kABytes);
-                            const uint32_t nkb = g.kt64 - 4 * kt;
-                            for (uint32_t kb = 0; kb < nkb; ++kb) {
-                                pair_cp_scales_elect(sf + 4 * kb, scale_desc(sfa + 512 * kb));
-                                pair_cp_scales_elect(sf + 16 + 8 * kb, scale_desc(sfb + 512 * kb));
-                                pair_cp_scales_elect(sf + 16 + 8 * kb + 4, scale_desc(sfb + 2048 + 512 * kb));
-                            }
-                            for (uint32_t kb = 0; kb < nkb; ++kb)
-                                pair_mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, (kt | kb) != 0);
-                            pair_commit_elect(bar_empty + 8 * stage);
-                        }
-                        if (++stage == kStages) stage = 0, phase ^= 1;
-                    }
-                } else
                 for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
                     if constexpr (SLICED) {
                         if (kt == slice_end) { // (never true at the last slice's end, where the loop ends)
@@ -662,10 +720,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     }
                     mma_commit_elect(bar_empty + 8 * s); // the stage may be overwritten once these MMAs have read it
                 }
-                if (ok) {
-                    if constexpr (PAIR) pair_commit_elect(bar_acc_full), pair_commit_elect(peer_acc_full);
-                    else mma_commit_elect(bar_acc_full);
-                }
+                if (ok) mma_commit_elect(bar_acc_full);
             }
             if (lane == 0) { PROF_FLUSH(1) }
             if (!ok && lane == 0) {
