@@ -1218,8 +1218,8 @@ muser_cuda_status decode_autotune(Ctx *ctx, const Weight *const *w, const Weight
 // batched kernels.  Of the batched kernels the one on the warp-level instructions (kquant_mma.cu) has the
 // smaller fixed part and pads token columns to 8, the tcgen05 one (kquant_tc.cu, to 16, 32 or 64; Q4_K and Q6_K) the
 // cheaper column: see takes_tcgen05.  At 13 to 16 tokens the decode kernel's integer products are bound by their scale
-// arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 35, 5120 x 27648 Q6_K 68 -> 42, 5120 x 5120 21 -> 14,
-// 1024 x 5120 18.5 -> 10).  At 9 to 12 it depends on the weight (40 / 40, 55 / 43 for the long Q6_K rows, 17 / 15, but
+// arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 28, 5120 x 27648 Q6_K 68 -> 41, 5120 x 5120 21 -> 11,
+// 1024 x 5120 18.5 -> 8.4).  At 9 to 12 it depends on the weight (40 / 40, 55 / 43 for the long Q6_K rows, 17 / 15, but
 // 8192 x 5120 17 / 20), which one line for all of them does not follow; below it wins (27648 x 5120 at 8: 27 / 34).
 // The decode kernel also keeps, and its forms for 13 to 16 tokens (fused gate/up among them) are there for,
 //   - K shards up to 16 tokens, whose partial sums must carry the same bits with and without the all-reduce fused in,
@@ -1229,15 +1229,15 @@ static bool takes_mma(const Ctx *ctx, const Weight *w, uint32_t tokens) {
     return tokens > 16 || w->shard.axis != MUSER_SHARD_K || w->shard.world <= 1;
 }
 
-// The tcgen05 kernel for large Q4_K weights at token counts that fill its columns (us, tcgen05 / warp-level: 27648 x 5120
-// 44 / 46 at 32 tokens, 61 / 70 at 64, 55 / 61 at 32 in f32, which take two columns each; 61 / 56 at 48; 13824 x 5120 37 / 40
-// at 64; 8192 x 5120 22 / 22 and 33 / 31; 5120 x 5120 19 / 17 and 29 / 23).  Q6_K: 63 / 52 at 32 and 78 / 76 at 64 for
-// 5120 x 27648.  A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves, which is
+// The tcgen05 kernel for large Q4_K weights at token counts that fill its columns (us, tcgen05 / warp-level, 27648 x 5120:
+// 35 / 32 at 17 to 24 tokens, 35 / 38 at 32, 54 / 48 at 48, 55 / 61 at 64; f32 activations, two columns a token, 47 / 44 at
+// 17 to 24 and 48 / 56 at 32.  Smaller weights, before both kernels' present forms: 13824 x 5120 37 / 40 at 64, 8192 x 5120
+// 22 / 22 at 32 and 33 / 31, 5120 x 5120 19 / 17 and 29 / 23).  Q6_K: 63 / 52 at 32 and 78 / 76 at 64 for 5120 x 27648.  A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves, which is
 // what its Q6_K form is kept for: the caller's choice of range and rounding against another kernel's.
 static bool takes_tcgen05(const Weight *w, uint32_t tokens, bool two_columns, uint32_t tc_from) {
     if (tc_from < 17) return true;
     const uint32_t cols = two_columns ? 2 * tokens : tokens;
-    return w->dtype == MUSER_DTYPE_Q4_K && (uint64_t)w->row_tiles * w->nsb > 12000 && (cols <= 32 || cols > 48);
+    return w->dtype == MUSER_DTYPE_Q4_K && (uint64_t)w->row_tiles * w->nsb > 12000 && (cols > 48 || (cols > 24 && cols <= 32));
 }
 
 // Up to four projections of one input (or a fused gate/up pair), 1..64 tokens.

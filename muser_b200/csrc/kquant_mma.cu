@@ -9,7 +9,7 @@
 // A kernel of its own first turns the activations into f16 fragments: every (token, 256 inputs) is scaled by a power of
 // two that puts its largest magnitude between 2^9 and 2^10 (no range limit; bf16 inputs are exact down to 2^-24 of that
 // maximum), f32 inputs become a head and a remainder (22 bits).  The contraction kernel's operands are then exact:
-//   Q4_K, Q5_K  the integer sc * q (6-bit scale x 4- or 5-bit quant, at most 1953) as f16.  Sixteen m16n8k16 products
+//   Q4_K, Q5_K  the integer sc * q (6-bit scale x 4- or 5-bit quant, at most 1953) times 2^-24 as f16.  Sixteen m16n8k16 products
 //               accumulate a super-block of 256 inputs in f32 registers, one more product multiplies the 6-bit mins
 //               with the sub-block sums (f16 head + remainder), and acc += s * (d * sum - dmin * mins) once per 256.
 //   Q6_K        up to 16 tokens q - 32 as f16; one product is one 16-input sub-block, whose int8 scale is applied to the
@@ -75,8 +75,14 @@ __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<ui
 __device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
 __device__ __forceinline__ uint32_t gw(const uint4 &v, int i) { return (&v.x)[i]; } // compile-time i only
 __device__ __forceinline__ uint32_t spread_bit4(uint32_t x) { return (x * 0x02040810u) & 0x10101010u; } // four fifth bits onto bit 4 of four bytes
-// byte i of w as the f16 pair (v, v): 0x6400 | v is 1024 + v
-__device__ __forceinline__ __half2 byte_pair(uint32_t w, uint32_t i) {
+// bytes 2 i, 2 i + 1 of w as an f16 pair: 0x6400 | v is 1024 + v
+__device__ __forceinline__ __half2 byte_pair(uint32_t w, uint32_t i, float bias = 1024.0f) {
+    return __hsub2(u2h(__byte_perm(w, 0x64646464u, i ? 0x4342u : 0x4140u)), __float2half2_rn(bias));
+}
+// one of a pair's halves on both sides (an operand's half selection, not an instruction)
+__device__ __forceinline__ __half2 both(__half2 v, int half) { return half ? __high2half2(v) : __low2half2(v); }
+// byte i of w on both sides
+__device__ __forceinline__ __half2 byte_twice(uint32_t w, uint32_t i) {
     return __hsub2(u2h(__byte_perm(w, 0x64646464u, 0x4040u | i | (i << 8))), __float2half2_rn(1024.0f));
 }
 // int8 byte i of w (biased by 128: b ^ 0x80) as f32
@@ -121,25 +127,38 @@ __device__ __forceinline__ void tile_q45(const uint8_t *tile, const uint8_t *blo
     for (int gp = 0; gp < NG; ++gp) acc[gp][0] = acc[gp][1] = acc[gp][2] = acc[gp][3] = 0.0f;
 #pragma unroll
     for (int gp = 0; gp < (kApart ? NG : 1); ++gp) rem[gp][0] = rem[gp][1] = rem[gp][2] = rem[gp][3] = 0.0f;
+    // Scales two sub-blocks at a time from 17 tokens on (27648 x 5120 at 48 tokens 49.7 -> 48.6 us, 5120 x 27648 Q6_K at 32
+    // 49.8 -> 48.3); below, where the kernel's Q6_K form keeps its scales in f32, that form lost its registers to it (5120 x
+    // 27648 at 16 tokens 41.6 -> 44.2).
+    constexpr bool kPairs = NG > 2;
+    __half2 scales[2], scales16[2]; // kPairs: of sub-blocks j and j + 1, rows g and g + 8
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+        if (kPairs && j % 2 == 0) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                scales[r] = byte_pair(r ? hb.sc[j >> 2] : ha.sc[j >> 2], (j >> 1) & 1);
+                scales16[r] = __hmul2(scales[r], __float2half2_rn(0.0625f));
+            }
+        }
         uint32_t av[2][4]; // [product][a0..a3]
 #pragma unroll
         for (int r = 0; r < 2; ++r) { // row g, row g + 8
             const uint32_t w = gw(q[2 * r + (j >> 2)], j & 3);
-            const __half2 sc = byte_pair(r ? hb.sc[j >> 2] : ha.sc[j >> 2], j & 3), off = __hmul2(sc, __float2half2_rn(-1024.0f));
-            // (1024 + q) * sc - 1024 * sc in one rounding: exactly sc * q
-            auto pair = [&](uint32_t bits) { return h2u(__hfma2(u2h(bits | 0x64006400u), sc, off)); };
+            // A quant in the low bits of an f16 is that many of its smallest subnormals, 2^-24: the operand is sc * q * 2^-24,
+            // exact, one mask and one product a pair.  (From 1024 + q by a fused multiply-add with -1024 sc, 27648 x 5120 at 16
+            // tokens took 32.5 us instead of 28.3, 5120 x 5120 12.3 instead of 11.1.)
+            const __half2 sc = kPairs ? both(scales[r], j & 1) : byte_twice(r ? hb.sc[j >> 2] : ha.sc[j >> 2], j & 3);
+            auto pair = [&](uint32_t bits) { return h2u(__hmul2(u2h(bits), sc)); };
             if constexpr (Q5) {
                 const uint32_t hi = (gw(hbits, 2 * r + (j >> 2)) >> (8 * (j & 3))) & 0xFFu;
                 const uint32_t wl = (w & 0x0F0F0F0Fu) | spread_bit4(hi & 15u), wh = ((w >> 4) & 0x0F0F0F0Fu) | spread_bit4(hi >> 4);
                 av[0][r] = pair(wl & 0x00FF00FFu), av[0][2 + r] = pair(wh & 0x00FF00FFu);
                 av[1][r] = pair((wl >> 8) & 0x00FF00FFu), av[1][2 + r] = pair((wh >> 8) & 0x00FF00FFu);
             } else {
-                // the nibbles at bits 4-7 and 20-23 stay where they are: (1024 + 16 q) * (sc / 16) - 64 sc (the
-                // byte-and-logic pipe is the fullest one here)
-                const __half2 sc16 = __hmul2(sc, __float2half2_rn(0.0625f)), off16 = __hmul2(sc, __float2half2_rn(-64.0f));
-                auto pair16 = [&](uint32_t bits) { return h2u(__hfma2(u2h(bits | 0x64006400u), sc16, off16)); };
+                // the nibbles at bits 4-7 and 20-23 stay where they are, sixteen times as large
+                const __half2 sc16 = kPairs ? both(scales16[r], j & 1) : __hmul2(sc, __float2half2_rn(0.0625f));
+                auto pair16 = [&](uint32_t bits) { return h2u(__hmul2(u2h(bits), sc16)); };
                 const uint32_t w8 = w >> 8;
                 av[0][r] = pair(w & 0x000F000Fu), av[0][2 + r] = pair16(w & 0x00F000F0u);
                 av[1][r] = pair(w8 & 0x000F000Fu), av[1][2 + r] = pair16(w8 & 0x00F000F0u);
@@ -161,6 +180,7 @@ __device__ __forceinline__ void tile_q45(const uint8_t *tile, const uint8_t *blo
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[gp][i] += rem[gp][i];
     }
+    const float da = ha.d * 16777216.0f, db = hb.d * 16777216.0f;
     const uint32_t sel = 0x4140u + (t & 1) * 0x0202u; // bytes 2t, 2t + 1 of the eight mins
     const uint32_t ma = h2u(__hsub2(u2h(__byte_perm(t & 2 ? ha.mn[1] : ha.mn[0], 0x64646464u, sel)), __float2half2_rn(1024.0f)));
     const uint32_t mb = h2u(__hsub2(u2h(__byte_perm(t & 2 ? hb.mn[1] : hb.mn[0], 0x64646464u, sel)), __float2half2_rn(1024.0f)));
@@ -170,10 +190,10 @@ __device__ __forceinline__ void tile_q45(const uint8_t *tile, const uint8_t *blo
         float m[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         hmma16(m, ma, mb, ma, mb, b.x, b.y);
         const float2 s = *reinterpret_cast<const float2 *>(blob + B::kScales + (gp * 8 + 2 * t) * 4);
-        out[gp][0] = fmaf(s.x, fmaf(-ha.dmin, m[0], ha.d * acc[gp][0]), out[gp][0]);
-        out[gp][1] = fmaf(s.y, fmaf(-ha.dmin, m[1], ha.d * acc[gp][1]), out[gp][1]);
-        out[gp][2] = fmaf(s.x, fmaf(-hb.dmin, m[2], hb.d * acc[gp][2]), out[gp][2]);
-        out[gp][3] = fmaf(s.y, fmaf(-hb.dmin, m[3], hb.d * acc[gp][3]), out[gp][3]);
+        out[gp][0] = fmaf(s.x, fmaf(-ha.dmin, m[0], da * acc[gp][0]), out[gp][0]);
+        out[gp][1] = fmaf(s.y, fmaf(-ha.dmin, m[1], da * acc[gp][1]), out[gp][1]);
+        out[gp][2] = fmaf(s.x, fmaf(-hb.dmin, m[2], db * acc[gp][2]), out[gp][2]);
+        out[gp][3] = fmaf(s.y, fmaf(-hb.dmin, m[3], db * acc[gp][3]), out[gp][3]);
     }
 }
 
@@ -202,8 +222,16 @@ __device__ __forceinline__ void tile_q6(const uint8_t *tile, const uint8_t *blob
     float acc[NG][4];
 #pragma unroll
     for (int gp = 0; gp < NG; ++gp) acc[gp][0] = acc[gp][1] = acc[gp][2] = acc[gp][3] = 0.0f;
+    __half2 scales4[2], offsets[2]; // kScaled: sc / 4 and -288 sc of sub-blocks s and s + 1, rows g and g + 8
 #pragma unroll
     for (int s = 0; s < 16; ++s) {
+        if (kScaled && s % 2 == 0) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const __half2 k = byte_pair(gw(sc[r], s >> 2), (s >> 1) & 1, 1152.0f);
+                scales4[r] = __hmul2(k, __float2half2_rn(0.25f)), offsets[r] = __hmul2(k, __float2half2_rn(-288.0f));
+            }
+        }
         uint32_t a[4];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -213,9 +241,7 @@ __device__ __forceinline__ void tile_q6(const uint8_t *tile, const uint8_t *blob
             const uint32_t b = ((tp & 0xF0F0F0F0u) | (lo & 0x0C0C0C0Cu)) ^ 0x80808080u; // 4 (q - 32) + 128 per byte
             const __half2 b01 = u2h(__byte_perm(b, 0x64646464u, 0x4140u)), b23 = u2h(__byte_perm(b, 0x64646464u, 0x4342u)); // 1024 + b
             if constexpr (kScaled) { // (1024 + b) * (sc / 4) - 288 sc = sc (q - 32), rounded once
-                const uint32_t i = s & 3;
-                const __half2 k = __hsub2(u2h(__byte_perm(gw(sc[r], s >> 2), 0x64646464u, 0x4040u | i | (i << 8))), __float2half2_rn(1152.0f));
-                const __half2 k4 = __hmul2(k, __float2half2_rn(0.25f)), off = __hmul2(k, __float2half2_rn(-288.0f));
+                const __half2 k4 = both(scales4[r], s & 1), off = both(offsets[r], s & 1);
                 a[r] = h2u(__hfma2(b01, k4, off)), a[2 + r] = h2u(__hfma2(b23, k4, off));
             } else {
                 a[r] = h2u(__hsub2(b01, __float2half2_rn(1152.0f))), a[2 + r] = h2u(__hsub2(b23, __float2half2_rn(1152.0f)));
