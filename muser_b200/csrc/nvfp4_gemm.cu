@@ -391,6 +391,8 @@ __device__ __forceinline__ void pair_first_products_elect(uint32_t tmem_d, uint3
 #undef PAIR_MMAS
 #undef PAIR_ARGS
 
+enum : int { kWhole = 0, kCluster = 1, kSliced = 2 }; // how a tile's K is cut (SPLIT)
+
 // Tensor maps of a launch beside the activations': the weights (one, gate and up, or a group's), and for PAIR the outputs, the
 // residual and all scales
 // (tiled loads with the pair's qualifier run a little faster than untiled bulk copies: 560 against 594 cycles per 32 KB).
@@ -413,20 +415,20 @@ struct GemmMaps {
 // GROUP: several projections that read the same quantized activations (q | k | v) share one launch: their weight-row
 // tiles form one tile space, so the small ones fill the SMs that a launch of their own would leave idle.  Plain
 // outputs only (no fused tail, row scale or residual).
-// SPLIT: the slabs of one output tile are cut between the CTAs of a cluster (gemm_ksplit()): each leaves its f32 sums in
+// SPLIT = kCluster: the slabs of one output tile are cut between the CTAs of a cluster (gemm_ksplit()): each leaves its f32 sums in
 // its shared memory, and all of them add the slices up in slice order, every CTA finishing a share of the tile's outputs.
-// SLICED (SPLIT with GROUP): a group that holds weights which SPLIT cuts when they are called alone.  Tiles are whole, but
-// the accumulator starts anew with every slice of such a weight and the epilogue adds the slices up as SPLIT does: the bits
-// of the single call in the group's one launch (where that is the faster way: group_in_one_launch).
+// SPLIT = kSliced (with GROUP): a group that holds weights which SPLIT cuts when they are called alone.  Tiles are whole, but
+// the accumulator starts anew with every slice of such a weight and the epilogue adds the slices up as kCluster does: the bits
+// of the single call in the group's one launch (where that is the faster way: group_cost).
 // PAIR: pairs of SMs on 256-token tiles (above).  Each CTA's loads report to its own barrier; the second CTA (rank 1) passes
 // "landed" on with an arrival on the leader's barrier of that stage (loads that report to the other CTA's barrier themselves
 // take 1600 cycles per 32 KB instead of 560); the leader issues the scale copies and the products for both and commits to
 // both CTAs' barriers.
-template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, bool SPLIT = false, bool PAIR = false>
+template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, int SPLIT = kWhole, bool PAIR = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ GemmMaps maps, const GemmArgs g) {
     constexpr uint32_t kTileRows = DUAL ? BN / 2 : BN; // output columns (weight rows) per tile
-    constexpr bool CLUSTER = SPLIT && !GROUP, SLICED = SPLIT && GROUP;
+    constexpr bool CLUSTER = SPLIT == kCluster, SLICED = SPLIT == kSliced;
     constexpr uint32_t kStages = PAIR ? kPStages : muser::kStages, kStageBytes = PAIR ? kPStageBytes : muser::kStageBytes;
     constexpr uint32_t kBBytes = PAIR ? kPBBytes : muser::kBBytes;
     extern __shared__ uint8_t smem_raw[];
@@ -1014,10 +1016,18 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         uint32_t tile_m, tile_n;
         tile_coords(GEMM_TILE_FIRST, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
         const uint32_t rows = min((uint32_t)BM, g.tokens - tile_m * BM);
+        uint32_t n_out = g.n_out; // (of this tile's projection)
+        void *y = g.y;
+        float scale2 = g.scale2;
+        if constexpr (GROUP) {
+            const uint32_t p = (tile_n >= g.grp_tile0[1]) + (tile_n >= g.grp_tile0[2]) + (tile_n >= g.grp_tile0[3]);
+            tile_n -= g.grp_tile0[p];
+            n_out = g.grp_n_out[p], y = g.grp_y[p], scale2 = g.grp_scale2[p];
+        }
         // eight columns of one row at a time: neighbouring lanes read and store neighbouring pieces
         for (uint32_t e = GEMM_SLICE * blockDim.x + threadIdx.x; e < rows * (BN / 8); e += g.ksplit * blockDim.x) {
             const uint32_t row = e / (BN / 8), c0 = (e % (BN / 8)) * 8, tok = tile_m * BM + row, n0 = tile_n * BN + c0;
-            if (n0 >= g.n_out) continue;
+            if (n0 >= n_out) continue;
             float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 4
             for (uint32_t p = 0; p < g.ksplit; ++p) {
@@ -1027,17 +1037,17 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             const float rs = g.row_scale ? g.row_scale[tok] : 1.0f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], g.scale2), g.inv_input_scale) * rs;
-            const size_t o = (size_t)tok * g.n_out + n0;
-            const uint32_t valid = min(8u, g.n_out - n0);
-            const bool vec_ok = (g.n_out & 7) == 0 && ((reinterpret_cast<uintptr_t>(g.y) | reinterpret_cast<uintptr_t>(g.residual)) & 15) == 0;
+            for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fmul_rn(v[i], scale2), g.inv_input_scale) * rs;
+            const size_t o = (size_t)tok * n_out + n0;
+            const uint32_t valid = min(8u, n_out - n0);
+            const bool vec_ok = (n_out & 7) == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(g.residual)) & 15) == 0;
             if (g.y_dtype == MUSER_DTYPE_F32)
-                store_strip<float, 8>(v, reinterpret_cast<float *>(g.y) + o, g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
+                store_strip<float, 8>(v, reinterpret_cast<float *>(y) + o, g.residual ? reinterpret_cast<const float *>(g.residual) + o : nullptr, valid, vec_ok);
             else if (g.y_dtype == MUSER_DTYPE_BF16)
-                store_strip<__nv_bfloat16, 8>(v, reinterpret_cast<__nv_bfloat16 *>(g.y) + o,
+                store_strip<__nv_bfloat16, 8>(v, reinterpret_cast<__nv_bfloat16 *>(y) + o,
                                               g.residual ? reinterpret_cast<const __nv_bfloat16 *>(g.residual) + o : nullptr, valid, vec_ok);
             else
-                store_strip<__half, 8>(v, reinterpret_cast<__half *>(g.y) + o, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
+                store_strip<__half, 8>(v, reinterpret_cast<__half *>(y) + o, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
         }
         split_barrier(); // no CTA leaves while another may read its sums
     }
@@ -1309,19 +1319,22 @@ static uint32_t box_tokens(uint32_t tokens) { return std::min<uint32_t>(BM, (tok
 
 // CTAs that share the K of one output tile.  A slab takes a CTA 0.45 us, so a long K over few tiles leaves most SMs idle:
 // 5120 x 27648 has 20 tiles of 108 slabs per 128 tokens.  Split where all tiles with all their slices are on the GPU at once
-// (clusters stay inside a GPC) and a slice keeps eight slabs.  Rows below 48 slabs are left whole: measured are 108 slabs
+// (clusters stay inside a GPC).  From 48 slabs on as often as a slice keeps eight slabs: measured are 108 slabs
 // (us, whole -> split: 48 -> 20 at 16 tokens, 52 -> 29 at 128, 52 -> 34 at 384; 509 tokens are 80 tiles, whole) and rows of
-// 48 (1024 x 12288 24 -> 10 at 16 tokens, 28 -> 17 at 128), not shorter ones.
+// 48 (1024 x 12288 24 -> 10 at 16 tokens, 28 -> 17 at 128).  Rows of kSplitMin to 47 slabs in four or two where there are so
+// few tokens that the meeting costs less than the slabs: 20 slabs up to 59 tokens (5120 + 1024 + 1024 rows of 5120 inputs
+// 9.9 -> 6.8 us at one token, 8.7 at 16, 9.0 at 32, 9.9 at 48; 5120 x 5120 with residual 10.3 -> 8.5 at 16), 12 slabs up to 21
+// (3072 x 3072 7.4 -> 6.8 at 16).
 // What the bits of a result depend on: the number of slices, i.e. the weight's rows and row length, the token count and the
 // device (its SMs, and how many clusters of a size it holds).  Calls with a logit scale or soft cap, the fused gate/up form
 // and contexts that use the paired kernel never split; a group gives the bits of the single calls.
+constexpr uint32_t kSplitMin = 12;
 struct SplitRoom {
     bool asked = false;
     int n[9] = {}; // clusters of n CTAs the device holds at once
 };
-static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
-    const uint32_t k_tiles = (uint32_t)((w->n_in + BK - 1) / BK), tiles = (uint32_t)(w->n_out_pad / BN) * ((tokens + BM - 1) / BM);
-    if (k_tiles < 48 || tiles * 2 > (uint32_t)ctx->sm_count || ctx->device < 0 || ctx->device >= kMaxDevices) return 1;
+static SplitRoom split_room(Ctx *ctx) {
+    if (ctx->device < 0 || ctx->device >= kMaxDevices) return SplitRoom{};
     static PerDevice<SplitRoom> rooms;
     std::lock_guard<std::mutex> lock(rooms.mu);
     SplitRoom &room = rooms.slot[ctx->device];
@@ -1329,7 +1342,7 @@ static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
         // Asked once and kept whatever the answer, so that the process's calls agree: a device that cannot say holds no
         // clusters.  (Its error is taken off: whole tiles need no clusters, and the launch reports errors of its own.)
         room.asked = true;
-        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, true>;
+        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, kCluster>;
         cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes);
         for (int n = 2; n <= 8 && e == cudaSuccess; ++n) {
             cudaLaunchConfig_t cfg = {};
@@ -1344,9 +1357,32 @@ static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
             for (int &n : room.n) n = 0;
         }
     }
+    return room;
+}
+// us of a tile in `ks` slices beside its launch: a slab 0.43, the meeting of the slices 0.6 and 0.075 per token row
+static double split_us(uint32_t k_tiles, uint32_t ks, uint32_t tokens) {
+    return std::ceil((double)k_tiles / ks) * 0.43 + (ks > 1 ? 0.6 + 0.075 * std::min<uint32_t>(tokens, BM) : 0.0);
+}
+static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
+    const uint32_t k_tiles = (uint32_t)((w->n_in + BK - 1) / BK), tiles = (uint32_t)(w->n_out_pad / BN) * ((tokens + BM - 1) / BM);
+    if (k_tiles < kSplitMin || tiles * 2 > (uint32_t)ctx->sm_count) return 1;
+    const SplitRoom room = split_room(ctx);
+    if (k_tiles < 48) {
+        for (uint32_t ks = 4; ks >= 2; ks -= 2)
+            if (tokens <= (uint32_t)BM && tiles <= (uint32_t)room.n[ks] && split_us(k_tiles, ks, tokens) <= 0.8 * split_us(k_tiles, 1, tokens)) return ks;
+        return 1;
+    }
     for (uint32_t ks = 8; ks >= 2; --ks)
         if (tiles <= (uint32_t)room.n[ks] && k_tiles / ks >= 8) return ks;
     return 1;
+}
+static void cluster_launch(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], uint32_t ctas, uint32_t size, size_t smem, cudaStream_t stream) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = size, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ctas), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+    cfg.attrs = attr, cfg.numAttrs = 2;
 }
 
 // ------------------------------------------------------------------------------------------ paired CTAs
@@ -1358,7 +1394,7 @@ static uint32_t pair_room(Ctx *ctx) {
     std::lock_guard<std::mutex> lock(rooms.mu);
     Room &room = rooms.slot[ctx->device];
     if (room.n < 0) {
-        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, false, true>;
+        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, kWhole, true>;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1387,19 +1423,14 @@ static bool takes_pairs(Ctx *ctx, uint32_t n_tiles, uint32_t m_blocks) {
 }
 template <bool DUAL, bool TAIL, bool QOUT, bool GROUP>
 static cudaError_t launch_pairs(Ctx *ctx, const CUtensorMap &map_a, const GemmMaps &maps, const GemmArgs &g, cudaStream_t stream) {
-    const auto kernel = nvfp4_gemm_kernel<DUAL, TAIL, QOUT, GROUP, false, true>;
+    const auto kernel = nvfp4_gemm_kernel<DUAL, TAIL, QOUT, GROUP, kWhole, true>;
     const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kPSmemBytes);
     if (e != cudaSuccess) return e;
     const uint32_t room = pair_room(ctx);
     if (!room) return cudaErrorNotSupported;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 2, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2 * std::min(room, g.n_tiles * ((g.tokens + 2 * BM - 1) / (2 * BM))));
-    cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kPSmemBytes, cfg.stream = stream, cfg.attrs = attr, cfg.numAttrs = 2;
+    cluster_launch(cfg, attr, 2 * std::min(room, g.n_tiles * ((g.tokens + 2 * BM - 1) / (2 * BM))), 2, kPSmemBytes, stream);
     return cudaLaunchKernelEx(&cfg, kernel, map_a, maps, g);
 }
 
@@ -1468,16 +1499,11 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     const uint32_t tiles = g.n_tiles * m_blocks;
     if (ks > 1) {
         g.ksplit = ks;
-        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, true>;
+        const auto kernel = nvfp4_gemm_kernel<false, false, false, false, kCluster>;
         MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes));
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = ks, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(tiles * ks), cfg.blockDim = dim3(kGemmThreads), cfg.dynamicSmemBytes = kSmemBytes, cfg.stream = stream;
-        cfg.attrs = attr, cfg.numAttrs = 2;
+        cluster_launch(cfg, attr, tiles * ks, ks, kSmemBytes, stream);
         MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, map_a, maps, g));
         return MUSER_CUDA_OK;
     }
@@ -1507,9 +1533,11 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
 // launch / apart: 3 x 1024 rows of 27648 inputs 53 / 40 at 16 tokens, 54 / 54 at 100, 55 / 64 at 200; 2048 + 512 + 512 of
 // 12288 27 / 25 at 8, 26 / 29 at 16, 28 / 51 at 128; 12288 + 1024 + 1024 of 12288 28 / 36 at 8, 31 / 63 at 256.  (Not split
 // at all, with other bits than the single calls': 50, 51, 52; 25, 25, 27; 28, 32.)
-static bool group_in_one_launch(const uint32_t *slices, const Weight *const *ws, uint32_t n, uint32_t tokens, int sm_count) {
-    const uint32_t m_tiles = (tokens + BM - 1) / BM;
-    const double k_tiles = (double)((ws[0]->n_in + BK - 1) / BK), rows = std::min<uint32_t>(tokens, BM);
+struct GroupCost {
+    double one_launch, apart;
+};
+static GroupCost group_cost(const uint32_t *slices, const Weight *const *ws, uint32_t n, uint32_t tokens, int sm_count) {
+    const uint32_t m_tiles = (tokens + BM - 1) / BM, k_tiles = (uint32_t)((ws[0]->n_in + BK - 1) / BK);
     const auto bytes_us = [&](uint32_t tiles) { return (double)tiles / m_tiles * BN * ws[0]->n_in * 0.5625 / 6.5e6; };
     const auto whole_us = [&](uint32_t tiles) { return tiles ? std::max(std::ceil((double)tiles / sm_count) * k_tiles * 0.43, bytes_us(tiles)) + 4.0 : 0.0; };
     uint32_t all = 0, unsplit = 0, most = 1;
@@ -1517,10 +1545,10 @@ static bool group_in_one_launch(const uint32_t *slices, const Weight *const *ws,
     for (uint32_t p = 0; p < n; ++p) {
         const uint32_t tiles = (uint32_t)(ws[p]->n_out_pad / BN) * m_tiles;
         all += tiles, most = std::max(most, slices[p]);
-        if (slices[p] > 1) apart += std::max(std::ceil(k_tiles / slices[p]) * 0.43, bytes_us(tiles)) + 4.6 + 0.075 * rows;
+        if (slices[p] > 1) apart += std::max(std::ceil((double)k_tiles / slices[p]) * 0.43, bytes_us(tiles)) + 4.6 + 0.075 * std::min<uint32_t>(tokens, BM);
         else unsplit += tiles;
     }
-    return whole_us(all) + (most - 1) * 0.5 <= apart + whole_us(unsplit);
+    return GroupCost{whole_us(all) + (most - 1) * 0.5, apart + whole_us(unsplit)};
 }
 
 // Up to four projections of the same quantized activations in one launch (GROUP form of the kernel).
@@ -1530,7 +1558,19 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     uint32_t slices[4] = {1, 1, 1, 1}; // (the paired kernel, which serves single calls where it is on, never splits)
     bool sliced = false;
     for (uint32_t p = 0; p < n && ctx->nvfp4_pair != 1; ++p) slices[p] = gemm_ksplit(ctx, ws[p], tokens), sliced = sliced || slices[p] > 1;
-    if (sliced && !group_in_one_launch(slices, ws, n, tokens, ctx->sm_count)) {
+    // All of them in the same number of slices and all clusters on the GPU at once: clusters.  (In two rounds 5120 + 2560 + 2560
+    // rows of 5120 inputs took 15.4 us at 16 tokens, whole tiles with sliced sums 12.)
+    const uint32_t m_blocks = (tokens + BM - 1) / BM;
+    uint32_t tiles_n = 0;
+    for (uint32_t p = 0; p < n; ++p) tiles_n += (uint32_t)(ws[p]->n_out_pad / BN);
+    bool clusters = sliced;
+    for (uint32_t p = 1; p < n; ++p) clusters = clusters && slices[p] == slices[0];
+    const GroupCost cost = group_cost(slices, ws, n, tokens, ctx->sm_count);
+    if (clusters) {
+        const uint32_t k_tiles = (uint32_t)((w0->n_in + BK - 1) / BK);
+        clusters = tiles_n * m_blocks <= (uint32_t)split_room(ctx).n[slices[0]] && split_us(k_tiles, slices[0], tokens) + 4.0 <= std::min(cost.one_launch, cost.apart);
+    }
+    if (sliced && !clusters && cost.one_launch > cost.apart) {
         const Weight *rest[4];
         void *rest_y[4];
         uint32_t n_rest = 0;
@@ -1544,9 +1584,6 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
         }
         return n_rest ? launch_nvfp4_gemm_group(ctx, rest, n_rest, x_packed, x_scales, rest_y, y_dtype, tokens, stream) : MUSER_CUDA_OK;
     }
-    const uint32_t m_blocks = (tokens + BM - 1) / BM;
-    uint32_t tiles_n = 0;
-    for (uint32_t p = 0; p < n; ++p) tiles_n += (uint32_t)(ws[p]->n_out_pad / BN);
     bool pair = !sliced && takes_pairs(ctx, tiles_n, m_blocks);
     for (uint32_t p = 0; p < n; ++p) pair = pair && pair_rows_fit(ys[p], nullptr, ws[p]->n_out, y_dtype);
     const uint32_t a_rows = pair ? BM : box_tokens(tokens);
@@ -1591,7 +1628,17 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
     }
     const uint32_t tiles = tiles_n * m_blocks;
     const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
-    const auto kernel = sliced ? nvfp4_gemm_kernel<false, false, false, true, true> : nvfp4_gemm_kernel<false, false, false, true>;
+    if (clusters) {
+        const auto kernel = nvfp4_gemm_kernel<false, false, false, true, kCluster>;
+        MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes));
+        g.ksplit = slices[0];
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[2];
+        cluster_launch(cfg, attr, tiles * slices[0], slices[0], kSmemBytes, stream);
+        MUSER_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, map_a, maps, g));
+        return MUSER_CUDA_OK;
+    }
+    const auto kernel = sliced ? nvfp4_gemm_kernel<false, false, false, true, kSliced> : nvfp4_gemm_kernel<false, false, false, true>;
     MUSER_CUDA_TRY(ctx, ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kSmemBytes));
     MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(grid), dim3(kGemmThreads), kSmemBytes, stream, map_a, maps, g));
     MUSER_CUDA_TRY(ctx, cudaGetLastError());
