@@ -1322,9 +1322,9 @@ static uint32_t box_tokens(uint32_t tokens) { return std::min<uint32_t>(BM, (tok
 // (clusters stay inside a GPC).  From 48 slabs on as often as a slice keeps eight slabs: measured are 108 slabs
 // (us, whole -> split: 48 -> 20 at 16 tokens, 52 -> 29 at 128, 52 -> 34 at 384; 509 tokens are 80 tiles, whole) and rows of
 // 48 (1024 x 12288 24 -> 10 at 16 tokens, 28 -> 17 at 128).  Rows of kSplitMin to 47 slabs in four or two where there are so
-// few tokens that the meeting costs less than the slabs: 20 slabs up to 59 tokens (5120 + 1024 + 1024 rows of 5120 inputs
-// 9.9 -> 6.8 us at one token, 8.7 at 16, 9.0 at 32, 9.9 at 48; 5120 x 5120 with residual 10.3 -> 8.5 at 16), 12 slabs up to 21
-// (3072 x 3072 7.4 -> 6.8 at 16).
+// few tokens that the meeting costs clearly less than the slabs: 20 slabs up to 43 tokens (5120 + 1024 + 1024 rows of 5120
+// inputs 9.9 -> 6.8 us at one token, 8.7 at 16, 9.0 at 32, 9.9 at 48; 5120 x 5120 with residual 10.3 -> 8.5 at 16), 12 slabs up
+// to 22 (3072 x 3072 7.4 -> 5.2 at one, 6.8 at 16).
 // What the bits of a result depend on: the number of slices, i.e. the weight's rows and row length, the token count and the
 // device (its SMs, and how many clusters of a size it holds).  Calls with a logit scale or soft cap, the fused gate/up form
 // and contexts that use the paired kernel never split; a group gives the bits of the single calls.
@@ -1369,7 +1369,7 @@ static uint32_t gemm_ksplit(Ctx *ctx, const Weight *w, uint32_t tokens) {
     const SplitRoom room = split_room(ctx);
     if (k_tiles < 48) {
         for (uint32_t ks = 4; ks >= 2; ks -= 2)
-            if (tokens <= (uint32_t)BM && tiles <= (uint32_t)room.n[ks] && split_us(k_tiles, ks, tokens) <= 0.8 * split_us(k_tiles, 1, tokens)) return ks;
+            if (tokens <= (uint32_t)BM && tiles <= (uint32_t)room.n[ks] && split_us(k_tiles, ks, tokens) <= 0.7 * split_us(k_tiles, 1, tokens)) return ks;
         return 1;
     }
     for (uint32_t ks = 8; ks >= 2; --ks)

@@ -639,3 +639,33 @@ def test_paired_forms_equal_the_single_sm_forms(gpu, n_in, tokens):
         assert torch.equal(a, b), f"output {i} differs between the two forms"
     for w in ws:
         w.free()
+
+
+@pytest.mark.parametrize("n_in, shapes", [(3072, (300, 256)), (3136, (37, 700, 256)), (5120, (5120, 1024, 1024)), (5120, (5120, 2560, 2560)), (12032, (300, 37))])
+@pytest.mark.parametrize("tokens", [1, 16, 22, 23, 43, 44, 128])
+def test_groups_of_shorter_rows_split_as_the_single_calls(gpu, n_in, shapes, tokens):
+    """Rows of 12 to 47 slabs, cut between the CTAs of a cluster up to a number of tokens, ragged ones among them: a group, as
+    one launch of clusters or (too many of them for the GPU) of whole tiles with sliced sums, carries the single calls' bits,
+    and they are the exact products' (f32 sums: some 1e-6 of their norm)."""
+    op, ctx, k = gpu
+    from muser_b200 import synth
+    x = synth.normal_activations(tokens, n_in, seed=13)
+    isi = synth.activation_input_scale_inv(x)
+    made = [make_weight(op, ctx, min(n, 300), n_in, seed=60 + i) for i, n in enumerate(shapes)]
+    made = [(np.resize(p, (n, n_in // 2)), np.resize(s, (n, n_in // 16)), s2) for (p, s, s2), n in zip(made, shapes)]
+    ws = [op.Weight(ctx, op.TensorView(p, O.NVFP4, n_in, n, s, s2, isi)) for (p, s, s2), n in zip(made, shapes)]
+    q = k.quantize_nvfp4_activation(x.cuda(), isi)
+    alone, grouped = ([torch.full((tokens, n), float("nan"), device="cuda") for n in shapes] for _ in range(2))
+    for w, y in zip(ws, alone):
+        k.encode_nvfp4_prequant(w, *q, y, tokens)
+    k.encode_nvfp4_group_prequant(ws, *q, grouped, tokens)
+    ctx.sync_status()
+    for a, b in zip(alone, grouped):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    xp, xs = synth.quantize_nvfp4(x.float(), isi)
+    p, s, s2 = made[-1]
+    rows = min(shapes[-1], 300)
+    want = O.dequant_nvfp4(xp.numpy(), xs.numpy(), 1.0).astype(np.float64) @ O.dequant_nvfp4(p[:rows], s[:rows], s2).astype(np.float64).T / isi
+    assert H.rel_l2(alone[-1][:, :rows].double().cpu().numpy(), want) <= 3e-6
+    for w in ws:
+        w.free()
