@@ -257,7 +257,7 @@ struct Q4Regs {
 };
 struct Q5Regs {
     uint4 q[4];
-    uint4 hbits; // [2*rowsel + half]: byte jj = the fifth bits of the lane's eight elements of sub-block 4*half + jj
+    uint4 hbits; // [2*rowsel + half]: the fifth bits of the lane's elements of sub-blocks 4*half .. + 3 (q5_fifth)
     uint4 ha, hb;
 };
 __device__ __forceinline__ Q5Regs load_regs(const uint8_t *tile, int lane, Q5Regs *) { // tile: shared memory
@@ -271,8 +271,6 @@ __device__ __forceinline__ Q5Regs load_regs(const uint8_t *tile, int lane, Q5Reg
     r.hb = h[(lane >> 2) + 8];
     return r;
 }
-// four fifth bits (x < 16) onto bit 4 of four bytes
-__device__ __forceinline__ uint32_t spread_bit4(uint32_t x) { return (x * 0x02040810u) & 0x10101010u; }
 __device__ __forceinline__ Q4Regs load_regs(const uint8_t *tile, int lane, Q4Regs *) { // tile: shared memory
     Q4Regs r;
     const uint4 *q = reinterpret_cast<const uint4 *>(tile);
@@ -320,9 +318,9 @@ __device__ __forceinline__ void q45_compute(const Regs &r, const uint4 *fb, cons
             uint32_t a0 = wa & 0x0F0F0F0Fu, a2 = (wa >> 4) & 0x0F0F0F0Fu;
             uint32_t a1 = wb & 0x0F0F0F0Fu, a3 = (wb >> 4) & 0x0F0F0F0Fu;
             if constexpr (Q5) {
-                const uint32_t ba = (uint32_t)ubyte(gw(r.hbits, j >> 2), j & 3), bb = (uint32_t)ubyte(gw(r.hbits, 2 + (j >> 2)), j & 3);
-                a0 |= spread_bit4(ba & 15u), a2 |= spread_bit4(ba >> 4);
-                a1 |= spread_bit4(bb & 15u), a3 |= spread_bit4(bb >> 4);
+                const uint32_t fa = gw(r.hbits, j >> 2), fb = gw(r.hbits, 2 + (j >> 2));
+                a0 |= q5_fifth(fa, 2 * (j & 3)), a2 |= q5_fifth(fa, 2 * (j & 3) + 1);
+                a1 |= q5_fifth(fb, 2 * (j & 3)), a3 |= q5_fifth(fb, 2 * (j & 3) + 1);
             }
             const int sa = ubyte(ha.sc[j >> 2], j & 3), sb = ubyte(hb.sc[j >> 2], j & 3);
 #pragma unroll

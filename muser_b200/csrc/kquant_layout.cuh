@@ -15,9 +15,9 @@
 // Q5_K tile (2816 bytes): the Q4_K tile with a plane of fifth bits between the nibbles and the headers.
 //   [0, 2048)   the low four bits of every weight, exactly as in a Q4_K tile.
 //   [2048,2560) uint4 (lane): word 0 = row g, sub-blocks 0-3; word 1 = row g, sub-blocks 4-7; words 2, 3 = row g + 8.
-//               Byte jj of a word holds the fifth bits of the lane's eight elements of that sub-block in the order the
-//               nibble word yields them: bit b (0..3) belongs to the element in the LOW nibble of byte b, bit 4 + b to
-//               the one in the HIGH nibble, so (x * 0x02040810) & 0x10101010 drops four of them onto bit 4 of four bytes.
+//               Bit 2 jj + h of byte b belongs to the element of the half's sub-block jj in the low (h = 0) or high (h = 1)
+//               nibble of byte b of the nibble word, so one shift and one mask (q5_fifth) put four of them onto bit 4 of four
+//               bytes.  (With a sub-block's eight bits in one byte it took a byte extraction, a mask and a product.)
 //   [2560,2816) 16 x the block's 16-byte header (d, dmin, 6-bit scales and mins), as in Q4_K.
 // Q6_K tile (3360 bytes).  A weight is stored as v = (q - 32) & 63 (six-bit two's complement), split into its top
 // four bits T = v >> 2 and low two bits L = v & 3, so that (T << 4) | (L << 2) is the signed byte 4 * (q - 32).
@@ -52,6 +52,8 @@ inline KqGeom kq_geom(const Weight &w) {
     return g;
 }
 
+// Q5_K: bits x = 2 jj + h of a word of the fifth-bit plane on bit 4 of the four bytes (no other byte's bit reaches a bit 4)
+__host__ __device__ __forceinline__ uint32_t q5_fifth(uint32_t plane, int x) { return (x < 4 ? plane << (4 - x) : plane >> (x - 4)) & 0x10101010u; }
 __host__ __device__ __forceinline__ int q4_nibble_pos(int i) { return (i & 1) * 4 + (i >> 1); }
 
 } // namespace muser

@@ -74,7 +74,6 @@ namespace mm {
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
 __device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
 __device__ __forceinline__ uint32_t gw(const uint4 &v, int i) { return (&v.x)[i]; } // compile-time i only
-__device__ __forceinline__ uint32_t spread_bit4(uint32_t x) { return (x * 0x02040810u) & 0x10101010u; } // four fifth bits onto bit 4 of four bytes
 // bytes 2 i, 2 i + 1 of w as an f16 pair: 0x6400 | v is 1024 + v
 __device__ __forceinline__ __half2 byte_pair(uint32_t w, uint32_t i, float bias = 1024.0f) {
     return __hsub2(u2h(__byte_perm(w, 0x64646464u, i ? 0x4342u : 0x4140u)), __float2half2_rn(bias));
@@ -151,8 +150,8 @@ __device__ __forceinline__ void tile_q45(const uint8_t *tile, const uint8_t *blo
             const __half2 sc = kPairs ? both(scales[r], j & 1) : byte_twice(r ? hb.sc[j >> 2] : ha.sc[j >> 2], j & 3);
             auto pair = [&](uint32_t bits) { return h2u(__hmul2(u2h(bits), sc)); };
             if constexpr (Q5) {
-                const uint32_t hi = (gw(hbits, 2 * r + (j >> 2)) >> (8 * (j & 3))) & 0xFFu;
-                const uint32_t wl = (w & 0x0F0F0F0Fu) | spread_bit4(hi & 15u), wh = ((w >> 4) & 0x0F0F0F0Fu) | spread_bit4(hi >> 4);
+                const uint32_t fifth = gw(hbits, 2 * r + (j >> 2));
+                const uint32_t wl = (w & 0x0F0F0F0Fu) | q5_fifth(fifth, 2 * (j & 3)), wh = ((w >> 4) & 0x0F0F0F0Fu) | q5_fifth(fifth, 2 * (j & 3) + 1);
                 av[0][r] = pair(wl & 0x00FF00FFu), av[0][2 + r] = pair(wh & 0x00FF00FFu);
                 av[1][r] = pair((wl >> 8) & 0x00FF00FFu), av[1][2 + r] = pair((wh >> 8) & 0x00FF00FFu);
             } else {

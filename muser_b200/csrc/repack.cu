@@ -53,7 +53,7 @@ __global__ void repack_q4k_kernel(const uint8_t *__restrict__ raw, uint8_t *__re
             }
         }
         reinterpret_cast<uint32_t *>(tile_ptr)[(u * 32 + lane) * 4 + jj] = word;
-    } else if (Q5 && unit < 512 + 128) { // one word of the fifth-bit plane: (lane, rowsel, half) -> four sub-blocks' bytes
+    } else if (Q5 && unit < 512 + 128) { // one word of the fifth-bit plane: (lane, rowsel, half) -> four sub-blocks' bits
         uint32_t v = unit - 512, lane = v >> 2, wi = v & 3;
         uint32_t g = lane >> 2, t = lane & 3;
         uint32_t row = rt * 16 + g + 8 * (wi >> 1), half = wi & 1;
@@ -68,7 +68,7 @@ __global__ void repack_q4k_kernel(const uint8_t *__restrict__ raw, uint8_t *__re
                     uint32_t bit = (blk[16 + (e & 31)] >> j) & 1u;
                     // element i sits in nibble q4_nibble_pos(i) of the nibble word: byte pos / 2, low or high nibble
                     uint32_t pos = q4_nibble_pos(i), b = pos >> 1, hi = pos & 1;
-                    word |= bit << (8 * jj + 4 * hi + b);
+                    word |= bit << (8 * b + 2 * jj + hi);
                 }
             }
         }
@@ -240,10 +240,10 @@ __device__ __forceinline__ float q4k_weight(const uint8_t *__restrict__ image, u
     uint32_t q = rowsel * 2 + (j >> 2);
     uint32_t word = reinterpret_cast<const uint32_t *>(tile)[(q * 32 + g * 4 + wi) * 4 + (j & 3)]; // lane (g, 8-element group), word = sub-block % 4
     uint32_t nib = (word >> (4 * q4_nibble_pos(i))) & 15u;
-    if constexpr (Q5) { // the fifth bit: byte (j % 4) of word (2 * rowsel + j / 4) of the lane's uint4, see kquant_layout.cuh
+    if constexpr (Q5) { // the fifth bit: in word 2 * rowsel + j / 4 of the lane's uint4, see kquant_layout.cuh
         uint32_t hw = reinterpret_cast<const uint32_t *>(tile + kQ5OffHi)[(g * 4 + wi) * 4 + rowsel * 2 + (j >> 2)];
         uint32_t pos = q4_nibble_pos(i);
-        nib |= ((hw >> (8 * (j & 3) + 4 * (pos & 1) + (pos >> 1))) & 1u) << 4;
+        nib |= ((hw >> (8 * (pos >> 1) + 2 * (j & 3) + (pos & 1))) & 1u) << 4;
     }
     const uint8_t *hdr = tile + (Q5 ? kQ5OffHdr : 2048) + r * 16;
     float d = __half2float(*reinterpret_cast<const __half *>(hdr));
