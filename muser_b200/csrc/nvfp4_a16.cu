@@ -70,16 +70,18 @@ struct A16Args {
     uint32_t n_out, n_in, kt, tokens, y_dtype, ksplit, row_tiles;
 };
 
-// Four E2M1 codes (the low 16 bits of w, one per nibble) -> four int8 of the codes' values in halves
-// (quant/nvfp4.rs:16-30).  A byte permute looks the magnitude up by the nibble's low three bits; with the nibble's
-// sign bit set it replicates the looked-up byte's top bit instead, i.e. gives 0.  One permute on the codes as they are
-// yields the positive values, one on the codes with their sign bits flipped the negative ones' magnitudes; the bias
-// keeps the borrows of the 32-bit difference inside their bytes.
+// Four E2M1 codes (the low 16 bits of w, one per nibble) -> the positive ones' values in halves as four bytes
+// (quant/nvfp4.rs:16-30).  A byte permute looks the magnitude up by the nibble's low three bits; with the nibble's sign bit
+// set it replicates the looked-up byte's top bit instead, i.e. gives 0.
+__device__ __forceinline__ uint32_t e2m1_positive(uint32_t w) {
+    uint32_t v; // (the __byte_perm intrinsic uses three bits of a selector)
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(0x03020100u), "r"(0x0C080604u), "r"(w));
+    return v;
+}
+// Four int8 of the codes' values: on the codes with their sign bits flipped the permute yields the negative ones' magnitudes;
+// the bias keeps the borrows of the 32-bit difference inside their bytes.
 __device__ __forceinline__ uint32_t e2m1_halves(uint32_t w, uint32_t w_flipped) {
-    uint32_t pos, neg; // (the __byte_perm intrinsic uses three bits of a selector)
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(pos) : "r"(0x03020100u), "r"(0x0C080604u), "r"(w));
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(neg) : "r"(0x03020100u), "r"(0x0C080604u), "r"(w_flipped));
-    return (pos + 0x80808080u - neg) ^ 0x80808080u;
+    return (e2m1_positive(w) + 0x80808080u - e2m1_positive(w_flipped)) ^ 0x80808080u;
 }
 __device__ __forceinline__ void imma_k32(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -118,6 +120,11 @@ constexpr int a16_ctas_per_sm(int pairs) { return pairs == 1 ? 3 : 2; } // what 
 // instructions per weight.
 template <int PAIRS, int CTAS>
 __global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const __grid_constant__ A16Args a) {
+    // With three CTAs an SM the byte-and-logic pipe bounds the kernel, and positive and negative values in products of their
+    // own, which meet in the sums, cost it four instructions less per eight codes (us at two tokens: 27648 x 5120 30.9 -> 28.3,
+    // 5120 x 27648 40.5 -> 36.6); with fewer warps or more tokens the products do (1024 x 5120 5.9 -> 6.4, 27648 x 5120 at 8
+    // tokens 62 -> 73).
+    constexpr bool kApart = CTAS == 3;
     __shared__ float contrib[2][kA16Warps][2 * PAIRS * 16];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t slot = warp / a.ksplit, part = warp % a.ksplit, slots = kA16Warps / a.ksplit;
@@ -169,14 +176,19 @@ __global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const _
                 for (int p = 0; p < PAIRS; ++p) sum[p][0] = sum[p][1] = 0;
 #pragma unroll
                 for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t av[4][4];
+                    uint32_t av[4][4], neg[4][4]; // kApart: the positive values, and the negative ones' magnitudes
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
 #pragma unroll
                         for (int r = 0; r < 2; ++r) {
                             const uint32_t w = word(cur.c[ch][r], i), f = w ^ 0x88888888u;
-                            av[i][r] = e2m1_halves(w, f);
-                            av[i][2 + r] = e2m1_halves(w >> 16, f >> 16);
+                            if constexpr (kApart) {
+                                av[i][r] = e2m1_positive(w), neg[i][r] = e2m1_positive(f);
+                                av[i][2 + r] = e2m1_positive(w >> 16), neg[i][2 + r] = e2m1_positive(f >> 16);
+                            } else {
+                                av[i][r] = e2m1_halves(w, f);
+                                av[i][2 + r] = e2m1_halves(w >> 16, f >> 16);
+                            }
                         }
                     int q0[4], q1[4]; // groups 4 (t & 1) .. + 3 of the chunk, rows g and g + 8
                     e4m3_q9(cur.s[ch][0], q0);
@@ -195,6 +207,13 @@ __global__ void __launch_bounds__(kA16Warps * 32, CTAS) nvfp4_a16_kernel(const _
                             const uint4 &x = h ? x1 : x0;
                             imma_k32(d, av[2 * h][0], av[2 * h][1], av[2 * h][2], av[2 * h][3], x.x, x.y);
                             imma_k32(d, av[2 * h + 1][0], av[2 * h + 1][1], av[2 * h + 1][2], av[2 * h + 1][3], x.z, x.w);
+                            if constexpr (kApart) {
+                                int n[4] = {0, 0, 0, 0};
+                                imma_k32(n, neg[2 * h][0], neg[2 * h][1], neg[2 * h][2], neg[2 * h][3], x.x, x.y);
+                                imma_k32(n, neg[2 * h + 1][0], neg[2 * h + 1][1], neg[2 * h + 1][2], neg[2 * h + 1][3], x.z, x.w);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) d[i] -= n[i];
+                            }
                             sum[p][0] += (long long)d[0] * q0[h] + (long long)d[1] * q0[2 + h];
                             sum[p][1] += (long long)d[2] * q1[h] + (long long)d[3] * q1[2 + h];
                         }
