@@ -176,31 +176,7 @@ __global__ void __launch_bounds__(kRmsThreads) rms_rows_staged_kernel(const void
         inv_rms[row0 + threadIdx.x] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)n_in), eps)));
 }
 
-// Up to so many rows of bf16.  f32 rows carry twice the bytes per value and the crew falls behind the chains earlier
-// (norm + quantize, us, staged / one warp per 32 chains: 2048 values 28 / 30 at 4096 rows; 5120 values 48 / 59 at 2048,
-// 73 / 66 at 3072; 8192 values 77 / 86 at 1536, 98 / 92 at 2048; 27648 values 234 / 282 at 1536, 339 / 305 at 2048).
-constexpr uint32_t kRmsStagedRows = 4096;
-static uint32_t rms_staged_rows(uint32_t x_dtype, uint32_t n_in) {
-    if (x_dtype != MUSER_DTYPE_F32 || n_in <= 2048) return kRmsStagedRows;
-    return n_in <= 5120 ? 2048 : 1536;
-}
-
-static cudaError_t launch_rms_rows_sequential(Ctx *ctx, const void *x, uint32_t x_dtype, uint32_t tokens, uint32_t n_in, float eps,
-                                              float *inv_rms, cudaStream_t stream) {
-    if (tokens <= rms_staged_rows(x_dtype, n_in)) {
-        const auto kernel = x_dtype == MUSER_DTYPE_F32 ? rms_rows_staged_kernel<true> : rms_rows_staged_kernel<false>;
-        const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kRmsSmem);
-        if (e != cudaSuccess) return e;
-        return launch_pdl(kernel, dim3((tokens + kRmsRows - 1) / kRmsRows), dim3(kRmsThreads), kRmsSmem, stream, x, tokens, n_in, eps, inv_rms);
-    }
-    const unsigned blocks = (tokens + 31) / 32;
-    const bool f32 = x_dtype == MUSER_DTYPE_F32;
-    const size_t smem = (size_t)2 * 32 * ((f32 ? 64 : 32) + 1) * sizeof(uint4);
-    const void *fn = f32 ? reinterpret_cast<const void *>(rms_rows_sequential_kernel<true>) : reinterpret_cast<const void *>(rms_rows_sequential_kernel<false>);
-    const cudaError_t e = ensure_dynamic_smem(fn, ctx->device, smem);
-    if (e != cudaSuccess) return e;
-    return launch_pdl(f32 ? rms_rows_sequential_kernel<true> : rms_rows_sequential_kernel<false>, dim3(blocks), dim3(32), smem, stream, x, tokens, n_in, eps, inv_rms);
-}
+constexpr uint32_t kRmsStagedRows = 4096; // beyond: the warp per 32 chains above
 
 // ---- the chain without its latency ----------------------------------------------------------------------------------
 // A chain of n dependent additions takes 4 cycles each at best.  A block cuts the row into one segment per thread.  While
@@ -219,9 +195,34 @@ struct ChainShared {
     float warp_sum[32];
     float inv_rms;
 };
+constexpr int kChainResident = 1152; // threads an SM holds (56 registers each)
 constexpr uint32_t kNoBinade = 256;
+static uint32_t chain_threads(uint32_t n_in, uint32_t eights) { return ((n_in / 8 + eights - 1) / eights + 31) / 32 * 32; }
 __device__ __forceinline__ uint2 chain_compose(uint2 first, uint2 then) {
     return make_uint2(first.x + ((first.x & 1) ? then.y : then.x), first.y + ((first.y & 1) ? then.x : then.y)); // (odd + odd: even)
+}
+// What a segment of `n` squares adds to an even and to an odd pattern, if the sum is about `before` in front of it and `after`
+// behind it and stays in the binade that is returned with it.
+__device__ __forceinline__ uint2 chain_segment(float before, float after, const float *v, int n, uint32_t &binade) {
+    binade = __float_as_uint(before) >> 23; // (sums of squares: no sign; infinities and NaN are 255)
+    if (binade != __float_as_uint(after) >> 23 || binade == 255) binade = kNoBinade;
+    const uint32_t bottom = binade << 23; // (no binade: sums that nobody looks at)
+    float even = __uint_as_float(bottom), odd = __uint_as_float(bottom + 1);
+#pragma unroll
+    for (int i = 0; i < n; ++i) even = __fadd_rn(even, v[i]), odd = __fadd_rn(odd, v[i]);
+    return make_uint2(__float_as_uint(even) - bottom, __float_as_uint(odd) - (bottom + 1));
+}
+// The lanes that begin a run of segments of one binade; `add` becomes the run's up to and with the lane's segment.
+__device__ __forceinline__ uint32_t chain_runs(uint32_t binade, uint2 &add) {
+    const uint32_t lane = threadIdx.x & 31, left = __shfl_up_sync(0xffffffffu, binade, 1);
+    const uint32_t starts = __ballot_sync(0xffffffffu, lane == 0 || binade != left || binade == kNoBinade);
+    const uint32_t start = 31 - __clz(starts & (0xffffffffu >> (31 - lane))); // of this lane's run
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint2 l = make_uint2(__shfl_up_sync(0xffffffffu, add.x, o), __shfl_up_sync(0xffffffffu, add.y, o));
+        if (lane >= start + o) add = chain_compose(l, add);
+    }
+    return starts;
 }
 // 1 / sqrt(mean(x^2) + eps) of one row of n_in <= 8 K blockDim values, for every thread of the block.
 template <bool XF32, int K>
@@ -252,26 +253,9 @@ __device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, fl
     float carry = 0.0f;
     for (uint32_t w = 0; w < warp; ++w) carry += sh.warp_sum[w];
     before += carry, after += carry;
-    uint32_t binade = __float_as_uint(before) >> 23; // (sums of squares: no sign; infinities and NaN are 255)
-    if (binade != __float_as_uint(after) >> 23 || binade == 255) binade = kNoBinade;
-    uint2 add = make_uint2(0, 0);
-    if (binade != kNoBinade) {
-        const uint32_t bottom = binade << 23;
-        float even = __uint_as_float(bottom), odd = __uint_as_float(bottom + 1);
-#pragma unroll
-        for (int i = 0; i < K; ++i)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) even = __fadd_rn(even, v[i][k]), odd = __fadd_rn(odd, v[i][k]);
-        add = make_uint2(__float_as_uint(even) - bottom, __float_as_uint(odd) - (bottom + 1));
-    }
-    const uint32_t left = __shfl_up_sync(0xffffffffu, binade, 1);
-    const uint32_t starts = __ballot_sync(0xffffffffu, lane == 0 || binade != left || binade == kNoBinade);
-    const uint32_t start = 31 - __clz(starts & (0xffffffffu >> (31 - lane))); // of this lane's run
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint2 l = make_uint2(__shfl_up_sync(0xffffffffu, add.x, o), __shfl_up_sync(0xffffffffu, add.y, o));
-        if (lane >= start + o) add = chain_compose(l, add);
-    }
+    uint32_t binade;
+    uint2 add = chain_segment(before, after, &v[0][0], 8 * K, binade);
+    const uint32_t starts = chain_runs(binade, add);
     sh.add[tid] = add, sh.binade[tid] = binade;
     if (lane == 0) sh.starts[warp] = starts;
     __syncthreads();
@@ -320,6 +304,103 @@ __device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, fl
     }
     __syncthreads();
     return sh.inv_rms;
+}
+
+// The same factors for many rows: a warp takes a row, 1024 values at a time (a segment of 32 per lane), and knows the running
+// sum at the start of each step, so nothing waits for another warp.  Each square is added twice and the 31 lanes' prefixes
+// are scanned twice per step: more work than a chain of plain additions, but 32 lanes share it and no value passes through
+// shared memory.  Segments of 8 or 16 values cost more scans for the same row (2048 rows of 2048 values, norm and quantizer:
+// 15.5 and 12.2 us against 11.5) and gain nothing on short rows (512 values: 7.8, 7.2, 7.4).
+constexpr int kChainRowWarps = 4;
+template <bool XF32>
+__global__ void __launch_bounds__(32 * kChainRowWarps) rms_rows_chain_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms) {
+    constexpr int K = 4; // eights per lane and step
+    pdl_wait();
+    pdl_release();
+    const uint32_t lane = threadIdx.x & 31, row = blockIdx.x * kChainRowWarps + (threadIdx.x >> 5), n8 = n_in / 8;
+    if (row >= tokens) return; // (whole warps)
+    const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
+                          : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
+    constexpr int kWords = XF32 ? 2 : 1; // 16-byte pieces of eight values
+    uint4 next[K][kWords];
+    auto fetch = [&](uint32_t first8) {
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            const uint32_t at = first8 + lane * K + i;
+#pragma unroll
+            for (int k = 0; k < kWords; ++k)
+                next[i][k] = at < n8 ? ld_after_wait(reinterpret_cast<const uint4 *>(xr) + (size_t)at * kWords + k) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    uint32_t s = 0; // the running sum's bit pattern, the same in every lane
+    fetch(0);
+    for (uint32_t first8 = 0; first8 < n8; first8 += 32 * K) {
+        float v[K][8], sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t w = XF32 ? (&next[i][(k / 4) % kWords].x)[k % 4] : (&next[i][0].x)[k / 2];
+                const float f = __uint_as_float(XF32 ? w : (k & 1) ? w & 0xFFFF0000u : w << 16);
+                v[i][k] = __fmul_rn(f, f), sum += v[i][k];
+            }
+        if (first8 + 32 * K < n8) fetch(first8 + 32 * K);
+        float after = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float up = __shfl_up_sync(0xffffffffu, after, o);
+            if (lane >= (uint32_t)o) after += up;
+        }
+        float before = __shfl_up_sync(0xffffffffu, after, 1);
+        before = __uint_as_float(s) + (lane ? before : 0.0f), after += __uint_as_float(s);
+        uint32_t binade;
+        uint2 add = chain_segment(before, after, &v[0][0], 8 * K, binade);
+        const uint32_t starts = chain_runs(binade, add);
+        for (uint32_t pos = 0; pos < 32;) {
+            const uint32_t rest = starts & ~(0xffffffffu >> (31 - pos)), end = rest ? __ffs(rest) - 1 : 32;
+            const uint32_t e = __shfl_sync(0xffffffffu, binade, end - 1);
+            const uint32_t even = __shfl_sync(0xffffffffu, add.x, end - 1), odd = __shfl_sync(0xffffffffu, add.y, end - 1);
+            const uint32_t sum_bits = s + ((s & 1) ? odd : even);
+            if (((starts >> pos) & 1) && (s >> 23) == e && (sum_bits >> 23) == e) {
+                s = sum_bits, pos = end;
+                continue;
+            }
+            float t = __uint_as_float(s); // (every lane adds its own squares, the segment's lane is heard)
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) t = __fadd_rn(t, v[i][k]);
+            s = __shfl_sync(0xffffffffu, __float_as_uint(t), pos);
+            ++pos;
+        }
+    }
+    if (lane == 0) inv_rms[row] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(__uint_as_float(s), (float)n_in), eps)));
+}
+
+// Which of the three leaves the factors.  The plain chains (few values per row, or enough rows that a lane each fills the chip)
+// do half the additions.  us with the quantizer, plain / warp per row, bf16: 512 values 4.5 / 4.8 at 148 rows, 6.4 / 7.4 at
+// 2048; 1024 values 6.6 / 5.4 at 449, 9.0 / 8.7 at 2048, 11.8 / 12.5 at 4096; 2048 values 14.3 / 11.5 at 2048, 18.3 / 16.9 at
+// 4096, 28.4 / 29 at 8192; 3136 values 27.5 / 23.6 at 4096, 42.6 / 40.2 at 8192, 139 / 153 at 32768; 5120 values 45 / 32 at
+// 4096, 66 / 57 at 8192, 224 / 212 at 32768; 12288 values 77 / 46 at 2048.  f32: 5120 values 72 / 52 at 4096, 352 / 353 at
+// 32768; 12288 values 136 / 72 at 2048; 27648 values 304 / 160 at 2048.
+static cudaError_t launch_rms_rows(Ctx *ctx, const void *x, uint32_t x_dtype, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms,
+                                   cudaStream_t stream) {
+    const bool f32 = x_dtype == MUSER_DTYPE_F32;
+    if (n_in >= 5120 || (n_in >= 1024 && tokens <= 2 * n_in))
+        return launch_pdl(f32 ? rms_rows_chain_kernel<true> : rms_rows_chain_kernel<false>, dim3((tokens + kChainRowWarps - 1) / kChainRowWarps),
+                          dim3(32 * kChainRowWarps), 0, stream, x, tokens, n_in, eps, inv_rms);
+    if (tokens <= kRmsStagedRows) {
+        const auto kernel = f32 ? rms_rows_staged_kernel<true> : rms_rows_staged_kernel<false>;
+        const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kRmsSmem);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(kernel, dim3((tokens + kRmsRows - 1) / kRmsRows), dim3(kRmsThreads), kRmsSmem, stream, x, tokens, n_in, eps, inv_rms);
+    }
+    const unsigned blocks = (tokens + 31) / 32;
+    const size_t smem = (size_t)2 * 32 * ((f32 ? 64 : 32) + 1) * sizeof(uint4);
+    const void *fn = f32 ? reinterpret_cast<const void *>(rms_rows_sequential_kernel<true>) : reinterpret_cast<const void *>(rms_rows_sequential_kernel<false>);
+    const cudaError_t e = ensure_dynamic_smem(fn, ctx->device, smem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(f32 ? rms_rows_sequential_kernel<true> : rms_rows_sequential_kernel<false>, dim3(blocks), dim3(32), smem, stream, x, tokens, n_in, eps, inv_rms);
 }
 
 // (x * inv_rms) * w of one row, quantized group by group by the whole block; rows past `tokens` only clear their scales.
@@ -381,16 +462,19 @@ __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
 }
 
-// Eights a thread holds in the kernel above, 0: the chains run as chains in a kernel of their own, which take their length
-// in latency but less work per row.  us with bf16 rows, chains and quantizer (or, below 449 rows, segments whose additions one
-// warp composed one after another) / this kernel: 5120 values 14.6 / 8.1 at 16 rows, 18.7 / 11.1 at 512, 28.4 / 13.9 at 1024,
-// 35.7 / 29.2 at 2048, 45 / 43 at 4096; 3136 values 12.0 / 6.9, 13.1 / 9.6, 18.2 / 12.4, 21.6 / 19.1, 27.5 / 36; 2048 values
-// 8.3 / 6.3 at 16, 11.6 / 9.3 at 1024, 14.4 / 14.4 at 2048; 1024 values 5.4 / 5.8 at 16; 8192 values 46 / 23 at 1024, 46 / 55
-// at 2048; 27648 values 33 / 14 at 16, 135 / 86 at 1024, 153 / 173 at 2048.  Two eights or four (5120 values): 8.1 / 9.3 at 16
-// rows, 10.0 / 10.3 at 300, 18 / 11 at 512.
-static uint32_t chain_eights(uint32_t tokens, uint32_t n_in) {
-    if (n_in < 1536 || n_in > 32 * kChainThreads || tokens > (n_in >= 3072 && n_in <= 6144 ? 2048u : 1024u)) return 0;
-    return tokens <= 448 && n_in <= 16 * kChainThreads ? 2 : 4;
+// Eights a thread holds in the kernel above, 0: a kernel of its own leaves the rows' factors and the quantizer reads the rows
+// again.  One block per row pays where one round of blocks takes all rows: a second round waits for the first one's chains.
+// us, factors on their own / two eights / four, bf16 rows of 5120 values: 7.8 / 7.4 / 9.3 at 1 row, 9.4 / 8.2 / 10 at 148,
+// 17.5 / 18 / 13.7 at 1024, 18.3 / - / 21.1 at 1500 (a second round); 12288 values: 15.7 / 9.7 / - at 148, 17.5 / 26 / - at
+// 300 (two eights: the second round of three); 27648 values: 23.8 / - / 13.4 at 1 row, 28.1 / - / 13.3 at 148, 31.8 / - / 38
+// at 300.  Shorter rows are the warp's: 2048 values 4.7 / 6.0 / - at 1 row, 6.4 / 6.6 / - at 148.
+static uint32_t chain_eights(const Ctx *ctx, uint32_t tokens, uint32_t n_in) {
+    if (n_in < 2560) return 0;
+    for (uint32_t eights = 2; eights <= 4; eights *= 2) {
+        const uint32_t threads = chain_threads(n_in, eights);
+        if (threads <= kChainThreads && tokens <= (uint32_t)ctx->sm_count * (kChainResident / threads)) return eights;
+    }
+    return 0;
 }
 
 // Plain rows: out[t][k] = (x[t][k] * inv_rms_t) * w[k] in f32, for the kernels that read their activations as they go.
@@ -418,7 +502,7 @@ muser_cuda_status launch_rmsnorm_rows(Ctx *ctx, const void *x, uint32_t x_dtype,
     // the factors sit behind the rows in the same scratch (the caller sized it for tokens x n_in floats and more)
     float *inv = ctx->inv_rms;
     if (tokens > ctx->inv_rms_rows) return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: more rows than the context's per-row scratch holds");
-    MUSER_CUDA_TRY(ctx, launch_rms_rows_sequential(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
+    MUSER_CUDA_TRY(ctx, launch_rms_rows(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
     if (x_dtype == MUSER_DTYPE_F32)
         rmsnorm_rows_kernel<true><<<tokens, 256, 0, stream>>>(x, (uint32_t)n_in, norm_weight, inv, out);
     else
@@ -435,10 +519,10 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
     if (norm_weight) {
         float *inv = ctx->inv_rms;
         if (!inv || tokens > ctx->inv_rms_rows) return fail(ctx, MUSER_CUDA_WORKSPACE_TOO_SMALL, "fused input norm: more rows than the context's per-row scratch holds");
-        const uint32_t eights = chain_eights(tokens, (uint32_t)n_in);
+        const uint32_t eights = chain_eights(ctx, tokens, (uint32_t)n_in);
         const bool f32 = x_dtype == MUSER_DTYPE_F32;
         if (!eights) {
-            MUSER_CUDA_TRY(ctx, launch_rms_rows_sequential(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
+            MUSER_CUDA_TRY(ctx, launch_rms_rows(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
             const auto kernel = f32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
             MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(256), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, (const float *)inv,
                                            packed, scales));
@@ -446,7 +530,7 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
         }
         const auto kernel = eights == 2 ? (f32 ? nvfp4_norm_quantize_kernel<true, 2> : nvfp4_norm_quantize_kernel<false, 2>)
                                         : (f32 ? nvfp4_norm_quantize_kernel<true, 4> : nvfp4_norm_quantize_kernel<false, 4>);
-        const uint32_t threads = ((uint32_t)((n_in / 8 + eights - 1) / eights) + 31) / 32 * 32;
+        const uint32_t threads = chain_threads((uint32_t)n_in, eights);
         MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(threads), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps, packed, scales));
         return MUSER_CUDA_OK;
     }

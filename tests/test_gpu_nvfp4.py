@@ -424,6 +424,30 @@ def test_fused_norm_adds_the_squares_front_to_back(gpu, n_in, x_dtype):
         assert np.array_equal(got_s[0].cpu().numpy(), want_s)
 
 
+@pytest.mark.parametrize("n_in,tokens", [(1024, 1), (1024, 2047), (1024, 2049), (2496, 45), (2560, 45), (12288, 148), (12288, 149), (12288, 450),
+                                         (16448, 5), (32768, 3), (32832, 6)])
+def test_norm_kernels_agree_on_either_side_of_their_lines(gpu, n_in, tokens):
+    """The block per row (eights by two and by four, to its longest row), the warp per row (ragged last step and block) and
+    the plain chains give the CPU lane's bytes where one takes over from the other."""
+    op, ctx, k = gpu
+    g = torch.Generator().manual_seed(n_in + tokens)
+    x = torch.randn((4, n_in), generator=g)
+    x[1] = torch.exp2(torch.linspace(-30, 15, n_in))       # a binade every few values
+    x[2, :-3] = 0.0                                        # all of the sum in the last segment
+    x[3] = 1.0 + torch.arange(n_in).remainder(3) * 0.0078125  # ties
+    nw = 1.0 + 0.1 * torch.randn(n_in, generator=g)
+    isi, eps = 41.5, 1e-6
+    for dt in (torch.float32, torch.bfloat16):
+        rows = x.to(dt)
+        want_p, want_s = O.quantize_nvfp4_activation(O.rms_norm_mul(rows.float().numpy(), eps, nw.numpy()), isi)
+        at = torch.arange(tokens) % 4
+        got_p, got_s = k.quantize_nvfp4_activation(rows[at].cuda(), isi, norm_weight=nw.cuda(), norm_eps=eps)
+        ctx.sync_status()
+        assert torch.equal(got_p.cpu().reshape(tokens, -1), torch.from_numpy(want_p).reshape(4, -1)[at])
+        got_s = op.unswizzle_scales(got_s, tokens, n_in)
+        assert torch.equal(torch.as_tensor(got_s).cpu().reshape(tokens, -1), torch.as_tensor(want_s).reshape(4, -1)[at])
+
+
 def test_nvfp4_tensor_parallel_shards(gpu):
     op, ctx, k = gpu
     from muser_b200 import synth
