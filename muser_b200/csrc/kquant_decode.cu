@@ -1258,8 +1258,9 @@ static bool takes_mma(const Ctx *ctx, const Weight *w, uint32_t tokens) {
 // The tcgen05 kernel for large Q4_K weights at token counts that fill its columns (us, tcgen05 / warp-level, 27648 x 5120:
 // 35 / 32 at 17 to 24 tokens, 35 / 38 at 32, 54 / 48 at 48, 55 / 61 at 64; f32 activations, two columns a token, 47 / 44 at
 // 17 to 24 and 48 / 56 at 32.  Smaller weights, before both kernels' present forms: 13824 x 5120 37 / 40 at 64, 8192 x 5120
-// 22 / 22 at 32 and 33 / 31, 5120 x 5120 19 / 17 and 29 / 23).  Q6_K: 63 / 52 at 32 and 78 / 76 at 64 for 5120 x 27648.  A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves, which is
-// what its Q6_K form is kept for: the caller's choice of range and rounding against another kernel's.
+// 22 / 22 at 32 and 33 / 31, 5120 x 5120 19 / 17 and 29 / 23).  Q6_K: 63 / 52 at 32 and 78 / 76 at 64 for 5120 x 27648.
+// A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves, which is what its Q6_K form
+// is kept for: the caller's choice of range and rounding against another kernel's.
 static bool takes_tcgen05(const Weight *w, uint32_t tokens, bool two_columns, uint32_t tc_from) {
     if (tc_from < 17) return true;
     const uint32_t cols = two_columns ? 2 * tokens : tokens;

@@ -23,10 +23,8 @@
 // (a full and an empty barrier each).  K is cut between the CTAs of a cluster; the slices meet through distributed shared
 // memory and are added in slice order, every CTA finishing its share of the outputs.
 //
-// What bounds it: no one unit.  A tile costs a warp about 450 instructions besides its products; at 16 tokens of
-// 27648 x 5120 the issue slots are 44 % used, the byte-and-logic pipe 37 %, the tensor pipe 23 %, with three warps a
-// scheduler in chains of unpack, product and scale.  m16n8k16 takes the tensor pipe 8.3 cycles: from 48 tokens the
-// products are the largest part.  Figures beside takes_mma() in kquant_decode.cu.
+// What bounds it: no one unit.  Three or four warps a scheduler run chains of unpack, product and scale whose latencies are only
+// partly covered.  m16n8k16 takes the tensor pipe 8.3 cycles: from 48 tokens the products are the largest part.  Figures beside takes_mma() in kquant_decode.cu.
 #include <algorithm>
 #include <cmath>
 

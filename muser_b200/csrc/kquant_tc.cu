@@ -1,5 +1,6 @@
 // Skinny GEMM for Q4_K / Q6_K weights on the 5th-generation tensor cores: y[t][r] = dot(W_r, x_t), 3..64 tokens (by default
-// 17..64 tokens of large Q4_K weights; kquant_mma.cu serves the other batches, see the dispatch in kquant_decode.cu).
+// large Q4_K weights with 25 to 32 or 49 to 64 token columns; kquant_mma.cu serves the other batches, see the dispatch in
+// kquant_decode.cu).
 //
 // Stands in for the batched routes of MetalKernels::encode_quantized_matmul and the speculative-verify batches of
 // encode_quantized_decode_group (crates/muser-engine/src/metal/encode/qkv.rs:234-281,414-449); on the CPU lane,

@@ -31,7 +31,7 @@ __device__ __forceinline__ uint32_t e2m1_word(const float (&q)[8]) {
 // midpoint only where m met it.  It is made without a divide, by the residual of a product with the rounded
 // reciprocal (tests/test_nvfp4_codec_cpu.py runs every scale against the floats around every bound).  The chain (seven
 // multiplies, compares and adds a value) bounded both quantizer kernels and the GEMM epilogue that quantizes: quantize
-// of 32768 x 5120 237 -> 117 us (the memory alone: 66), behind the norm 334 -> 227, gate/up + quantize 6.14 -> 4.82 ms.
+// of 32768 x 5120 237 -> 117 us (the memory alone: 66; 79 with four rows a thread), behind the norm 334 -> 227, gate/up + quantize 6.14 -> 4.82 ms.
 __device__ __forceinline__ uint32_t quantize_group(const float (&r)[16], float isi, uint32_t &codes_lo, uint32_t &codes_hi) {
     __half2 h[8], top = __floats2half2_rn(0.0f, 0.0f);
 #pragma unroll

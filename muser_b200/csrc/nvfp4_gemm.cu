@@ -5,10 +5,11 @@
 // (src/weights.rs:111-121, quant/nvfp4.rs:304-338): E2M1 codes of activations and weights, one E4M3 scale per
 // 16 values on each side, then (acc * weight_scale2) * (1 / input_scale_inv) in that order.
 //
-// Shape of the kernel: persistent CTAs, one per SM, each walking 128-token x 256-row output tiles.  Warp 0 streams 128-byte-swizzled
+// Shape of the kernel: persistent CTAs, one per SM, each walking 128-token x 256-row output tiles, or pairs of CTAs on
+// 256 tokens x 256 rows where that is faster (takes_pairs; the PAIR form below).  Warp 0 streams 128-byte-swizzled
 // K slabs (256 values) of both operands with TMA plus their scale factors with bulk copies through a
 // 4-stage shared-memory ring; warp 1 copies each K = 64 block's scale factors into tensor memory (tcgen05.cp) and
-// issues its tcgen05.mma kind::mxf4nvf4 right behind them into a 128 x 256 f32 accumulator in tensor memory (both
+// issues its tcgen05.mma kind::mxf4nvf4 right behind them (for pairs: a slab's copies, then its products) into a 128 x 256 f32 accumulator in tensor memory (both
 // warps run their loops converged and issue through an elected lane: tcgen05.cuh);
 // warps 2-17 read the accumulator back (tcgen05.ld), apply the two tensor scales and the fused epilogue, and
 // store.  Every mbarrier wait is bounded: on expiry the CTA records a code in the context's status word,
@@ -1327,7 +1328,7 @@ static uint32_t box_tokens(uint32_t tokens) { return std::min<uint32_t>(BM, (tok
 // to 22 (3072 x 3072 7.4 -> 5.2 at one, 6.8 at 16).
 // What the bits of a result depend on: the number of slices, i.e. the weight's rows and row length, the token count and the
 // device (its SMs, and how many clusters of a size it holds).  Calls with a logit scale or soft cap, the fused gate/up form
-// and contexts that use the paired kernel never split; a group gives the bits of the single calls.
+// and contexts told to use pairs never split; a group gives the bits of the single calls.
 constexpr uint32_t kSplitMin = 12;
 struct SplitRoom {
     bool asked = false;

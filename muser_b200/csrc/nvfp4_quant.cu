@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(32 * kChainRowWarps) rms_rows_chain_kernel(con
 }
 
 // Which of the three leaves the factors.  The plain chains (few values per row, or enough rows that a lane each fills the chip)
-// do half the additions.  us with the quantizer, plain / warp per row, bf16: 512 values 4.5 / 4.8 at 148 rows, 6.4 / 7.4 at
+// do half the additions.  us with the quantizer of a row a block, plain / warp per row, bf16: 512 values 4.5 / 4.8 at 148 rows, 6.4 / 7.4 at
 // 2048; 1024 values 6.6 / 5.4 at 449, 9.0 / 8.7 at 2048, 11.8 / 12.5 at 4096; 2048 values 14.3 / 11.5 at 2048, 18.3 / 16.9 at
 // 4096, 28.4 / 29 at 8192; 3136 values 27.5 / 23.6 at 4096, 42.6 / 40.2 at 8192, 139 / 153 at 32768; 5120 values 45 / 32 at
 // 4096, 66 / 57 at 8192, 224 / 212 at 32768; 12288 values 77 / 46 at 2048.  f32: 5120 values 72 / 52 at 4096, 352 / 353 at
@@ -449,7 +449,8 @@ __global__ void __launch_bounds__(kChainThreads) nvfp4_norm_quantize_kernel(cons
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, inv, packed, scales);
 }
 
-// The quantizer behind a kernel that leaves the rows' factors in memory (chain_eights).
+// The quantizer behind a kernel that leaves the rows' factors in memory (chain_eights).  Blocks of a row's own size (64 threads
+// for 1024 values) were slower from 700 rows on: 9.9 against 8.7 us at 2048 rows.
 template <bool XF32>
 __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
                                                                     const float *norm_w, const float *inv_rms, uint8_t *packed,
@@ -460,6 +461,69 @@ __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
+}
+
+// Both quantizers for many rows: a thread takes one group of the four rows whose scales are neighbours in the swizzled plane
+// (r, r + 32, r + 64, r + 96 of a 128-row block), all of them on their way before the first is used, and four lanes' scale bytes
+// leave as 16 bytes instead of four times 4 (a sector each); the norm's weights are read once for four rows.  32768 rows of
+// 5120 values: 117 -> 79 us from bf16 (5.5 TB/s), 135 -> 109 from f32 (7 TB/s); behind the norm 212 -> 180 and 353 -> 297 with
+// the norm's own kernel.  (Blocks of 256 threads 85 and 127; two of the four rows ahead 87 and 120.)
+template <bool XF32, bool NORM>
+__global__ void __launch_bounds__(128) nvfp4_quantize_quads_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
+                                                                   const float *norm_w, const float *inv_rms, uint8_t *packed, uint8_t *scales) {
+    pdl_wait();
+    pdl_release();
+    const uint32_t groups_pad = kt * 4;
+    const uint64_t idx = blockIdx.x * (uint64_t)128 + threadIdx.x; // (128 x kt of them per 128 rows: whole blocks)
+    const uint32_t quad = (uint32_t)(idx / groups_pad), grp = (uint32_t)(idx % groups_pad);
+    const uint32_t row0 = quad / 32 * 128 + quad % 32;
+    constexpr int kWords = XF32 ? 4 : 2; // 16-byte pieces of a group
+    const bool live = grp * 16 < n_in;
+    uint4 raw[4][kWords];
+    float inv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t row = row0 + 32 * i;
+        const bool there = live && row < tokens;
+        const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(x) + ((size_t)row * n_in + grp * 16) * (XF32 ? 4 : 2));
+#pragma unroll
+        for (int k = 0; k < kWords; ++k) raw[i][k] = there ? ld_after_wait(p + k) : make_uint4(0, 0, 0, 0);
+        if (NORM) inv[i] = there ? ld_after_wait(inv_rms + row) : 0.0f;
+    }
+    float4 w[4];
+    if (NORM && live) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[k] = ld_after_wait(reinterpret_cast<const float4 *>(norm_w + grp * 16) + k);
+    }
+    uint32_t word[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t row = row0 + 32 * i;
+        word[i] = 0;
+        if (live && row < tokens) {
+            float r[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const uint32_t bits = XF32 ? (&raw[i][(k / 4) % kWords].x)[k % 4] : (&raw[i][(k / 8) % kWords].x)[(k % 8) / 2];
+                const float f = __uint_as_float(XF32 ? bits : (k & 1) ? bits & 0xFFFF0000u : bits << 16);
+                r[k] = NORM ? __fmul_rn(__fmul_rn(f, inv[i]), (&w[k / 4].x)[k % 4]) : f;
+            }
+            word[i] = quantize_group(r, isi, packed + (size_t)row * (n_in / 2) + grp * 8);
+        }
+        word[i] |= __shfl_down_sync(0xffffffffu, word[i], 1) << 8;
+        word[i] |= __shfl_down_sync(0xffffffffu, word[i], 2) << 16;
+    }
+    if ((grp & 3) == 0) // (the four rows' words are neighbours)
+        *reinterpret_cast<uint4 *>(scales + (size_t)(row0 / 128) * ((size_t)kt * 512) + (size_t)(grp / 4) * 512 + (row0 % 32) * 16) =
+            make_uint4(word[0], word[1], word[2], word[3]);
+}
+// Where a quarter of the threads still fills the chip: us, a row / four rows a thread, bf16 rows of 2048 values 3.9 / 3.9 at 2048
+// rows, 6.4 / 5.4 at 4096; 5120 values 4.5 / 5.2 at 1024, 7.7 / 6.6 at 2048; f32 rows, whose loads are twice as many, 2048 values
+// 7.0 / 7.3 at 4096, 12.6 / 11.8 at 8192; 5120 values 8.3 / 8.6 at 2048, 17.0 / 15.0 at 4096.  Behind a norm, which leaves the
+// SMs unevenly free for a grid of one round: bf16 2048 values 11.6 / 13.6 at 2048 rows, 17.1 / 15.7 at 4096; f32 1024 values
+// 14.1 / 16.9 at 4096, 23.0 / 20.1 at 8192; 5120 values 30.6 / 22.4 at 1500.
+static bool takes_quads(uint32_t tokens_pad, uint32_t kt, bool f32, bool norm) {
+    return (uint64_t)tokens_pad * kt >= (f32 && !norm ? 16u << 14 : 8u << 14); // (in 64 values)
 }
 
 // Eights a thread holds in the kernel above, 0: a kernel of its own leaves the rows' factors and the quantizer reads the rows
@@ -523,6 +587,12 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
         const bool f32 = x_dtype == MUSER_DTYPE_F32;
         if (!eights) {
             MUSER_CUDA_TRY(ctx, launch_rms_rows(ctx, x, x_dtype, tokens, (uint32_t)n_in, norm_eps, inv, stream));
+            if (takes_quads(tokens_pad, kt, f32, true)) {
+                const auto kernel = f32 ? nvfp4_quantize_quads_kernel<true, true> : nvfp4_quantize_quads_kernel<false, true>;
+                MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad / 128 * kt), dim3(128), 0, stream, x, tokens, (uint32_t)n_in, kt, isi,
+                                               norm_weight, (const float *)inv, packed, scales));
+                return MUSER_CUDA_OK;
+            }
             const auto kernel = f32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
             MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(256), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, (const float *)inv,
                                            packed, scales));
@@ -532,6 +602,12 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
                                         : (f32 ? nvfp4_norm_quantize_kernel<true, 4> : nvfp4_norm_quantize_kernel<false, 4>);
         const uint32_t threads = chain_threads((uint32_t)n_in, eights);
         MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(threads), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps, packed, scales));
+        return MUSER_CUDA_OK;
+    }
+    if (takes_quads(tokens_pad, kt, x_dtype == MUSER_DTYPE_F32, false)) {
+        const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_quantize_quads_kernel<true, false> : nvfp4_quantize_quads_kernel<false, false>;
+        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad / 128 * kt), dim3(128), 0, stream, x, tokens, (uint32_t)n_in, kt, isi,
+                                       (const float *)nullptr, (const float *)nullptr, packed, scales));
         return MUSER_CUDA_OK;
     }
     const uint64_t total = (uint64_t)tokens_pad * kt * 4;

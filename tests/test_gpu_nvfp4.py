@@ -448,6 +448,30 @@ def test_norm_kernels_agree_on_either_side_of_their_lines(gpu, n_in, tokens):
         assert torch.equal(torch.as_tensor(got_s).cpu().reshape(tokens, -1), torch.as_tensor(want_s).reshape(4, -1)[at])
 
 
+@pytest.mark.parametrize("n_in,tokens", [(2032, 4097), (2032, 8200), (272, 30850), (5200, 1600)])
+def test_quantizers_of_four_rows_a_thread(gpu, n_in, tokens):
+    """Many rows, plain and behind the norm, a ragged last block of rows and rows that end inside a 64-value chunk: the CPU
+    lane's bytes in every row, zeros in the scale slots of rows and groups that are not there."""
+    op, ctx, k = gpu
+    g = torch.Generator().manual_seed(tokens)
+    x = torch.randn((7, n_in), generator=g)
+    x[3] = 0.0
+    x[4, ::16] = 1e30
+    nw = 1.0 + 0.1 * torch.randn(n_in, generator=g)
+    isi, eps = 41.5, 1e-6
+    at = torch.arange(tokens) % 7
+    for dt in (torch.float32, torch.bfloat16):
+        rows = x.to(dt).float()
+        for norm in (False, True):
+            want_p, want_s = O.quantize_nvfp4_activation(O.rms_norm_mul(rows.numpy(), eps, nw.numpy()) if norm else rows.numpy(), isi)
+            got_p, got_s = k.quantize_nvfp4_activation(x.to(dt)[at].cuda(), isi, **({"norm_weight": nw.cuda(), "norm_eps": eps} if norm else {}))
+            ctx.sync_status()
+            assert torch.equal(got_p.cpu().reshape(tokens, -1), torch.from_numpy(want_p).reshape(7, -1)[at]), (dt, norm)
+            plain = torch.as_tensor(op.unswizzle_scales(got_s, tokens, n_in)).cpu().reshape(tokens, -1)
+            assert torch.equal(plain, torch.as_tensor(want_s).reshape(7, -1)[at]), (dt, norm)
+            assert int(got_s.cpu().long().sum()) == int(plain.long().sum()), (dt, norm)
+
+
 def test_nvfp4_tensor_parallel_shards(gpu):
     op, ctx, k = gpu
     from muser_b200 import synth
