@@ -113,6 +113,13 @@ extern thread_local std::string g_create_error;
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The two in the order that `early` asks for: released first, the kernel behind this one starts (and its successor, if it
+// does the same) while the kernel in FRONT of this one is still running.
+__device__ __forceinline__ void pdl_turn(bool early) {
+    if (early) pdl_release();
+    pdl_wait();
+    if (!early) pdl_release();
+}
 // Loads of what an earlier kernel may have written, kept behind pdl_wait(), which makes its writes visible to every load
 // that follows: __ldg and loads through const __restrict__ pointers count as reads of constant memory, which the compiler
 // may move across it and the hardware may serve from a line fetched before (none of 43 million lines read with ld.global by

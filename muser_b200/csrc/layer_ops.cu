@@ -13,10 +13,12 @@
 namespace muser {
 
 // These kernels are a few microseconds of latency between two projections.  Up to one block an SM (decode: a row per token)
-// each lets its successor launch as soon as it has its own inputs' go-ahead (`early`: pdl_release behind pdl_wait): the
-// projection that follows sets up and starts its weight copies under it.  Larger grids do not: the successor's blocks only
-// took the slots of their own later ones (head norm, gate and tail of 512 rows of 2048, us: 12.6 with the release, 10.6
-// without; of 16 rows of 5120: 6.0 and 6.9).  They work in place: rows are read behind the wait (ld_after_wait).
+// each lets its successor launch in front of its own wait (`early`): the launches of a chain of them, and the set-up and first
+// weight copies of the projection that follows, lie under the projection before (a layer at one token 88.1 -> 87.1 us, at eight
+// 126.2 -> 124.6, against a release behind the wait).  Larger grids do not: the successor's blocks only took the slots of
+// their own later ones (head norm, gate and tail of 512 rows of 2048, us: 12.6 with the release, 10.6 without; of 16 rows of
+// 5120: 6.0 and 6.9).  They work in place, and a caller may make the norm weights on the stream: both are read behind the wait
+// (ld_after_wait).
 
 // Sum over the block of one value per thread; `red` holds 33 floats; every thread gets the total.
 __device__ __forceinline__ float block_sum(float v, float *red) {
@@ -43,23 +45,29 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
 // and have their trips covered by other blocks (512 rows of 2048: 7.2 us held, 5.7 read again).
 template <bool HELD>
 __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, const float *src, float *output,
-                                                                 const float *__restrict__ w1, const float *__restrict__ w2, uint32_t n, float eps1,
+                                                                 const float *w1, const float *w2, uint32_t n, float eps1,
                                                                  float eps2) {
     __shared__ float red[33];
-    pdl_wait();
     if constexpr (HELD) pdl_release();
+    pdl_wait();
     const uint32_t n4 = n / 4;
     float4 *h4 = reinterpret_cast<float4 *>(hidden + (size_t)blockIdx.x * n);
     const float4 *s4 = reinterpret_cast<const float4 *>(src + (size_t)blockIdx.x * n);
     const float4 *w14 = reinterpret_cast<const float4 *>(w1), *w24 = reinterpret_cast<const float4 *>(w2);
     constexpr uint32_t kHeld = HELD ? 4 : 0;
-    float4 s[kHeld + 1], h[kHeld + 1];
+    float4 s[kHeld + 1], h[kHeld + 1], u1[kHeld + 1], u2[kHeld + 1]; // (the weights' pieces with them)
     float ss = 0.0f;
 #pragma unroll
     for (uint32_t k = 0; k < kHeld; ++k) {
         const uint32_t i = threadIdx.x + k * blockDim.x;
         s[k] = h[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (i < n4) s[k] = ld_after_wait(s4 + i), h[k] = ld_after_wait(h4 + i);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kHeld; ++k) {
+        const uint32_t i = threadIdx.x + k * blockDim.x;
+        if (i < n4) u1[k] = ld_after_wait(w14 + i);
+        if (i < n4 && output) u2[k] = ld_after_wait(w24 + i);
     }
 #pragma unroll
     for (uint32_t k = 0; k < kHeld; ++k) ss += s[k].x * s[k].x + s[k].y * s[k].y + s[k].z * s[k].z + s[k].w * s[k].w;
@@ -69,8 +77,7 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, 
     }
     const float inv_src = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(ss, red), (float)n) + eps1));
     float sh = 0.0f;
-    auto tail = [&](uint32_t i, const float4 &sv, float4 &hv) {
-        const float4 w = w14[i];
+    auto tail = [&](uint32_t i, const float4 &sv, float4 &hv, const float4 &w) {
         hv.x += sv.x * inv_src * w.x, hv.y += sv.y * inv_src * w.y, hv.z += sv.z * inv_src * w.z, hv.w += sv.w * inv_src * w.w;
         h4[i] = hv;
         sh += hv.x * hv.x + hv.y * hv.y + hv.z * hv.z + hv.w * hv.w;
@@ -78,31 +85,30 @@ __global__ void __launch_bounds__(512) norm_residual_norm_kernel(float *hidden, 
 #pragma unroll
     for (uint32_t k = 0; k < kHeld; ++k) {
         const uint32_t i = threadIdx.x + k * blockDim.x;
-        if (i < n4) tail(i, s[k], h[k]);
+        if (i < n4) tail(i, s[k], h[k], u1[k]);
     }
     for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) {
         float4 hv = ld_after_wait(h4 + i);
-        tail(i, ld_after_wait(s4 + i), hv);
+        tail(i, ld_after_wait(s4 + i), hv, ld_after_wait(w14 + i));
     }
     if (!output) return;
     const float inv_h = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(block_sum(sh, red), (float)n) + eps2));
     float4 *o4 = reinterpret_cast<float4 *>(output + (size_t)blockIdx.x * n);
-    auto out = [&](uint32_t i, const float4 &hv) {
-        const float4 w = w24[i];
+    auto out = [&](uint32_t i, const float4 &hv, const float4 &w) {
         o4[i] = make_float4(hv.x * inv_h * w.x, hv.y * inv_h * w.y, hv.z * inv_h * w.z, hv.w * inv_h * w.w);
     };
 #pragma unroll
     for (uint32_t k = 0; k < kHeld; ++k) {
         const uint32_t i = threadIdx.x + k * blockDim.x;
-        if (i < n4) out(i, h[k]);
+        if (i < n4) out(i, h[k], u2[k]);
     }
-    for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) out(i, ld_after_wait(h4 + i)); // (this thread's own)
+    for (uint32_t i = threadIdx.x + kHeld * blockDim.x; i < n4; i += blockDim.x) out(i, ld_after_wait(h4 + i), ld_after_wait(w24 + i)); // (this thread's own)
 }
 
 // x[i] *= 1 / (1 + exp(-gate[i])), four at a time.
 __global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *x, const float *gate, size_t n4, bool early) {
-    pdl_wait();
     if (early) pdl_release();
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
         float4 v = ld_after_wait(reinterpret_cast<const float4 *>(x) + i);
         const float4 g = ld_after_wait(reinterpret_cast<const float4 *>(gate) + i);
@@ -113,15 +119,16 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(float *x, const float
 }
 
 // One warp per (token, head): x <- x * 1/sqrt(mean(x^2) + eps) * w, head_dim % 4 == 0, head_dim <= 1024.
-__global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const float *__restrict__ w, float eps, uint32_t heads_total,
+__global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const float *w, float eps, uint32_t heads_total,
                                                             uint32_t head_dim, bool early) {
-    pdl_wait();
     if (early) pdl_release();
+    pdl_wait();
     const uint32_t head = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (head >= heads_total) return;
     float4 *row = reinterpret_cast<float4 *>(x + (size_t)head * head_dim);
     const float4 *w4 = reinterpret_cast<const float4 *>(w);
     const uint32_t n4 = head_dim / 4;
+    const float4 w0 = lane < n4 ? ld_after_wait(w4 + lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); // (all of it up to heads of 128)
     float ss = 0.0f;
     for (uint32_t i = lane; i < n4; i += 32) {
         const float4 v = ld_after_wait(row + i);
@@ -131,7 +138,7 @@ __global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const floa
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(ss, (float)head_dim) + eps));
     for (uint32_t i = lane; i < n4; i += 32) {
-        const float4 v = ld_after_wait(row + i), ww = w4[i];
+        const float4 v = ld_after_wait(row + i), ww = i == lane ? w0 : ld_after_wait(w4 + i);
         row[i] = make_float4(v.x * inv * ww.x, v.y * inv * ww.y, v.z * inv * ww.z, v.w * inv * ww.w);
     }
 }

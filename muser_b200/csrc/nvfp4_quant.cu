@@ -12,6 +12,10 @@
 
 namespace muser {
 
+// Grids of up to two blocks an SM release their successor in front of their own wait (pdl_turn): norm, q | k | v, quantizer and o of
+// a 5120-wide layer 29.5 -> 26.8 us at 16 tokens, 34.1 -> 33.3 at 200; larger ones gain nothing (509 tokens 40.0 / 39.9) or, with
+// the whole layer, lose (168.5 -> 173).
+static bool few_blocks(const Ctx *ctx, uint32_t blocks) { return blocks <= 2 * (uint32_t)ctx->sm_count; }
 // Four neighbouring threads (groups 4q .. 4q+3 of one row) merge their scale bytes into one aligned 32-bit store.
 // Every lane of the warp calls this; lanes past the row's last group slot pass live = false.
 __device__ __forceinline__ void store_scale_quad(uint32_t scale_code, uint32_t row, uint32_t grp, uint32_t kt, uint8_t *scales,
@@ -30,9 +34,8 @@ __device__ __forceinline__ void store_scale_quad(uint32_t scale_code, uint32_t r
 // aligned 32-bit store.  Rows tokens..tokens_pad-1 only clear their scale slots.
 template <bool XF32>
 __global__ void nvfp4_quantize_kernel(const void *x, uint32_t tokens, uint32_t tokens_pad, uint32_t n_in, uint32_t kt, float isi, uint8_t *packed,
-                                      uint8_t *scales) {
-    pdl_wait();
-    pdl_release();
+                                      uint8_t *scales, bool early) {
+    pdl_turn(early);
     const uint32_t groups_pad = kt * 4; // group slots per row in the swizzled plane
     const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (idx >= (uint64_t)tokens_pad * groups_pad) return; // groups_pad % 4 == 0: quads never straddle the edge
@@ -59,9 +62,8 @@ __global__ void nvfp4_quantize_kernel(const void *x, uint32_t tokens, uint32_t t
 // rows at a time through shared memory (asynchronous copies, two buffers), so that global loads stay coalesced
 // (consecutive threads read consecutive 16 bytes of one row) while the sums stay sequential.
 template <bool XF32>
-__global__ void __launch_bounds__(32) rms_rows_sequential_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms) {
-    pdl_wait();
-    pdl_release();
+__global__ void __launch_bounds__(32) rms_rows_sequential_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms, bool early) {
+    pdl_turn(early);
     constexpr int kRows = 32, kChunk = 256;                       // rows per block (one warp), inputs per row and step
     constexpr int kParts = kChunk * (XF32 ? 4 : 2) / 16;          // 16-byte pieces per row and step
     constexpr int kStride = kParts + 1;                           // row stride in pieces: conflict-free 16-byte reads down a column
@@ -129,10 +131,9 @@ constexpr int kRmsPitch = kRmsRows + 1;                                     // f
 constexpr int kRmsBuffer = kRmsChunk / 4 * kRmsPitch;                       // float4 of one buffer
 constexpr size_t kRmsSmem = 2 * kRmsBuffer * sizeof(float4);
 template <bool XF32>
-__global__ void __launch_bounds__(kRmsThreads) rms_rows_staged_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms) {
+__global__ void __launch_bounds__(kRmsThreads) rms_rows_staged_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms, bool early) {
     extern __shared__ float4 rms_squares[]; // two buffers
-    pdl_wait();
-    pdl_release();
+    pdl_turn(early);
     const uint32_t row0 = blockIdx.x * kRmsRows, steps = (n_in + kRmsChunk - 1) / kRmsChunk;
     // warps 1 .. 7: pieces of eight inputs, neighbouring lanes along a row; all of a thread's loads before the first is used
     constexpr uint32_t kPieces = kRmsRows * (kRmsChunk / 8), kLoaders = kRmsThreads - 32, kPer = (kPieces + kLoaders - 1) / kLoaders;
@@ -313,10 +314,9 @@ __device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, fl
 // 15.5 and 12.2 us against 11.5) and gain nothing on short rows (512 values: 7.8, 7.2, 7.4).
 constexpr int kChainRowWarps = 4;
 template <bool XF32>
-__global__ void __launch_bounds__(32 * kChainRowWarps) rms_rows_chain_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms) {
+__global__ void __launch_bounds__(32 * kChainRowWarps) rms_rows_chain_kernel(const void *x, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms, bool early) {
     constexpr int K = 4; // eights per lane and step
-    pdl_wait();
-    pdl_release();
+    pdl_turn(early);
     const uint32_t lane = threadIdx.x & 31, row = blockIdx.x * kChainRowWarps + (threadIdx.x >> 5), n8 = n_in / 8;
     if (row >= tokens) return; // (whole warps)
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
@@ -388,19 +388,22 @@ static cudaError_t launch_rms_rows(Ctx *ctx, const void *x, uint32_t x_dtype, ui
     const bool f32 = x_dtype == MUSER_DTYPE_F32;
     if (n_in >= 5120 || (n_in >= 1024 && tokens <= 2 * n_in))
         return launch_pdl(f32 ? rms_rows_chain_kernel<true> : rms_rows_chain_kernel<false>, dim3((tokens + kChainRowWarps - 1) / kChainRowWarps),
-                          dim3(32 * kChainRowWarps), 0, stream, x, tokens, n_in, eps, inv_rms);
+                          dim3(32 * kChainRowWarps), 0, stream, x, tokens, n_in, eps, inv_rms,
+                          few_blocks(ctx, (tokens + kChainRowWarps - 1) / kChainRowWarps));
     if (tokens <= kRmsStagedRows) {
         const auto kernel = f32 ? rms_rows_staged_kernel<true> : rms_rows_staged_kernel<false>;
         const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), ctx->device, kRmsSmem);
         if (e != cudaSuccess) return e;
-        return launch_pdl(kernel, dim3((tokens + kRmsRows - 1) / kRmsRows), dim3(kRmsThreads), kRmsSmem, stream, x, tokens, n_in, eps, inv_rms);
+        return launch_pdl(kernel, dim3((tokens + kRmsRows - 1) / kRmsRows), dim3(kRmsThreads), kRmsSmem, stream, x, tokens, n_in, eps, inv_rms,
+                          few_blocks(ctx, (tokens + kRmsRows - 1) / kRmsRows));
     }
     const unsigned blocks = (tokens + 31) / 32;
     const size_t smem = (size_t)2 * 32 * ((f32 ? 64 : 32) + 1) * sizeof(uint4);
     const void *fn = f32 ? reinterpret_cast<const void *>(rms_rows_sequential_kernel<true>) : reinterpret_cast<const void *>(rms_rows_sequential_kernel<false>);
     const cudaError_t e = ensure_dynamic_smem(fn, ctx->device, smem);
     if (e != cudaSuccess) return e;
-    return launch_pdl(f32 ? rms_rows_sequential_kernel<true> : rms_rows_sequential_kernel<false>, dim3(blocks), dim3(32), smem, stream, x, tokens, n_in, eps, inv_rms);
+    return launch_pdl(f32 ? rms_rows_sequential_kernel<true> : rms_rows_sequential_kernel<false>, dim3(blocks), dim3(32), smem, stream, x, tokens, n_in, eps, inv_rms,
+                      few_blocks(ctx, blocks));
 }
 
 // (x * inv_rms) * w of one row, quantized group by group by the whole block; rows past `tokens` only clear their scales.
@@ -435,14 +438,13 @@ __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, 
 // (chain_inv_rms) and quantizes (x * inv_rms) * w group by group.
 template <bool XF32, int K>
 __global__ void __launch_bounds__(kChainThreads) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
-                                                                            const float *norm_w, float eps, uint8_t *packed, uint8_t *scales) {
+                                                                            const float *norm_w, float eps, uint8_t *packed, uint8_t *scales, bool early) {
     __shared__ ChainShared sh;
     const uint32_t row = blockIdx.x;
     // the norm weights are read last, from L2 if they are asked for now (between two layers' weights they go to memory)
     if (row < min(tokens, 16u))
         for (uint32_t i = 32 * threadIdx.x; i < n_in; i += 32 * blockDim.x) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + i));
-    pdl_wait();
-    pdl_release();
+    pdl_turn(early);
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     const float inv = row < tokens ? chain_inv_rms<XF32, K>(xr, n_in, eps, sh) : 0.0f; // (uniform over the block)
@@ -454,10 +456,9 @@ __global__ void __launch_bounds__(kChainThreads) nvfp4_norm_quantize_kernel(cons
 template <bool XF32>
 __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
                                                                     const float *norm_w, const float *inv_rms, uint8_t *packed,
-                                                                    uint8_t *scales) {
+                                                                    uint8_t *scales, bool early) {
     const uint32_t row = blockIdx.x;
-    pdl_wait();
-    pdl_release();
+    pdl_turn(early);
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, row < tokens ? ld_after_wait(inv_rms + row) : 0.0f, packed, scales);
@@ -470,9 +471,8 @@ __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *
 // the norm's own kernel.  (Blocks of 256 threads 85 and 127; two of the four rows ahead 87 and 120.)
 template <bool XF32, bool NORM>
 __global__ void __launch_bounds__(128) nvfp4_quantize_quads_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
-                                                                   const float *norm_w, const float *inv_rms, uint8_t *packed, uint8_t *scales) {
-    pdl_wait();
-    pdl_release();
+                                                                   const float *norm_w, const float *inv_rms, uint8_t *packed, uint8_t *scales, bool early) {
+    pdl_turn(early);
     const uint32_t groups_pad = kt * 4;
     const uint64_t idx = blockIdx.x * (uint64_t)128 + threadIdx.x; // (128 x kt of them per 128 rows: whole blocks)
     const uint32_t quad = (uint32_t)(idx / groups_pad), grp = (uint32_t)(idx % groups_pad);
@@ -590,30 +590,32 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
             if (takes_quads(tokens_pad, kt, f32, true)) {
                 const auto kernel = f32 ? nvfp4_quantize_quads_kernel<true, true> : nvfp4_quantize_quads_kernel<false, true>;
                 MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad / 128 * kt), dim3(128), 0, stream, x, tokens, (uint32_t)n_in, kt, isi,
-                                               norm_weight, (const float *)inv, packed, scales));
+                                               norm_weight, (const float *)inv, packed, scales, false));
                 return MUSER_CUDA_OK;
             }
             const auto kernel = f32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
             MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(256), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, (const float *)inv,
-                                           packed, scales));
+                                           packed, scales, few_blocks(ctx, tokens_pad)));
             return MUSER_CUDA_OK;
         }
         const auto kernel = eights == 2 ? (f32 ? nvfp4_norm_quantize_kernel<true, 2> : nvfp4_norm_quantize_kernel<false, 2>)
                                         : (f32 ? nvfp4_norm_quantize_kernel<true, 4> : nvfp4_norm_quantize_kernel<false, 4>);
         const uint32_t threads = chain_threads((uint32_t)n_in, eights);
-        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(threads), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps, packed, scales));
+        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(threads), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps, packed,
+                                       scales, few_blocks(ctx, tokens_pad)));
         return MUSER_CUDA_OK;
     }
     if (takes_quads(tokens_pad, kt, x_dtype == MUSER_DTYPE_F32, false)) {
         const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_quantize_quads_kernel<true, false> : nvfp4_quantize_quads_kernel<false, false>;
         MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad / 128 * kt), dim3(128), 0, stream, x, tokens, (uint32_t)n_in, kt, isi,
-                                       (const float *)nullptr, (const float *)nullptr, packed, scales));
+                                       (const float *)nullptr, (const float *)nullptr, packed, scales, false));
         return MUSER_CUDA_OK;
     }
     const uint64_t total = (uint64_t)tokens_pad * kt * 4;
     const unsigned blocks = (unsigned)((total + 255) / 256);
     const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_quantize_kernel<true> : nvfp4_quantize_kernel<false>;
-    MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(blocks), dim3(256), 0, stream, x, tokens, tokens_pad, (uint32_t)n_in, kt, isi, packed, scales));
+    MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(blocks), dim3(256), 0, stream, x, tokens, tokens_pad, (uint32_t)n_in, kt, isi, packed, scales,
+                                   few_blocks(ctx, blocks)));
     return MUSER_CUDA_OK;
 }
 
