@@ -126,3 +126,31 @@ def test_a_decoder_layers_non_attention_work_stays_on_the_device(gpu):
     assert H.rel_l2(hd_.cpu().numpy(), h2) <= 1e-3, H.rel_l2(hd_.cpu().numpy(), h2)
     for ww in w.values():
         ww.free()
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 200])
+def test_chained_launches_see_what_their_predecessors_wrote(gpu, tokens):
+    """Launches that start under the two before them (rows in place, norm weights made two launches back) leave the bits of
+    the same calls with a synchronization between each two."""
+    op, ctx, k = gpu
+    n = 1024
+    x0, g0, w0 = _rand((tokens, n), 11).cuda(), _rand((tokens, n), 12).cuda(), (1.0 + 0.1 * _rand((n,), 13)).cuda()
+    gw = _rand((n,), 14).cuda()
+
+    def chain(sync):
+        x, w, hidden, out = x0.clone(), w0.clone(), g0.clone(), torch.empty_like(x0)
+        for _ in range(6):
+            for call in (lambda: k.encode_sigmoid_gate(w, gw), lambda: k.encode_sigmoid_gate(x, g0),
+                         lambda: k.encode_head_rms_norm(x.view(tokens, n), w[:128], 1e-6, n // 128),
+                         lambda: k.encode_fused_norm_residual_rms_norm(hidden, x, w, 1e-8, out, w, 1e-5),
+                         lambda: k.encode_sigmoid_gate(w, out[0])):
+                call()
+                if sync:
+                    torch.cuda.synchronize()
+        ctx.sync_status()
+        return x, w, hidden, out
+
+    want = chain(True)
+    assert all(torch.isfinite(t).all() for t in want)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(chain(False), want))

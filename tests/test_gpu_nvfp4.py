@@ -554,6 +554,31 @@ def test_weight_only_lane_is_bit_identical(gpu, golden):
         w.free()
 
 
+@pytest.mark.parametrize("n_in", [256, 1280])
+def test_weight_only_lane_of_many_rows(gpu, n_in):
+    """Weights with more row tiles than two CTAs an SM take the form that keeps positive and negative codes apart: the CPU
+    lane's f16 bits, signs, largest magnitudes and a ragged last row tile included."""
+    op, ctx, k = gpu
+    from muser_b200 import synth
+    n_out = 40001
+    g = torch.Generator().manual_seed(n_in)
+    packed = torch.randint(0, 256, (n_out, n_in // 2), dtype=torch.uint8, generator=g)  # every code, -0 among them
+    packed[:16] = 0x77                                                                  # +6 throughout
+    packed[16:32] = 0xFF                                                                # -6
+    scales = torch.randint(0, 0x7F, (n_out, n_in // 16), dtype=torch.uint8, generator=g)
+    scales[:32] = 0x7E                                                                  # 448
+    packed, scales = packed.numpy(), scales.numpy()
+    w = op.Weight(ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, 0.001, None))
+    for tokens in (1, 2):
+        x = synth.normal_activations(tokens, n_in, seed=15)
+        want = O.matmul(O.TensorView(packed, O.NVFP4, n_in, n_out, scales, 0.001, None), x.float().numpy(), threads=O.host_threads())
+        y = torch.empty((tokens, n_out), dtype=torch.float32, device="cuda")
+        k.encode_nvfp4_matmul(w, x.cuda(), y, tokens)
+        ctx.sync_status()
+        assert np.array_equal(y.cpu().numpy(), want), tokens
+    w.free()
+
+
 def test_workspace_and_dtype_misuse(gpu):
     op, ctx, k = gpu
     packed, scales, scale2 = make_weight(op, ctx, 64, 256, seed=1)
