@@ -285,7 +285,9 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t cta_addr, uint32_t rank
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+// "Accumulator read", the one arrival of a thread on the other CTA's barrier: relaxed, because all that it orders is tensor-memory
+// reads, which tcgen05.wait::ld has completed and the tcgen05 fences in front of it and behind the wait order.
+__device__ __forceinline__ void mbar_arrive_accumulator_read(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Staging buffer (64-byte rows, 64-byte swizzle) -> a box of the output; columns and rows past its end are not written.
@@ -307,23 +309,31 @@ __device__ __forceinline__ uint4 lds_16(uint32_t at) {
 __device__ __forceinline__ void sts_16(uint32_t at, const uint32_t (&v)[4]) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster_elect(uint32_t cluster_addr) {
-    asm volatile("{\n\t" MUSER_ELECT_PRED "@e mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n\t}" ::"r"(cluster_addr) : "memory");
-}
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// mbar_wait_warp for barriers that the other CTA of the pair arrives on.
+// mbar_wait_relaxed and mbar_wait_warp for barriers that the other CTA of the pair arrives on (by its loads, its products' commits or its warps).
+__device__ __forceinline__ bool mbar_try_pair(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done;
+}
+__device__ __forceinline__ bool mbar_wait_pair_relaxed(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t ns) {
+    for (uint32_t i = 0; i < kSpinLimit; ++i) {
+        if (mbar_try_pair(bar, parity)) return true;
+        if ((i & 255u) == 255u && *abort_flag) return false;
+        __nanosleep(ns);
+    }
+    return false;
+}
 __device__ __forceinline__ bool mbar_wait_pair_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
     bool ok = false;
     for (uint32_t i = 0; i < kSpinLimit && !ok; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}"
-            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        ok = done;
+        ok = mbar_try_pair(bar, parity);
         if ((i & 1023u) == 1023u && *abort_flag) break;
     }
     return __all_sync(0xffffffffu, ok);
@@ -350,12 +360,12 @@ __device__ __forceinline__ void pair_mma_nvf4_elect(uint32_t tmem_d, uint64_t de
         : "memory");
 }
 
-// A whole slab's twelve scale copies, four products and the commit behind ONE election: with an elect.sync each and a loop
-// around them the issuing warp took 1080 cycles a slab, unrolled 740, so about 400, and the products take 512.  Chunks of
-// 512 bytes follow one another in shared memory: four of the activations, then four of either half of the weight rows.  The
-// role is entered by a branch that does not tell the compiler that its warp runs converged: told so, as the other roles are
-// (they issue their loads in 128 cycles instead of 304, and the single CTAs' slabs are 10 % shorter), it takes 923 cycles to
-// issue these seventeen instructions.
+// A whole slab's twelve scale copies, four products and two commits ("stage consumed", to both CTAs) behind ONE election.  With
+// one commit an elect.sync each and a loop around them took the issuing warp 1080 cycles a slab, unrolled 740, one election
+// about 400, and the products take 512.  Chunks of 512 bytes follow one another in shared memory: four of the activations, then
+// four of either half of the weight rows.  The role is entered by a branch that does not tell the compiler that its warp runs
+// converged: told so, as the other roles are (they issue their loads in 128 cycles instead of 304, and the single CTAs' slabs
+// are 10 % shorter), it takes 923 cycles to issue them.
 #define PAIR_CP(COL, CHUNK)                                                                                                  \
     "add.u32 t, %4, " #COL ";\n\tadd.u32 v, %5, " #CHUNK " * 32;\n\tmov.b64 d, {v, %7};\n\t"                                     \
     "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [t], d;\n\t"
@@ -369,20 +379,21 @@ __device__ __forceinline__ void pair_mma_nvf4_elect(uint32_t tmem_d, uint64_t de
     PAIR_CP(8, 2) PAIR_CP(32, 6) PAIR_CP(36, 10) PAIR_CP(12, 3) PAIR_CP(40, 7) PAIR_CP(44, 11)
 #define PAIR_MMAS(FIRST)                                                                             \
     PAIR_MMA(0, 0, 16, FIRST) PAIR_MMA(1, 4, 24, "q") PAIR_MMA(2, 8, 32, "q") PAIR_MMA(3, 12, 40, "q") \
-    "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+    "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"                                      \
+    "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%9];\n\t}"
 // (shared-memory addresses lie below 256 KB: the low words of operand_desc() and scale_desc() are address / 16 and constants)
 #define PAIR_ARGS                                                                                                          \
     ::"r"(tmem_d), "r"((a >> 4) | (1u << 16)), "r"((b >> 4) | (1u << 16)), "r"(idesc), "r"(sf), "r"(scales >> 4),         \
-        "r"(empty), "n"((128 >> 4) | (1 << 14)), "n"((1024 >> 4) | (1 << 14) | (2 << 29))                         \
+        "r"(empty), "n"((128 >> 4) | (1 << 14)), "n"((1024 >> 4) | (1 << 14) | (2 << 29)), "r"(peer_empty)        \
         : "memory"
-__device__ __forceinline__ void pair_slab_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty) {
+__device__ __forceinline__ void pair_slab_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty, uint32_t peer_empty) {
     asm volatile(PAIR_HEAD PAIR_CPS PAIR_MMAS("q") PAIR_ARGS);
 }
 // A tile's first slab in two parts: its copies, and the products that start the accumulator anew.
-__device__ __forceinline__ void pair_first_copies_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty) {
+__device__ __forceinline__ void pair_first_copies_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty, uint32_t peer_empty) {
     asm volatile(PAIR_HEAD PAIR_CPS "}" PAIR_ARGS);
 }
-__device__ __forceinline__ void pair_first_products_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty) {
+__device__ __forceinline__ void pair_first_products_elect(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sf, uint32_t scales, uint32_t empty, uint32_t peer_empty) {
     asm volatile(PAIR_HEAD PAIR_MMAS("!q") PAIR_ARGS);
 }
 #undef PAIR_CP
@@ -421,10 +432,11 @@ struct GemmMaps {
 // SPLIT = kSliced (with GROUP): a group that holds weights which SPLIT cuts when they are called alone.  Tiles are whole, but
 // the accumulator starts anew with every slice of such a weight and the epilogue adds the slices up as kCluster does: the bits
 // of the single call in the group's one launch (where that is the faster way: group_cost).
-// PAIR: pairs of SMs on 256-token tiles (above).  Each CTA's loads report to its own barrier; the second CTA (rank 1) passes
-// "landed" on with an arrival on the leader's barrier of that stage (loads that report to the other CTA's barrier themselves
-// take 1600 cycles per 32 KB instead of 560); the leader issues the scale copies and the products for both and commits to
-// both CTAs' barriers.
+// PAIR: pairs of SMs on 256-token tiles (above).  Both CTAs' loads report to the leader's (rank 0's) barrier of their stage, which
+// expects the bytes of both; the leader issues the scale copies and the products for both and commits "stage consumed" and
+// "accumulator complete" to both CTAs' barriers.  So what either CTA acts on comes from the loads and products themselves.  (A
+// thread that passed its own CTA's observation on would have to release it at cluster scope: 1.7 times the time of the whole
+// GEMM for "landed", 1.9 times for "consumed", at 2048 tokens.)
 template <bool DUAL, bool TAIL, bool QOUT = false, bool GROUP = false, int SPLIT = kWhole, bool PAIR = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ GemmMaps maps, const GemmArgs g) {
@@ -456,7 +468,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kStages; ++s) {
-            mbar_init(bar_full + 8 * s, PAIR && rank == 0 ? 2 : 1); // the leader's: its own copies and the other CTA's "landed"
+            mbar_init(bar_full + 8 * s, 1);
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_acc_full, 1);
@@ -489,7 +501,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             uint32_t it = 0, issued = 0; // k slabs issued so far, over all tiles
             uint32_t stage = 0, phase = 1; // PAIR: of slab `it`
             bool ok = true; PROF_DECL
-            const uint32_t peer_empty = PAIR ? map_to_rank(bar_empty, 1) : 0u;
+            const uint32_t landed = PAIR ? map_to_rank(bar_full, 0) : bar_full; // where this CTA's loads report
             const CUtensorMap *ms = nullptr; // PAIR: the scales of `mb`
             uint32_t tile_m, tile_n;
             const uint8_t *sfa, *sfb0, *sfb1;
@@ -514,9 +526,9 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             // end, and only the scale chunks that exist are fetched
             auto sf_bytes = [&](uint32_t kt) { return min(4u, g.kt64 - 4 * kt) * 512; };
             auto load_weights = [&](uint32_t kt, uint32_t s) {
-                const uint32_t st = base + s * kStageBytes, full = bar_full + 8 * s;
+                const uint32_t st = base + s * kStageBytes, full = landed + 8 * s;
                 if constexpr (PAIR) { // (scale rows of 8-byte elements; what lies past a row's or the tensor's end arrives as zeros)
-                    mbar_expect_tx_elect(full, g.a_bytes + kBBytes + kSfaBytes + kSfbBytes);
+                    if (rank == 0) mbar_expect_tx_elect(bar_full + 8 * s, 2 * (g.a_bytes + kBBytes + kSfaBytes + kSfbBytes));
                     // the leader holds the tile's first 128 weight rows (the gate rows of the fused form), the other CTA the rest (up)
                     const CUtensorMap *half = DUAL ? &maps.b[rank] : mb;
                     tma_load_2d_pair_elect(st + kABytes, half, (int)(kt * (BK / 2)), (int)(DUAL ? tile_n * kTileRows : tile_n * BN + rank * (BN / 2)), full);
@@ -536,7 +548,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 bulk_load_elect(st + kABytes + kBBytes + kSfaBytes + 2048, sfb1 + (size_t)kt * 2048, sf_bytes(kt), full);
             };
             auto load_activations = [&](uint32_t kt, uint32_t s) {
-                const uint32_t st = base + s * kStageBytes, full = bar_full + 8 * s;
+                const uint32_t st = base + s * kStageBytes, full = landed + 8 * s;
                 if constexpr (PAIR) {
                     tma_load_2d_pair_elect(st, &map_a, (int)(kt * (BK / 2)), (int)((2 * tile_m + rank) * BM), full);
                     tma_load_2d_pair_elect(st + kABytes + kBBytes, &maps.a_scales, (int)(kt * (4 * 512 / 8)), (int)(2 * tile_m + rank), full);
@@ -555,9 +567,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 locate(tile);
                 for (uint32_t kt = GEMM_KT_FIRST; kt < GEMM_KT_END; ++kt, ++it) {
                     const uint32_t s = PAIR ? stage : it % kStages, round = it / kStages;
-                    PROF_BEGIN if (PAIR) { if (it >= kStages) ok = mbar_wait_warp(bar_empty + 8 * s, phase, abort_flag); } else if (round > 0) ok = mbar_wait_warp(bar_empty + 8 * s, (round - 1) & 1, abort_flag); PROF_END(0)
+                    PROF_BEGIN if (PAIR) { if (it >= kStages) ok = mbar_wait_pair_warp(bar_empty + 8 * s, phase, abort_flag); } else if (round > 0) ok = mbar_wait_warp(bar_empty + 8 * s, (round - 1) & 1, abort_flag); PROF_END(0)
                     if (!ok) break;
-                    if (PAIR && rank == 0 && it >= kStages) mbar_arrive_cluster_elect(peer_empty + 8 * s); // (a second commit a slab costs the tensor pipe 30 cycles)
                     if (it >= ahead) load_weights(kt, s);
                     load_activations(kt, s);
                     issued = it + 1;
@@ -566,10 +577,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             if (lane == 0) { PROF_FLUSH(0) }
             if constexpr (PAIR) { // the last commits have reached this CTA's barriers before it may leave
-                for (uint32_t k = issued > kStages ? issued - kStages : 0; k < issued && ok; ++k) {
-                    ok = mbar_wait_warp(bar_empty + 8 * (k % kStages), (k / kStages) & 1, abort_flag);
-                    if (ok && rank == 0) mbar_arrive_cluster_elect(peer_empty + 8 * (k % kStages));
-                }
+                for (uint32_t k = issued > kStages ? issued - kStages : 0; k < issued && ok; ++k)
+                    ok = mbar_wait_pair_warp(bar_empty + 8 * (k % kStages), (k / kStages) & 1, abort_flag);
             }
             if (!ok) {
                 if (lane == 0) {
@@ -577,8 +586,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     atomicExch(g.status + 1, 101);
                 }
                 // let the copies already in flight land before the CTA's shared memory goes away
+                // (the second CTA's report to the leader's barriers, which it cannot ask: it stays for one wait that runs out)
+                if (PAIR && rank) mbar_wait_alone(bar_full, 0);
                 const uint32_t first = issued > kStages ? issued - kStages : 0;
-                for (uint32_t k = first; k < issued; ++k) {
+                for (uint32_t k = first; k < issued && !(PAIR && rank); ++k) {
                     uint32_t done = 0;
                     for (uint32_t i = 0; i < kSpinLimit && !done; ++i)
                         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
@@ -586,20 +597,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
             }
         }
-    } else if (PAIR && warp == 1 && rank) {
-        // ---------------------------------------------------------------- the other CTA of a pair: "my stage has landed"
-        const uint32_t leader_full = map_to_rank(bar_full, 0);
-        const uint32_t slabs = GEMM_TILE_FIRST < n_tiles_total ? ((n_tiles_total - GEMM_TILE_FIRST - 1) / (GEMM_TILE_STEP) + 1) * g.k_tiles : 0;
-        bool ok = true;
-        for (uint32_t it = 0; it < slabs && ok; ++it) {
-            const uint32_t s = it % kStages;
-            ok = mbar_wait_warp(bar_full + 8 * s, (it / kStages) & 1, abort_flag);
-            if (ok) mbar_arrive_cluster_elect(leader_full + 8 * s);
-        }
-        if (!ok && lane == 0) {
-            *abort_flag = 1;
-            atomicCAS(g.status + 1, 0, 116);
-        }
+    } else if (PAIR && warp == 1 && rank) { // (the leader issues for both)
     } else if (PAIR && (threadIdx.x >> 5) == 1) { // (see pair_slab_elect)
         // ---------------------------------------------------------------- MMA issuer of a pair (whole warp; one elected lane issues)
         // A pair's copies run beside the products only when the slab's are issued together in front of them (512 cycles per
@@ -608,7 +606,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // cycles, and 30 more with one more flag to look at; now the products' 512 (gate/up at 2048 tokens 234 -> 220 us).
         // What is left is the change of tiles, about 1800 cycles from the last slab's issue to the next tile's first.
         const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
-        const uint32_t peer_acc_full = map_to_rank(bar_acc_full, 1), whole_slabs = g.kt64 / 4;
+        const uint32_t peer_empty = map_to_rank(bar_empty, 1), peer_acc_full = map_to_rank(bar_acc_full, 1), whole_slabs = g.kt64 / 4;
         uint32_t local = 0, stage = 0, phase = 0;
         bool ok = true;
         auto landed = [&] {
@@ -638,15 +636,16 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             for (uint32_t kb = 0; kb < g.kt64 % 4; ++kb)
                 pair_mma_nvf4_elect(tmem, da + 2 * kb, db + 2 * kb, idesc, sf + 4 * kb, sf + 16 + 8 * kb, !fresh || kb != 0);
             pair_commit_elect(bar_empty + 8 * stage);
+            pair_commit_elect(peer_empty + 8 * stage);
             next_stage();
         };
         for (uint32_t tile = GEMM_TILE_FIRST; tile < n_tiles_total; tile += GEMM_TILE_STEP, ++local) {
             if (!landed()) break;
             if (whole_slabs) {
                 // the first copies go into the tensor pipe's queue behind the last tile's products, before the accumulator is free
-                pair_first_copies_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, 0);
+                pair_first_copies_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, 0, 0);
                 if (!drained()) break;
-                pair_first_products_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, bar_empty + 8 * stage);
+                pair_first_products_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, bar_empty + 8 * stage, peer_empty + 8 * stage);
                 next_stage();
             } else {
                 if (!drained()) break;
@@ -654,7 +653,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             for (uint32_t i = 1; i < whole_slabs; ++i) {
                 if (!landed()) break;
-                pair_slab_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, bar_empty + 8 * stage);
+                pair_slab_elect(tmem, PAIR_STAGE, idesc, PAIR_SCALES, bar_empty + 8 * stage, peer_empty + 8 * stage);
                 next_stage();
             }
             if (!ok) break;
@@ -793,7 +792,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     for (uint32_t at = 64; at < kPartCols * (is_f32 ? 4 : 2); at += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(res_at + at));
             }
             // (with a sleep between the polls: sixteen polling warps cost the SM power that the products could use)
-            bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, PAIR ? 20 : 64));
+            bool ok = __all_sync(0xffffffffu, (PAIR ? mbar_wait_pair_relaxed(bar_acc_full, local & 1, abort_flag, 20) : mbar_wait_relaxed(bar_acc_full, local & 1, abort_flag, 64)));
             if (!ok) {
                 if (lane == 0) {
                     *abort_flag = 1;
@@ -849,7 +848,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
-                if constexpr (PAIR) mbar_arrive_cluster(leader_acc_empty);
+                if constexpr (PAIR) mbar_arrive_accumulator_read(leader_acc_empty);
                 else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty) : "memory");
             }
             if constexpr (CLUSTER) {
