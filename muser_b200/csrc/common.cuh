@@ -58,7 +58,7 @@ struct Ctx {
     unsigned int *amax_flags = nullptr;
     uint32_t host_direct_output = 2;           // host-group entry: 2 one copy per output on the copy stream (beside the next launches), 1 a kernel
                                                // stores the outputs into mapped host buffers, 0 one copy per output on the launches' stream
-    uint32_t nvfp4_pair = 2;                   // NVFP4 GEMM on pairs of SMs (cta_group::2): 0 never, 1 always, 2 where they are faster
+    uint32_t nvfp4_pair = 2;                   // NVFP4 GEMM on pairs of SMs (cta_group::2): 0 never, 1 wherever rows allow, 2 where they are faster
     uint32_t nvfp4_group_m = 0;                // NVFP4 GEMM: token tiles per raster group, 0 = automatic
     uint32_t oneshot_max_bytes = 1536u << 10;  // all-reduce payloads up to this size take the one-shot peer exchange
     std::string last_error;

@@ -69,6 +69,22 @@ def make_weight(op, ctx, n_out, n_in, seed, negative_scales=False):
     return packed, scales, scale2
 
 
+def rounding_operands(op, k, n_in, tokens, rows, seed):
+    """Quantized activations and weights (one per entry of `rows`) whose f32 sums round: random codes, scales over some
+    thirteen binades on both sides, so that a sum spans more bits than f32 has and shows the order and the slices it was
+    added in."""
+    g = torch.Generator("cuda").manual_seed(seed)
+    x = torch.randn((tokens, n_in // 16, 16), device="cuda", generator=g)
+    x = x * torch.exp2(torch.randint(-6, 7, (tokens, n_in // 16, 1), device="cuda", generator=g).float())
+    isi = 0.25
+    ws = []
+    for n_out in rows:
+        packed = torch.randint(0, 256, (n_out, n_in // 2), dtype=torch.uint8, device="cuda", generator=g)
+        scales = torch.randint(0x10, 0x78, (n_out, n_in // 16), dtype=torch.uint8, device="cuda", generator=g)
+        ws.append(op.Weight(k.ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, 0.01, isi)))
+    return (*k.quantize_nvfp4_activation(x.reshape(tokens, n_in), isi), ws)
+
+
 def test_weight_repack_dequantises_bit_exactly(gpu, golden):
     op, ctx, k = gpu
     packed, scales, scale2 = make_weight(op, ctx, 37, 320, seed=2, negative_scales=True)
@@ -205,7 +221,7 @@ def test_paired_sm_gemm_equals_the_single_sm_gemm(gpu, n_out, n_in, tokens):
             ctx.sync_status()
             out[mode] = [y.cpu() for y in ys]
     finally:
-        ctx.tuning_set(TUNE_NVFP4_PAIR, 0)
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 2)
     for i, (a, b) in enumerate(zip(out[0], out[1])):
         assert torch.equal(a.view(torch.int32 if a.dtype == torch.float32 else torch.int16),
                            b.view(torch.int32 if b.dtype == torch.float32 else torch.int16)), f"output {i} differs between the two kernels"
@@ -707,7 +723,7 @@ def test_paired_forms_equal_the_single_sm_forms(gpu, n_in, tokens):
             ctx.sync_status()
             out[mode] = [y.cpu() for y in got]
     finally:
-        ctx.tuning_set(TUNE_NVFP4_PAIR, 0)
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 2)
     for i, (a, b) in enumerate(zip(out[0], out[1])):
         assert torch.equal(a, b), f"output {i} differs between the two forms"
     for w in ws:
@@ -742,3 +758,30 @@ def test_groups_of_shorter_rows_split_as_the_single_calls(gpu, n_in, shapes, tok
     assert H.rel_l2(alone[-1][:, :rows].double().cpu().numpy(), want) <= 3e-6
     for w in ws:
         w.free()
+
+
+def test_the_choice_between_the_forms_can_be_given_back_to_the_library(gpu):
+    """Told to use pairs, a context does not cut a row's sum; told to choose again, it does as a new context does."""
+    from muser_b200._lib import TUNE_NVFP4_PAIR
+    op, ctx, k = gpu
+    n_in, tokens = 12288, 16
+    xp, xs, (w,) = rounding_operands(op, k, n_in, tokens, [256], seed=5)
+
+    def call(kern):
+        y = torch.full((tokens, 256), float("nan"), device="cuda")
+        kern.encode_nvfp4_prequant(w, xp, xs, y, tokens)
+        kern.ctx.sync_status()
+        return y
+    fresh_ctx = op.Context(0, workspace_bytes=1 << 20)
+    fresh = call(op.CudaKernels(fresh_ctx))
+    try:
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 1)
+        assert not torch.equal(call(k), fresh), "these operands do not tell a cut sum from a whole one"
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 2)
+        assert torch.equal(call(k), fresh)
+    finally:
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 2)
+    with pytest.raises(op.MuserCudaError):
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 3)
+    fresh_ctx.close()
+    w.free()
