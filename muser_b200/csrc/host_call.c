@@ -177,18 +177,9 @@ static PyObject *matmul(PyObject *const *a, Py_ssize_t argc, int nvfp4) {
 static PyObject *quantized_matmul(PyObject *self, PyObject *const *a, Py_ssize_t argc) { return matmul(a, argc, 0); }
 static PyObject *nvfp4_matmul(PyObject *self, PyObject *const *a, Py_ssize_t argc) { return matmul(a, argc, 1); }
 
-/* (ctx, device, weights, x, outputs, tokens, epilogues): epilogues a sequence of keyword dictionaries or None each, or None */
-static int epilogue_of(PyObject *dict, muser_cuda_epilogue *ep, int *used) {
+static int epilogue_of_dict(PyObject *dict, muser_cuda_epilogue *ep, int *used) {
     PyObject *v[7];
     Py_ssize_t found = 0;
-    const int given = dict != Py_None ? PyObject_IsTrue(dict) : 0;
-    if (given < 0) return -1;
-    *used = 0;
-    if (!given) return 0;
-    if (!PyDict_Check(dict)) {
-        PyErr_Format(PyExc_TypeError, "an epilogue is a dict or None, not %s", Py_TYPE(dict)->tp_name);
-        return -1;
-    }
     for (int i = 0; i < 7; ++i) {
         v[i] = PyDict_GetItemWithError(dict, s_keys[i]);
         if (!v[i] && PyErr_Occurred()) return -1;
@@ -201,6 +192,22 @@ static int epilogue_of(PyObject *dict, muser_cuda_epilogue *ep, int *used) {
     }
     return to_epilogue(v[0], v[1], v[2], v[3], v[4], v[5], v[6], ep, used);
 }
+/* (ctx, device, weights, x, outputs, tokens, epilogues): weights as len() and iteration give them, outputs any iterable; epilogues
+ * None or epilogues[i], a mapping of keywords or None each */
+static int epilogue_of(PyObject *given_as, muser_cuda_epilogue *ep, int *used) {
+    const int given = given_as != Py_None ? PyObject_IsTrue(given_as) : 0;
+    if (given < 0) return -1;
+    *used = 0;
+    if (!given) return 0;
+    if (PyDict_Check(given_as)) return epilogue_of_dict(given_as, ep, used);
+    PyObject *dict = PyDict_New(); /* (lives until the tensors' addresses are read, as they do) */
+    int st = dict ? PyDict_Update(dict, given_as) : -1;
+    if (st && PyErr_ExceptionMatches(PyExc_AttributeError)) /* it has no keys() */
+        PyErr_Format(PyExc_TypeError, "an epilogue is a mapping or None, not %s", Py_TYPE(given_as)->tp_name);
+    if (!st) st = epilogue_of_dict(dict, ep, used);
+    Py_XDECREF(dict);
+    return st;
+}
 static PyObject *quantized_matmul_group(PyObject *self, PyObject *const *a, Py_ssize_t argc) {
     enum { kMost = 16 }; /* (the library takes four; longer lists are its to refuse) */
     muser_cuda_group_item items[kMost];
@@ -208,29 +215,29 @@ static PyObject *quantized_matmul_group(PyObject *self, PyObject *const *a, Py_s
     void *ctx, *x, *stream;
     uint32_t xd, tokens;
     ARGS(7)
-    PyObject *ws = PySequence_Fast(a[2], "weights must be a sequence"), *ys = ws ? PySequence_Fast(a[4], "outputs must be a sequence") : NULL;
+    PyObject *ws = PyObject_Size(a[2]) < 0 ? NULL : PySequence_Fast(a[2], "weights must be a sequence");
+    PyObject *ys = ws ? PySequence_Fast(a[4], "outputs must be a sequence") : NULL;
     const int given = ys && a[6] != Py_None ? PyObject_IsTrue(a[6]) : 0;
-    PyObject *es = given > 0 ? PySequence_Fast(a[6], "epilogues must be a sequence") : NULL;
     const Py_ssize_t n = ws ? PySequence_Fast_GET_SIZE(ws) : 0;
-    int ok = ws && ys && given >= 0 && (given == 0 || es);
+    int ok = ws && ys && given >= 0;
     memset(items, 0, sizeof(items));
     for (Py_ssize_t i = 0; ok && i < n && i < kMost && i < PySequence_Fast_GET_SIZE(ys); ++i) {
         int used = 0;
-        if (es && i >= PySequence_Fast_GET_SIZE(es)) {
-            PyErr_SetString(PyExc_IndexError, "list index out of range");
-            ok = 0;
-            break;
-        }
         PyObject *y = PySequence_Fast_GET_ITEM(ys, i);
         void *w, *yp;
-        ok = !(es && epilogue_of(PySequence_Fast_GET_ITEM(es, i), &eps[i], &used)) && !to_handle(PySequence_Fast_GET_ITEM(ws, i), &w) && !to_ptr(y, &yp) &&
+        if (given) {
+            PyObject *at = PyLong_FromSsize_t(i), *e = at ? PyObject_GetItem(a[6], at) : NULL;
+            ok = e && !epilogue_of(e, &eps[i], &used);
+            Py_XDECREF(at);
+            Py_XDECREF(e);
+        }
+        ok = ok && !to_handle(PySequence_Fast_GET_ITEM(ws, i), &w) && !to_ptr(y, &yp) &&
              !to_dtype(y, &items[i].y_dtype);
         if (!ok) break;
         items[i].w = w, items[i].y = yp, items[i].epilogue = used ? &eps[i] : NULL;
     }
     Py_XDECREF(ws);
     Py_XDECREF(ys);
-    Py_XDECREF(es);
     if (!ok || to_handle(a[0], &ctx) || to_ptr(a[3], &x) || to_dtype(a[3], &xd) || to_u32(a[5], &tokens) || to_stream(a[1], &stream)) return NULL;
     CALL(f_group(ctx, items, (uint32_t)n, x, xd, tokens, stream));
 }
@@ -268,7 +275,10 @@ static PyObject *nvfp4_group_prequant(PyObject *self, PyObject *const *a, Py_ssi
     void *y[kMost] = {NULL}, *ctx, *packed, *scales, *stream;
     uint32_t yd = 0, tokens;
     ARGS(7)
-    PyObject *ws = PySequence_Fast(a[2], "weights must be a sequence"), *ys = ws ? PySequence_Fast(a[5], "outputs must be a sequence") : NULL;
+    PyObject *ws = PyObject_Size(a[2]) < 0 ? NULL : PySequence_Fast(a[2], "weights must be a sequence");
+    PyObject *ys = ws && !PySequence_Check(a[5]) ? PyErr_Format(PyExc_TypeError, "'%s' object is not subscriptable", Py_TYPE(a[5])->tp_name)
+                   : ws                          ? PySequence_Fast(a[5], "outputs must be a sequence")
+                                                 : NULL;
     const Py_ssize_t n = ws ? PySequence_Fast_GET_SIZE(ws) : 0, n_y = ys ? PySequence_Fast_GET_SIZE(ys) : 0;
     int ok = ys != NULL;
     if (ok && (n_y == 0 || n_y > n)) {

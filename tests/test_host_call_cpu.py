@@ -1,5 +1,6 @@
 """The per-call binding (csrc/host_call.c) on the CPU: what it hands to the library and what it refuses.  The library's own
 argument checks come first, so a call with a freed handle ends in them without a GPU."""
+import collections
 import ctypes as C
 import types
 
@@ -60,6 +61,49 @@ def test_arguments_are_refused_as_before(kern):
                  lambda: k.encode_nvfp4_ffn_gate_up_silu_requant(w, w, x, x, 2, 1.0, out_packed=x, out_scales=x)):
         with pytest.raises(op.MuserCudaError):
             call()
+    assert k.launches == 0
+
+
+def test_a_groups_arguments_may_be_what_python_takes_for_them(kern):
+    """weights: len() and iteration; outputs: iteration (indexing too for NVFP4 groups); epilogues: epilogues[i], each a mapping
+    or None.  The library refuses a call without a context, so BAD_ARG says that the arguments passed."""
+    k, w = kern
+    x, y = torch.zeros((2, 256)), torch.zeros((2, 16))
+    taken = {"norm_weight": torch.ones(256), "norm_eps": 1e-5}
+    wrong = {"norm_weight": torch.ones(256, dtype=torch.float64)}
+
+    def group(weights, outputs, epilogues=None):
+        k.encode_quantized_matmul_group(weights, x, outputs, 2, epilogues=epilogues)
+
+    def nvfp4(weights, outputs):
+        k.encode_nvfp4_group_prequant(weights, x, x, outputs, 2)
+    two = {0: w, 1: w}
+    for weights, outputs in ((two.values(), (y, y)), ((w, w), {0: y, 1: y}.values()), (collections.deque([w, w]), iter([y, y]))):
+        for epilogues in (None, [None, taken], (taken, None), {0: None, 1: taken}, [types.MappingProxyType(taken), collections.UserDict(taken)],
+                          collections.defaultdict(lambda: None)):
+            with pytest.raises(op.MuserCudaError) as e:
+                group(weights, outputs if not hasattr(outputs, "__next__") else iter([y, y]), epilogues)
+            assert e.value.status_name == "BAD_ARG" and "norm_weight" not in str(e.value)
+    for epilogue in (types.MappingProxyType(wrong), collections.UserDict(wrong)):
+        with pytest.raises(op.MuserCudaError, match="norm_weight must be f32"):
+            group([w, w], [y, y], [None, epilogue])
+    with pytest.raises(op.MuserCudaError, match="norm_weight must be f32"):
+        group([w, w], [y, y], {0: None, 1: wrong})
+    with pytest.raises(KeyError):
+        group([w, w], [y, y], {0: taken})
+    for epilogue in (types.MappingProxyType({"no_such_argument": 1}), 5, [1, 2]):
+        with pytest.raises(TypeError):
+            group([w, w], [y, y], [None, epilogue])
+    with pytest.raises(TypeError):
+        group((v for v in [w, w]), [y, y])
+    for weights in (two.values(), collections.deque([w, w])):
+        with pytest.raises(op.MuserCudaError):
+            nvfp4(weights, (y, y))
+    with pytest.raises(TypeError):
+        nvfp4((v for v in [w, w]), [y, y])
+    for outputs in (iter([y, y]), {0: y, 1: y}.values()):
+        with pytest.raises(TypeError):
+            nvfp4([w, w], outputs)
     assert k.launches == 0
 
 
