@@ -61,6 +61,13 @@ static int to_f32(PyObject *o, float *out) {
     *out = (float)v;
     return 0;
 }
+/* what c_float(o) gives, for the arguments that the interface wraps so: TypeError, not ArgumentError, where it is no number */
+static int to_c_float(PyObject *o, float *out) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) return -1;
+    *out = (float)v;
+    return 0;
+}
 /* what float(o) gives, for the arguments that the interface converts itself */
 static int to_float(PyObject *o, float *out) {
     double v;
@@ -301,7 +308,7 @@ static PyObject *nvfp4_gate_up_requant(PyObject *self, PyObject *const *a, Py_ss
     float isi;
     ARGS(10)
     if (to_handle(a[0], &ctx) || to_handle(a[2], &gate) || to_handle(a[3], &up) || to_ptr(a[4], &packed) || to_ptr(a[5], &scales) || to_u32(a[6], &tokens) ||
-        to_f32(a[7], &isi) || to_ptr(a[8], &op) || to_ptr(a[9], &os) || to_stream(a[1], &stream))
+        to_c_float(a[7], &isi) || to_ptr(a[8], &op) || to_ptr(a[9], &os) || to_stream(a[1], &stream))
         return NULL;
     CALL(f_nv_requant(ctx, gate, up, packed, scales, tokens, isi, op, os, stream));
 }
@@ -327,7 +334,7 @@ static PyObject *norm_residual_norm(PyObject *self, PyObject *const *a, Py_ssize
     float eps1, eps2;
     ARGS(11)
     if (to_handle(a[0], &ctx) || to_ptr(a[2], &hidden) || to_ptr(a[3], &src) || to_ptr_or_null(a[4], &out) || to_ptr(a[5], &w1) || to_ptr_or_null(a[6], &w2) ||
-        to_u32(a[7], &tokens) || to_u32(a[8], &n) || to_f32(a[9], &eps1) || to_f32(a[10], &eps2) || to_stream(a[1], &stream))
+        to_u32(a[7], &tokens) || to_u32(a[8], &n) || to_c_float(a[9], &eps1) || to_c_float(a[10], &eps2) || to_stream(a[1], &stream))
         return NULL;
     CALL(f_norm_residual(ctx, hidden, src, out, w1, w2, tokens, n, eps1, eps2, stream));
 }
@@ -347,7 +354,7 @@ static PyObject *head_rms_norm(PyObject *self, PyObject *const *a, Py_ssize_t ar
     uint32_t tokens, heads, head_dim;
     float eps;
     ARGS(8)
-    if (to_handle(a[0], &ctx) || to_ptr(a[2], &x) || to_ptr(a[3], &w) || to_f32(a[4], &eps) || to_u32(a[5], &tokens) || to_u32(a[6], &heads) ||
+    if (to_handle(a[0], &ctx) || to_ptr(a[2], &x) || to_ptr(a[3], &w) || to_c_float(a[4], &eps) || to_u32(a[5], &tokens) || to_u32(a[6], &heads) ||
         to_u32(a[7], &head_dim) || to_stream(a[1], &stream))
         return NULL;
     CALL(f_head_norm(ctx, x, w, eps, tokens, heads, head_dim, stream));

@@ -54,6 +54,14 @@ def test_arguments_are_refused_as_before(kern):
         k.encode_nvfp4_group_prequant([w], x, x, [y, y], 2)
     with pytest.raises(C.ArgumentError):
         k.quantize_nvfp4_activation(x, "1.0", out=(x, x))
+    for eps in ("1e-5", None, x):
+        with pytest.raises(Exception) as want:
+            C.c_float(eps)
+        for call in (lambda: k.encode_head_rms_norm(x, y, eps, 2), lambda: k.encode_fused_norm_residual_rms_norm(x, x, x[0], eps),
+                     lambda: k.encode_fused_norm_residual_rms_norm(x, x, x[0], 1e-5, x, x[0], eps),
+                     lambda: k.encode_nvfp4_ffn_gate_up_silu_requant(w, w, x, x, 2, eps, out_packed=x, out_scales=x)):
+            with pytest.raises(want.type):
+                call()
     with pytest.raises(op.MuserCudaError):
         k.quantize_nvfp4_activation(x, 1, norm_weight=torch.ones(256), norm_eps=1e-5, out=(x, x))
     for call in (lambda: k.encode_sigmoid_gate(x, x), lambda: k.encode_head_rms_norm(x, y, 1e-5, 2), lambda: k.encode_nvfp4_prequant(w, x, x, y, 2, residual=y),
