@@ -11,7 +11,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libmuser_cuda.so"
-CALL = PKG / "_call.so"  # the Python binding's per-call half (csrc/host_call.c)
+CALL = PKG / ("_call" + sysconfig.get_config_var("EXT_SUFFIX"))  # the Python binding's per-call half (csrc/host_call.c), for this Python
 SOURCES = ["api.cu", "repack.cu", "kquant_decode.cu", "kquant_tc.cu", "kquant_mma.cu", "nvfp4_quant.cu", "nvfp4_gemm.cu", "nvfp4_static.cu", "nvfp4_a16.cu", "collective.cu", "layer_ops.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -27,14 +27,18 @@ def _newest(paths) -> float:
     return max(p.stat().st_mtime for p in paths)
 
 
-def build_call(force: bool = False) -> Path:
-    src = CSRC / "host_call.c"
+def build_call(force: bool = False) -> Path | None:
+    src, include = CSRC / "host_call.c", Path(sysconfig.get_paths()["include"])
+    (PKG / "_call.so").unlink(missing_ok=True)  # (its former name, which any Python takes for its own)
+    if not (include / "Python.h").exists():
+        print(f"{include} has no Python.h: calls from Python go through ctypes (_call_py.py), some microseconds slower", file=sys.stderr)
+        return None
     if not force and CALL.exists() and CALL.stat().st_mtime >= _newest([src, PKG.parent / "include" / "muser_cuda.h"]):
         return CALL
-    cmd = [os.environ.get("CC", "gcc"), "-shared", "-fPIC", "-O2", "-Wall", "-Wno-unused-parameter", "-I" + sysconfig.get_paths()["include"], str(src), "-o", str(CALL), "-ldl"]
+    cmd = [nvcc(), "-shared", "-cudart", "none", "-O2", "-Xcompiler", "-fPIC,-Wall,-Wno-unused-parameter", f"-I{include}", str(src), "-o", str(CALL), "-ldl"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError("gcc failed for host_call.c:\n" + r.stderr[-4000:])
+        raise RuntimeError("nvcc failed for host_call.c:\n" + r.stderr[-4000:])
     return CALL
 
 

@@ -4,7 +4,7 @@
  * 3 in the launch, 1 to 1.6 in ctypes' argument conversion, 1 in building an epilogue structure, 1.2 in
  * torch.cuda.current_stream().  Here a call costs some tenths of a microsecond besides the launch.  Nothing is kept between
  * calls: addresses, dtypes and the stream are asked for every time, and the library is entered without the GIL, as ctypes
- * does it.  What ctypes refused with ArgumentError is refused with it here.
+ * does it.  What ctypes refuses with ArgumentError is refused with it here.  muser_b200/_call_py.py is the same over ctypes.
  */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -392,6 +392,7 @@ static PyObject *bind(PyObject *self, PyObject *args) {
         Py_INCREF(o[i]);
         Py_XSETREF(*slots[i], o[i]);
     }
+    g.stream_ready = 0;
     Py_RETURN_NONE;
 }
 

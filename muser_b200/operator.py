@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
-from . import _call, _lib
+from . import _call_py, _lib
 from ._lib import (BF16, F16, F32, NVFP4, Q4_K, Q6_K, SHARD_K, SHARD_NONE, SHARD_ROWS, TUNE_DECODE_KSPLIT, TUNE_DECODE_RING,
                    TUNE_DECODE_WARPS, TUNE_DECODE_WSPLIT, TUNE_TC_MIN_ROWS, TUNE_TC_MIN_TOKENS_Q4_K, TUNE_TC_MIN_TOKENS_Q6_K, MuserCudaError)
 
@@ -33,8 +33,15 @@ def _stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-# the calls that a decode step makes go through csrc/host_call.c
-_call.bind(str(_lib.LIB_PATH), _TORCH_DTYPE, torch.float32, torch._C._cuda_getCurrentRawStream, _stream_ptr, MuserCudaError, C.ArgumentError)
+# the calls that a decode step makes go through csrc/host_call.c, or ctypes where that could not be built
+try:
+    from . import _call
+except ImportError:
+    _call = _call_py
+# (the first stream is asked for through torch.cuda, which initializes it; a torch without CUDA lacks the quicker way)
+for _binding in {_call, _call_py}:
+    _binding.bind(str(_lib.LIB_PATH), _TORCH_DTYPE, torch.float32, getattr(torch._C, "_cuda_getCurrentRawStream", _stream_ptr), _stream_ptr,
+                  MuserCudaError, C.ArgumentError)
 
 
 @dataclass
@@ -161,18 +168,6 @@ def _row_bytes(dtype: int, n_in: int) -> int:
     raise MuserCudaError(4, f"dtype {dtype} has no CUDA projection kernel")
 
 
-def _epilogue(row_scale=None, residual=None, norm_weight=None, norm_eps=0.0, out_scale=1.0, softcap=0.0, all_reduce=False):
-    """muser_cuda_epilogue; `norm_weight` (f32 [n_in], device) fuses rms_norm_mul(x, eps, norm_weight) in front,
-    `out_scale` / `softcap` the LM-head tail y <- softcap * tanh(y * out_scale / softcap) behind."""
-    if row_scale is None and residual is None and norm_weight is None and out_scale == 1.0 and softcap == 0.0 and not all_reduce:
-        return None
-    if norm_weight is not None and norm_weight.dtype != torch.float32:
-        raise MuserCudaError(1, "norm_weight must be f32")
-    return _lib.Epilogue(row_scale.data_ptr() if row_scale is not None else None,
-                         residual.data_ptr() if residual is not None else None, 0, float(norm_eps),
-                         norm_weight.data_ptr() if norm_weight is not None else None, float(out_scale), float(softcap), int(bool(all_reduce)))
-
-
 class CudaKernels:
     """Counterpart of the reference's `MetalKernels` for the projections of one device."""
 
@@ -238,7 +233,7 @@ class CudaKernels:
         index = torch.empty(tokens, dtype=torch.int32, device=dev)
         value = torch.empty(tokens, dtype=torch.float32, device=dev)
         nonfinite = torch.empty(tokens, dtype=torch.int32, device=dev)
-        ep = _epilogue(None, None, norm_weight, norm_eps, out_scale, softcap)
+        ep = _call_py.epilogue(None, None, norm_weight, norm_eps, out_scale, softcap)
         self.ctx.check(_L.muser_cuda_lm_head_argmax(
             self.ctx._h, weights._h, input.data_ptr(), _TORCH_DTYPE[input.dtype], tokens, C.byref(ep) if ep else None,
             logits.data_ptr() if logits is not None else None, _TORCH_DTYPE[logits.dtype] if logits is not None else F32,

@@ -1,19 +1,24 @@
-"""The per-call binding (csrc/host_call.c) on the CPU: what it hands to the library and what it refuses.  The library's own
-argument checks come first, so a call with a freed handle ends in them without a GPU."""
+"""The per-call binding (csrc/host_call.c, and _call_py.py, which stands in for it) on the CPU: what it hands to the library and
+what it refuses.  The library's own argument checks come first, so a call with a freed handle ends in them without a GPU."""
 import collections
 import ctypes as C
+import importlib.util
+import subprocess
+import sys
 import types
 
 import pytest
 import torch
 
-from muser_b200 import _call, _lib, operator as op
+from muser_b200 import _call, _call_py, _lib, build, operator as op
 
 
-@pytest.fixture
-def kern():
+@pytest.fixture(params=[_call, _call_py], ids=["c", "ctypes"])
+def kern(request, monkeypatch):
+    monkeypatch.setattr(op, "_call", request.param)
+
     def bind(raw, slow):
-        _call.bind(str(_lib.LIB_PATH), op._TORCH_DTYPE, torch.float32, raw, slow, op.MuserCudaError, C.ArgumentError)
+        op._call.bind(str(_lib.LIB_PATH), op._TORCH_DTYPE, torch.float32, raw, slow, op.MuserCudaError, C.ArgumentError)
     bind(lambda device: 0, lambda device: 0)
     ctx = op.Context.__new__(op.Context)
     ctx.device, ctx._h = 0, None
@@ -118,10 +123,25 @@ def test_a_groups_arguments_may_be_what_python_takes_for_them(kern):
 def test_the_stream_is_asked_for_on_every_call(kern):
     k, w = kern
     asked = []
-    _call.bind(str(_lib.LIB_PATH), op._TORCH_DTYPE, torch.float32, lambda d: asked.append(d) or 0, lambda d: asked.append(d) or 0, op.MuserCudaError, C.ArgumentError)
+    op._call.bind(str(_lib.LIB_PATH), op._TORCH_DTYPE, torch.float32, lambda d: asked.append(d) or 0, lambda d: asked.append(d) or 0, op.MuserCudaError, C.ArgumentError)
     x = torch.zeros((2, 256))
     for device in (0, 3):
         k.ctx.device = device
         with pytest.raises(op.MuserCudaError):
             k.encode_sigmoid_gate(x, x)
     assert asked == [0, 3]
+
+
+def test_binding_needs_no_more_than_the_library(monkeypatch, tmp_path):
+    """A torch without CUDA imports the operators; a Python without headers builds, and calls through ctypes; the extension
+    carries the tag of the Python it was built for, so that no other loads it."""
+    for hide, want in (("", "_call"), ("sys.modules['muser_b200._call'] = None\n", "_call_py")):
+        prog = ("import sys, torch\n"
+                "if hasattr(torch._C, '_cuda_getCurrentRawStream'): del torch._C._cuda_getCurrentRawStream\n" + hide +
+                f"from muser_b200 import operator as op\nassert op._call.__name__ == 'muser_b200.{want}'\n")
+        r = subprocess.run([sys.executable, "-c", prog], capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr
+    assert importlib.util.find_spec("muser_b200._call").origin.endswith(build.sysconfig.get_config_var("EXT_SUFFIX"))
+    monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    monkeypatch.setattr(build, "CALL", tmp_path / "none.so")
+    assert build.build_call(force=True) is None and not (tmp_path / "none.so").exists()
