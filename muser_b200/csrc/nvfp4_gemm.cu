@@ -6,7 +6,7 @@
 // 16 values on each side, then (acc * weight_scale2) * (1 / input_scale_inv) in that order.
 //
 // Shape of the kernel: persistent CTAs, one per SM, each walking 128-token x 256-row output tiles, or pairs of CTAs on
-// 256 tokens x 256 rows where that is faster (takes_pairs; the PAIR form below).  Warp 0 streams 128-byte-swizzled
+// 256 tokens x 256 rows where that is faster (pairs_pay; the PAIR form below).  Warp 0 streams 128-byte-swizzled
 // K slabs (256 values) of both operands with TMA plus their scale factors with bulk copies through a
 // 4-stage shared-memory ring; warp 1 copies each K = 64 block's scale factors into tensor memory (tcgen05.cp) and
 // issues its tcgen05.mma kind::mxf4nvf4 right behind them (for pairs: a slab's copies, then its products) into a 128 x 256 f32 accumulator in tensor memory (both
@@ -22,6 +22,7 @@
 
 #include "common.cuh"
 #include "nvfp4_codec.cuh"
+#include "nvfp4_pairs_rule.h"
 #include "tcgen05.cuh"
 
 namespace muser {
@@ -1409,17 +1410,9 @@ static uint32_t pair_room(Ctx *ctx) {
     }
     return (uint32_t)std::max(0, std::min(room.n, ctx->sm_count / 2));
 }
-// Pairs of SMs or single CTAs for `n_tiles` weight-row tiles of `m_blocks` 128-token blocks?  The same bits either way.  A
-// round of pairs takes 0.86 to 0.93 of a round of single CTAs (us, single / pairs at 2048 tokens: 5120 x 5120 32.3 / 27.7,
-// 7168 x 5120 in a group 37.7 / 32.4, 5120 x 27648 138 / 120, gate/up 237 / 220), but an odd block of tokens is half of a
-// pair's tile (gate/up at 384 tokens, five rounds against six: 55 / 60).
-static bool takes_pairs(Ctx *ctx, uint32_t n_tiles, uint32_t m_blocks) {
+static bool takes_pairs(Ctx *ctx, uint32_t n_tiles, uint32_t tokens, uint64_t n_in, PairForm form) {
     if (ctx->nvfp4_pair != 2) return ctx->nvfp4_pair == 1;
-    const uint32_t room = pair_room(ctx);
-    if (!room) return false;
-    const uint64_t pair_rounds = ((uint64_t)n_tiles * ((m_blocks + 1) / 2) + room - 1) / room;
-    const uint64_t single_rounds = ((uint64_t)n_tiles * m_blocks + ctx->sm_count - 1) / ctx->sm_count;
-    return pair_rounds * 9 <= single_rounds * 10;
+    return pairs_pay((uint32_t)ctx->sm_count, pair_room(ctx), n_tiles, tokens, (uint32_t)((n_in + BK - 1) / BK), form);
 }
 template <bool DUAL, bool TAIL, bool QOUT, bool GROUP>
 static cudaError_t launch_pairs(Ctx *ctx, const CUtensorMap &map_a, const GemmMaps &maps, const GemmArgs &g, cudaStream_t stream) {
@@ -1449,7 +1442,7 @@ muser_cuda_status launch_nvfp4_gemm(Ctx *ctx, const Weight *w, const uint8_t *x_
     const uint32_t m_blocks = (tokens + BM - 1) / BM, n_tiles = w_up ? (uint32_t)((w->n_out + BN / 2 - 1) / (BN / 2)) : (uint32_t)(w->n_out_pad / BN);
     const bool tail = ep.out_scale != 1.0f || ep.softcap > 0.0f;
     const uint32_t ks = w_up || tail || ctx->nvfp4_pair == 1 ? 1 : gemm_ksplit(ctx, w, tokens);
-    const bool pair = ks == 1 && takes_pairs(ctx, n_tiles, m_blocks) && (qout || pair_rows_fit(y, ep.residual, w->n_out, y_dtype));
+    const bool pair = ks == 1 && takes_pairs(ctx, n_tiles, tokens, w->n_in, w_up ? PairForm::fused : PairForm::plain) && (qout || pair_rows_fit(y, ep.residual, w->n_out, y_dtype));
     const uint32_t a_rows = pair ? BM : box_tokens(tokens);
     CUtensorMap map_a;
     GemmMaps maps;
@@ -1584,7 +1577,7 @@ muser_cuda_status launch_nvfp4_gemm_group(Ctx *ctx, const Weight *const *ws, uin
         }
         return n_rest ? launch_nvfp4_gemm_group(ctx, rest, n_rest, x_packed, x_scales, rest_y, y_dtype, tokens, stream) : MUSER_CUDA_OK;
     }
-    bool pair = !sliced && takes_pairs(ctx, tiles_n, m_blocks);
+    bool pair = !sliced && takes_pairs(ctx, tiles_n, tokens, w0->n_in, PairForm::group);
     for (uint32_t p = 0; p < n; ++p) pair = pair && pair_rows_fit(ys[p], nullptr, ws[p]->n_out, y_dtype);
     const uint32_t a_rows = pair ? BM : box_tokens(tokens);
     CUtensorMap map_a;
