@@ -128,19 +128,20 @@ __global__ void __launch_bounds__(256) head_rms_norm_kernel(float *x, const floa
     float4 *row = reinterpret_cast<float4 *>(x + (size_t)head * head_dim);
     const float4 *w4 = reinterpret_cast<const float4 *>(w);
     const uint32_t n4 = head_dim / 4;
-    const float4 w0 = lane < n4 ? ld_after_wait(w4 + lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); // (all of it up to heads of 128)
-    float ss = 0.0f;
-    for (uint32_t i = lane; i < n4; i += 32) {
+    // A lane's first piece of the row and of the weights, all of them up to heads of 128, are fetched together and held.  (us, weights
+    // fetched ahead and the row read twice / held: 40 heads 1.63 / 1.45 at one token, 5.46 / 3.97 at 512, 16.9 / 12.1 at 2048.)
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f), v0 = lane < n4 ? ld_after_wait(row + lane) : zero, w0 = lane < n4 ? ld_after_wait(w4 + lane) : zero;
+    float ss = v0.x * v0.x + v0.y * v0.y + v0.z * v0.z + v0.w * v0.w;
+    for (uint32_t i = lane + 32; i < n4; i += 32) {
         const float4 v = ld_after_wait(row + i);
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(ss, (float)head_dim) + eps));
-    for (uint32_t i = lane; i < n4; i += 32) {
-        const float4 v = ld_after_wait(row + i), ww = i == lane ? w0 : ld_after_wait(w4 + i);
-        row[i] = make_float4(v.x * inv * ww.x, v.y * inv * ww.y, v.z * inv * ww.z, v.w * inv * ww.w);
-    }
+    auto scaled = [&](const float4 &v, const float4 &ww) { return make_float4(v.x * inv * ww.x, v.y * inv * ww.y, v.z * inv * ww.z, v.w * inv * ww.w); };
+    if (lane < n4) row[lane] = scaled(v0, w0);
+    for (uint32_t i = lane + 32; i < n4; i += 32) row[i] = scaled(ld_after_wait(row + i), ld_after_wait(w4 + i));
 }
 
 muser_cuda_status launch_norm_residual_norm(Ctx *ctx, float *hidden, const float *src, float *output, const float *w1, const float *w2,
