@@ -464,6 +464,28 @@ def test_norm_kernels_agree_on_either_side_of_their_lines(gpu, n_in, tokens):
         assert torch.equal(torch.as_tensor(got_s).cpu().reshape(tokens, -1), torch.as_tensor(want_s).reshape(4, -1)[at])
 
 
+@pytest.mark.parametrize("n_in,tokens", [(1024, 3), (1024, 600), (4096, 3), (4096, 600), (12288, 3)])
+def test_norm_where_the_guess_parts_from_the_sum_at_a_runs_start(gpu, n_in, tokens):
+    """A row whose sum stays one unit below a power of two over values too small to move it: a prefix sum says that the next
+    segments lie in the binade above, and a run of them fails at its first.  The CPU lane's bytes all the same."""
+    op, ctx, k = gpu
+    rows = torch.ones((3, n_in))
+    v = np.float32(32.0)
+    while np.float32(v * v) >= np.float32(1024.0):
+        v = np.nextafter(v, np.float32(0.0))
+    rows[:, 0] = float(v)
+    rows[:, 1:64] = 2.0 ** -8                                 # (a quarter of a unit below 1024 and less)
+    rows[1, 1:200] = 2.0 ** -8                                # several segments long
+    rows[2] = rows[1].roll(n_in // 2)                         # in the middle of the row
+    nw = torch.linspace(0.5, 1.5, n_in)
+    want_p, want_s = O.quantize_nvfp4_activation(O.rms_norm_mul(rows.numpy(), 1e-6, nw.numpy()), 41.5)
+    at = torch.arange(tokens) % 3
+    got_p, got_s = k.quantize_nvfp4_activation(rows[at].cuda(), 41.5, norm_weight=nw.cuda(), norm_eps=1e-6)
+    ctx.sync_status()
+    assert torch.equal(got_p.cpu().reshape(tokens, -1), torch.from_numpy(want_p).reshape(3, -1)[at])
+    assert torch.equal(torch.as_tensor(op.unswizzle_scales(got_s, tokens, n_in)).cpu().reshape(tokens, -1), torch.as_tensor(want_s).reshape(3, -1)[at])
+
+
 @pytest.mark.parametrize("n_in,tokens", [(2032, 4097), (2032, 8200), (272, 30850), (5200, 1600)])
 def test_quantizers_of_four_rows_a_thread(gpu, n_in, tokens):
     """Many rows, plain and behind the norm, a ragged last block of rows and rows that end inside a 64-value chunk: the CPU
