@@ -483,8 +483,8 @@ __global__ void __launch_bounds__(256) nvfp4_scaled_quantize_kernel(const void *
 // the norm's own kernel.  (Blocks of 256 threads 85 and 127; two of the four rows ahead 87 and 120.)
 template <bool XF32, bool NORM>
 __global__ void __launch_bounds__(128) nvfp4_quantize_quads_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
-                                                                   const float *norm_w, const float *inv_rms, uint8_t *packed, uint8_t *scales, bool early) {
-    pdl_turn(early);
+                                                                   const float *norm_w, const float *inv_rms, uint8_t *packed, uint8_t *scales) {
+    pdl_turn(false); // (thousands of blocks)
     const uint32_t groups_pad = kt * 4;
     const uint64_t idx = blockIdx.x * (uint64_t)128 + threadIdx.x; // (128 x kt of them per 128 rows: whole blocks)
     const uint32_t quad = (uint32_t)(idx / groups_pad), grp = (uint32_t)(idx % groups_pad);
@@ -602,7 +602,7 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
             if (takes_quads(tokens_pad, kt, f32, true)) {
                 const auto kernel = f32 ? nvfp4_quantize_quads_kernel<true, true> : nvfp4_quantize_quads_kernel<false, true>;
                 MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad / 128 * kt), dim3(128), 0, stream, x, tokens, (uint32_t)n_in, kt, isi,
-                                               norm_weight, (const float *)inv, packed, scales, false));
+                                               norm_weight, (const float *)inv, packed, scales));
                 return MUSER_CUDA_OK;
             }
             const auto kernel = f32 ? nvfp4_scaled_quantize_kernel<true> : nvfp4_scaled_quantize_kernel<false>;
@@ -620,7 +620,7 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
     if (takes_quads(tokens_pad, kt, x_dtype == MUSER_DTYPE_F32, false)) {
         const auto kernel = x_dtype == MUSER_DTYPE_F32 ? nvfp4_quantize_quads_kernel<true, false> : nvfp4_quantize_quads_kernel<false, false>;
         MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad / 128 * kt), dim3(128), 0, stream, x, tokens, (uint32_t)n_in, kt, isi,
-                                       (const float *)nullptr, (const float *)nullptr, packed, scales, false));
+                                       (const float *)nullptr, (const float *)nullptr, packed, scales));
         return MUSER_CUDA_OK;
     }
     const uint64_t total = (uint64_t)tokens_pad * kt * 4;

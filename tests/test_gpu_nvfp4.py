@@ -807,3 +807,53 @@ def test_the_choice_between_the_forms_can_be_given_back_to_the_library(gpu):
         ctx.tuning_set(TUNE_NVFP4_PAIR, 3)
     fresh_ctx.close()
     w.free()
+
+
+@pytest.mark.parametrize("n", [1024, 5120])
+@pytest.mark.parametrize("tokens", [1, 16, 200])
+def test_chained_nvfp4_launches_see_what_their_predecessors_wrote(gpu, n, tokens):
+    """Quantizers, norms and GEMMs that start under the launches before them, buffers and the context's row factors used again
+    and again, norm weights made on the stream two launches back: the bits of the same calls with a synchronization between
+    each two.  Rows of 1024 take the factor kernel and a quantizer, rows of 5120 a block each up to 148."""
+    op, ctx, k = gpu
+    isi = 3.0
+    g = torch.Generator("cuda").manual_seed(n + tokens)
+    weights = []
+    for i in range(4):
+        packed = torch.randint(0, 256, (n, n // 2), dtype=torch.uint8, device="cuda", generator=g)
+        scales = torch.randint(0x28, 0x38, (n, n // 16), dtype=torch.uint8, device="cuda", generator=g)
+        weights.append(op.Weight(ctx, op.TensorView(packed, O.NVFP4, n, n, scales, 0.02, isi)))
+    x0 = torch.randn((tokens, n), device="cuda", generator=g)
+    w0, gate = 1.0 + 0.1 * torch.randn(n, device="cuda", generator=g), 2.0 + torch.randn(n, device="cuda", generator=g)
+
+    def chain(sync):
+        x, xb, w, w2 = x0.clone(), x0.bfloat16(), w0.clone(), w0.clone()
+        ys = [torch.zeros((tokens, n), dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+        yf = torch.zeros((tokens, n), device="cuda")
+        q = k.quantize_nvfp4_activation(x, isi)
+        kept = []
+        for _ in range(4):
+            for call in (lambda: k.encode_sigmoid_gate(w, gate), lambda: k.encode_sigmoid_gate(w2, gate),
+                         lambda: k.quantize_nvfp4_activation(x, isi, norm_weight=w, norm_eps=1e-5, out=q),
+                         lambda: k.quantize_nvfp4_activation(xb, isi, norm_weight=w2, norm_eps=1e-5, out=q),
+                         lambda: k.encode_nvfp4_group_prequant(weights[:3], *q, ys, tokens),
+                         lambda: k.quantize_nvfp4_activation(ys[1], isi, norm_weight=w, norm_eps=1e-5, out=q),
+                         lambda: k.encode_nvfp4_prequant(weights[3], *q, yf, tokens, residual=x),
+                         lambda: k.quantize_nvfp4_activation(yf, isi, out=q),
+                         lambda: k.encode_nvfp4_prequant(weights[0], *q, xb, tokens),
+                         lambda: k.quantize_nvfp4_activation(xb, isi, norm_weight=w0, norm_eps=1e-5, out=q),
+                         lambda: k.encode_nvfp4_ffn_gate_up_silu_requant(weights[1], weights[2], *q, tokens, isi, out_packed=q2[0], out_scales=q2[1]),
+                         lambda: k.encode_nvfp4_prequant(weights[2], *q2, x, tokens)):
+                call()
+                if sync:
+                    torch.cuda.synchronize()
+            kept.append([t.clone() for t in (*ys, yf, x, xb, *q2)])
+        ctx.sync_status()
+        return [t for step in kept for t in step]
+    q2 = tuple(torch.zeros_like(t) for t in k.quantize_nvfp4_activation(x0, isi))
+    want = chain(True)
+    assert all(torch.isfinite(t.float()).all() for t in want) and all(t.any() for t in want)
+    for _ in range(10):
+        assert all(torch.equal(a, b) for a, b in zip(chain(False), want))
+    for w in weights:
+        w.free()
