@@ -349,19 +349,22 @@ def test_long_rows_split_between_the_ctas_of_a_cluster(gpu, n_out, n_in, tokens)
 @pytest.mark.parametrize("shapes, tokens", [((9600, 300, 37), 131), ((300, 9600), 250), ((700, 37, 300, 256), 16), ((300, 37, 37888), 9)])
 def test_groups_of_long_rows_sum_in_the_single_calls_slices(gpu, shapes, tokens):
     """A group of long rows is one launch of whole tiles, some of its weights summed in the slices that the single call
-    splits them into, in different numbers of slices, beside weights that are never split: equal bits.  (The last group is
-    launched in parts: one launch would take a round of tiles more.)"""
+    splits them into, in different numbers of slices, beside weights that are never split: equal bits, on sums that round.
+    (The last group is launched in parts: one launch would take a round of tiles more.)"""
+    from muser_b200._lib import TUNE_NVFP4_PAIR
     op, ctx, k = gpu
-    from muser_b200 import synth
     n_in = 12352  # (49 slabs, the last one short)
-    x = synth.normal_activations(tokens, n_in, seed=11)
-    isi = synth.activation_input_scale_inv(x)
-    ws = []
-    for i, n_out in enumerate(shapes):
-        packed, scales, scale2 = make_weight(op, ctx, min(n_out, 700), n_in, seed=40 + i, negative_scales=(i == 0))
-        packed, scales = np.resize(packed, (n_out, n_in // 2)), np.resize(scales, (n_out, n_in // 16))
-        ws.append(op.Weight(ctx, op.TensorView(packed, O.NVFP4, n_in, n_out, scales, scale2, isi)))
-    q = k.quantize_nvfp4_activation(x.cuda(), isi)
+    *q, ws = rounding_operands(op, k, n_in, tokens, shapes, seed=11)
+    try:  # the operands tell cut sums from whole ones (the forced pairs')
+        sums = []
+        for mode in (1, 2):
+            ctx.tuning_set(TUNE_NVFP4_PAIR, mode)
+            sums.append([torch.empty((tokens, n), device="cuda") for n in shapes])
+            for w, y in zip(ws, sums[-1]):
+                k.encode_nvfp4_prequant(w, *q, y, tokens)
+        assert any(not torch.equal(a, b) for a, b in zip(*sums))
+    finally:
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 2)
     for dt in (torch.float32, torch.bfloat16):
         alone, grouped = ([torch.full((tokens, n), float("nan"), dtype=dt, device="cuda") for n in shapes] for _ in range(2))
         for w, y in zip(ws, alone):
@@ -647,13 +650,14 @@ def test_workspace_and_dtype_misuse(gpu):
     small.close()
 
 
+@pytest.mark.parametrize("pairs", [0, 1])
 @pytest.mark.parametrize("group_m", [1, 2, 3])
-def test_raster_groups_do_not_change_the_outputs(gpu, group_m):
+def test_raster_groups_do_not_change_the_outputs(gpu, group_m, pairs):
     """MUSER_TUNE_NVFP4_GROUP_M only reorders the output tiles (groups of token tiles; the last group short when the
     tile count is no multiple): every output must carry the same bits as with all token tiles in one group, in the
-    plain, the fused gate/up and the quantized-output forms."""
+    plain, the fused gate/up and the quantized-output forms, on single CTAs and on pairs (whose groups are half as many tiles)."""
     from muser_b200 import synth
-    from muser_b200._lib import TUNE_NVFP4_GROUP_M
+    from muser_b200._lib import TUNE_NVFP4_GROUP_M, TUNE_NVFP4_PAIR
     op, ctx, k = gpu
     n_out, n_in, tokens = 768, 512, 900  # 8 token tiles (the last one ragged), 3 weight-row tiles
     packed, scales, scale2 = make_weight(op, ctx, n_out, n_in, seed=91, negative_scales=True)
@@ -665,6 +669,7 @@ def test_raster_groups_do_not_change_the_outputs(gpu, group_m):
     xp, xs = k.quantize_nvfp4_activation(x.cuda(), isi)
     out = {}
     try:
+        ctx.tuning_set(TUNE_NVFP4_PAIR, pairs)
         for gm in (0, group_m):
             ctx.tuning_set(TUNE_NVFP4_GROUP_M, gm)
             y = torch.full((tokens, n_out), float("nan"), dtype=torch.float32, device="cuda")
@@ -676,6 +681,7 @@ def test_raster_groups_do_not_change_the_outputs(gpu, group_m):
             out[gm] = [t.cpu() for t in (y, y2, qp, qs)]
     finally:
         ctx.tuning_set(TUNE_NVFP4_GROUP_M, 0)
+        ctx.tuning_set(TUNE_NVFP4_PAIR, 2)
     for i, (a, b) in enumerate(zip(out[0], out[group_m])):
         assert torch.equal(a.view(torch.int32) if a.dtype == torch.float32 else a, b.view(torch.int32) if b.dtype == torch.float32 else b), f"output {i}"
     assert not torch.isnan(out[group_m][0]).any()
