@@ -112,19 +112,7 @@ __device__ __forceinline__ uint64_t scale_desc(uint32_t smem_addr) {
     return d;
 }
 
-__device__ __forceinline__ void tmem_cp_scales(uint32_t tmem_addr, uint64_t desc) {
-    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_addr), "l"(desc) : "memory");
-}
-__device__ __forceinline__ void mma_nvf4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                         uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
-        : "memory");
-}
-// The same two, issued by the elected lane of a warp that runs its role converged (tcgen05.cuh).
+// A scale copy and a product, issued by the elected lane of a warp that runs its role converged (tcgen05.cuh).
 __device__ __forceinline__ void tmem_cp_scales_elect(uint32_t tmem_addr, uint64_t desc) {
     asm volatile("{\n\t" MUSER_ELECT_PRED "@e tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n\t}" ::"r"(tmem_addr), "l"(desc) : "memory");
 }
@@ -249,18 +237,20 @@ __device__ __forceinline__ void store_strip(const float (&v)[N], T *y, const T *
     }
 }
 
-// SPLIT form: f32 sums of a tile as [row][256 columns + padding] in shared memory.
-constexpr uint32_t kRedPitch = BN + 4;
-static_assert((uint32_t)BM * kRedPitch * 4 <= (uint32_t)(kStages * kStageBytes), "the slices' sums exceed the stage ring");
-__device__ __forceinline__ void split_barrier() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t split_map(uint32_t cta_addr, uint32_t rank) {
+// Clusters (SPLIT and PAIR): an address in another CTA's shared memory, and all threads of all CTAs meeting.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t cta_addr, uint32_t rank) { // shared::cta address -> that CTA's window
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
     return r;
 }
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// SPLIT form: f32 sums of a tile as [row][256 columns + padding] in shared memory.
+constexpr uint32_t kRedPitch = BN + 4;
+static_assert((uint32_t)BM * kRedPitch * 4 <= (uint32_t)(kStages * kStageBytes), "the slices' sums exceed the stage ring");
 __device__ __forceinline__ float4 split_load(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -279,11 +269,6 @@ static_assert(kPSmemBytes <= 227 * 1024, "stage ring exceeds the shared memory o
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t cta_addr, uint32_t rank) { // shared::cta address -> that CTA's window
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
     return r;
 }
 // "Accumulator read", the one arrival of a thread on the other CTA's barrier: relaxed, because all that it orders is tensor-memory
@@ -309,9 +294,6 @@ __device__ __forceinline__ uint4 lds_16(uint32_t at) {
 }
 __device__ __forceinline__ void sts_16(uint32_t at, const uint32_t (&v)[4]) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // mbar_wait_relaxed and mbar_wait_warp for barriers that the other CTA of the pair arrives on (by its loads, its products' commits or its warps).
 __device__ __forceinline__ bool mbar_try_pair(uint32_t bar, uint32_t parity) {
@@ -422,9 +404,9 @@ struct GemmMaps {
 // each factor first rounded to f16 as the unfused W4A4 lane returns it (quant/nvfp4.rs:337).
 // TAIL compiles the LM-head tail (logit scale, tanh soft cap) into the epilogue; the common instantiation has none of it.
 // QOUT (with DUAL): silu(gate) * up is not stored but quantized on the spot for the down projection, exactly as
-// quant::quantize_nvfp4_activation would quantize the f32 product (quant/nvfp4.rs:173-238): a thread holds 64
-// consecutive outputs of its token, i.e. four 16-value groups = one chunk of the swizzled scale plane, and writes
-// 32 bytes of codes and one word of scales.  The 27648-wide intermediate is never written or read as numbers.
+// quant::quantize_nvfp4_activation would quantize the f32 product (quant/nvfp4.rs:173-238): a thread holds 32
+// consecutive outputs of its token, i.e. two 16-value groups = half a chunk of the swizzled scale plane, and writes
+// 16 bytes of codes and two of scales.  The 27648-wide intermediate is never written or read as numbers.
 // GROUP: several projections that read the same quantized activations (q | k | v) share one launch: their weight-row
 // tiles form one tile space, so the small ones fill the SMs that a launch of their own would leave idle.  Plain
 // outputs only (no fused tail, row scale or residual).
@@ -1012,7 +994,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     if constexpr (PAIR && !QOUT) // the stores are done with the staging buffers
         if (warp >= 2) asm volatile("{\n\t" MUSER_ELECT_PRED "@e cp.async.bulk.wait_group 0;\n\t}" ::: "memory");
     if constexpr (CLUSTER) {
-        split_barrier();
+        cluster_barrier();
         pdl_wait(); // (every warp stores here)
         uint32_t tile_m, tile_n;
         tile_coords(GEMM_TILE_FIRST, m_tiles, g.n_tiles, g.group_m, tile_m, tile_n);
@@ -1032,7 +1014,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 4
             for (uint32_t p = 0; p < g.ksplit; ++p) {
-                const uint32_t at = split_map(base + (row * kRedPitch + c0) * 4, p);
+                const uint32_t at = map_to_rank(base + (row * kRedPitch + c0) * 4, p);
                 const float4 q0 = split_load(at), q1 = split_load(at + 16);
                 v[0] += q0.x, v[1] += q0.y, v[2] += q0.z, v[3] += q0.w, v[4] += q1.x, v[5] += q1.y, v[6] += q1.z, v[7] += q1.w;
             }
@@ -1050,7 +1032,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             else
                 store_strip<__half, 8>(v, reinterpret_cast<__half *>(y) + o, g.residual ? reinterpret_cast<const __half *>(g.residual) + o : nullptr, valid, vec_ok);
         }
-        split_barrier(); // no CTA leaves while another may read its sums
+        cluster_barrier(); // no CTA leaves while another may read its sums
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
