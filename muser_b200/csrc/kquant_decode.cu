@@ -1247,9 +1247,13 @@ muser_cuda_status decode_autotune(Ctx *ctx, const Weight *const *w, const Weight
 // batched kernels.  Of the batched kernels the one on the warp-level instructions (kquant_mma.cu) has the
 // smaller fixed part and pads token columns to 8, the tcgen05 one (kquant_tc.cu, to 16, 32 or 64; Q4_K and Q6_K) the
 // cheaper column: see takes_tcgen05.  At 13 to 16 tokens the decode kernel's integer products are bound by their scale
-// arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 28, 5120 x 27648 Q6_K 68 -> 41, 5120 x 5120 21 -> 11,
-// 1024 x 5120 18.5 -> 8.4).  At 9 to 12 it depends on the weight (40 / 40, 55 / 43 for the long Q6_K rows, 17 / 15, but
-// 8192 x 5120 17 / 20), which one line for all of them does not follow; below it wins (27648 x 5120 at 8: 27 / 34).
+// arithmetic (us, decode kernel -> batched: 27648 x 5120 Q4_K 53 -> 29, 5120 x 27648 Q6_K 68 -> 42, 5120 x 5120 21 -> 11.5,
+// 1024 x 5120 18.5 -> 9).  The line at 13 was drawn for an earlier form of the batched kernel; at 9 to 12 tokens it would now be
+// the faster one for bf16 rows (decode / batched: 27648 x 5120 Q4_K 40.7 / 28.7, 5120 x 27648 Q6_K 55 / 42, Q5_K 52 / 37,
+// 5120 x 5120 17.4 / 11.7, 8192 x 5120 17.4 / 15.9, 1024 x 5120 15.6 / 9.1), and for f32 rows by the weight (40 / 37, 54 / 52,
+// 51 / 44, 17 / 14, but 8192 x 5120 16.9 / 18.3, 5120 x 27648 Q4_K 38.9 / 41.5); the fused gate/up 76 / 70.  At eight the
+// decode kernel wins on large weights and f32 rows (5120 x 27648 27.0 / 30.8, Q6_K 31.7 / 39.7) and loses on small ones
+// (5120 x 5120 13.1 / 11.4, 1024 x 5120 11.1 / 8.6).
 // The decode kernel also keeps, and its forms for 13 to 16 tokens (fused gate/up among them) are there for,
 //   - K shards up to 16 tokens, whose partial sums must carry the same bits with and without the all-reduce fused in,
 //   - calls under a forced launch plan (MUSER_TUNE_DECODE_*), and shapes the batched kernels refuse.
@@ -1259,9 +1263,10 @@ static bool takes_mma(const Ctx *ctx, const Weight *w, uint32_t tokens) {
 }
 
 // The tcgen05 kernel for large Q4_K weights at token counts that fill its columns (us, tcgen05 / warp-level, 27648 x 5120:
-// 35 / 32 at 17 to 24 tokens, 35 / 38 at 32, 54 / 48 at 48, 55 / 61 at 64; f32 activations, two columns a token, 47 / 44 at
-// 17 to 24 and 48 / 56 at 32.  Smaller weights, before both kernels' present forms: 13824 x 5120 37 / 40 at 64, 8192 x 5120
-// 22 / 22 at 32 and 33 / 31, 5120 x 5120 19 / 17 and 29 / 23).  Q6_K: 63 / 52 at 32 and 78 / 76 at 64 for 5120 x 27648.
+// 35 / 32 at 17 to 24 tokens, 35 / 38 at 32, 55 / 48 at 48, 55 / 61 at 64; f32 activations, two columns a token, 48 / 44 at
+// 17 to 24 and 48 / 56 at 32.  At 24, 32, 48, 64: 13824 x 5120 23 / 22, 23 / 24.5, 31 / 30, 32 / 36; 8192 x 8192 23.5 / 22,
+// 23.5 / 25.5, 35 / 30, 35 / 38; below the line 8192 x 5120 19 / 17, 19 / 19.5, 29 / 22, 29 / 27.5, 5120 x 5120 16 / 13, 16.5 / 14.5,
+// 25 / 18, 26.5 / 21).  Q6_K, 5120 x 27648: 51 / 43, 51 / 49, 70 / 59, 72 / 73; 27648 x 5120 44 / 40, 44 / 43.5, 66 / 53, 67 / 65.
 // A threshold set below 17 tokens (MUSER_TUNE_TC_MIN_TOKENS_*) asks for it wherever it serves, which is what its Q6_K form
 // is kept for: the caller's choice of range and rounding against another kernel's.
 static bool takes_tcgen05(const Weight *w, uint32_t tokens, bool two_columns, uint32_t tc_from) {
