@@ -192,15 +192,18 @@ constexpr uint32_t kRmsStagedRows = 4096; // beyond: the warp per 32 chains abov
 // value by value to its end it took the kernel from 7 to 18 us at rows of 4096, segment by segment 10.7.)  The sum that results
 // is the chain's.
 constexpr int kChainThreads = 1024; // most threads of a block, one segment each
-struct ChainShared {
-    uint2 add[kChainThreads];      // per thread: its run's units up to and with its segment, from an even and an odd pattern
-    uint2 own[kChainThreads];      // and its segment's alone
-    uint32_t binade[kChainThreads]; // exponent field that the segment's additions hold for, kNoBinade: one by one
-    uint32_t starts[32];           // per warp: the lanes that begin a run
+struct ChainThread {
+    uint2 add, own;  // units of its run up to and with its segment, and of the segment alone, from an even and an odd pattern
+    uint32_t binade; // exponent field that the segment's additions hold for, kNoBinade: one by one
+    uint32_t unused;
+};
+struct ChainBlock {
+    uint32_t starts[32]; // per warp: the lanes that begin a run
     float warp_sum[32];
     float inv_rms;
 };
 constexpr int kChainResident = 1152; // threads an SM holds (56 registers each)
+static_assert(kChainResident * sizeof(ChainThread) + kChainResident / 32 * (sizeof(ChainBlock) + 1024) < 227 * 1024, "shared memory holds fewer blocks than registers");
 constexpr uint32_t kNoBinade = 256;
 static uint32_t chain_threads(uint32_t n_in, uint32_t eights) { return ((n_in / 8 + eights - 1) / eights + 31) / 32 * 32; }
 __device__ __forceinline__ uint2 chain_compose(uint2 first, uint2 then) {
@@ -231,7 +234,7 @@ __device__ __forceinline__ uint32_t chain_runs(uint32_t binade, uint2 &add) {
 }
 // 1 / sqrt(mean(x^2) + eps) of one row of n_in <= 8 K blockDim values, for every thread of the block.
 template <bool XF32, int K>
-__device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, float eps, ChainShared &sh) {
+__device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, float eps, ChainThread *th, ChainBlock &sh) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5, n8 = n_in / 8;
     float v[K][8];
 #pragma unroll
@@ -260,9 +263,9 @@ __device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, fl
     before += carry, after += carry;
     uint32_t binade;
     uint2 add = chain_segment(before, after, &v[0][0], 8 * K, binade);
-    sh.own[tid] = add;
+    th[tid].own = add;
     const uint32_t starts = chain_runs(binade, add);
-    sh.add[tid] = add, sh.binade[tid] = binade;
+    th[tid].add = add, th[tid].binade = binade;
     if (lane == 0) sh.starts[warp] = starts;
     __syncthreads();
     if (warp == 0) {
@@ -275,14 +278,14 @@ __device__ __forceinline__ float chain_inv_rms(const void *xr, uint32_t n_in, fl
         };
         // what there is to know of a warp that is one run, a warp per lane
         const uint32_t w_starts = lane < warps ? sh.starts[lane] : 0u, w_last = min(lane, warps - 1) * 32 + 31;
-        const uint32_t w_binade = sh.binade[w_last];
-        const uint2 w_add = sh.add[w_last];
+        const uint32_t w_binade = th[w_last].binade;
+        const uint2 w_add = th[w_last].add;
         for (uint32_t w = 0; w < warps; ++w) {
             uint32_t runs = __shfl_sync(0xffffffffu, w_starts, w);
             const uint32_t e = __shfl_sync(0xffffffffu, w_binade, w), x = __shfl_sync(0xffffffffu, w_add.x, w), y = __shfl_sync(0xffffffffu, w_add.y, w);
             if (runs == 1 && step(e, x, y)) continue;
-            const uint2 my_add = sh.add[w * 32 + lane], my_own = sh.own[w * 32 + lane];
-            const uint32_t my_binade = sh.binade[w * 32 + lane];
+            const uint2 my_add = th[w * 32 + lane].add, my_own = th[w * 32 + lane].own;
+            const uint32_t my_binade = th[w * 32 + lane].binade;
             for (uint32_t pos = 0; pos < 32;) {
                 const uint32_t rest = runs & ~(0xffffffffu >> (31 - pos)); // starts behind `pos`
                 const uint32_t end = rest ? __ffs(rest) - 1 : 32;
@@ -360,21 +363,14 @@ __global__ void __launch_bounds__(32 * kChainRowWarps) rms_rows_chain_kernel(con
         before = __uint_as_float(s) + (lane ? before : 0.0f), after += __uint_as_float(s);
         uint32_t binade;
         uint2 add = chain_segment(before, after, &v[0][0], 8 * K, binade);
-        const uint2 own = add;
         const uint32_t starts = chain_runs(binade, add);
-        const auto step = [&](uint2 units, uint32_t last) { // what lane `last` holds, if the sum stays in its binade
-            const uint32_t e = __shfl_sync(0xffffffffu, binade, last);
-            const uint32_t even = __shfl_sync(0xffffffffu, units.x, last), odd = __shfl_sync(0xffffffffu, units.y, last);
-            const uint32_t next = s + ((s & 1) ? odd : even);
-            const bool holds = (s >> 23) == e && (next >> 23) == e;
-            if (holds) s = next;
-            return holds;
-        };
         for (uint32_t pos = 0; pos < 32;) {
             const uint32_t rest = starts & ~(0xffffffffu >> (31 - pos)), end = rest ? __ffs(rest) - 1 : 32;
-            const bool start = (starts >> pos) & 1; // (uniform over the warp)
-            if (step(start ? add : own, start ? end - 1 : pos)) {
-                pos = start ? end : pos + 1;
+            const uint32_t e = __shfl_sync(0xffffffffu, binade, end - 1);
+            const uint32_t even = __shfl_sync(0xffffffffu, add.x, end - 1), odd = __shfl_sync(0xffffffffu, add.y, end - 1);
+            const uint32_t sum_bits = s + ((s & 1) ? odd : even);
+            if (((starts >> pos) & 1) && (s >> 23) == e && (sum_bits >> 23) == e) {
+                s = sum_bits, pos = end;
                 continue;
             }
             float t = __uint_as_float(s); // (every lane adds its own squares, the segment's lane is heard)
@@ -449,9 +445,10 @@ __device__ __forceinline__ void norm_quantize_row(const void *xr, uint32_t row, 
 // The same quantizer behind a fused input RMSNorm (reference.rs:59-80): one block per token row takes the row's factor
 // (chain_inv_rms) and quantizes (x * inv_rms) * w group by group.
 template <bool XF32, int K>
-__global__ void __launch_bounds__(kChainThreads) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
+__global__ void __maxnreg__(56) nvfp4_norm_quantize_kernel(const void *x, uint32_t tokens, uint32_t n_in, uint32_t kt, float isi,
                                                                             const float *norm_w, float eps, uint8_t *packed, uint8_t *scales, bool early) {
-    __shared__ ChainShared sh;
+    extern __shared__ ChainThread chain_threads_shared[]; // (by the block's size: 1024 of them left room for ten blocks of 96 where twelve are counted on)
+    __shared__ ChainBlock sh;
     const uint32_t row = blockIdx.x;
     // the norm weights are read last, from L2 if they are asked for now (between two layers' weights they go to memory)
     if (row < min(tokens, 16u))
@@ -459,7 +456,7 @@ __global__ void __launch_bounds__(kChainThreads) nvfp4_norm_quantize_kernel(cons
     pdl_turn(early);
     const void *xr = XF32 ? (const void *)(reinterpret_cast<const float *>(x) + (size_t)row * n_in)
                           : (const void *)(reinterpret_cast<const __nv_bfloat16 *>(x) + (size_t)row * n_in);
-    const float inv = row < tokens ? chain_inv_rms<XF32, K>(xr, n_in, eps, sh) : 0.0f; // (uniform over the block)
+    const float inv = row < tokens ? chain_inv_rms<XF32, K>(xr, n_in, eps, chain_threads_shared, sh) : 0.0f; // (uniform over the block)
     norm_quantize_row<XF32>(xr, row, tokens, n_in, kt, isi, norm_w, inv, packed, scales);
 }
 
@@ -613,7 +610,7 @@ muser_cuda_status launch_nvfp4_quantize(Ctx *ctx, const void *x, uint32_t x_dtyp
         const auto kernel = eights == 2 ? (f32 ? nvfp4_norm_quantize_kernel<true, 2> : nvfp4_norm_quantize_kernel<false, 2>)
                                         : (f32 ? nvfp4_norm_quantize_kernel<true, 4> : nvfp4_norm_quantize_kernel<false, 4>);
         const uint32_t threads = chain_threads((uint32_t)n_in, eights);
-        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(threads), 0, stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps, packed,
+        MUSER_CUDA_TRY(ctx, launch_pdl(kernel, dim3(tokens_pad), dim3(threads), threads * sizeof(ChainThread), stream, x, tokens, (uint32_t)n_in, kt, isi, norm_weight, norm_eps, packed,
                                        scales, few_blocks(ctx, tokens_pad)));
         return MUSER_CUDA_OK;
     }
