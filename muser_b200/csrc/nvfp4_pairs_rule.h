@@ -24,8 +24,10 @@ enum class PairForm { plain, group, fused }; // single outputs, projections in o
 //            128         4 slabs 7.7 / 8.1 at 16; 20 slabs 13.4 / 12.8 at 16, 14.4 / 14.8 at 40, 16.9 / 16.0 at 74
 //   group, single over pairs: at 64 tokens 0.91 to 0.99 up to 11 slabs, 1.02 to 1.07 with 20; at 128 up to 37 tiles 1.01 to 1.12,
 //            with 74 tiles 0.78 to 0.93; at 384 with 74 tiles 0.91 (5 slabs); at 512 with 37 tiles 0.90 (4), 0.97 (11), 1.01 (20)
-// Over 2520 points (4 to 22 slabs, 4 to 108 tiles, 1 to 1000 tokens, the three forms) the choice took 1.0005 times the faster
-// form's time on average and 1.08 times at worst, calls that cut K aside.
+//   long rows: 32 slabs, plain at 32 and 48 tokens 18.4 / 16.9 at 56; SwiGLU of 108 slabs at 16 tokens 43.7 / 38.1 at 20, 54.6 /
+//            49.2 at 56; a group of 32 slabs and 72 tiles at 128 tokens 20.5 / 18.7
+// Over 4000 points (4 to 108 slabs, 4 to 108 tiles, 1 to 1000 tokens, the three forms) the choice took 1.002 times the faster
+// form's time on average and 1.1 times at worst, calls that cut K aside.
 inline bool pairs_pay(uint32_t sms, uint32_t room, uint32_t n_tiles, uint32_t tokens, uint32_t slabs, PairForm form) {
     if (!room) return false;
     const uint64_t blocks = ((uint64_t)tokens + 127) / 128, pair_tiles = n_tiles * ((blocks + 1) / 2);
@@ -36,13 +38,15 @@ inline bool pairs_pay(uint32_t sms, uint32_t room, uint32_t n_tiles, uint32_t to
     const bool odd = blocks % 2, wasted = odd && blocks > 1 && pair_rounds == single_rounds; // an odd block's pairs gain no round
     switch (form) {
     case PairForm::plain:
-        if (tokens < 64 && (slabs < 9 || of_sms(tokens < 40 ? 8 : 4))) return false;
-        return !crowded || !odd || slabs >= (tokens < 96 ? 14 : tokens < 112 ? 10 : 8);
+        if (tokens < 64 && (slabs < 9 || (of_sms(tokens < 40 ? 8 : 4) && slabs < (tokens < 32 ? ~0u : tokens < 40 ? 30u : 24u)))) return false;
+        return !crowded || !odd || slabs >= (tokens < 96 ? 14 : tokens < 112 ? 10 : 7 * pair_tiles > 2 * sms ? 8 : 0);
     case PairForm::group:
-        if (tokens < 112 && (slabs < (tokens < 96 ? 16 : 11) || of_sms(tokens < 64 ? 8 : 4))) return false;
-        return crowded ? blocks > 1 && slabs >= (odd ? 16 : 10) : slabs >= (wasted && pair_rounds > 1 ? 9 : 0);
+        if (tokens < 112 && (slabs < (tokens < 96 ? 16 : 11) || (of_sms(tokens < 64 ? 8 : 4) && slabs < (tokens < 96 ? ~0u : 24u)))) return false;
+        if (crowded && blocks == 1) return slabs >= 24 || (slabs >= 10 && 8 * pair_tiles <= 3 * sms);
+        return crowded ? slabs >= (odd ? 16 : 10) : slabs >= (wasted && pair_rounds > 1 ? 9 : 0);
     case PairForm::fused:
-        if (tokens < 64 && of_sms(tokens < 48 ? 8 : 5)) return false;
+        if (tokens < 64 && of_sms(tokens >= 48 ? 5 : slabs < 16 ? 8 : slabs < 40 || tokens < 8 ? 6 : 4) &&
+            slabs < (tokens < 16 ? ~0u : tokens < 32 ? 80u : tokens < 48 ? 40u : 24u)) return false;
         return slabs >= (crowded ? 20 : wasted ? 16 : 12);
     }
     return false;

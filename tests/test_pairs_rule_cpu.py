@@ -18,7 +18,9 @@ MEASURED = [
     (FUSED, 4, 4, 1, 7.11, 7.53), (FUSED, 74, 4, 16, 7.44, 9.91), (FUSED, 74, 4, 256, 9.18, 9.98), (FUSED, 16, 20, 16, 13.11, 12.68),
     (FUSED, 40, 20, 16, 14.12, 18.00), (FUSED, 74, 20, 1, 16.48, 19.16), (FUSED, 74, 20, 48, 16.72, 18.61), (FUSED, 74, 20, 128, 16.85, 16.01),
     (FUSED, 74, 12, 300, 17.31, 18.42), (FUSED, 216, 20, 384, 55, 60), (FUSED, 216, 20, 2048, 237, 220),
-    (GROUP, 37, 4, 100, 5.51, 5.96), (GROUP, 8, 11, 384, 8.58, 7.72), (GROUP, 37, 12, 384, 9.93, 10.58), (GROUP, 28, 13, 96, 8.78, 8.34),
+    (PLAIN, 40, 4, 128, 6.64, 6.29), (PLAIN, 56, 32, 32, 18.37, 16.90), (PLAIN, 54, 32, 48, 18.4, 17.0), (FUSED, 56, 108, 16, 54.59, 49.18),
+    (FUSED, 20, 108, 16, 43.7, 38.1), (FUSED, 56, 108, 48, 51.0, 46.3),
+    (GROUP, 72, 32, 128, 20.5, 18.7), (GROUP, 52, 20, 128, 13.2, 12.8), (GROUP, 37, 4, 100, 5.51, 5.96), (GROUP, 8, 11, 384, 8.58, 7.72), (GROUP, 37, 12, 384, 9.93, 10.58), (GROUP, 28, 13, 96, 8.78, 8.34),
     (GROUP, 74, 5, 384, 9.41, 10.30), (GROUP, 28, 20, 2048, 37.7, 32.4),
 ]
 
