@@ -272,6 +272,12 @@ MUSER_CUDA_API muser_cuda_status muser_cuda_rmsnorm_quantize_nvfp4_activation(mu
  * i.e. weights::matmul's W4A4 lane (src/weights.rs:111-121, quant/nvfp4.rs:304-338): quantizes x
  * into the context workspace, then runs the block-scaled tensor-core GEMM.  y_dtype F32, F16 or BF16
  * (F16 is the reference's output boundary, nvfp4.rs:337).
+ * What the bits of a result depend on besides its operands: rows of 3072 inputs or more over few rows and tokens are
+ * summed in two to eight slices that are added in order, and the number of slices follows the weight's rows and row
+ * length, the token count and the device.  So a token's outputs can differ in their last bits between batches of
+ * different sizes (5120 inputs: up to about 43 tokens and beyond).  A call repeated on the same device, and a group
+ * (muser_cuda_nvfp4_matmul_group_prequant) against the single calls, give the same bits.  Calls with a logit scale or
+ * soft cap, the fused gate/up forms and contexts told to use pairs (MUSER_TUNE_NVFP4_PAIR 1) never cut a sum.
  * A weight repacked WITHOUT input_scale_inv takes the reference's weight-only lane instead (input_scale_inv = None,
  * src/weights.rs:117-121, quant::dot_nvfp4_a16_q8_f32 src/quant/nvfp4.rs:348-379): activations go to int8 per 256
  * inputs, the contraction is exact integer arithmetic, and the f16-rounded result equals the reference's bit for bit
