@@ -391,7 +391,8 @@ __global__ void __launch_bounds__(32 * kChainRowWarps) rms_rows_chain_kernel(con
 // Which of the three leaves the factors.  The plain chains (few values per row, or enough rows that a lane each fills the chip)
 // do half the additions.  us with the quantizer of a row a block, plain / warp per row, bf16: 512 values 4.5 / 4.8 at 148 rows, 6.4 / 7.4 at
 // 2048; 1024 values 6.6 / 5.4 at 449, 9.0 / 8.7 at 2048, 11.8 / 12.5 at 4096; 2048 values 14.3 / 11.5 at 2048, 18.3 / 16.9 at
-// 4096, 28.4 / 29 at 8192; 3136 values 27.5 / 23.6 at 4096, 42.6 / 40.2 at 8192, 139 / 153 at 32768; 5120 values 45 / 32 at
+// 4096, 28.4 / 29 at 8192; 3136 values 27.5 / 23.6 at 4096, 42.6 / 40.2 at 8192, 139 / 153 at 32768; 4608
+// values 59 / 58 at 10000, 82 / 89 at 16384, 168 / 169 at 32768 (f32, where the line could lie lower: 90 / 90, 161 / 141, 279 / 269); 5120 values 45 / 32 at
 // 4096, 66 / 57 at 8192, 224 / 212 at 32768; 12288 values 77 / 46 at 2048.  f32: 5120 values 72 / 52 at 4096, 352 / 353 at
 // 32768; 12288 values 136 / 72 at 2048; 27648 values 304 / 160 at 2048.
 static cudaError_t launch_rms_rows(Ctx *ctx, const void *x, uint32_t x_dtype, uint32_t tokens, uint32_t n_in, float eps, float *inv_rms,
